@@ -98,4 +98,16 @@ struct fe3d_solver {
     float2 *vals2 = nullptr, *p2 = nullptr;  // split-FP32 (hi, lo) values and direction
     int have2 = 0;
     unsigned int *counter = nullptr;      // last-block-done counter of the reductions
+    // FP64 solves: the non-zero values in slices of 32 rows (entry k of row i
+    // at 32 (soff[i / 32] + k) + i % 32, rows padded with zeros to the slice's
+    // longest), rebuilt from the caller's values by every solve; sell_on: the
+    // current solve uses it
+    int64_t *soff = nullptr;
+    int32_t *slen = nullptr;
+    double *sval = nullptr;
+    uint16_t *scol = nullptr;             // offsets from the pattern's colbase
+    int64_t sell_cap = 0;                 // entries allocated in sval / scol
+    unsigned long long *sell_total = nullptr;
+    int sell_on = 0;
+    int sell_grid = 0;                    // blocks of the slice kernels (one wave of resident ones)
 };

@@ -136,6 +136,114 @@ __global__ void __launch_bounds__(RED_BS) spmv_kernel(int64_t n, const int64_t *
     }
 }
 
+// ---- non-zero values in slices of 32 rows (FP64 solves) -----------------
+// A flat plate couples (u, v, rz) and (w, rx, ry) only, so half of the
+// entries its pattern stores are exact zeros.  Every FP64 solve first lays the
+// non-zero values out in slices of 32 rows, entry by entry (one row per lane):
+// zeros cost neither bytes nor FP64 instructions (an FP64 instruction takes
+// the pipe for 64 cycles per sub-partition whatever its active lanes), loads
+// are coalesced and a row needs no shuffle reduction.  501x501-node plate
+// (80.5 M stored entries): one PCG iteration 0.286 -> 0.17 ms, 50 iterations
+// with set-up and residuals 18.5 -> 10.5 ms.
+
+// Longest non-zero row of each slice, its place in the slice layout (taken
+// from *total, so the slices' order may vary but not what they hold).
+__global__ void __launch_bounds__(RED_BS) sell_count_kernel(int64_t n, const int64_t *__restrict__ rowptr,
+                                                            const double *__restrict__ vals,
+                                                            int32_t *__restrict__ slen, int64_t *__restrict__ soff,
+                                                            unsigned long long *total) {
+    const int64_t slice = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    if (slice * 32 >= n) return;
+    const int lane = threadIdx.x & 31;
+    const int64_t row = slice * 32 + lane;
+    const int64_t rb = rowptr[row < n ? row : n], re = rowptr[row < n ? row + 1 : n];
+    unsigned longest = 0;
+    // row by row with the lanes along the entries: coalesced reads
+#pragma unroll 4
+    for (int r = 0; r < 32; r++) {
+        const int64_t b = __shfl_sync(0xffffffffu, rb, r), e = __shfl_sync(0xffffffffu, re, r);
+        unsigned cnt = 0;
+        for (int64_t k = b; k < e; k += 32)
+            cnt += __popc(__ballot_sync(0xffffffffu, k + lane < e && vals[k + lane < e ? k + lane : b] != 0.));
+        longest = cnt > longest ? cnt : longest;
+    }
+    if (lane == 0) {
+        slen[slice] = (int32_t)longest;
+        soff[slice] = (int64_t)atomicAdd(total, (unsigned long long)longest);
+    }
+}
+
+// Fills the slices; a row shorter than its slice repeats its last column with
+// the value 0 (a non-finite x there is met by the row's own entry as well).
+__global__ void __launch_bounds__(RED_BS) sell_fill_kernel(int64_t n, const int64_t *__restrict__ rowptr,
+                                                           const uint16_t *__restrict__ col16,
+                                                           const double *__restrict__ vals,
+                                                           const int32_t *__restrict__ slen,
+                                                           const int64_t *__restrict__ soff,
+                                                           double *__restrict__ sval, uint16_t *__restrict__ scol) {
+    const int64_t slice = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    if (slice * 32 >= n) return;
+    const int lane = threadIdx.x & 31;
+    const int64_t row = slice * 32 + lane;
+    const int len = slen[slice];
+    double *sv = sval + soff[slice] * 32 + lane;
+    uint16_t *sc = scol + soff[slice] * 32 + lane;
+    int at = 0;
+    uint16_t c = 0;
+    if (row < n) {
+        const int64_t re = rowptr[row + 1];
+        for (int64_t k = rowptr[row]; k < re; k++) {
+            const double v = vals[k];
+            if (v != 0.) {
+                c = col16[k];
+                sv[32 * at] = v;
+                sc[32 * at] = c;
+                at++;
+            }
+        }
+    }
+    for (; at < len; at++) {
+        sv[32 * at] = 0.;
+        sc[32 * at] = c;
+    }
+}
+
+// spmv_kernel on the slices: one row per lane.
+__global__ void __launch_bounds__(RED_BS) spmv_sell_kernel(int64_t n, const int32_t *__restrict__ slen,
+                                                           const int64_t *__restrict__ soff,
+                                                           const int32_t *__restrict__ colbase,
+                                                           const uint16_t *__restrict__ scol,
+                                                           const double *__restrict__ sval,
+                                                           const double *__restrict__ x, double *__restrict__ y,
+                                                           double *partial_dot, unsigned int *counter,
+                                                           const double *rz, double *alpha_out) {
+    __shared__ double sh[34];
+    double dot = 0.;
+    for (int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; row < n;
+         row += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t slice = row >> 5;
+        const int len = slen[slice];
+        const int64_t o = soff[slice] * 32 + (row & 31);
+        const double *sv = sval + o;
+        const uint16_t *sc = scol + o;
+        const double *xb = x + colbase[row];
+        double acc = 0.;
+#pragma unroll 9
+        for (int k = 0; k < len; k++) acc += sv[32 * k] * xb[sc[32 * k]];
+        y[row] = acc;
+        dot += x[row] * acc;
+    }
+    const double s = block_sum(dot, sh);
+    if (threadIdx.x == 0) partial_dot[blockIdx.x] = s;
+    if (last_block(counter)) {
+        const double pq = reduce_partials_l2(partial_dot, gridDim.x, sh);
+        if (threadIdx.x == 0) {
+            *alpha_out = pq != 0. ? *rz / pq : 0.;
+            *counter = 0u;
+        }
+    }
+}
+
 // y = K x with the products on the FP32 pipe: values and x are held as
 // float pairs (hi + lo, ~48 significant bits), each product is split exactly
 // with an FMA plus the two cross terms, and the row sums are carried in
@@ -578,6 +686,46 @@ __global__ void __launch_bounds__(RED_BS) dd_residual_kernel(int64_t n, const in
     if (threadIdx.x == 0) partial_rr[blockIdx.x] = s;
 }
 
+// dd_residual_kernel on the slices, one row per lane (an exact zero changes
+// neither part of a double-double sum).
+__global__ void __launch_bounds__(RED_BS) dd_residual_sell_kernel(int64_t n, const int32_t *__restrict__ slen,
+                                                                  const int64_t *__restrict__ soff,
+                                                                  const int32_t *__restrict__ colbase,
+                                                                  const uint16_t *__restrict__ scol,
+                                                                  const double *__restrict__ sval,
+                                                                  const double *__restrict__ xhi,
+                                                                  const double *__restrict__ xlo,
+                                                                  const double *__restrict__ f,
+                                                                  double *__restrict__ r, double *partial_rr) {
+    __shared__ double sh[33];
+    double rr = 0.;
+    for (int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; row < n;
+         row += (int64_t)gridDim.x * blockDim.x) {
+        const int len = slen[row >> 5];
+        const int64_t o = soff[row >> 5] * 32 + (row & 31);
+        const int32_t base = colbase[row];
+        double hi = 0., lo = 0.;
+#pragma unroll 3
+        for (int k = 0; k < len; k++) {
+            const double a = sval[o + 32 * k];
+            const int c = base + scol[o + 32 * k];
+            const double xh = xhi[c];
+            const double pr = a * xh;
+            const double pe = fma(a, xh, -pr);
+            double e;
+            two_sum(hi, pr, hi, e);
+            lo = fma(a, xlo[c], lo + (e + pe));
+        }
+        double sm, e;
+        two_sum(f[row], -hi, sm, e);
+        const double ri = sm + (e - lo);
+        r[row] = ri;
+        rr += ri * ri;
+    }
+    const double s = block_sum(rr, sh);
+    if (threadIdx.x == 0) partial_rr[blockIdx.x] = s;
+}
+
 __global__ void combine_kernel(int64_t n, const double *xhi, const double *xlo, double *u) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         u[i] = xhi[i] + xlo[i];
@@ -768,6 +916,7 @@ extern "C" int fe3d_solver_free(fe3d_solver *s) {
     cudaFree(s->z32); cudaFree(s->p32); cudaFree(s->q32); cudaFree(s->ppq); cudaFree(s->prz);
     cudaFree(s->prr); cudaFree(s->prf); cudaFree(s->scal); cudaFree(s->nonpos);
     cudaFree(s->vals2); cudaFree(s->p2);
+    cudaFree(s->soff); cudaFree(s->slen); cudaFree(s->sval); cudaFree(s->scol); cudaFree(s->sell_total);
     delete s;
     return FE3D_OK;
 }
@@ -901,14 +1050,79 @@ extern "C" int fe3d_spmv(const fe3d_pattern *p, const double *vals, const double
 
 namespace {
 
+// Slice layout of the solve's values: counts the non-zeros on st (sell_plan),
+// and once the caller has read *sell_total and synchronised, decides and
+// fills it (sell_build).  The layout is used when it holds at most 3/4 of the
+// stored entries; otherwise (curved shells, laminates with coupling) the CSR
+// kernels read the caller's values as they are.  Below kSellMinRows one row
+// per lane leaves too few warps and the row's serial FP64 chain shows (clamped
+// perturbed plates, us per iteration CSR / slices: 2,166 rows 20.8 / 23.3,
+// 9,126 rows 22.2 / 24.1, 14,406 rows 24.0 / 23.8, 20,886 rows 25.5 / 24.2,
+// 58,806 rows 30.1 / 25.5, 133,206 rows 42.9 / 30.5, 536,406 rows 114 / 69.5).
+constexpr int64_t kSellMinRows = 16384;
+
+int sell_plan(fe3d_solver *s, cudaStream_t st) {
+    s->sell_on = 0;
+    if (!s->pat->col16 || s->n < kSellMinRows) return FE3D_OK;
+    const int64_t slices = (s->n + 31) / 32;
+    if (!s->sell_total) {
+        const int res = resident_per_sm(spmv_sell_kernel, RED_BS, 0);
+        s->sell_grid = grid_cap(s->n, RED_BS, kSMs * (res < 8 ? res : 8));
+        if (alloc(&s->slen, slices) || alloc(&s->soff, slices) || alloc(&s->sell_total, 1)) return FE3D_ERR_NOMEM;
+    }
+    FE3D_CUDA(cudaMemsetAsync(s->sell_total, 0, sizeof(unsigned long long), st));
+    sell_count_kernel<<<grid_cap(slices * 32, RED_BS, 1 << 30), RED_BS, 0, st>>>(s->n, s->pat->rowptr, s->vals,
+                                                                                 s->slen, s->soff, s->sell_total);
+    FE3D_CHECK_LAUNCH();
+    return FE3D_OK;
+}
+
+int sell_build(fe3d_solver *s, unsigned long long total, cudaStream_t st) {
+    const int64_t entries = 32 * (int64_t)total;
+    int on = s->pat->col16 && s->n >= kSellMinRows && 4 * entries <= 3 * s->pat->nnz;
+    if (on && entries > s->sell_cap) {
+        cudaFree(s->sval);
+        cudaFree(s->scol);
+        s->sval = nullptr;
+        s->scol = nullptr;
+        s->sell_cap = 0;
+        if (alloc(&s->sval, entries) || alloc(&s->scol, entries)) {
+            // no room for the copy: the CSR kernels need none
+            (void)cudaGetLastError();
+            cudaFree(s->sval);
+            s->sval = nullptr;
+            on = 0;
+        } else {
+            s->sell_cap = entries;
+        }
+        // the captured iterations hold the old arrays' addresses
+        for (int j = 0; j < 2; j++)
+            if (s->graph[0][j]) {
+                cudaGraphExecDestroy(s->graph[0][j]);
+                s->graph[0][j] = nullptr;
+            }
+    }
+    s->sell_on = on;
+    if (!on) return FE3D_OK;
+    sell_fill_kernel<<<grid_cap((s->n + 31) / 32 * 32, RED_BS, 1 << 30), RED_BS, 0, st>>>(
+        s->n, s->pat->rowptr, s->pat->col16, s->vals, s->slen, s->soff, s->sval, s->scol);
+    FE3D_CHECK_LAUNCH();
+    return FE3D_OK;
+}
+
 // FP64 residual r = f - K u; returns ||r||^2 (synchronises).
 int true_residual(fe3d_solver *s, const double *f, double *u, cudaStream_t st, double *rr) {
     // the increment u since the last replacement joins the double-double
     // base, whose residual is evaluated with compensated sums
     fold_kernel<<<s->vec_grid, RED_BS, 0, st>>>(s->n, s->xhi, s->xlo, u);
-    dd_residual_kernel<<<s->spmv_grid, RED_BS, 0, st>>>(s->n, s->pat->rowptr, s->pat->colind, s->vals, s->xhi,
-                                                         s->xlo, f, s->r, s->prr);
-    finalize_sum_kernel<<<1, RED_BS, 0, st>>>(s->prr, s->spmv_grid, s->scal + 2);
+    const int grid = s->sell_on ? s->sell_grid : s->spmv_grid;
+    if (s->sell_on)
+        dd_residual_sell_kernel<<<grid, RED_BS, 0, st>>>(s->n, s->slen, s->soff, s->pat->colbase, s->scol, s->sval,
+                                                         s->xhi, s->xlo, f, s->r, s->prr);
+    else
+        dd_residual_kernel<<<grid, RED_BS, 0, st>>>(s->n, s->pat->rowptr, s->pat->colind, s->vals, s->xhi, s->xlo,
+                                                    f, s->r, s->prr);
+    finalize_sum_kernel<<<1, RED_BS, 0, st>>>(s->prr, grid, s->scal + 2);
     FE3D_CHECK_LAUNCH();
     FE3D_CUDA(cudaMemcpyAsync(rr, s->scal + 2, sizeof(double), cudaMemcpyDeviceToHost, st));
     FE3D_CUDA(cudaStreamSynchronize(st));
@@ -931,14 +1145,21 @@ int run_cg(fe3d_solver *s, const double *f, double *u, const fe3d_solve_opts *o,
     const double *sck = mixed ? s->sc : nullptr;  // the FP32 recurrence runs on S^-1 K S^-1
     const double *isck = mixed ? s->sc + n : nullptr;
     double ff = 0.;
+    int rc = 0;
     {
-        // ||f||
+        // ||f||, and the non-zero count of the FP64 recurrence's matrix
+        unsigned long long total = 0;
+        s->sell_on = 0;
+        if (prec == 0 && (rc = sell_plan(s, st))) return rc;
         precond_kernel<double, double><<<s->node_grid, RED_BS, 0, st>>>(
             s->nnodes, s->start, s->size, s->Dinv, f, s->z, s->prz, s->prr, nullptr, nullptr);
         finalize_sum_kernel<<<1, RED_BS, 0, st>>>(s->prr, s->node_grid, s->scal + 4);
         FE3D_CHECK_LAUNCH();
         FE3D_CUDA(cudaMemcpyAsync(&ff, s->scal + 4, sizeof(double), cudaMemcpyDeviceToHost, st));
+        if (prec == 0 && s->sell_total)
+            FE3D_CUDA(cudaMemcpyAsync(&total, s->sell_total, sizeof(total), cudaMemcpyDeviceToHost, st));
         FE3D_CUDA(cudaStreamSynchronize(st));
+        if (prec == 0 && ff != 0. && (rc = sell_build(s, total, st))) return rc;
     }
     stats->iterations = 0;
     stats->replacements = 0;
@@ -958,8 +1179,7 @@ int run_cg(fe3d_solver *s, const double *f, double *u, const fe3d_solve_opts *o,
         FE3D_CUDA(cudaMemsetAsync(u, 0, sizeof(double) * n, st));
     }
     double rr = 0.;
-    int rc = true_residual(s, f, u, st, &rr);
-    if (rc) return rc;
+    if ((rc = true_residual(s, f, u, st, &rr))) return rc;
     if (!(rr == rr)) {
         combine_kernel<<<s->vec_grid, RED_BS, 0, st>>>(n, s->xhi, s->xlo, u);
         FE3D_CHECK_LAUNCH();
@@ -993,12 +1213,17 @@ int run_cg(fe3d_solver *s, const double *f, double *u, const fe3d_solve_opts *o,
     const int pidx = prec == 3 ? 1 : prec;  // the nested inner iterations are the precision-1 graphs
     double *prf = o->flexible ? s->prf : nullptr;
     const int gflex = o->flexible ? 1 : 0;
-    const int lanes = s->lanes[pidx] ? s->lanes[pidx] : 4;
+    // lanes per row of the SpMV; 1 marks the slice layout
+    const int lanes = s->sell_on ? 1 : s->lanes[pidx] ? s->lanes[pidx] : 4;
     auto launch_iteration = [&](int pr) {
         // scal: [pr] rz, [pr ^ 1] rz_new, [2] r.r, [3] alpha, [5] beta
         if (prec == 2)
             launch_spmv_split(lanes, st, n, s->pat, s->vals2, p2, (const double *)p, (double *)q, s->ppq, s->counter,
                               s->scal + pr, s->scal + 3);
+        else if (s->sell_on)
+            spmv_sell_kernel<<<s->sell_grid, RED_BS, 0, st>>>(n, s->slen, s->soff, s->pat->colbase, s->scol, s->sval,
+                                                             (const double *)p, (double *)q, s->ppq, s->counter,
+                                                             s->scal + pr, s->scal + 3);
         else
             launch_spmv<VT, PT>(lanes, st, n, s->pat, vals_k, p, q, s->ppq, s->counter, s->scal + pr, s->scal + 3);
         update_kernel<PT, PT><<<s->node_grid, RED_BS, 0, st>>>(s->nnodes, s->start, s->size, Dk, s->scal + 3,
