@@ -60,6 +60,34 @@ struct fe3d_fmap {
     fe3d_fmap_group g[kFmapMaxGroups];
 };
 
+// Resident PCG of one system (team_pcg.cu): its split over co-resident blocks,
+// the slice layout of the non-zero values and the exchange words.
+// Rows per block wanted while blocks are left: 16 rather than 64 at 2,166 rows
+// takes 6.2 instead of 8.0 us per iteration (fewer FP64 instructions per block
+// against a slower exchange).
+constexpr int kTeamRows = 16;
+constexpr int64_t kTeamMaxRows = 1 << 20;
+
+struct fe3d_team {
+    int G = 0, L = 1;                  // blocks, lanes per row
+    int nmax = 0, wmax = 0;            // largest row count and column window of a block
+    size_t smem = 0;
+    bool reg = false;                  // the rows fit the blocks' registers
+    int32_t *r0 = nullptr;             // [G + 1] first row of each block
+    int32_t *slice0 = nullptr;         // [G + 1] first slice
+    int32_t *cmin = nullptr, *cmax = nullptr;  // [G] column window
+    int32_t *slen = nullptr;
+    int64_t *soff = nullptr;
+    double *sval = nullptr;
+    uint16_t *scol = nullptr;
+    int64_t cap = 0;
+    unsigned long long *total = nullptr;
+    ulonglong2 *z = nullptr, *slots = nullptr;
+    double *dval = nullptr;            // [6][n] non-zeros of the rows of the block inverses
+    uint32_t *dinf = nullptr;          // [n]
+    unsigned epoch = 1;
+};
+
 // Block-Jacobi PCG state (pcg.cu); the batched solver (bpcg.cu) reuses its
 // node blocks, block inverses, work vectors and private stream.
 struct fe3d_solver {
@@ -110,4 +138,22 @@ struct fe3d_solver {
     unsigned long long *sell_total = nullptr;
     int sell_on = 0;
     int sell_grid = 0;                    // blocks of the slice kernels (one wave of resident ones)
+    fe3d_team *team = nullptr;            // resident iterations (FP64, systems that fit)
+    int team_tried = 0;
 };
+
+namespace fe3d {
+void team_free(fe3d_team *t);
+fe3d_team *team_create(const fe3d_solver *s, cudaStream_t st);
+// Counts the non-zeros into t->total (and the longest slice into t->total[1]);
+// team_build lays them out once the caller has read both.
+int team_plan(fe3d_team *t, const fe3d_solver *s, cudaStream_t st);
+int team_build(fe3d_team *t, const fe3d_solver *s, unsigned long long total, unsigned long long longest,
+               cudaStream_t st);
+// Up to maxiter iterations from s->r, s->p, u and scal[rz_index], ended where
+// phase + iterations is a multiple of chunk and r.r <= stop2 or not finite;
+// scal[2] = r.r, scal[6] = iterations run, scal[7] = 1 when a block gave up
+// waiting.
+int team_run(fe3d_team *t, const fe3d_solver *s, double *u, int rz_index, int maxiter, int chunk, int phase,
+             double stop2, cudaStream_t st);
+}  // namespace fe3d

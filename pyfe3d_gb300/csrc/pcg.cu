@@ -10,6 +10,8 @@
 //   K2  alpha = rz / p.q;  u += alpha p;  r -= alpha q;  z = Minv r
 //                                        partial sums of r.z and r.r
 //   K3  beta = rz_new / rz;  p = z + beta p
+// Plain FP64 solves whose vectors fit the SMs' shared memory run the same
+// recurrence in one launch for many iterations instead (team_pcg.cu).
 // Every block of a consumer kernel reduces the producer's per-block partial
 // sums in the same order, so all blocks see identical scalars and the result
 // does not depend on scheduling.
@@ -916,6 +918,7 @@ extern "C" int fe3d_solver_free(fe3d_solver *s) {
     cudaFree(s->z32); cudaFree(s->p32); cudaFree(s->q32); cudaFree(s->ppq); cudaFree(s->prz);
     cudaFree(s->prr); cudaFree(s->prf); cudaFree(s->scal); cudaFree(s->nonpos);
     cudaFree(s->vals2); cudaFree(s->p2);
+    team_free(s->team);
     cudaFree(s->soff); cudaFree(s->slen); cudaFree(s->sval); cudaFree(s->scol); cudaFree(s->sell_total);
     delete s;
     return FE3D_OK;
@@ -1110,6 +1113,8 @@ int sell_build(fe3d_solver *s, unsigned long long total, cudaStream_t st) {
     return FE3D_OK;
 }
 
+constexpr int64_t kTeamIters = 4096;  // iterations of one resident launch at most (a quarter of a second)
+
 // FP64 residual r = f - K u; returns ||r||^2 (synchronises).
 int true_residual(fe3d_solver *s, const double *f, double *u, cudaStream_t st, double *rr) {
     // the increment u since the last replacement joins the double-double
@@ -1146,20 +1151,31 @@ int run_cg(fe3d_solver *s, const double *f, double *u, const fe3d_solve_opts *o,
     const double *isck = mixed ? s->sc + n : nullptr;
     double ff = 0.;
     int rc = 0;
+    // plain FP64 recurrence: resident iterations where the system fits
+    const bool resident = prec == 0 && !o->flexible;
+    if (resident && !s->team_tried) {
+        s->team = team_create(s, st);
+        s->team_tried = 1;
+    }
+    fe3d_team *team = nullptr;
     {
         // ||f||, and the non-zero count of the FP64 recurrence's matrix
-        unsigned long long total = 0;
+        unsigned long long total[2] = {0, 0};
         s->sell_on = 0;
-        if (prec == 0 && (rc = sell_plan(s, st))) return rc;
+        team = resident ? s->team : nullptr;
+        if (team ? (rc = team_plan(team, s, st)) : prec == 0 && (rc = sell_plan(s, st))) return rc;
         precond_kernel<double, double><<<s->node_grid, RED_BS, 0, st>>>(
             s->nnodes, s->start, s->size, s->Dinv, f, s->z, s->prz, s->prr, nullptr, nullptr);
         finalize_sum_kernel<<<1, RED_BS, 0, st>>>(s->prr, s->node_grid, s->scal + 4);
         FE3D_CHECK_LAUNCH();
         FE3D_CUDA(cudaMemcpyAsync(&ff, s->scal + 4, sizeof(double), cudaMemcpyDeviceToHost, st));
-        if (prec == 0 && s->sell_total)
-            FE3D_CUDA(cudaMemcpyAsync(&total, s->sell_total, sizeof(total), cudaMemcpyDeviceToHost, st));
+        if (team || (prec == 0 && s->sell_total))
+            FE3D_CUDA(cudaMemcpyAsync(total, team ? team->total : s->sell_total, (team ? 2 : 1) * sizeof(total[0]),
+                                      cudaMemcpyDeviceToHost, st));
         FE3D_CUDA(cudaStreamSynchronize(st));
-        if (prec == 0 && ff != 0. && (rc = sell_build(s, total, st))) return rc;
+        // no memory for the copy: the launch-per-kernel iteration needs none
+        if (team && ff != 0. && team_build(team, s, total[0], total[1], st)) team = nullptr;
+        else if (!team && prec == 0 && ff != 0. && (rc = sell_build(s, total[0], st))) return rc;
     }
     stats->iterations = 0;
     stats->replacements = 0;
@@ -1290,16 +1306,31 @@ int run_cg(fe3d_solver *s, const double *f, double *u, const fe3d_solve_opts *o,
     double rr_replaced = rr;
     int stalls = 0;
     while (it < o->maxiter) {
-        const int len = (int)((o->maxiter - it) < chunk ? (o->maxiter - it) : chunk);
-        if ((rc = run_chunk(len))) return rc;
+        int64_t len = (o->maxiter - it) < chunk ? (o->maxiter - it) : chunk;
+        if (team) {
+            // many chunks in one launch: it ends where the host has to act
+            // (the conditions below), at kTeamIters iterations at most
+            double h[8];
+            const int64_t most = (o->maxiter - it) < kTeamIters ? (o->maxiter - it) : kTeamIters;
+            const double stop2 = target > inner2 * rr_replaced ? target : inner2 * rr_replaced;
+            if ((rc = team_run(team, s, u, par, (int)most, chunk, (int)(it % chunk), stop2, st))) return rc;
+            FE3D_CUDA(cudaMemcpyAsync(h, s->scal, sizeof(h), cudaMemcpyDeviceToHost, st));
+            FE3D_CUDA(cudaStreamSynchronize(st));
+            if (h[7] != 0.) return FE3D_ERR_LAUNCH;
+            rr = h[2];
+            len = (int64_t)h[6];
+        } else {
+            if ((rc = run_chunk((int)len))) return rc;
+            FE3D_CUDA(cudaMemcpyAsync(&rr, s->scal + 2, sizeof(double), cudaMemcpyDeviceToHost, st));
+            FE3D_CUDA(cudaStreamSynchronize(st));
+        }
         it += len;
         since_replace += len;
-        FE3D_CUDA(cudaMemcpyAsync(&rr, s->scal + 2, sizeof(double), cudaMemcpyDeviceToHost, st));
-        FE3D_CUDA(cudaStreamSynchronize(st));
         if (!(rr == rr) || isinf(rr)) {
             stats->status = 3;
             break;
         }
+        if (team && it % chunk && it < o->maxiter) continue;  // a launch that ended between two checks
         const bool periodic = replace && since_replace >= replace;
         if (periodic || rr <= target || rr <= inner2 * rr_replaced) {
             double rt = 0.;

@@ -1,5 +1,6 @@
-"""FP64 solves of matrices whose pattern stores exact zeros (the solver drops them): slice remainders, sizes on
-both sides of the layout's limit, and values changed in place between two solves."""
+"""FP64 solves of matrices whose pattern stores exact zeros (the solver drops them), resident and launch by launch:
+remainders of blocks and slices, sizes on both sides of the layouts' limits, and values changed in place between two
+solves."""
 import numpy as np
 import pytest
 
@@ -28,7 +29,8 @@ def _triplets(nodes, coupled, seed):
 
 @pytest.mark.parametrize('nodes', [1, 5, 6, 11, 16, 171, 2730, 2731, 3001])
 @pytest.mark.parametrize('coupled', [False, True])
-def test_solve_with_stored_zeros(gpulib, nodes, coupled):
+@pytest.mark.parametrize('flexible', [False, True])  # flexible CG runs launch by launch
+def test_solve_with_stored_zeros(gpulib, nodes, coupled, flexible):
     import torch
     from scipy.sparse.linalg import spsolve
     from pyfe3d_gb300.solver import CSRPattern, Solver
@@ -39,10 +41,42 @@ def test_solve_with_stored_zeros(gpulib, nodes, coupled):
     s = Solver(pat).setup(vals)
     f = np.random.default_rng(1).normal(size=6 * nodes)
     for _ in range(2):  # the second solve sees values changed in place, one more of them non-zero
-        u, st = s.solve(torch.from_numpy(f).cuda(), tol=1e-13, check_every=2)
+        u, st = s.solve(torch.from_numpy(f).cuda(), tol=1e-13, check_every=2, flexible=flexible)
         assert st['status'] == 'converged'
         ref = spsolve(pat.to_scipy(vals).tocsc(), f)
         assert np.linalg.norm(u.cpu().numpy() - ref) <= 1e-11 * np.linalg.norm(ref)  # condition number below 100
         v = 3. * v
         v[((r == 0) & (c == 8)) | ((r == 8) & (c == 0))] = 0.25
         pat.assemble(v, out=vals)
+
+
+@pytest.mark.parametrize('nodes', [40, 5000])
+@pytest.mark.parametrize('order', ['shuffled', 'fixed'])
+def test_numbering_and_partial_nodes(gpulib, nodes, order):
+    """Nodes in random order (5000: a block's columns no longer fit shared memory) and nodes with fixed DOFs."""
+    import torch
+    from scipy.sparse.linalg import spsolve
+    from pyfe3d_gb300.solver import CSRPattern, Solver
+    rng = np.random.default_rng(7)
+    r, c, v = _triplets(nodes, False, 3)
+    bk = None
+    if order == 'shuffled':
+        perm = rng.permutation(nodes)
+        r, c = 6 * perm[r // 6] + r % 6, 6 * perm[c // 6] + c % 6
+    else:
+        bk = rng.random(6 * nodes) < 0.3
+        bk[60:90] = True
+    pat = CSRPattern(r, c, 6 * nodes, bk)
+    vals = pat.assemble(v)
+    s = Solver(pat).setup(vals)
+    f = rng.normal(size=pat.nrows)
+    u, st = s.solve(torch.from_numpy(f).cuda(), tol=1e-13)
+    assert st['status'] == 'converged'
+    ref = spsolve(pat.to_scipy(vals).tocsc(), f)
+    assert np.linalg.norm(u.cpu().numpy() - ref) <= 1e-11 * np.linalg.norm(ref)
+    # few iterations and a restart from their iterate: the same recurrence cut short
+    u1, st1 = s.solve(torch.from_numpy(f).cuda(), tol=1e-300, maxiter=5, check_every=2)
+    assert st1['iterations'] == 5
+    u2, st2 = s.solve(torch.from_numpy(f).cuda(), u0=u1, tol=1e-13, check_every=7)
+    assert st2['status'] == 'converged'
+    assert np.linalg.norm(u2.cpu().numpy() - ref) <= 1e-11 * np.linalg.norm(ref)
