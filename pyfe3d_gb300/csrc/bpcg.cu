@@ -604,8 +604,10 @@ __global__ void __launch_bounds__(CT) bcta_kernel(CtaArgs a) {
                     break;
                 }
                 if (rr <= lim) {
+                    // 5 % below the tolerance: the reported residual is summed in
+                    // another order, which moves it by up to a percent here
                     const double rt = cta_rows(a, r0, r1, a.u, 0, a.r, 0, a.f, red);
-                    if (rt <= lim) {
+                    if (rt <= 0.9 * lim) {
                         status = 0;
                         break;
                     }
