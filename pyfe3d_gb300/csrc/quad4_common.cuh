@@ -140,9 +140,10 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // the element axes when m12 != 0 (quad4.pyx:845-899), shear correction on E
 // (quad4.pyx:903-905), then, for flat elements evaluated in the global frame,
 // the in-plane rotation element -> global of ABD and of the shear matrix.
-__device__ void q4_constitutive(const double *P, const double *m, const double *R,
-                                bool global_frame, double *abd36, double *es) {
-    double A[6], B[6], D[6];
+// A, B and D come packed as 11 12 16 22 26 66.
+__device__ __forceinline__ void q4_constitutive_packed(const double *P, const double *m, const double *R,
+                                                       bool global_frame, double *A, double *B, double *D,
+                                                       double *es) {
     if (m[1] == 0.) {
 #pragma unroll
         for (int i = 0; i < 6; i++) {
@@ -181,7 +182,16 @@ __device__ void q4_constitutive(const double *P, const double *m, const double *
         E45 = g01;
         E44 = g11;
     }
-    // full symmetric 6x6 [[A, B], [B, D]]
+    es[0] = E44;
+    es[1] = E45;
+    es[2] = E55;
+}
+
+// The same as the full symmetric 6x6 [[A, B], [B, D]].
+__device__ void q4_constitutive(const double *P, const double *m, const double *R,
+                                bool global_frame, double *abd36, double *es) {
+    double A[6], B[6], D[6];
+    q4_constitutive_packed(P, m, R, global_frame, A, B, D, es);
     const int idx[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
 #pragma unroll
     for (int i = 0; i < 3; i++)
@@ -192,9 +202,6 @@ __device__ void q4_constitutive(const double *P, const double *m, const double *
             abd36[6 * (i + 3) + j] = B[idx[i][j]];
             abd36[6 * (i + 3) + j + 3] = D[idx[i][j]];
         }
-    es[0] = E44;
-    es[1] = E45;
-    es[2] = E55;
 }
 
 // --- KC0 pair block -------------------------------------------------------

@@ -7,7 +7,8 @@
 //
 //   phase A   one thread per element (FP64): frame R (and material cosines),
 //             flatness test, constitutive matrices in the evaluation frame,
-//             nodal coordinates relative to node 1, thin/thick flag.
+//             nodal coordinates relative to node 1, thin/thick flag.  Flat
+//             isotropic elements need no frame (kc0_setup_flat_iso).
 //   phase A2  one thread per (element, point) at the 4 Gauss points and the
 //             centre: Jacobian and Cartesian shape derivatives, computed in
 //             float-float (FP32 pipe) for flat elements.
@@ -19,12 +20,20 @@
 //             in row groups (no lane holds a whole block: for isotropic
 //             sections -- rotation-invariant A, D, E and B = 0 -- the 18
 //             non-zeros in two groups, otherwise three rows at a time);
+//             current values that are all zeros are not added to but stored
+//             over, and entries that are exact zeros are not multiplied out;
 //   write-out each warp streams its two staged elements (576 values each)
 //             with the coalesced += read-modify-write and the indices.
 //
-// CTAs of 8 warps (FE3D_KC0_WARPS), two per SM (FE3D_KC0_MINB, 128
-// registers): 16 warps per SM; phase A runs on warp 0 while the other warps
-// write out their last round of the previous tile.
+// CTAs of 8 warps, two per SM (128 registers): the last warp runs phase A one
+// tile ahead into the other half of a double buffer, the 7 others run A2 and B
+// and write out, four elements each per tile, with one barrier per tile.  (With
+// phase A on a warp of the same tile the others waited for it: 20,000 of a
+// tile's 70,000 cycles.)  1,000,000 flat isotropic elements with indices onto
+// cleared values 3.56 -> 3.09 ms, 0.88 of the 2.95 ms that reading and writing
+// the values and writing the indices take with the same stores and no element
+// work; DRAM at 5.8 TB/s.  90,000 elements into CSR 0.73 -> 0.50 ms, 28,800
+// laminated elements of a cylinder 0.42 -> 0.38 ms.
 //
 // Flat elements whose normal is +Z (r13 = r23 = r31 = r32 = 0) are evaluated
 // in the global frame with in-plane rotated constitutive matrices (no
@@ -38,20 +47,18 @@
 namespace fe3d {
 namespace {
 
-#ifndef FE3D_KC0_TILE
-#define FE3D_KC0_TILE 32
-#endif
-#ifndef FE3D_KC0_WARPS
-#define FE3D_KC0_WARPS 8
-#endif
-constexpr int KT = FE3D_KC0_TILE;  // elements per CTA iteration (phase A: one lane each)
-constexpr int KNT = 32 * FE3D_KC0_WARPS;  // threads per CTA
-constexpr int KRND = 2 * FE3D_KC0_WARPS;  // elements per phase-B round (two per warp)
-static_assert(KT % KRND == 0 && KT <= 32, "a tile is whole rounds of elements, phase A one warp");
+constexpr int KCW = 7;                  // consumer warps of a CTA; one more runs phase A
+constexpr int KNT = 32 * (KCW + 1);     // threads per CTA
+constexpr int KPER = 4;                 // elements per consumer warp and tile at most (two per round)
+constexpr int KT = KCW * KPER;          // elements per tile at most (phase A: one lane each)
+constexpr int KMINB = 2;                // CTAs per SM
+static_assert(KT <= 32, "phase A is one warp");
 constexpr int KPTS = 5;   // 4 Gauss points + centre
 constexpr int KSLOT = 9;  // per point: w detJ, Nx[4], Ny[4] (N is the same for every element)
 
-enum : int { KF_VALID = 1, KF_THICK = 2, KF_FP64 = 4, KF_ISO = 8 };
+// KF_SPLIT: (u, v, rz) and (w, rx, ry) do not couple (evaluated in the global
+// frame with B = 0); KF_B0: B = 0
+enum : int { KF_VALID = 1, KF_THICK = 2, KF_FP64 = 4, KF_ISO = 8, KF_B0 = 16, KF_SPLIT = 32 };
 
 union Slot {
     double d;
@@ -60,7 +67,8 @@ union Slot {
 
 struct __align__(16) KElem {
     double R[9];
-    double abd[36];
+    double A[6], B[6], D[6];  // 11 12 16 22 26 66
+    double ap, am;            // A66 + 1/4, A66 - 1/4: with the unit drilling weight
     double es[3];
     Slot xy[8];
     long long init_k;
@@ -70,15 +78,104 @@ struct __align__(16) KElem {
 };
 
 struct KSmem {
-    KElem el[KT];
+    KElem el[2][KT];  // the tile in work, and the next one that phase A fills
     Slot gp[KT][KPTS][KSLOT];
     ff shape[KPTS][3][4];
-    double stage[KNT / 32][2][24 * KROW];
+    double stage[KCW][2][24 * KROW];
 };
 
 // shape-function values and natural derivatives at the 5 points, float-float:
 // [point][0: N, 1: dN/dxi, 2: dN/deta][node]
 __constant__ ff c_shape[KPTS][3][4];
+
+// Comparisons of doubles with integer operations (a DSETP takes the FP64 pipe
+// for 64 cycles): the results of ==, == 0 and > 0.
+__device__ __forceinline__ unsigned long long dbits(double v) { return (unsigned long long)__double_as_longlong(v); }
+__device__ __forceinline__ bool is_zero(double v) { return (dbits(v) << 1) == 0; }
+__device__ __forceinline__ bool is_nan(double v) { return (dbits(v) << 1) > 0xffe0000000000000ull; }
+__device__ __forceinline__ bool is_eq(double a, double b) {
+    return (dbits(a) == dbits(b) && !is_nan(a)) || (is_zero(a) && is_zero(b));
+}
+__device__ __forceinline__ bool is_pos(double v) { return (long long)dbits(v) > 0 && !is_nan(v); }
+__device__ __forceinline__ bool is_finite(double v) { return (dbits(v) << 1) < 0xffe0000000000000ull; }
+
+// Set-up of a flat isotropic element with its normal along +z, which needs no
+// frame: the decisions of q4_rotation + is_flat + iso_section, taken from the
+// coordinates and the record with 20 FP64 instructions instead of about 200.
+// Phase A is the serial part of a tile (one warp works, each FP64 instruction
+// takes it 64 cycles), so this is what small meshes and the tile rate wait for.
+// Returns false, with nothing decided, for any other element.
+__device__ __forceinline__ bool kc0_setup_flat_iso(const Q4Args &a, const long long *c, const double *P, KElem &s) {
+    double X[4], Y[4], Z[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const double *q = a.x + c[i] / 2;
+        X[i] = q[0];
+        Y[i] = q[1];
+        Z[i] = q[2];
+    }
+    // r13 = r23 = r31 = r32 = 0: the diagonals have no z component
+    bool flat = is_eq(Z[0], Z[2]) && is_eq(Z[1], Z[3]) && is_finite(Z[0]) && is_finite(Z[1]);
+    double xy[8];
+    bool safe = true;
+    xy[0] = xy[1] = 0.;
+#pragma unroll
+    for (int i = 1; i < 4; i++) {
+        xy[2 * i] = X[i] - X[0];
+        xy[2 * i + 1] = Y[i] - Y[0];
+        safe &= ff_safe(xy[2 * i]) && ff_safe(xy[2 * i + 1]);
+    }
+    const double vx = X[1] - X[3], vy = Y[1] - Y[3];
+    flat &= is_pos(vx * xy[5] - vy * xy[4]);
+    if (!flat || !safe) return false;
+    const double E44 = P[SP_E44] * P[SP_SCF23];
+    const double E45 = P[SP_E45] * 0.5 * (P[SP_SCF13] + P[SP_SCF23]);
+    const double E55 = P[SP_E55] * P[SP_SCF13];
+    const double A11 = P[SP_A11], A12 = P[SP_A12], A66 = P[SP_A66];
+    const double D11 = P[SP_D11], D12 = P[SP_D12], D66 = P[SP_D66];
+    bool iso = is_zero(P[SP_A16]) && is_zero(P[SP_A26]) && is_zero(P[SP_D16]) && is_zero(P[SP_D26]);
+#pragma unroll
+    for (int i = 0; i < 6; i++) iso &= is_zero(P[SP_B11 + i]);
+    iso &= is_eq(A11, P[SP_A22]) && is_eq(D11, P[SP_D22]) && is_zero(E45) && is_eq(E44, E55);
+    const double eps = 64. * 2.220446049250313e-16;
+    // |x| <= y of non-negative doubles compares their bits
+    iso &= dbits(fabs(A66 - 0.5 * (A11 - A12))) <= dbits(eps * fabs(A11));
+    iso &= dbits(fabs(D66 - 0.5 * (D11 - D12))) <= dbits(eps * fabs(D11));
+    if (!iso) return false;
+    s.A[0] = A11;
+    s.A[1] = A12;
+    s.D[0] = D11;
+    s.D[1] = D12;
+    s.D[5] = D66;
+    s.ap = A66 + 0.25;
+    s.am = A66 - 0.25;
+    s.es[0] = E44;
+    s.es[1] = 0.;
+    s.es[2] = E55;
+    ff q[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        q[i] = i < 2 ? ff{0.f, 0.f} : ff_from_double(xy[i]);
+        s.xy[i].f = q[i];
+    }
+    // h / sqrt(area) >= 1, in floats where they decide it
+    const double h = P[SP_H];
+    const float hf = (float)h;
+    const float t1 = q[2].h * q[5].h, t2 = q[4].h * q[3].h, t3 = q[4].h * q[7].h, t4 = q[6].h * q[5].h;
+    const float ar = 0.5f * fabsf((t1 - t2) + (t3 - t4));
+    const float er = 1e-6f * (fabsf(t1) + fabsf(t2) + fabsf(t3) + fabsf(t4)), hh = hf * hf;
+    bool thick = false;
+    if (!(hf > 0.f && hh * 1.00001f < ar - er)) {
+        if (hf > 0.f && hh > (ar + er) * 1.00001f) {
+            thick = true;
+        } else {
+            const double sq = sqrt(shoelace(xy));
+            thick = h >= sq || h / sq >= 1.;
+        }
+    }
+    s.flags = KF_VALID | KF_ISO | KF_B0 | KF_SPLIT | (thick ? KF_THICK : 0);
+    return true;
+}
 
 // Element set-up shared by the triplet and the CSR kernels: frame,
 // flatness, constitutive data and nodal coordinates of element e with DOF
@@ -93,9 +190,10 @@ __device__ void kc0_elem_setup(const Q4Args &a, int64_t e, const long long *c, b
         raise_error(a.err, kErrBounds);
         return;
     }
+    if (a.x && kc0_setup_flat_iso(a, c, a.props + (int64_t)SP_STRIDE * p, s)) return;
     const double *P = a.props + (int64_t)SP_STRIDE * p;
     double R[9], m[4] = {1., 0., 0., 1.}, xy[8], ar;
-    bool fp64 = true, iso = false;
+    bool fp64 = true;
     if (a.x) {
         const double *pp[4] = {a.x + c[0] / 2, a.x + c[1] / 2, a.x + c[2] / 2, a.x + c[3] / 2};
         q4_rotation(pp[0], pp[1], pp[2], pp[3], a.xmat ? a.xmat + (int64_t)a.xmat_stride * e : nullptr,
@@ -110,27 +208,7 @@ __device__ void kc0_elem_setup(const Q4Args &a, int64_t e, const long long *c, b
             }
             fp64 = !safe;
         }
-        if (!fp64) {
-            const double E44 = P[SP_E44] * P[SP_SCF23];
-            const double E45 = P[SP_E45] * 0.5 * (P[SP_SCF13] + P[SP_SCF23]);
-            const double E55 = P[SP_E55] * P[SP_SCF13];
-            iso = iso_section(P, E44, E45, E55);
-            if (iso) {
-                // rotation-invariant section: the material values are the
-                // global-frame values (A11 A12 A66, D11 D12 D66, E44)
-                s.abd[0] = P[SP_A11];
-                s.abd[1] = P[SP_A12];
-                s.abd[2] = P[SP_A66];
-                s.abd[3] = P[SP_D11];
-                s.abd[4] = P[SP_D12];
-                s.abd[5] = P[SP_D66];
-                s.es[0] = E44;
-                s.es[1] = 0.;
-                s.es[2] = E55;
-            } else {
-                q4_constitutive(P, m, R, true, s.abd, s.es);
-            }
-        } else {
+        if (fp64) {
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 double q[3];
@@ -138,8 +216,8 @@ __device__ void kc0_elem_setup(const Q4Args &a, int64_t e, const long long *c, b
                 xy[2 * i] = q[0];
                 xy[2 * i + 1] = q[1];
             }
-            q4_constitutive(P, m, R, false, s.abd, s.es);
         }
+        q4_constitutive_packed(P, m, R, !fp64, s.A, s.B, s.D, s.es);
         ar = shoelace(xy);
     } else {
 #pragma unroll
@@ -151,9 +229,14 @@ __device__ void kc0_elem_setup(const Q4Args &a, int64_t e, const long long *c, b
             xy[2 * i] = a.xe[12 * e + 3 * i];
             xy[2 * i + 1] = a.xe[12 * e + 3 * i + 1];
         }
-        q4_constitutive(P, m, R, false, s.abd, s.es);
+        q4_constitutive_packed(P, m, R, false, s.A, s.B, s.D, s.es);
         ar = a.area[e];
     }
+    s.ap = s.A[5] + 0.25;
+    s.am = s.A[5] - 0.25;
+    bool b0 = true;
+#pragma unroll
+    for (int i = 0; i < 6; i++) b0 &= is_zero(s.B[i]);
 #pragma unroll
     for (int i = 0; i < 9; i++) s.R[i] = R[i];
     if (fp64) {
@@ -168,7 +251,8 @@ __device__ void kc0_elem_setup(const Q4Args &a, int64_t e, const long long *c, b
     // quotient is >= 1)
     const double sq = sqrt(ar);
     const bool thick = P[SP_H] >= sq || P[SP_H] / sq >= 1.;
-    s.flags = KF_VALID | (thick ? KF_THICK : 0) | (fp64 ? KF_FP64 : 0) | (iso ? KF_ISO : 0);
+    s.flags = KF_VALID | (thick ? KF_THICK : 0) | (fp64 ? KF_FP64 : 0) | (b0 ? KF_B0 : 0) |
+              (b0 && !fp64 ? KF_SPLIT : 0);
 }
 
 __device__ void kc0_phase_a2(const Q4Args &a, int64_t e, KElem &s) {
@@ -261,26 +345,6 @@ __device__ __forceinline__ void write_staged(const Q4Args &a, const double *sv, 
     }
 }
 
-// The element data of a staged element whose write-out is deferred, kept in
-// the stage's padding columns (24, 25), which the values never use.
-__device__ __forceinline__ long long *stage_meta(double *sv, int i) {
-    return reinterpret_cast<long long *>(sv + (i >> 1) * KROW + 24 + (i & 1));
-}
-
-// Writes out a warp's two deferred elements.
-__device__ __forceinline__ void flush_deferred(const Q4Args &a, double (*stage)[24 * KROW], int lane) {
-#pragma unroll
-    for (int hh = 0; hh < 2; hh++) {
-        double *sv = stage[hh];
-        if (!(*stage_meta(sv, 0) & KF_VALID)) continue;
-        long long c[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) c[i] = *stage_meta(sv, 2 + i);
-        write_staged(a, sv, *stage_meta(sv, 1), c, lane);
-    }
-    __syncwarp();
-}
-
 // N_i at point g in FP64, the expression of quad_derivs (elements evaluated
 // in FP64 only).
 __device__ __forceinline__ double shape_n(int g, int i) {
@@ -293,7 +357,8 @@ __device__ __forceinline__ double shape_n(int g, int i) {
 // The 4-point tensor H^pq_ab = sum_g w detJ D^p N_a D^q N_b (p, q in
 // {N, d/dx, d/dy}) of node pair (na, nb) of element slot el: accumulated in
 // float-float and rounded to double, or in FP64 for elements evaluated in
-// FP64 (FF = false).
+// FP64 (FF = false).  The entries (N, d) and (d, N) are halved, as the drilling
+// penalty uses them.
 template <bool FF>
 __device__ __forceinline__ void pair_h(const KSmem &S, int el, int na, int nb, double H[3][3]) {
     if (FF) {
@@ -302,7 +367,9 @@ __device__ __forceinline__ void pair_h(const KSmem &S, int el, int na, int nb, d
         for (int p = 0; p < 3; p++)
 #pragma unroll
             for (int q = 0; q < 3; q++) h[p][q] = ffz();
-#pragma unroll
+        // (rolled: a quarter of the code, which the kernel otherwise fetches
+        // from beyond the instruction cache: 4.27 -> 4.12 ms per 1M elements)
+#pragma unroll 1
         for (int g = 0; g < 4; g++) {
             const Slot *o = S.gp[el][g];
             const ff w = o[0].f;
@@ -316,7 +383,8 @@ __device__ __forceinline__ void pair_h(const KSmem &S, int el, int na, int nb, d
 #pragma unroll
         for (int p = 0; p < 3; p++)
 #pragma unroll
-            for (int q = 0; q < 3; q++) H[p][q] = ff_to_double(h[p][q]);
+            for (int q = 0; q < 3; q++)
+                H[p][q] = ff_to_double((p == 0) != (q == 0) ? ff_scale(h[p][q], 0.5f) : h[p][q]);
     } else {
 #pragma unroll
         for (int p = 0; p < 3; p++)
@@ -333,6 +401,10 @@ __device__ __forceinline__ void pair_h(const KSmem &S, int el, int na, int nb, d
 #pragma unroll
                 for (int q = 0; q < 3; q++) H[p][q] += va[p] * vb[q];
         }
+        H[0][1] *= 0.5;
+        H[0][2] *= 0.5;
+        H[1][0] *= 0.5;
+        H[2][0] *= 0.5;
     }
 }
 
@@ -353,6 +425,8 @@ struct CentreH<true> {
         b[2] = o[5 + nb].f;
     }
     __device__ __forceinline__ double operator()(int p, int q) const { return ff_to_double(ff_mul(a[p], b[q])); }
+    // H0^xx + H0^yy
+    __device__ __forceinline__ double trace() const { return ff_to_double(ff_fma(a[1], b[1], ff_mul(a[2], b[2]))); }
 };
 template <>
 struct CentreH<false> {
@@ -370,104 +444,254 @@ struct CentreH<false> {
     __device__ __forceinline__ double operator()(int p, int q) const { return a[p] * b[q]; }
 };
 
+__device__ __forceinline__ double2 *staged(double *st, int na, int nb, int m, int n) {
+    return reinterpret_cast<double2 *>(st + (6 * na + m) * KROW + 6 * nb + n);
+}
+
+// Adds (x, y) onto the staged pair (row m of node na, columns n, n + 1 of node
+// nb); X, Y false: that entry of the block is an exact zero and stays as it
+// is.  CLEAR: the lane's staged entries are known to be zeros, so the sum is
+// the entry itself.
+template <bool CLEAR, bool X = true, bool Y = true>
 __device__ __forceinline__ void add2(double *st, int na, int nb, int m, int n, double x, double y) {
-    double2 *q = reinterpret_cast<double2 *>(st + (6 * na + m) * KROW + 6 * nb + n);
-    double2 o = *q;
-    o.x += x;
-    o.y += y;
-    *q = o;
+    double2 *q = staged(st, na, nb, m, n);
+    if (CLEAR && X && Y) {
+        *q = make_double2(x, y);
+    } else if (CLEAR) {
+        if (X) q->x = x;
+        if (Y) q->y = y;
+    } else {
+        double2 o = *q;
+        if (X) o.x += x;
+        if (Y) o.y += y;
+        *q = o;
+    }
+}
+
+// Whether the current values that the block of every lane adds to are zeros (a
+// cleared array, assigned CSR blocks): the FP64 additions are left out then
+// (36 or 18 instructions of 64 cycles each).  SPLIT: only the entries within
+// (u, v, rz) and (w, rx, ry) count.
+template <bool SPLIT>
+__device__ __forceinline__ bool stage_clear(double *st, int na, int nb) {
+    unsigned long long any = 0;
+#pragma unroll
+    for (int m = 0; m < 6; m++)
+#pragma unroll
+        for (int n = 0; n < 6; n += 2) {
+            const bool mid = m >= 2 && m <= 4;  // rows w, rx, ry
+            const bool x = !SPLIT || (mid ? n >= 2 : n == 0), y = !SPLIT || (mid ? n == 2 : n != 2);
+            if (!x && !y) continue;
+            const double2 o = *staged(st, na, nb, m, n);
+            if (x) any |= dbits(o.x) << 1;
+            if (y) any |= dbits(o.y) << 1;
+        }
+    return __all_sync(__activemask(), any == 0);
 }
 
 // Adds the 6x6 block K_ab of a flat isotropic element in the global frame
-// (B = 0, E45 = 0; abd holds A11 A12 A66 D11 D12 D66, es E44 0 E55) onto the
-// staged values: the non-zero terms of kc0_block for A11 = A22,
-// A16 = A26 = 0 (same for D), with the unit drilling weight folded into the
-// A66 terms.  The block couples (u, v, rz) and (w, rx, ry) only: the slot
-// pairs that hold exact zeros (cols 2-3 of rows u, v, rz; cols 0-1 of rows
-// w, rx, ry) are left as they are, and each group is added as soon as it is
-// formed.
+// (B = 0, E45 = 0, E44 = E55) onto the staged values: the non-zero terms for
+// A11 = A22, A16 = A26 = 0 (same for D).  The block couples (u, v, rz) and
+// (w, rx, ry) only, and each group is added as soon as it is formed.
+template <bool CLEAR>
 __device__ __forceinline__ void pair_add_iso(const KElem &s, const double H[3][3], const CentreH<true> &h0,
                                              double *st, int na, int nb) {
-    const double *abd = s.abd;
-    const double A11 = abd[0], A12 = abd[1], A66 = abd[2];
-    const double am = A66 + 0.25, an = A66 - 0.25;
+    const double A11 = s.A[0], A12 = s.A[1], ap = s.ap, am = s.am;
     // membrane and drilling: rows and columns u, v, rz
-    add2(st, na, nb, 0, 0, A11 * H[1][1] + am * H[2][2], A12 * H[1][2] + an * H[2][1]);
-    add2(st, na, nb, 0, 4, 0., 0.5 * H[2][0]);
-    add2(st, na, nb, 1, 0, an * H[1][2] + A12 * H[2][1], am * H[1][1] + A11 * H[2][2]);
-    add2(st, na, nb, 1, 4, 0., -0.5 * H[1][0]);
-    add2(st, na, nb, 5, 0, 0.5 * H[0][2], -0.5 * H[0][1]);
-    add2(st, na, nb, 5, 4, 0., H[0][0]);
+    add2<CLEAR>(st, na, nb, 0, 0, A11 * H[1][1] + ap * H[2][2], A12 * H[1][2] + am * H[2][1]);
+    add2<CLEAR, false, true>(st, na, nb, 0, 4, 0., H[2][0]);
+    add2<CLEAR>(st, na, nb, 1, 0, am * H[1][2] + A12 * H[2][1], ap * H[1][1] + A11 * H[2][2]);
+    add2<CLEAR, false, true>(st, na, nb, 1, 4, 0., -H[1][0]);
+    add2<CLEAR>(st, na, nb, 5, 0, H[0][2], -H[0][1]);
+    add2<CLEAR, false, true>(st, na, nb, 5, 4, 0., H[0][0]);
     // bending and transverse shear: rows and columns w, rx, ry
-    const double D11 = abd[3], D12 = abd[4], D66 = abd[5];
-    const double E44 = s.es[0], E55 = s.es[2];
-    const bool thick = s.flags & KF_THICK;
-    const double c00 = h0(0, 0);
-    const double hs22 = thick ? H[2][2] : h0(2, 2), hs11 = thick ? H[1][1] : h0(1, 1);
-    add2(st, na, nb, 2, 2, E44 * hs22 + E55 * hs11, -E44 * h0(2, 0));
-    add2(st, na, nb, 2, 4, E55 * h0(1, 0), 0.);
-    add2(st, na, nb, 3, 2, -E44 * h0(0, 2), D66 * H[1][1] + D11 * H[2][2] + E44 * c00);
-    add2(st, na, nb, 3, 4, -(D66 * H[1][2] + D12 * H[2][1]), 0.);
-    add2(st, na, nb, 4, 2, E55 * h0(0, 1), -(D12 * H[1][2] + D66 * H[2][1]));
-    add2(st, na, nb, 4, 4, D11 * H[1][1] + D66 * H[2][2] + E55 * c00, 0.);
+    const double D11 = s.D[0], D12 = s.D[1], D66 = s.D[5], E = s.es[0];
+    const double ec = E * h0(0, 0);
+    add2<CLEAR>(st, na, nb, 2, 2, E * ((s.flags & KF_THICK) ? H[1][1] + H[2][2] : h0.trace()), -E * h0(2, 0));
+    add2<CLEAR, true, false>(st, na, nb, 2, 4, E * h0(1, 0), 0.);
+    add2<CLEAR>(st, na, nb, 3, 2, -E * h0(0, 2), D66 * H[1][1] + (D11 * H[2][2] + ec));
+    add2<CLEAR, true, false>(st, na, nb, 3, 4, -(D66 * H[1][2] + D12 * H[2][1]), 0.);
+    add2<CLEAR>(st, na, nb, 4, 2, E * h0(0, 1), -(D12 * H[1][2] + D66 * H[2][1]));
+    add2<CLEAR, true, false>(st, na, nb, 4, 4, D11 * H[1][1] + (D66 * H[2][2] + ec), 0.);
 }
 
-// Adds the general 6x6 block K_ab (kc0_block; rotated to the global frame
-// for elements evaluated in the element frame) onto the staged values,
-// three rows at a time (a row block of T K T^T needs only the same row
-// block of K).
-template <bool FF>
+// sum_pq X[s_p t_q] H^pq over p, q in {x, y}: the coupling by X (11 12 16 22
+// 26 66) of the strains (s_x, s_y) and (t_x, t_y) that the two DOFs'
+// derivatives make (0 xx, 1 yy, 2 xy); the xy-xy term takes x66.
+__device__ __forceinline__ constexpr int sym3(int i, int j) {
+    return i > j ? sym3(j, i) : i == 0 ? j : i == 1 ? 2 + j : 5;
+}
+template <int SX, int SY, int TX, int TY>
+__device__ __forceinline__ double couple(const double *X, double x66, const double H[3][3]) {
+    auto c = [&](int i, int j) { return sym3(i, j) == 5 ? x66 : X[sym3(i, j)]; };
+    return (c(SX, TX) * H[1][1] + c(SX, TY) * H[1][2]) + (c(SY, TX) * H[2][1] + c(SY, TY) * H[2][2]);
+}
+
+// out = tmp R^T: three rows of a 3x3 part turned to the global axes, from
+// tmp = R K.
+__device__ __forceinline__ void turn(const double *R, const double (&tmp)[3][3], double (&out)[3][3]) {
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++)
+            out[i][j] = tmp[i][0] * R[3 * j] + tmp[i][1] * R[3 * j + 1] + tmp[i][2] * R[3 * j + 2];
+}
+
+// Adds the general 6x6 block K_ab onto the staged values, three rows at a
+// time.  Strains: u -> (xx, xy), v -> (xy, yy), rx -> -(xy, yy), ry -> (xx, xy)
+// for the x and y derivatives (quad4.pyx:958-1000), drilling with unit weight
+// d = u N_y / 2 - v N_x / 2 + rz N, shear (gyz, gxz) = (w_y - rx N, w_x + ry N).
+// Of the block's 36 entries 10 are exact zeros, 18 with B = 0 (B0); elements
+// evaluated in the element frame turn the 3x3 parts without multiplying them
+// (FP64 instructions per lane, B = 0: 260 instead of 400), the others leave
+// them out.
+template <bool FF, bool B0, bool CLEAR>
 __device__ __forceinline__ void pair_add_general(const KElem &s, const double H[3][3], const CentreH<FF> &h0,
                                                  double *st, int na, int nb) {
     const bool thick = s.flags & KF_THICK;
-    double H0[3][3], Hs[3][3];
-#pragma unroll
-    for (int p = 0; p < 3; p++)
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-            H0[p][q] = h0(p, q);
-            Hs[p][q] = thick ? H[p][q] : H0[p][q];
-        }
+    const double E44 = s.es[0], E45 = s.es[1], E55 = s.es[2];
+    const double *R = s.R, *A = s.A, *B = s.B, *D = s.D;
 #pragma unroll
     for (int hb = 0; hb < 2; hb++) {
-        double K[6][6];
-        kc0_block(H, H0, Hs, s.abd, s.es, K);
-        if (!FF) rotate_block(s.R, K);
+        // the rows' 3x3 parts: columns u v w and rx ry rz
+        double P[3][3], Q[3][3];
+        if (hb == 0) {
+            const double s22 = thick ? H[2][2] : h0(2, 2), s11 = thick ? H[1][1] : h0(1, 1);
+            const double s21 = thick ? H[2][1] : h0(2, 1), s12 = thick ? H[1][2] : h0(1, 2);
+            P[0][0] = couple<0, 2, 0, 2>(A, s.ap, H);
+            P[0][1] = couple<0, 2, 2, 1>(A, s.am, H);
+            P[1][0] = couple<2, 1, 0, 2>(A, s.am, H);
+            P[1][1] = couple<2, 1, 2, 1>(A, s.ap, H);
+            P[2][2] = E44 * s22 + E45 * (s21 + s12) + E55 * s11;
+            if (!B0) {
+                Q[0][0] = -couple<0, 2, 2, 1>(B, B[5], H);
+                Q[0][1] = couple<0, 2, 0, 2>(B, B[5], H);
+                Q[1][0] = -couple<2, 1, 2, 1>(B, B[5], H);
+                Q[1][1] = couple<2, 1, 0, 2>(B, B[5], H);
+            }
+            Q[0][2] = H[2][0];
+            Q[1][2] = -H[1][0];
+            const double h20 = h0(2, 0), h10 = h0(1, 0);
+            Q[2][0] = -(E44 * h20 + E45 * h10);
+            Q[2][1] = E45 * h20 + E55 * h10;
+        } else {
+            if (!B0) {
+                P[0][0] = -couple<2, 1, 0, 2>(B, B[5], H);
+                P[0][1] = -couple<2, 1, 2, 1>(B, B[5], H);
+                P[1][0] = couple<0, 2, 0, 2>(B, B[5], H);
+                P[1][1] = couple<0, 2, 2, 1>(B, B[5], H);
+            }
+            const double h02 = h0(0, 2), h01 = h0(0, 1), h00 = h0(0, 0);
+            P[0][2] = -(E44 * h02 + E45 * h01);
+            P[1][2] = E45 * h02 + E55 * h01;
+            P[2][0] = H[0][2];
+            P[2][1] = -H[0][1];
+            const double e45 = E45 * h00;
+            Q[0][0] = couple<2, 1, 2, 1>(D, D[5], H) + E44 * h00;
+            Q[0][1] = -(couple<2, 1, 0, 2>(D, D[5], H) + e45);
+            Q[1][0] = -(couple<0, 2, 2, 1>(D, D[5], H) + e45);
+            Q[1][1] = couple<0, 2, 0, 2>(D, D[5], H) + E55 * h00;
+            Q[2][2] = H[0][0];
+        }
+        if (FF) {
+            if (hb == 0) {
+                add2<CLEAR>(st, na, nb, 0, 0, P[0][0], P[0][1]);
+                add2<CLEAR>(st, na, nb, 1, 0, P[1][0], P[1][1]);
+                if (B0) {
+                    add2<CLEAR, false, true>(st, na, nb, 0, 4, 0., Q[0][2]);
+                    add2<CLEAR, false, true>(st, na, nb, 1, 4, 0., Q[1][2]);
+                } else {
+                    add2<CLEAR, false, true>(st, na, nb, 0, 2, 0., Q[0][0]);
+                    add2<CLEAR, false, true>(st, na, nb, 1, 2, 0., Q[1][0]);
+                    add2<CLEAR>(st, na, nb, 0, 4, Q[0][1], Q[0][2]);
+                    add2<CLEAR>(st, na, nb, 1, 4, Q[1][1], Q[1][2]);
+                }
+                add2<CLEAR>(st, na, nb, 2, 2, P[2][2], Q[2][0]);
+                add2<CLEAR, true, false>(st, na, nb, 2, 4, Q[2][1], 0.);
+            } else {
+                if (!B0) {
+                    add2<CLEAR>(st, na, nb, 3, 0, P[0][0], P[0][1]);
+                    add2<CLEAR>(st, na, nb, 4, 0, P[1][0], P[1][1]);
+                }
+                add2<CLEAR>(st, na, nb, 3, 2, P[0][2], Q[0][0]);
+                add2<CLEAR>(st, na, nb, 4, 2, P[1][2], Q[1][0]);
+                add2<CLEAR, true, false>(st, na, nb, 3, 4, Q[0][1], 0.);
+                add2<CLEAR, true, false>(st, na, nb, 4, 4, Q[1][1], 0.);
+                add2<CLEAR>(st, na, nb, 5, 0, P[2][0], P[2][1]);
+                add2<CLEAR, false, true>(st, na, nb, 5, 4, 0., Q[2][2]);
+            }
+        } else {
+            double tp[3][3], tq[3][3], op[3][3], oq[3][3];
 #pragma unroll
-        for (int m = 3 * hb; m < 3 * hb + 3; m++)
+            for (int i = 0; i < 3; i++) {
+                const double x = R[3 * i], y = R[3 * i + 1], z = R[3 * i + 2];
 #pragma unroll
-            for (int n = 0; n < 6; n += 2) add2(st, na, nb, m, n, K[m][n], K[m][n + 1]);
+                for (int j = 0; j < 2; j++) {
+                    const double inP = hb == 0 || !B0 ? x * P[0][j] + y * P[1][j] : 0.;
+                    const double inQ = hb == 1 || !B0 ? x * Q[0][j] + y * Q[1][j] : 0.;
+                    tp[i][j] = hb == 0 ? inP : B0 ? z * P[2][j] : inP + z * P[2][j];
+                    tq[i][j] = hb == 1 ? inQ : B0 ? z * Q[2][j] : inQ + z * Q[2][j];
+                }
+                tp[i][2] = hb == 0 ? z * P[2][2] : x * P[0][2] + y * P[1][2];
+                tq[i][2] = hb == 1 ? z * Q[2][2] : x * Q[0][2] + y * Q[1][2];
+            }
+            turn(R, tp, op);
+            turn(R, tq, oq);
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                add2<CLEAR>(st, na, nb, 3 * hb + i, 0, op[i][0], op[i][1]);
+                add2<CLEAR>(st, na, nb, 3 * hb + i, 2, op[i][2], oq[i][0]);
+                add2<CLEAR>(st, na, nb, 3 * hb + i, 4, oq[i][1], oq[i][2]);
+            }
+        }
     }
 }
 
 // Phase B work of one lane: the node-pair tensor (before the caller's
 // values are known to be staged) and the block added onto them (after).
-__device__ __forceinline__ void pair_tensor(const KSmem &S, int el, int na, int nb, double H[3][3]) {
-    const KElem &s = S.el[el];
+__device__ __forceinline__ void pair_tensor(const KSmem &S, const KElem &s, int el, int na, int nb, double H[3][3]) {
     if (!(s.flags & KF_VALID)) return;
     if (s.flags & KF_FP64) pair_h<false>(S, el, na, nb, H);
     else pair_h<true>(S, el, na, nb, H);
 }
 
-__device__ __forceinline__ void pair_add(const KSmem &S, int el, int na, int nb, const double H[3][3], double *st) {
-    const KElem &s = S.el[el];
+__device__ __forceinline__ void pair_add(const KSmem &S, const KElem &s, int el, int na, int nb,
+                                         const double H[3][3], double *st) {
     if (!(s.flags & KF_VALID)) return;
     if (s.flags & KF_FP64) {
         const CentreH<false> h0(S, el, na, nb);
-        pair_add_general<false>(s, H, h0, st, na, nb);
+        const bool clear = stage_clear<false>(st, na, nb);
+        if (s.flags & KF_B0) {
+            if (clear) pair_add_general<false, true, true>(s, H, h0, st, na, nb);
+            else pair_add_general<false, true, false>(s, H, h0, st, na, nb);
+        } else {
+            if (clear) pair_add_general<false, false, true>(s, H, h0, st, na, nb);
+            else pair_add_general<false, false, false>(s, H, h0, st, na, nb);
+        }
     } else {
         const CentreH<true> h0(S, el, na, nb);
-        if (s.flags & KF_ISO) pair_add_iso(s, H, h0, st, na, nb);
-        else pair_add_general<true>(s, H, h0, st, na, nb);
+        if (s.flags & KF_SPLIT) {
+            const bool clear = stage_clear<true>(st, na, nb);
+            if (s.flags & KF_ISO) {
+                if (clear) pair_add_iso<true>(s, H, h0, st, na, nb);
+                else pair_add_iso<false>(s, H, h0, st, na, nb);
+            } else {
+                if (clear) pair_add_general<true, true, true>(s, H, h0, st, na, nb);
+                else pair_add_general<true, true, false>(s, H, h0, st, na, nb);
+            }
+        } else {
+            if (stage_clear<false>(st, na, nb)) pair_add_general<true, false, true>(s, H, h0, st, na, nb);
+            else pair_add_general<true, false, false>(s, H, h0, st, na, nb);
+        }
     }
 }
 
-// Phase B of one round for a warp: the elements el0 (lanes 0-15) and el0 + 1
-// (lanes 16-31), one lane per node pair: the caller's current values are
-// prefetched into stage[0..1] with cp.async while the 6x6 blocks are
+// Phase B of one round for a warp: the tile's elements el0 (lanes 0-15) and
+// el0 + 1 (lanes 16-31), one lane per node pair: the caller's current values
+// are prefetched into stage[0..1] with cp.async while the 6x6 blocks are
 // computed, then the blocks are added onto them (ready for the write-out).
-__device__ __forceinline__ void kc0_round(const Q4Args &a, KSmem &S, int el0, double (*stage)[24 * KROW],
-                                          int lane) {
+__device__ __forceinline__ void kc0_round(const Q4Args &a, KSmem &S, const KElem *els, int el0,
+                                          double (*stage)[24 * KROW], int lane) {
     const int half = lane >> 4, pair = lane & 15;
     const int na = pair >> 2, nb = pair & 3;
     const int el = el0 + half;
@@ -475,7 +699,7 @@ __device__ __forceinline__ void kc0_round(const Q4Args &a, KSmem &S, int el0, do
     // prefetch the two elements' current values into the stage
 #pragma unroll
     for (int hh = 0; hh < 2; hh++) {
-        const KElem &t = S.el[el0 + hh];
+        const KElem &t = els[el0 + hh];
         if (!(t.flags & KF_VALID)) continue;
         const double *kv = a.Kv + t.init_k;
         double *sv = stage[hh];
@@ -502,19 +726,18 @@ __device__ __forceinline__ void kc0_round(const Q4Args &a, KSmem &S, int el0, do
     }
     cp_async_commit();
     double H[3][3];
-    pair_tensor(S, el, na, nb, H);
+    pair_tensor(S, els[el], el, na, nb, H);
     // all lanes' prefetches of both staged elements have landed
     cp_async_wait_all();
     __syncwarp();
-    pair_add(S, el, na, nb, H, st);
+    pair_add(S, els[el], el, na, nb, H, st);
     __syncwarp();
 }
 
 // Phase A2 for element slot el at point g: w detJ and the shape functions
 // with their Cartesian derivatives (float-float for flat elements, FP64
 // otherwise).
-__device__ __forceinline__ void kc0_point(KSmem &S, int el, int g) {
-    const KElem &s = S.el[el];
+__device__ __forceinline__ void kc0_point(KSmem &S, const KElem &s, int el, int g) {
     if (!(s.flags & KF_VALID)) return;
     Slot *o = S.gp[el][g];
     if (s.flags & KF_FP64) {
@@ -539,59 +762,67 @@ __device__ __forceinline__ void kc0_tables(KSmem &S, int tid) {
     for (int i = tid; i < KPTS * 12; i += KNT) (&S.shape[0][0][0])[i] = (&c_shape[0][0][0])[i];
 }
 
-#ifndef FE3D_KC0_MINB
-#define FE3D_KC0_MINB 2
-#endif
-__global__ void __launch_bounds__(KNT, FE3D_KC0_MINB) quad4_kc0_ff_kernel(Q4Args a) {
+// Phase A2 of a consumer warp: the points of its per (2 or 4) elements from
+// el0 on, one lane each.
+__device__ __forceinline__ void kc0_points(KSmem &S, const KElem *els, int el0, int per, int lane) {
+    if (lane < per * KPTS) kc0_point(S, els[el0 + lane / KPTS], el0 + lane / KPTS, lane % KPTS);
+    __syncwarp();
+}
+
+// The tiles of a CTA over cnt elements: full tiles of KT, interleaved over the
+// CTAs, then one smaller tile each that shares what is left evenly.
+struct KTiles {
+    int64_t full, rest0, left;
+    __device__ __forceinline__ KTiles(int64_t cnt) {
+        full = cnt / ((int64_t)KT * gridDim.x);
+        rest0 = full * KT * gridDim.x;
+        left = cnt - rest0;
+    }
+    // first element and number of elements of the CTA's t-th tile (0: none)
+    __device__ __forceinline__ int64_t first(int64_t t) const {
+        return t < full ? (t * gridDim.x + blockIdx.x) * KT : rest0 + left * blockIdx.x / gridDim.x;
+    }
+    __device__ __forceinline__ int count(int64_t t) const {
+        if (t < full) return KT;
+        return t > full ? 0 : (int)(left * (blockIdx.x + 1) / gridDim.x - left * blockIdx.x / gridDim.x);
+    }
+};
+
+__global__ void __launch_bounds__(KNT, KMINB) quad4_kc0_ff_kernel(Q4Args a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     KSmem &S = *reinterpret_cast<KSmem *>(smem_raw);
     const int tid = threadIdx.x;
     kc0_tables(S, tid);
-    const int64_t ntiles = (a.E + KT - 1) / KT;
     const int lane = tid & 31, warp = tid >> 5;
-    // warps other than 0 defer the write-out of their last round of a tile
-    // and do it while warp 0 runs phase A of the next tile
-    bool pending = false;
-    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int64_t e0 = tile * KT;
+    const KTiles tiles(a.E);
+    // the last warp runs phase A one tile ahead of the others
+    auto phase_a = [&](int64_t t, int buf) {
+        if (warp != KCW || lane >= KT) return;
+        if (lane < tiles.count(t)) kc0_phase_a2(a, tiles.first(t) + lane, S.el[buf][lane]);
+        else S.el[buf][lane].flags = 0;
+    };
+    phase_a(0, 0);
+    int buf = 0, n;
+    for (int64_t t = 0; (n = tiles.count(t)) > 0; t++, buf ^= 1) {
         __syncthreads();
-        if (tid < KT) {
-            const int64_t e = e0 + tid;
-            if (e < a.E) kc0_phase_a2(a, e, S.el[tid]);
-            else S.el[tid].flags = 0;
-        } else if (pending) {
-            flush_deferred(a, S.stage[warp], lane);
-            pending = false;
+        if (warp == KCW) {
+            phase_a(t + 1, buf ^ 1);
+            continue;
         }
-        __syncthreads();
-        // phase A2: integration points
-        for (int it = tid; it < KT * KPTS; it += KNT) {
-            const int el = it / KPTS, g = it - el * KPTS;
-            kc0_point(S, el, g);
-        }
-        __syncthreads();
-        // phase B: each warp owns 2 elements per round, one lane per node
-        // pair; blocks are staged and then streamed out coalesced
-        for (int round = 0; round < KT / KRND; round++) {
-            kc0_round(a, S, round * KRND + warp * 2, S.stage[warp], lane);
-            const bool defer = round == KT / KRND - 1 && warp != 0;
+        const int per = n > 2 * KCW ? 4 : 2, first = warp * per;
+        if (first >= n) continue;
+        const KElem *els = S.el[buf];
+        kc0_points(S, els, first, per, lane);
+        for (int el0 = first; el0 < first + per && el0 < n; el0 += 2) {
+            kc0_round(a, S, els, el0, S.stage[warp], lane);
 #pragma unroll
             for (int hh = 0; hh < 2; hh++) {
-                const KElem &t = S.el[round * KRND + warp * 2 + hh];
-                if (defer) {
-                    double *sv = S.stage[warp][hh];
-                    if (lane < 6) *stage_meta(sv, lane) = lane == 0 ? (long long)t.flags
-                                                          : lane == 1 ? t.init_k : t.c[lane - 2];
-                    continue;
-                }
-                if (!(t.flags & KF_VALID)) continue;
-                write_staged(a, S.stage[warp][hh], t.init_k, t.c, lane);
+                const KElem &e = els[el0 + hh];
+                if (e.flags & KF_VALID) write_staged(a, S.stage[warp][hh], e.init_k, e.c, lane);
             }
-            pending = defer;
             __syncwarp();
         }
     }
-    if (pending) flush_deferred(a, S.stage[warp], lane);
 }
 
 
@@ -628,13 +859,13 @@ struct __align__(8) CsrElem {
 
 struct KSmemCsr {
     KSmem s;
-    CsrElem cm[KT];
+    CsrElem cm[2][KT];
 };
 
-// FE3D_KC0_MINB CTAs per SM must fit the SM's 228 KB of shared memory
-// (1 KB of it reserved per CTA)
-static_assert(FE3D_KC0_MINB * (sizeof(KSmem) + 1024) <= 228 * 1024, "triplet kernel: shared memory per SM");
-static_assert(FE3D_KC0_MINB * (sizeof(KSmemCsr) + 1024) <= 228 * 1024, "CSR kernel: shared memory per SM");
+// KMINB CTAs per SM must fit the SM's 228 KB of shared memory (1 KB of it
+// reserved per CTA)
+static_assert(KMINB * (sizeof(KSmem) + 1024) <= 228 * 1024, "triplet kernel: shared memory per SM");
+static_assert(KMINB * (sizeof(KSmemCsr) + 1024) <= 228 * 1024, "CSR kernel: shared memory per SM");
 
 // A staged element's scatter data in the stage's padding columns (24, 25):
 // slots 0-23 the CSR position of each row's first entry (-1: fixed DOF),
@@ -708,7 +939,8 @@ __device__ __forceinline__ void csr_meta_build(const KElem &t, const CsrElem &q,
 }
 
 // The slots of a staged element that move: free row and column, and not an
-// exact isotropic zero of a block that is added (assigned blocks store all).
+// exact zero between (u, v, rz) and (w, rx, ry) of a block that is added
+// (assigned blocks store all).
 // Lane l < 24 takes column l of the element for all 24 rows, so the column's
 // rank, its block offsets and assign bits are hoisted out of the row loop;
 // every row is one warp-wide access of its 4 runs of 6 entries.
@@ -722,8 +954,8 @@ __device__ __forceinline__ void csr_slots(const double *sv, int lane, F &&f) {
     if (cr < 0) return;  // fixed column
     const unsigned first = (unsigned)((unsigned long long)fl >> 32);
     const int b = lane / 6, n = lane - 6 * b;
-    const bool iso = flags & KF_ISO;
-    const bool z_mid = iso && n < 2, z_out = iso && (n == 2 || n == 3);
+    const bool split = flags & KF_SPLIT;
+    const bool z_mid = split && (n < 2 || n == 5), z_out = split && n >= 2 && n <= 4;
     long long colpart[4];
     bool asg[4];
 #pragma unroll
@@ -763,70 +995,64 @@ __device__ __forceinline__ void csr_write(const CsrArgs &m, const double *sv, in
     });
 }
 
-__device__ __forceinline__ void kc0_round_csr(const Q4Args &a, const CsrArgs &m, KSmem &S, const CsrElem *cm,
-                                              int el0, double (*stage)[24 * KROW], int lane) {
+__device__ __forceinline__ void kc0_round_csr(const Q4Args &a, const CsrArgs &m, KSmem &S, const KElem *els,
+                                              const CsrElem *cm, int el0, double (*stage)[24 * KROW], int lane) {
     const int half = lane >> 4, pair = lane & 15;
     const int na = pair >> 2, nb = pair & 3;
     const int el = el0 + half;
     double *st = stage[half];
 #pragma unroll
-    for (int hh = 0; hh < 2; hh++) csr_meta_build(S.el[el0 + hh], cm[el0 + hh], stage[hh], lane);
+    for (int hh = 0; hh < 2; hh++) csr_meta_build(els[el0 + hh], cm[el0 + hh], stage[hh], lane);
     __syncwarp();
 #pragma unroll
     for (int hh = 0; hh < 2; hh++) csr_prefetch(m, stage[hh], lane, a.err);
     cp_async_commit();
     double H[3][3];
-    pair_tensor(S, el, na, nb, H);
+    pair_tensor(S, els[el], el, na, nb, H);
     cp_async_wait_all();
     __syncwarp();
-    pair_add(S, el, na, nb, H, st);
+    pair_add(S, els[el], el, na, nb, H, st);
     __syncwarp();
 }
 
-__global__ void __launch_bounds__(KNT, FE3D_KC0_MINB) quad4_kc0_csr_kernel(Q4Args a, CsrArgs m) {
+__global__ void __launch_bounds__(KNT, KMINB) quad4_kc0_csr_kernel(Q4Args a, CsrArgs m) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     KSmemCsr &SC = *reinterpret_cast<KSmemCsr *>(smem_raw);
     KSmem &S = SC.s;
     const int tid = threadIdx.x;
     kc0_tables(S, tid);
-    const int64_t ntiles = (m.cnt + KT - 1) / KT;
     const int lane = tid & 31, warp = tid >> 5;
-    bool pending = false;
-    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int64_t t0 = tile * KT;
+    const KTiles tiles(m.cnt);
+    auto phase_a = [&](int64_t t, int buf) {
+        if (warp != KCW || lane >= KT) return;
+        if (lane < tiles.count(t)) kc0_phase_a_csr(a, m, tiles.first(t) + lane, S.el[buf][lane], SC.cm[buf][lane]);
+        else S.el[buf][lane].flags = 0;
+    };
+    phase_a(0, 0);
+    int buf = 0, n;
+    for (int64_t t = 0; (n = tiles.count(t)) > 0; t++, buf ^= 1) {
         __syncthreads();
-        if (tid < KT) {
-            const int64_t t = t0 + tid;
-            if (t < m.cnt) kc0_phase_a_csr(a, m, t, S.el[tid], SC.cm[tid]);
-            else S.el[tid].flags = 0;
-        } else if (pending) {
+        if (warp == KCW) {
+            phase_a(t + 1, buf ^ 1);
+            continue;
+        }
+        const int per = n > 2 * KCW ? 4 : 2, first = warp * per;
+        if (first >= n) continue;
+        const KElem *els = S.el[buf];
+        kc0_points(S, els, first, per, lane);
+        for (int el0 = first; el0 < first + per && el0 < n; el0 += 2) {
+            kc0_round_csr(a, m, S, els, SC.cm[buf], el0, S.stage[warp], lane);
 #pragma unroll
             for (int hh = 0; hh < 2; hh++) csr_write(m, S.stage[warp][hh], lane);
             __syncwarp();
-            pending = false;
-        }
-        __syncthreads();
-        for (int it = tid; it < KT * KPTS; it += KNT) {
-            const int el = it / KPTS, g = it - el * KPTS;
-            kc0_point(S, el, g);
-        }
-        __syncthreads();
-        for (int round = 0; round < KT / KRND; round++) {
-            kc0_round_csr(a, m, S, SC.cm, round * KRND + warp * 2, S.stage[warp], lane);
-            // warps other than 0 write their last round while warp 0 runs the next phase A
-            const bool defer = round == KT / KRND - 1 && warp != 0;
-            if (!defer) {
-#pragma unroll
-                for (int hh = 0; hh < 2; hh++) csr_write(m, S.stage[warp][hh], lane);
-            }
-            pending = defer;
-            __syncwarp();
         }
     }
-    if (pending) {
-#pragma unroll
-        for (int hh = 0; hh < 2; hh++) csr_write(m, S.stage[warp][hh], lane);
-    }
+}
+
+// One wave of CTAs; small meshes spread over the SMs (4 elements a CTA).
+int kc0_grid(int64_t E) {
+    const int64_t g = (E + 3) / 4, cap = (int64_t)kSMs * KMINB;
+    return (int)(g < cap ? g : cap);
 }
 
 int g_shape_ready[64] = {0};
@@ -890,10 +1116,7 @@ extern "C" int fe3d_quad4_kc0(int64_t E, const int64_t *cdof, const int64_t *ini
     // arrays are 16-byte aligned
     const auto al16 = [](const void *q) { return ((uintptr_t)q & 15u) == 0; };
     a.vec16 = al16(Kv) && (values_only || (al16(Kr) && al16(Kc)));
-    const int64_t tiles = (E + KT - 1) / KT;
-    const int64_t cap = (int64_t)kSMs * FE3D_KC0_MINB;
-    const int grid = (int)(tiles < cap ? tiles : cap);
-    quad4_kc0_ff_kernel<<<grid, KNT, sizeof(KSmem), as_stream(stream)>>>(a);
+    quad4_kc0_ff_kernel<<<kc0_grid(E), KNT, sizeof(KSmem), as_stream(stream)>>>(a);
     FE3D_CHECK_LAUNCH();
     return FE3D_OK;
 }
@@ -915,13 +1138,10 @@ extern "C" int fe3d_quad4_kc0_csr(const fe3d_fmap *fm, int g, const double *x, i
     Q4Args a{G.E, nullptr, nullptr, x, nx, xmat, xmat_stride, nullptr, nullptr, nullptr, nullptr, props, nprops, pid,
              nullptr, nullptr, nullptr, 0, 1, err};
     a.vec16 = 0;
-    const int64_t cap = (int64_t)kSMs * FE3D_KC0_MINB;
     if (mode == FE3D_CSR_ATOMIC) {
         CsrArgs m{nullptr, G.E, G.node, G.boff, G.first, fm->pat->noderow, fm->pat->nnodes,
                   vals, fm->pat->nnz, 0, 1};
-        const int64_t tiles = (G.E + KT - 1) / KT;
-        const int grid = (int)(tiles < cap ? tiles : cap);
-        quad4_kc0_csr_kernel<<<grid, KNT, sizeof(KSmemCsr), as_stream(stream)>>>(a, m);
+        quad4_kc0_csr_kernel<<<kc0_grid(G.E), KNT, sizeof(KSmemCsr), as_stream(stream)>>>(a, m);
         FE3D_CHECK_LAUNCH();
         return FE3D_OK;
     }
@@ -930,9 +1150,7 @@ extern "C" int fe3d_quad4_kc0_csr(const fe3d_fmap *fm, int g, const double *x, i
         if (cnt == 0) continue;
         CsrArgs m{G.order + G.cstart[c], cnt, G.node, G.boff, G.first, fm->pat->noderow, fm->pat->nnodes,
                   vals, fm->pat->nnz, mode == FE3D_CSR_ASSIGN, 0};
-        const int64_t tiles = (cnt + KT - 1) / KT;
-        const int grid = (int)(tiles < cap ? tiles : cap);
-        quad4_kc0_csr_kernel<<<grid, KNT, sizeof(KSmemCsr), as_stream(stream)>>>(a, m);
+        quad4_kc0_csr_kernel<<<kc0_grid(cnt), KNT, sizeof(KSmemCsr), as_stream(stream)>>>(a, m);
         FE3D_CHECK_LAUNCH();
     }
     return FE3D_OK;
