@@ -11,7 +11,12 @@
 // sorted slot permutation `perm` and the segment starts `seg`.
 // Numeric assembly (every update): vals[s] = sum of Kv[perm[t]] over the
 // segment t in [seg[s], seg[s+1]), summed in ascending slot order, so the
-// result is deterministic.
+// result is deterministic.  The six (free) columns of a node in a row of the
+// matrix come from six consecutive slots of every element that has both nodes,
+// so the segments of neighbouring entries are the same slots shifted by one:
+// the pattern describes such a run by one 32-byte record, and the numeric
+// assembly reads 5 instead of 11 bytes of indices per entry and two slots per
+// load.
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
@@ -112,7 +117,138 @@ __global__ void widen_kernel(int64_t n, const int32_t *a, int64_t *b) {
     if (i < n) b[i] = a[i];
 }
 
-// Numeric assembly: one thread per CSR entry (segment).
+// ---- runs of entries ----------------------------------------------------
+// A run is entries s, s + 1, .. of one row and one node's columns whose
+// segments are as long and whose slots are each one further.  Record: {first
+// entry, length | slots per entry << 8, 0, first place in perm}, {its first
+// four slots}.
+constexpr int RUN_SLOTS = 4;
+
+// flag[s] = 1 where entry s does not continue the run of entry s - 1 (rows:
+// run_rows_kernel).
+__global__ void run_flags_kernel(int64_t nnz, const int32_t *seg, const int32_t *perm, const int32_t *colind,
+                                 const int64_t *dof_of_row, int32_t *flag) {
+    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (s >= nnz) return;
+    bool head = s == 0;
+    if (!head) {
+        const int32_t b = seg[s], e = seg[s + 1], a = seg[s - 1];
+        head = e - b != b - a || colind[s] != colind[s - 1] + 1 || dof_of_row[colind[s]] % 6 == 0;
+        for (int32_t t = 0; !head && t < e - b; t++) head = perm[b + t] != perm[a + t] + 1;
+    }
+    flag[s] = head;
+}
+
+__global__ void run_rows_kernel(int64_t nrows, const int64_t *rowptr, int64_t nnz, int32_t *flag) {
+    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (r < nrows && rowptr[r] < nnz) flag[rowptr[r]] = 1;
+}
+
+__global__ void run_fill_kernel(int64_t nnz, const int32_t *flag, const int32_t *scan, const int32_t *seg,
+                                const int32_t *perm, int4 *runs) {
+    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (s >= nnz || !flag[s]) return;
+    const int32_t b = seg[s], k = seg[s + 1] - b;
+    int32_t q[RUN_SLOTS];
+    for (int t = 0; t < RUN_SLOTS; t++) q[t] = t < k ? perm[b + t] : 0;
+    runs[2 * (int64_t)scan[s]] = make_int4((int)s, k << 8, 0, b);
+    runs[2 * (int64_t)scan[s] + 1] = make_int4(q[0], q[1], q[2], q[3]);
+}
+
+__global__ void run_lengths_kernel(int64_t nruns, int64_t nnz, int4 *runs) {
+    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (r >= nruns) return;
+    const int next = r + 1 < nruns ? runs[2 * (r + 1)].x : (int)nnz;
+    runs[2 * r].y |= next - runs[2 * r].x;
+}
+
+// Sorts every RUN_CHUNK runs by their slots per entry (4 and more, 3, 2, 1;
+// stable).  An FP64 addition takes a sub-partition's pipe for 64 cycles
+// whatever its active lanes, and with the runs of a row side by side (1 2 1 2 4
+// 2 1 2 1 slots in a plate) every warp made the additions of the longest.
+constexpr int RUN_CHUNK = 256;
+__global__ void __launch_bounds__(RUN_CHUNK) run_sort_kernel(int64_t nruns, int4 *runs) {
+    __shared__ int cnt[4][RUN_CHUNK / 32];
+    const int64_t r = blockIdx.x * (int64_t)RUN_CHUNK + threadIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool in = r < nruns;
+    int4 h = make_int4(0, 0, 0, 0), q = h;
+    if (in) {
+        h = runs[2 * r];
+        q = runs[2 * r + 1];
+    }
+    const int k = h.y >> 8, cls = !in ? -1 : k >= 4 ? 0 : 4 - k;
+    int below = 0;
+    for (int c = 0; c < 4; c++) {
+        const unsigned m = __ballot_sync(0xffffffffu, cls == c);
+        if (lane == 0) cnt[c][warp] = __popc(m);
+        if (cls == c) below = __popc(m & ((1u << lane) - 1u));
+    }
+    __syncthreads();
+    if (!in) return;
+    int at = below;
+    for (int c = 0; c <= cls; c++)
+        for (int w = 0; w < RUN_CHUNK / 32; w++)
+            if (c < cls || w < warp) at += cnt[c][w];
+    const int64_t o = blockIdx.x * (int64_t)RUN_CHUNK + at;
+    runs[2 * o] = h;
+    runs[2 * o + 1] = q;
+}
+
+__device__ __forceinline__ double2 run_load(const double *a, bool two, bool wide) {
+    if (wide) return __ldg(reinterpret_cast<const double2 *>(a));
+    return make_double2(__ldg(a), two ? __ldg(a + 1) : 0.);
+}
+
+// Numeric assembly over runs: three lanes a run, two entries a lane; 8 bytes
+// per slot and per entry and 32 per run.  301x301-node plate (51.8 M slots, 29 M
+// entries): 0.354 ms by entries, 0.234 ms with the runs unsorted (78 % of the
+// FP64 pipe), 0.144 ms sorted (5.6 TB/s, 0.82 of the measured copy rate).
+__global__ void __launch_bounds__(256) assemble_runs_kernel(int64_t nruns, const int4 *__restrict__ runs,
+                                                            const int32_t *__restrict__ perm,
+                                                            const double *__restrict__ Kv, double *__restrict__ vals,
+                                                            int vec16) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, r = t / 3;
+    const int j = 2 * (int)(t - 3 * r);
+    int4 h = make_int4(0, 0, 0, 0), q = h;
+    if (r < nruns) {
+        h = __ldg(runs + 2 * r);
+        q = __ldg(runs + 2 * r + 1);
+    }
+    const int len = h.y & 0xff, k = h.y >> 8;
+    const bool in = j < len, two = j + 1 < len;
+    // one path per warp, its loads in flight together
+    const int most = __reduce_max_sync(0xffffffffu, in ? k : 0);
+    const bool wide = two && vec16;
+    double2 s = make_double2(0., 0.);
+    if (most == 0) return;
+    if (most == 1) {
+        if (in) s = run_load(Kv + q.x + j, two, wide && !(q.x & 1));
+    } else if (most == 2) {
+        double2 v = s;
+        if (in) s = run_load(Kv + q.x + j, two, wide && !(q.x & 1));
+        if (in && k > 1) v = run_load(Kv + q.y + j, two, wide && !(q.y & 1));
+        s.x += v.x;
+        s.y += v.y;
+    } else if (most <= RUN_SLOTS) {
+        double2 v1 = s, v2 = s, v3 = s;
+        if (in) s = run_load(Kv + q.x + j, two, wide && !(q.x & 1));
+        if (in && k > 1) v1 = run_load(Kv + q.y + j, two, wide && !(q.y & 1));
+        if (in && k > 2) v2 = run_load(Kv + q.z + j, two, wide && !(q.z & 1));
+        if (in && k > 3) v3 = run_load(Kv + q.w + j, two, wide && !(q.w & 1));
+        s.x = ((s.x + v1.x) + v2.x) + v3.x;
+        s.y = ((s.y + v1.y) + v2.y) + v3.y;
+    } else if (in) {
+        for (int i = 0; i < k; i++) {
+            s.x += __ldg(Kv + __ldg(perm + h.w + j * k + i));
+            if (two) s.y += __ldg(Kv + __ldg(perm + h.w + (j + 1) * k + i));
+        }
+    }
+    if (in) vals[h.x + j] = s.x;
+    if (two) vals[h.x + j + 1] = s.y;
+}
+
+// Numeric assembly without runs: one thread per CSR entry (segment).
 __global__ void __launch_bounds__(256) assemble_kernel(int64_t nseg, const int32_t *__restrict__ seg,
                                                        const int32_t *__restrict__ perm,
                                                        const double *__restrict__ Kv,
@@ -256,6 +392,32 @@ extern "C" int fe3d_pattern_build(const int64_t *Kr, const int64_t *Kc, int64_t 
     }
     TRYC(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, rc64, rscan, (int)(p->nrows + 1), st));
     rowptr_kernel<<<nblk(p->nrows + 1), 256, 0, st>>>(p->nrows, rscan, p->rowptr, p->nnz);
+    if (p->nnz > 0) {
+        // runs of entries (head and hscan are free again)
+        run_flags_kernel<<<nblk(p->nnz), 256, 0, st>>>(p->nnz, p->seg, p->perm, p->colind, p->dof_of_row, head);
+        run_rows_kernel<<<nblk(p->nrows), 256, 0, st>>>(p->nrows, p->rowptr, p->nnz, head);
+        TRYC(cub::DeviceScan::ExclusiveSum(nullptr, need, head, hscan, (int)p->nnz, st));
+        if (need > tmp_bytes) {
+            cudaFree(tmp);
+            tmp = nullptr;
+            tmp_bytes = need;
+            TRYC(cudaMalloc(&tmp, tmp_bytes));
+        }
+        TRYC(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, head, hscan, (int)p->nnz, st));
+        TRYC(cudaMemcpyAsync(&last_head, head + p->nnz - 1, 4, cudaMemcpyDeviceToHost, st));
+        TRYC(cudaMemcpyAsync(&last_hscan, hscan + p->nnz - 1, 4, cudaMemcpyDeviceToHost, st));
+        TRYC(cudaStreamSynchronize(st));
+        p->nruns = last_head + last_hscan;
+        // shorter than two entries on average: the records would be the larger part
+        if (2 * p->nruns <= p->nnz && dalloc(&p->runs, 2 * (size_t)p->nruns) == 0) {
+            run_fill_kernel<<<nblk(p->nnz), 256, 0, st>>>(p->nnz, head, hscan, p->seg, p->perm, p->runs);
+            run_lengths_kernel<<<nblk(p->nruns), 256, 0, st>>>(p->nruns, p->nnz, p->runs);
+            run_sort_kernel<<<nblk(p->nruns, RUN_CHUNK), RUN_CHUNK, 0, st>>>(p->nruns, p->runs);
+        } else {
+            (void)cudaGetLastError();
+            p->nruns = 0;
+        }
+    }
     if (p->nrows > 0 && p->nnz > 0) {
         // compressed columns for the SpMV (2 bytes per entry instead of 4)
         TRY(dalloc(&p->colbase, p->nrows));
@@ -296,6 +458,7 @@ extern "C" int fe3d_pattern_free(fe3d_pattern *p) {
     cudaFree(p->dof_of_row);
     cudaFree(p->perm);
     cudaFree(p->seg);
+    cudaFree(p->runs);
     cudaFree(p->colind);
     cudaFree(p->rowptr);
     cudaFree(p->colbase);
@@ -347,6 +510,12 @@ extern "C" int fe3d_assemble(const fe3d_pattern *p, const double *Kv, double *va
     if (!p || (p->nnz > 0 && (!Kv || !vals))) return FE3D_ERR_ARG;
     if (p->nnz > 0 && !p->perm) return FE3D_ERR_STATE;  // pattern built from elements: no COO slots
     if (p->nnz == 0) return FE3D_OK;
+    if (p->nruns) {
+        assemble_runs_kernel<<<nblk(3 * p->nruns), 256, 0, as_stream(stream)>>>(p->nruns, p->runs, p->perm, Kv, vals,
+                                                                               ((uintptr_t)Kv & 15u) == 0);
+        FE3D_CHECK_LAUNCH();
+        return FE3D_OK;
+    }
     const int64_t blocks = (p->nnz + 255) / 256;
     const unsigned grid = (unsigned)(blocks < kSMs * 16 ? blocks : kSMs * 16);
     assemble_kernel<<<grid, 256, 0, as_stream(stream)>>>(p->nnz, p->seg, p->perm, Kv, vals);

@@ -22,6 +22,8 @@ struct fe3d_pattern {
     int64_t *dof_of_row = nullptr;  // [nrows] full DOF of a reduced row
     int32_t *perm = nullptr;        // [nnz_in] COO slots sorted by (row, col)
     int32_t *seg = nullptr;         // [nnz + 1] segment starts in perm
+    int4 *runs = nullptr;           // [2 nruns] runs of entries summed alike (assembly.cu), or NULL
+    int64_t nruns = 0;
     int32_t *colind = nullptr;      // [nnz]
     int64_t *rowptr = nullptr;      // [nrows + 1]
     // compressed columns for the solver's SpMV when every row spans fewer than
