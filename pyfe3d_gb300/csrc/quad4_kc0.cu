@@ -57,8 +57,8 @@ constexpr int KPTS = 5;   // 4 Gauss points + centre
 constexpr int KSLOT = 9;  // per point: w detJ, Nx[4], Ny[4] (N is the same for every element)
 
 // KF_SPLIT: (u, v, rz) and (w, rx, ry) do not couple (evaluated in the global
-// frame with B = 0); KF_B0: B = 0
-enum : int { KF_VALID = 1, KF_THICK = 2, KF_FP64 = 4, KF_ISO = 8, KF_B0 = 16, KF_SPLIT = 32 };
+// frame with B = 0); KF_B0: B = 0; KF_FREE (CSR): no fixed DOF
+enum : int { KF_VALID = 1, KF_THICK = 2, KF_FP64 = 4, KF_ISO = 8, KF_B0 = 16, KF_SPLIT = 32, KF_FREE = 64 };
 
 union Slot {
     double d;
@@ -655,12 +655,12 @@ __device__ __forceinline__ void pair_tensor(const KSmem &S, const KElem &s, int 
     else pair_h<true>(S, el, na, nb, H);
 }
 
+// clear: the staged entries that the block adds to are zeros (every lane's).
 __device__ __forceinline__ void pair_add(const KSmem &S, const KElem &s, int el, int na, int nb,
-                                         const double H[3][3], double *st) {
+                                         const double H[3][3], double *st, bool clear) {
     if (!(s.flags & KF_VALID)) return;
     if (s.flags & KF_FP64) {
         const CentreH<false> h0(S, el, na, nb);
-        const bool clear = stage_clear<false>(st, na, nb);
         if (s.flags & KF_B0) {
             if (clear) pair_add_general<false, true, true>(s, H, h0, st, na, nb);
             else pair_add_general<false, true, false>(s, H, h0, st, na, nb);
@@ -670,17 +670,14 @@ __device__ __forceinline__ void pair_add(const KSmem &S, const KElem &s, int el,
         }
     } else {
         const CentreH<true> h0(S, el, na, nb);
-        if (s.flags & KF_SPLIT) {
-            const bool clear = stage_clear<true>(st, na, nb);
-            if (s.flags & KF_ISO) {
-                if (clear) pair_add_iso<true>(s, H, h0, st, na, nb);
-                else pair_add_iso<false>(s, H, h0, st, na, nb);
-            } else {
-                if (clear) pair_add_general<true, true, true>(s, H, h0, st, na, nb);
-                else pair_add_general<true, true, false>(s, H, h0, st, na, nb);
-            }
+        if (s.flags & KF_ISO) {
+            if (clear) pair_add_iso<true>(s, H, h0, st, na, nb);
+            else pair_add_iso<false>(s, H, h0, st, na, nb);
+        } else if (s.flags & KF_B0) {
+            if (clear) pair_add_general<true, true, true>(s, H, h0, st, na, nb);
+            else pair_add_general<true, true, false>(s, H, h0, st, na, nb);
         } else {
-            if (stage_clear<false>(st, na, nb)) pair_add_general<true, false, true>(s, H, h0, st, na, nb);
+            if (clear) pair_add_general<true, false, true>(s, H, h0, st, na, nb);
             else pair_add_general<true, false, false>(s, H, h0, st, na, nb);
         }
     }
@@ -730,7 +727,9 @@ __device__ __forceinline__ void kc0_round(const Q4Args &a, KSmem &S, const KElem
     // all lanes' prefetches of both staged elements have landed
     cp_async_wait_all();
     __syncwarp();
-    pair_add(S, els[el], el, na, nb, H, st);
+    const KElem &s = els[el];
+    const bool clear = (s.flags & KF_SPLIT) ? stage_clear<true>(st, na, nb) : stage_clear<false>(st, na, nb);
+    pair_add(S, s, el, na, nb, H, st, clear);
     __syncwarp();
 }
 
@@ -832,7 +831,13 @@ __global__ void __launch_bounds__(KNT, KMINB) quad4_kc0_ff_kernel(Q4Args a) {
 // per element colour (no two elements of a colour share a node), so the
 // read-add-write of the CSR entries needs no atomics and sums every entry
 // in a fixed order.  The node-pair blocks an element assigns (it is their
-// first contributor) are stored without reading.
+// first contributor) are stored without reading, and where a warp's blocks are
+// all assigned nothing is added.
+//
+// Bound by latency and instructions (1,261 per element on interior isotropic
+// elements, 2,123 with a test, a position and a bounds check per row and
+// entry), then by the colours' passes over the values (3 TB/s).  90,000
+// elements in 4 colours 0.50 -> 0.33 ms.
 
 struct CsrArgs {
     const int32_t *order;  // the colour's elements
@@ -866,23 +871,6 @@ struct KSmemCsr {
 // reserved per CTA)
 static_assert(KMINB * (sizeof(KSmem) + 1024) <= 228 * 1024, "triplet kernel: shared memory per SM");
 static_assert(KMINB * (sizeof(KSmemCsr) + 1024) <= 228 * 1024, "CSR kernel: shared memory per SM");
-
-// A staged element's scatter data in the stage's padding columns (24, 25):
-// slots 0-23 the CSR position of each row's first entry (-1: fixed DOF),
-// 24-27 the 16 block offsets (int16), 28-30 the rank of each column within
-// its node (int8, -1: fixed DOF), 31 flags | assign bits << 32.
-__device__ __forceinline__ long long *csr_meta(double *sv, int i) {
-    return reinterpret_cast<long long *>(sv + (i >> 1) * KROW + 24 + (i & 1));
-}
-__device__ __forceinline__ const long long *csr_meta(const double *sv, int i) {
-    return reinterpret_cast<const long long *>(sv + (i >> 1) * KROW + 24 + (i & 1));
-}
-__device__ __forceinline__ int csr_boff(const double *sv, int k) {
-    return reinterpret_cast<const short *>(csr_meta(sv, 24 + (k >> 2)))[k & 3];
-}
-__device__ __forceinline__ int csr_colrank(const double *sv, int col) {
-    return reinterpret_cast<const signed char *>(csr_meta(sv, 28 + (col >> 3)))[col & 7];
-}
 
 __device__ void kc0_phase_a_csr(const Q4Args &a, const CsrArgs &m, int64_t t, KElem &s, CsrElem &q) {
     s.flags = 0;
@@ -919,80 +907,97 @@ __device__ void kc0_phase_a_csr(const Q4Args &a, const CsrArgs &m, int64_t t, KE
     }
     q.first = m.assign ? m.first[e] : 0u;
     s.init_k = 0;
-    kc0_elem_setup(a, e, c, true, s);
-}
-
-__device__ __forceinline__ void csr_meta_build(const KElem &t, const CsrElem &q, double *sv, int lane) {
-    if (lane < 24) {
-        const int a = lane / 6, m = lane - 6 * a;
-        const int Lf = q.Lf[a], fm = Lf >> 16, L = Lf & 0xffff;
-        const bool fr = (fm >> m) & 1;
-        const int rank = __popc(fm & ((1 << m) - 1));
-        *csr_meta(sv, lane) = fr ? t.c[a] + (long long)rank * L : -1LL;
-        reinterpret_cast<signed char *>(csr_meta(sv, 28 + (lane >> 3)))[lane & 7] =
-            fr ? (signed char)rank : (signed char)-1;
-    } else if (lane < 28) {
-        *csr_meta(sv, lane) = reinterpret_cast<const long long *>(q.boff)[lane - 24];
-    } else if (lane == 28) {
-        *csr_meta(sv, 31) = (long long)(unsigned)t.flags | ((long long)q.first << 32);
+    // every row and column of the element inside the values
+    bool all = true;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int fm = q.Lf[i] >> 16, L = q.Lf[i] & 0xffff;
+        all &= fm == 63;
+        if (fm) ok &= s.c[i] >= 0 && s.c[i] + (long long)__popc(fm) * L <= m.nnz;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (fm) ok &= q.boff[4 * i + j] >= 0 && q.boff[4 * i + j] + __popc(q.Lf[j] >> 16) <= L;
     }
+    kc0_elem_setup(a, e, c, ok, s);
+    if (all && (s.flags & KF_VALID)) s.flags |= KF_FREE;
 }
 
-// The slots of a staged element that move: free row and column, and not an
-// exact zero between (u, v, rz) and (w, rx, ry) of a block that is added
-// (assigned blocks store all).
-// Lane l < 24 takes column l of the element for all 24 rows, so the column's
-// rank, its block offsets and assign bits are hoisted out of the row loop;
-// every row is one warp-wide access of its 4 runs of 6 entries.
-template <class F>
-__device__ __forceinline__ void csr_slots(const double *sv, int lane, F &&f) {
-    if (lane >= 24) return;
-    const long long fl = *csr_meta(sv, 31);
-    const int flags = (int)(fl & 0xffffffffLL);
-    if (!(flags & KF_VALID)) return;
-    const int cr = csr_colrank(sv, lane);
-    if (cr < 0) return;  // fixed column
-    const unsigned first = (unsigned)((unsigned long long)fl >> 32);
+// The entries of a staged element that move: lane l < 24 takes column l (column
+// n of node b) for the free rows of the four nodes, f(stage index, address)
+// each, in warp-wide accesses of a node's runs of columns.  The rows of a node
+// are L entries apart, so a lane forms one address per node.  Elements that do
+// not couple (u, v, rz) and (w, rx, ry) move a lane's three rows of its own
+// group; the other three are exact zeros, which only assigned blocks store:
+// z(address).  skip(assigned) leaves a node's rows out.
+template <class S, class F, class Z>
+__device__ __forceinline__ void csr_entries(const CsrArgs &m, const KElem &t, const CsrElem &q, int lane, S &&skip,
+                                            F &&f, Z &&z) {
     const int b = lane / 6, n = lane - 6 * b;
-    const bool split = flags & KF_SPLIT;
-    const bool z_mid = split && (n < 2 || n == 5), z_out = split && n >= 2 && n <= 4;
-    long long colpart[4];
-    bool asg[4];
+    if (lane >= 24 || !(t.flags & KF_VALID)) return;
+    const bool mid = n >= 2 && n <= 4;
+    if ((t.flags & (KF_SPLIT | KF_FREE)) == (KF_SPLIT | KF_FREE)) {
+        // the three rows of the lane's group and of the other one
+        const int i0 = mid ? 2 : 0, i2 = mid ? 4 : 5, o0 = mid ? 0 : 2, o2 = mid ? 5 : 4;
 #pragma unroll
+        for (int a = 0; a < 4; a++) {
+            const bool asg = (q.first >> (4 * a + b)) & 1;
+            if (skip(asg)) continue;
+            const int L = q.Lf[a] & 0xffff, si = 6 * a * KROW + lane;
+            double *p = m.vals + (t.c[a] + q.boff[4 * a + b] + n);
+            double *p0 = p + i0 * L;
+            f(si + i0 * KROW, p0);
+            f(si + (i0 + 1) * KROW, p0 + L);
+            f(si + i2 * KROW, p + i2 * L);
+            if (asg) {
+                double *z0 = p + o0 * L;
+                z(z0);
+                z(z0 + L);
+                z(p + o2 * L);
+            }
+        }
+        return;
+    }
+    const int fb = q.Lf[b] >> 16;
+    if (!((fb >> n) & 1)) return;  // fixed column
+    const int rank = __popc(fb & ((1 << n) - 1));
+    const bool split = t.flags & KF_SPLIT;
+#pragma unroll 1
     for (int a = 0; a < 4; a++) {
-        colpart[a] = csr_boff(sv, 4 * a + b) + cr;
-        asg[a] = (first >> (4 * a + b)) & 1;
-    }
+        const bool asg = (q.first >> (4 * a + b)) & 1;
+        const int Lf = q.Lf[a], fm = Lf >> 16, L = Lf & 0xffff;
+        if (skip(asg) || !fm) continue;
+        double *p = m.vals + (t.c[a] + q.boff[4 * a + b] + rank);
 #pragma unroll
-    for (int row = 0; row < 24; row++) {
-        const int a = row / 6, m = row - 6 * (row / 6);
-        const long long rb = *csr_meta(sv, row);
-        if (rb < 0) continue;
-        const bool zero = (m >= 2 && m <= 4) ? z_mid : z_out;
-        if (!asg[a] && zero) continue;
-        f(row * KROW + lane, rb + colpart[a], asg[a]);
+        for (int i = 0; i < 6; i++) {
+            if (!((fm >> i) & 1)) continue;
+            if (split && (i >= 2 && i <= 4) != mid) {
+                if (asg) z(p);
+            } else {
+                f((6 * a + i) * KROW + lane, p);
+            }
+            p += L;
+        }
     }
 }
 
-__device__ __forceinline__ void csr_prefetch(const CsrArgs &m, double *sv, int lane, int *err) {
-    csr_slots(sv, lane, [&](int si, long long pos, bool asg) {
-        if (asg || m.atomic) {
-            sv[si] = 0.;
-        } else if (pos >= 0 && pos < m.nnz) {
-            cp_async8(sv + si, m.vals + pos);
-        } else {
-            raise_error(err, kErrBounds);
-        }
-    });
+// Current values of the blocks that are added to.
+__device__ __forceinline__ void csr_prefetch(const CsrArgs &m, const KElem &t, const CsrElem &q, double *sv,
+                                             int lane) {
+    if (m.atomic) return;
+    csr_entries(m, t, q, lane, [](bool asg) { return asg; }, [&](int si, double *p) { cp_async8(sv + si, p); },
+                [](double *) {});
 }
 
-__device__ __forceinline__ void csr_write(const CsrArgs &m, const double *sv, int lane) {
-    csr_slots(sv, lane, [&](int si, long long pos, bool) {
-        if (pos >= 0 && pos < m.nnz) {
-            if (m.atomic) atomicAdd(m.vals + pos, sv[si]);
-            else m.vals[pos] = sv[si];
-        }
-    });
+// Stores the staged entries (assigned blocks with their exact zeros, which the
+// stage does not hold), or adds them with atomics.
+__device__ __forceinline__ void csr_write(const CsrArgs &m, const KElem &t, const CsrElem &q, const double *sv,
+                                          int lane) {
+    if (m.atomic)
+        csr_entries(m, t, q, lane, [](bool) { return false; },
+                    [&](int si, double *p) { atomicAdd(p, sv[si]); }, [](double *) {});
+    else
+        csr_entries(m, t, q, lane, [](bool) { return false; }, [&](int si, double *p) { *p = sv[si]; },
+                    [](double *p) { *p = 0.; });
 }
 
 __device__ __forceinline__ void kc0_round_csr(const Q4Args &a, const CsrArgs &m, KSmem &S, const KElem *els,
@@ -1000,18 +1005,25 @@ __device__ __forceinline__ void kc0_round_csr(const Q4Args &a, const CsrArgs &m,
     const int half = lane >> 4, pair = lane & 15;
     const int na = pair >> 2, nb = pair & 3;
     const int el = el0 + half;
+    const KElem &s = els[el];
     double *st = stage[half];
 #pragma unroll
-    for (int hh = 0; hh < 2; hh++) csr_meta_build(els[el0 + hh], cm[el0 + hh], stage[hh], lane);
-    __syncwarp();
-#pragma unroll
-    for (int hh = 0; hh < 2; hh++) csr_prefetch(m, stage[hh], lane, a.err);
+    for (int hh = 0; hh < 2; hh++) csr_prefetch(m, els[el0 + hh], cm[el0 + hh], stage[hh], lane);
     cp_async_commit();
     double H[3][3];
-    pair_tensor(S, els[el], el, na, nb, H);
+    pair_tensor(S, s, el, na, nb, H);
     cp_async_wait_all();
     __syncwarp();
-    pair_add(S, els[el], el, na, nb, H, st);
+    // a block that is assigned (or added with atomics) starts from zeros; a
+    // warp with such blocks only makes no additions
+    const bool own = m.atomic || ((cm[el].first >> (4 * na + nb)) & 1);
+    const bool clear = __all_sync(0xffffffffu, own || !(s.flags & KF_VALID));
+    if (own && !(clear && (s.flags & (KF_SPLIT | KF_FP64))))
+#pragma unroll
+        for (int i = 0; i < 6; i++)
+#pragma unroll
+            for (int j = 0; j < 6; j += 2) *staged(st, na, nb, i, j) = make_double2(0., 0.);
+    pair_add(S, s, el, na, nb, H, st, clear);
     __syncwarp();
 }
 
@@ -1029,6 +1041,10 @@ __global__ void __launch_bounds__(KNT, KMINB) quad4_kc0_csr_kernel(Q4Args a, Csr
         else S.el[buf][lane].flags = 0;
     };
     phase_a(0, 0);
+    // the next colour's CTAs may start as these end; this colour's values wait
+    // for the previous one (both no-ops in a launch without the attribute)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     int buf = 0, n;
     for (int64_t t = 0; (n = tiles.count(t)) > 0; t++, buf ^= 1) {
         __syncthreads();
@@ -1043,7 +1059,8 @@ __global__ void __launch_bounds__(KNT, KMINB) quad4_kc0_csr_kernel(Q4Args a, Csr
         for (int el0 = first; el0 < first + per && el0 < n; el0 += 2) {
             kc0_round_csr(a, m, S, els, SC.cm[buf], el0, S.stage[warp], lane);
 #pragma unroll
-            for (int hh = 0; hh < 2; hh++) csr_write(m, S.stage[warp][hh], lane);
+            for (int hh = 0; hh < 2; hh++)
+                csr_write(m, els[el0 + hh], SC.cm[buf][el0 + hh], S.stage[warp][hh], lane);
             __syncwarp();
         }
     }
@@ -1145,13 +1162,26 @@ extern "C" int fe3d_quad4_kc0_csr(const fe3d_fmap *fm, int g, const double *x, i
         FE3D_CHECK_LAUNCH();
         return FE3D_OK;
     }
+    bool launched = false;
     for (int c = 0; c < G.ncolors; c++) {
         const int64_t cnt = G.cstart[c + 1] - G.cstart[c];
         if (cnt == 0) continue;
         CsrArgs m{G.order + G.cstart[c], cnt, G.node, G.boff, G.first, fm->pat->noderow, fm->pat->nnodes,
                   vals, fm->pat->nnz, mode == FE3D_CSR_ASSIGN, 0};
-        quad4_kc0_csr_kernel<<<kc0_grid(cnt), KNT, sizeof(KSmemCsr), as_stream(stream)>>>(a, m);
-        FE3D_CHECK_LAUNCH();
+        // colours after the first overlap their set-up with the tail of the one
+        // before; the first waits for whatever the caller has queued
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kc0_grid(cnt));
+        cfg.blockDim = dim3(KNT);
+        cfg.dynamicSmemBytes = sizeof(KSmemCsr);
+        cfg.stream = as_stream(stream);
+        cfg.attrs = &at;
+        cfg.numAttrs = launched ? 1 : 0;
+        if (cudaLaunchKernelEx(&cfg, quad4_kc0_csr_kernel, a, m) != cudaSuccess) return FE3D_ERR_LAUNCH;
+        launched = true;
     }
     return FE3D_OK;
 }
