@@ -284,6 +284,39 @@ __device__ __forceinline__ void rotate_block(const double *R, double K[6][6]) {
         for (int j = 0; j < 6; j++) K[i][j] = T[i][j];
 }
 
+// Comparisons of doubles with integer operations (a DSETP takes the FP64 pipe
+// for 64 cycles): the results of ==, == 0 and > 0.
+__device__ __forceinline__ unsigned long long dbits(double v) { return (unsigned long long)__double_as_longlong(v); }
+__device__ __forceinline__ bool is_zero(double v) { return (dbits(v) << 1) == 0; }
+__device__ __forceinline__ bool is_nan(double v) { return (dbits(v) << 1) > 0xffe0000000000000ull; }
+__device__ __forceinline__ bool is_eq(double a, double b) {
+    return (dbits(a) == dbits(b) && !is_nan(a)) || (is_zero(a) && is_zero(b));
+}
+__device__ __forceinline__ bool is_pos(double v) { return (long long)dbits(v) > 0 && !is_nan(v); }
+__device__ __forceinline__ bool is_finite(double v) { return (dbits(v) << 1) < 0xffe0000000000000ull; }
+
+// sum_pq X[s_p t_q] H^pq over p, q in {x, y}: the coupling by X (11 12 16 22
+// 26 66) of the strains (s_x, s_y) and (t_x, t_y) that the two DOFs'
+// derivatives make (0 xx, 1 yy, 2 xy); the xy-xy term takes x66.
+__device__ __forceinline__ constexpr int sym3(int i, int j) {
+    return i > j ? sym3(j, i) : i == 0 ? j : i == 1 ? 2 + j : 5;
+}
+template <int SX, int SY, int TX, int TY>
+__device__ __forceinline__ double couple(const double *X, double x66, const double (*H)[3]) {
+    auto c = [&](int i, int j) { return sym3(i, j) == 5 ? x66 : X[sym3(i, j)]; };
+    return (c(SX, TX) * H[1][1] + c(SX, TY) * H[1][2]) + (c(SY, TX) * H[2][1] + c(SY, TY) * H[2][2]);
+}
+
+// out = tmp R^T: three rows of a 3x3 part turned to the global axes, from
+// tmp = R K.
+__device__ __forceinline__ void turn(const double *R, const double (&tmp)[3][3], double (&out)[3][3]) {
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++)
+            out[i][j] = tmp[i][0] * R[3 * j] + tmp[i][1] * R[3 * j + 1] + tmp[i][2] * R[3 * j + 2];
+}
+
 struct Q4Args {
     int64_t E;
     const int64_t *cdof;

@@ -88,17 +88,6 @@ struct KSmem {
 // [point][0: N, 1: dN/dxi, 2: dN/deta][node]
 __constant__ ff c_shape[KPTS][3][4];
 
-// Comparisons of doubles with integer operations (a DSETP takes the FP64 pipe
-// for 64 cycles): the results of ==, == 0 and > 0.
-__device__ __forceinline__ unsigned long long dbits(double v) { return (unsigned long long)__double_as_longlong(v); }
-__device__ __forceinline__ bool is_zero(double v) { return (dbits(v) << 1) == 0; }
-__device__ __forceinline__ bool is_nan(double v) { return (dbits(v) << 1) > 0xffe0000000000000ull; }
-__device__ __forceinline__ bool is_eq(double a, double b) {
-    return (dbits(a) == dbits(b) && !is_nan(a)) || (is_zero(a) && is_zero(b));
-}
-__device__ __forceinline__ bool is_pos(double v) { return (long long)dbits(v) > 0 && !is_nan(v); }
-__device__ __forceinline__ bool is_finite(double v) { return (dbits(v) << 1) < 0xffe0000000000000ull; }
-
 // Set-up of a flat isotropic element with its normal along +z, which needs no
 // frame: the decisions of q4_rotation + is_flat + iso_section, taken from the
 // coordinates and the record with 20 FP64 instructions instead of about 200.
@@ -513,28 +502,6 @@ __device__ __forceinline__ void pair_add_iso(const KElem &s, const double H[3][3
     add2<CLEAR, true, false>(st, na, nb, 3, 4, -(D66 * H[1][2] + D12 * H[2][1]), 0.);
     add2<CLEAR>(st, na, nb, 4, 2, E * h0(0, 1), -(D12 * H[1][2] + D66 * H[2][1]));
     add2<CLEAR, true, false>(st, na, nb, 4, 4, D11 * H[1][1] + (D66 * H[2][2] + ec), 0.);
-}
-
-// sum_pq X[s_p t_q] H^pq over p, q in {x, y}: the coupling by X (11 12 16 22
-// 26 66) of the strains (s_x, s_y) and (t_x, t_y) that the two DOFs'
-// derivatives make (0 xx, 1 yy, 2 xy); the xy-xy term takes x66.
-__device__ __forceinline__ constexpr int sym3(int i, int j) {
-    return i > j ? sym3(j, i) : i == 0 ? j : i == 1 ? 2 + j : 5;
-}
-template <int SX, int SY, int TX, int TY>
-__device__ __forceinline__ double couple(const double *X, double x66, const double H[3][3]) {
-    auto c = [&](int i, int j) { return sym3(i, j) == 5 ? x66 : X[sym3(i, j)]; };
-    return (c(SX, TX) * H[1][1] + c(SX, TY) * H[1][2]) + (c(SY, TX) * H[2][1] + c(SY, TY) * H[2][2]);
-}
-
-// out = tmp R^T: three rows of a 3x3 part turned to the global axes, from
-// tmp = R K.
-__device__ __forceinline__ void turn(const double *R, const double (&tmp)[3][3], double (&out)[3][3]) {
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++)
-            out[i][j] = tmp[i][0] * R[3 * j] + tmp[i][1] * R[3 * j + 1] + tmp[i][2] * R[3 * j + 2];
 }
 
 // Adds the general 6x6 block K_ab onto the staged values, three rows at a

@@ -9,7 +9,7 @@
 // Brockman's hourglass stiffness on u, v, w, rx, ry with the twist mode
 // gamma_a = N_a,xy at the centre (quad4r.pyx:1936-1981).
 //
-// KC0 kernels: phase A (one thread per element, plus one per Quad4R drilling
+// Quad4R KC0 kernel (Tria3R's: t3_kc0_kernel): phase A (one thread per element, plus one per Quad4R drilling
 // point) stages the element's frame, constitutive data and shape-function
 // derivatives in shared memory; phase B gives each thread one node pair
 // a <= b, builds the 6x6 block (and its transpose) and stages it; phase C
@@ -439,13 +439,10 @@ __device__ __forceinline__ void rs_drill_point(RSElem<NN> &s, const ff (*sh)[3][
     }
 }
 
-// 6x6 block of node pair (a, b) in the evaluation frame.  kc0_rule: the
-// Tria3R update_KC0 transformation (tria3r.pyx:2323-2960) keeps, of the
-// drilling DOF rz, only the diagonal rz_a - rz_a terms (its couplings with
-// u, v and with the rz of the other nodes do not reach KC0v), while
-// update_probe_finte uses the whole local matrix.
+// 6x6 block of node pair (a, b) in the evaluation frame (the whole local matrix;
+// Tria3R's update_KC0 leaves out couplings of rz: t3_pair_add).
 template <int NN>
-__device__ __forceinline__ void rs_block(const RSElem<NN> &s, const ff (*sh)[3][4], int a, int b, bool kc0_rule,
+__device__ __forceinline__ void rs_block(const RSElem<NN> &s, const ff (*sh)[3][4], int a, int b,
                                          double K[6][6]) {
     const double w = s.wc, Nc = NN == 3 ? 0.33333333333333333333 : 0.25;
     const double xa = s.Nx[a], ya = s.Ny[a], xb = s.Nx[b], yb = s.Ny[b];
@@ -575,15 +572,11 @@ __device__ __forceinline__ void rs_block(const RSElem<NN> &s, const ff (*sh)[3][
     K[0][1] -= kd * 0.25 * hyx;
     K[1][0] -= kd * 0.25 * hxy;
     K[1][1] += kd * 0.25 * hxx;
-    if (!(NN == 3 && kc0_rule)) {
-        K[0][5] += kd * 0.5 * hyn;
-        K[1][5] -= kd * 0.5 * hxn;
-        K[5][0] += kd * 0.5 * hny;
-        K[5][1] -= kd * 0.5 * hnx;
-        K[5][5] += kd * hnn;
-    } else if (a == b) {
-        K[5][5] += kd * hnn;
-    }
+    K[0][5] += kd * 0.5 * hyn;
+    K[1][5] -= kd * 0.5 * hxn;
+    K[5][0] += kd * 0.5 * hny;
+    K[5][1] -= kd * 0.5 * hnx;
+    K[5][5] += kd * hnn;
     if (NN == 4) {
         const double g = s.gam[a] * s.gam[b] * w;
         K[0][0] += g * s.hg[0];
@@ -598,14 +591,11 @@ __device__ __forceinline__ void rs_block(const RSElem<NN> &s, const ff (*sh)[3][
     }
 }
 
-// elements staged per pass: 8 (Quad4R) and 9 (Tria3R) keep the shared memory
-// of a block small enough for 3 and 4 blocks per SM (measured faster than
-// 12 and 18 at 2 and 3 blocks per SM, whose passes keep more threads busy)
+// elements staged per pass: 8 keep the shared memory of a block small enough
+// for 3 blocks per SM (measured faster than 12 at 2 blocks per SM, whose passes
+// keep more threads busy)
 #ifndef FE3D_RS_TB4
 #define FE3D_RS_TB4 8
-#endif
-#ifndef FE3D_RS_TB3
-#define FE3D_RS_TB3 9
 #endif
 template <int NN>
 struct RSTile {
@@ -614,14 +604,14 @@ struct RSTile {
     // staged row and element strides (doubles): rows 16-byte aligned; the
     // node pairs of a warp's stage updates spread over the banks (at most
     // 2-way conflicts), consecutive elements shifted by 4 or 12 banks
-    static constexpr int RS = NN == 4 ? 26 : S;
+    static constexpr int RS = S + 2;
     static constexpr int SP = S * RS + 2;
     static constexpr int P = NN * (NN + 1) / 2;      // node pairs a <= b
     // TE elements per tile: phase A runs on one full warp (the FP64 pipe
     // charges a warp instruction whatever its active lanes); the blocks are
     // staged TB elements at a time
     static constexpr int TE = 32;
-    static constexpr int TB = NN == 4 ? FE3D_RS_TB4 : FE3D_RS_TB3;
+    static constexpr int TB = FE3D_RS_TB4;
     static constexpr size_t smem = (size_t)TB * SP * sizeof(double) + (size_t)TE * sizeof(RSElem<NN>);
 };
 
@@ -704,7 +694,7 @@ __global__ void __launch_bounds__(RNT) rs_kc0_kernel(RSArgs a) {
                     int pa, pb;
                     pair_of<NN>(tid - el * Tl::P, pa, pb);
                     double K[6][6];
-                    rs_block<NN>(s, sh, pa, pb, true, K);
+                    rs_block<NN>(s, sh, pa, pb, K);
                     if (s.flags & RF_ROTATE) rotate_block(s.R, K);
                     double *st = stage + (size_t)el * Tl::SP;
                     // an isotropic block in the global frame couples (u, v,
@@ -799,7 +789,7 @@ __global__ void __launch_bounds__(RNT) rs_fint_kernel(RSArgs a, const double *ue
             const RSElem<NN> &s = se[el];
             if (s.flags & RF_VALID) {
                 double K[6][6];
-                rs_block<NN>(s, sh, pa, pb, false, K);
+                rs_block<NN>(s, sh, pa, pb, K);
                 const double *u = ue + 6 * NN * (e0 + el) + 6 * pb;
                 double ub[6];
 #pragma unroll
@@ -1168,6 +1158,534 @@ int launch_rs_kc0(const RSArgs &a, cudaStream_t st) {
     return FE3D_OK;
 }
 
+
+// ------------------------------------------------------------ Tria3R KC0
+// CTAs of 7 warps, two per SM: the last warp runs phase A (one lane per
+// element) one tile ahead into the other half of a double buffer; each of the
+// six others takes five elements of the tile, one lane per node pair a <= b
+// (30 of 32 lanes), adds the blocks and their transposes onto the staged values
+// and writes the elements out, with one barrier per tile.  Exact zeros are not
+// multiplied out, and nothing is added where the current values are zeros.
+// (With all warps in step over phase A, blocks and write-out, two of four
+// warps formed blocks and one ran phase A.)  120,000 flat isotropic triangles
+// with indices: 0.427 -> 0.213 ms
+// (5.9 TB/s, 0.87 of the measured copy rate).
+constexpr int TCW = 6;               // consumer warps
+constexpr int TEL = 5;               // elements per consumer warp and tile
+constexpr int TTE = TCW * TEL;       // elements per tile
+constexpr int TNT = 32 * (TCW + 1);
+constexpr int TROW = 18, TSP = 18 * TROW + 2;  // row and element strides of the stage (doubles)
+constexpr int TMINB = 2;
+static_assert(TTE <= 32 && 6 * TEL <= 32, "one warp per tile in phase A, one per round in phase B");
+
+// TF_ISO: isotropic section in the global frame (A16 = A26 = 0, A22 = A11, D
+// likewise, B = 0, E45 = 0, E44 = E55)
+enum : int { TF_VALID = 1, TF_ROTATE = 2, TF_B0 = 4, TF_ISO = 8 };
+
+struct __align__(16) T3Elem {
+    double R[9];
+    double A[6], B[6], D[6];  // 11 12 16 22 26 66, evaluation frame
+    double ap, am;            // A66 + kd / 4, A66 - kd / 4: with the drilling penalty
+    double es[3];             // E44 E45 E55 with the shear-locking factor
+    double Nx[3], Ny[3];
+    double w, kzz;            // w detJ of the centroid rule; drilling rz_a - rz_a
+    long long init_k;
+    long long c[3];
+    int flags;
+    int pad;
+};
+
+struct T3Smem {
+    T3Elem el[2][TTE];
+    double stage[TCW][TEL][TSP];
+};
+static_assert(TMINB * (sizeof(T3Smem) + 1024) <= 228 * 1024, "shared memory per SM");
+
+// Derivatives, shear-locking factor and drilling data of an element whose xy,
+// A and unscaled es are known.
+__device__ __forceinline__ void t3_finish(const RSArgs &a, int64_t e, const double *xy, double ar, double h, double a66,
+                                          T3Elem &s) {
+    t3_derivs(xy, ar, s.Nx, s.Ny);
+    s.w = 2 * ar * 0.5;
+    // alpha maxl^2 / h^2 (tria3r.pyx:2195-2210)
+    const double l12 = (xy[0] - xy[2]) * (xy[0] - xy[2]) + (xy[1] - xy[3]) * (xy[1] - xy[3]);
+    const double l23 = (xy[2] - xy[4]) * (xy[2] - xy[4]) + (xy[3] - xy[5]) * (xy[3] - xy[5]);
+    const double l31 = (xy[4] - xy[0]) * (xy[4] - xy[0]) + (xy[5] - xy[1]) * (xy[5] - xy[1]);
+    const double maxl2 = fmax(l12, fmax(l23, l31));
+    const double sf = h * h / (h * h + arg_at(a.aux, a.aux_stride, e, 0) * maxl2);
+#pragma unroll
+    for (int i = 0; i < 3; i++) s.es[i] = sf * s.es[i];
+    const double kd = 1e-6 * arg_at(a.k6rot, a.k6rot_stride, e, 0) * a66;
+    s.ap = s.A[5] + 0.25 * kd;
+    s.am = s.A[5] - 0.25 * kd;
+    s.kzz = kd * (s.w * 0.33333333333333333333 * 0.5);
+}
+
+__device__ void t3_phase_a(const RSArgs &a, int64_t e, T3Elem &s) {
+    s.flags = 0;
+    bool ok = true;
+    long long c[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        c[i] = a.cdof[3 * e + i];
+        s.c[i] = c[i];
+        if (c[i] < 0 || (a.x && c[i] / 2 + 3 > a.nx)) ok = false;
+    }
+    const long long k0 = a.init_k[e];
+    s.init_k = k0;
+    if (k0 < 0 || k0 + 324 > a.nk) ok = false;
+    const int64_t p = a.pid ? (int64_t)a.pid[e] : e;
+    if (p < 0 || p >= a.nprops) ok = false;
+    if (!ok) {
+        raise_error(a.err, kErrBounds);
+        return;
+    }
+    const double *P = a.props + (int64_t)SP_STRIDE * p;
+    const double h = P[SP_H];
+    const double E44 = P[SP_E44] * P[SP_SCF23];
+    const double E45 = P[SP_E45] * 0.5 * (P[SP_SCF13] + P[SP_SCF23]);
+    const double E55 = P[SP_E55] * P[SP_SCF13];
+    double xy[6], X[3], Y[3], Z[3];
+    if (a.x) {
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            const double *q = a.x + c[i] / 2;
+            X[i] = q[0];
+            Y[i] = q[1];
+            Z[i] = q[2];
+        }
+        // flat with the normal along +z and an isotropic section: no frame
+        // (the decisions of t3_rotation + is_flat + iso_section)
+        const double dx1 = X[1] - X[0], dy1 = Y[1] - Y[0], dx2 = X[2] - X[0], dy2 = Y[2] - Y[0];
+        bool iso = is_eq(Z[0], Z[1]) && is_eq(Z[0], Z[2]) && is_finite(Z[0]) && is_pos(dx1 * dy2 - dy1 * dx2);
+        iso = iso && is_zero(P[SP_A16]) && is_zero(P[SP_A26]) && is_zero(P[SP_D16]) && is_zero(P[SP_D26]);
+        if (iso) {
+            double v[12];
+#pragma unroll
+            for (int i = 0; i < 6; i++) iso &= is_zero(P[SP_B11 + i]);
+#pragma unroll
+            for (int i = 0; i < 6; i++) {
+                v[i] = P[SP_A11 + i];
+                v[6 + i] = P[SP_D11 + i];
+            }
+            const double eps = 64. * 2.220446049250313e-16;
+            iso &= is_eq(v[0], v[3]) && is_eq(v[6], v[9]) && is_zero(E45) && is_eq(E44, E55);
+            iso &= dbits(fabs(v[5] - 0.5 * (v[0] - v[1]))) <= dbits(eps * fabs(v[0]));
+            iso &= dbits(fabs(v[11] - 0.5 * (v[6] - v[7]))) <= dbits(eps * fabs(v[6]));
+            if (iso) {
+#pragma unroll
+                for (int i = 0; i < 6; i++) {
+                    s.A[i] = v[i];
+                    s.D[i] = v[6 + i];
+                }
+                s.es[0] = E44;
+                s.es[1] = E45;
+                s.es[2] = E55;
+                xy[0] = xy[1] = 0.;
+                xy[2] = dx1;
+                xy[3] = dy1;
+                xy[4] = dx2;
+                xy[5] = dy2;
+                t3_finish(a, e, xy, t3_area(xy), h, v[5], s);
+                s.flags = TF_VALID | TF_B0 | TF_ISO;
+                return;
+            }
+        }
+    }
+    double R[9], m[4] = {1., 0., 0., 1.}, ar;
+    bool global_frame = false;
+    if (a.x) {
+        const double *pp[3] = {a.x + c[0] / 2, a.x + c[1] / 2, a.x + c[2] / 2};
+        t3_rotation(pp[0], pp[1], pp[2], a.xmat ? a.xmat + (int64_t)a.xmat_stride * e : nullptr, R, m);
+        global_frame = is_flat(R);
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            if (global_frame) {
+                xy[2 * i] = pp[i][0] - pp[0][0];
+                xy[2 * i + 1] = pp[i][1] - pp[0][1];
+            } else {
+                double q[3];
+                to_local(R, pp[i], q);
+                xy[2 * i] = q[0];
+                xy[2 * i + 1] = q[1];
+            }
+        }
+        ar = t3_area(xy);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 9; i++) R[i] = a.R[9 * e + i];
+#pragma unroll
+        for (int i = 0; i < 4; i++) m[i] = a.m[4 * e + i];
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            xy[2 * i] = a.xe[9 * e + 3 * i];
+            xy[2 * i + 1] = a.xe[9 * e + 3 * i + 1];
+        }
+        ar = a.area[e];
+    }
+#pragma unroll
+    for (int i = 0; i < 9; i++) s.R[i] = R[i];
+    double a66 = P[SP_A66];  // element axes
+    if (m[1] != 0.) {
+        double A[6];
+        rotate_plane(m[0], m[1], m[2], m[3], P + SP_A11, A);
+        a66 = A[5];
+    }
+    q4_constitutive_packed(P, m, R, global_frame, s.A, s.B, s.D, s.es);
+    bool b0 = true;
+#pragma unroll
+    for (int i = 0; i < 6; i++) b0 &= is_zero(s.B[i]);
+    t3_finish(a, e, xy, ar, h, a66, s);
+    s.flags = TF_VALID | (global_frame ? 0 : TF_ROTATE) | (b0 ? TF_B0 : 0);
+}
+
+__device__ __forceinline__ double *t3_at(double *st, int na, int nb, int m, int n) {
+    return st + (6 * na + m) * TROW + 6 * nb + n;
+}
+
+// Adds (x, y) onto entries (m, n), (m, n + 1), n even, of block (na, nb); X, Y
+// false: left as it is (an exact zero); CLEAR: the entries are known zeros.
+template <bool CLEAR, bool X = true, bool Y = true>
+__device__ __forceinline__ void t3_add2(double *st, int na, int nb, int m, int n, double x, double y) {
+    double2 *q = reinterpret_cast<double2 *>(t3_at(st, na, nb, m, n));
+    if (CLEAR && X && Y) {
+        *q = make_double2(x, y);
+    } else if (CLEAR) {
+        if (X) q->x = x;
+        if (Y) q->y = y;
+    } else {
+        double2 o = *q;
+        if (X) o.x += x;
+        if (Y) o.y += y;
+        *q = o;
+    }
+}
+
+template <bool CLEAR>
+__device__ __forceinline__ void t3_add(double *st, int na, int nb, int m, int n, double v) {
+    double *q = t3_at(st, na, nb, m, n);
+    *q = CLEAR ? v : *q + v;
+}
+
+// The 14 non-zeros of an isotropic block in the global frame, formed while the
+// current values are on their way.
+struct T3Iso {
+    double uu, uv, vu, vv, ww, wx, wy, xw, yw, xx, xy, yx, yy, zz;
+    __device__ __forceinline__ T3Iso(const T3Elem &s, int na, int nb) {
+        const double Nc = 0.33333333333333333333, w = s.w, xb = s.Nx[nb], yb = s.Ny[nb];
+        const double wxa = w * s.Nx[na], wya = w * s.Ny[na], E = s.es[0];
+        const double hxx = wxa * xb, hxy = wxa * yb, hyx = wya * xb, hyy = wya * yb;
+        const double A11 = s.A[0], A12 = s.A[1], ap = s.ap, am = s.am, D11 = s.D[0], D12 = s.D[1], D66 = s.D[5];
+        uu = A11 * hxx + ap * hyy;
+        uv = A12 * hxy + am * hyx;
+        vu = A12 * hyx + am * hxy;
+        vv = ap * hxx + A11 * hyy;
+        ww = E * (hxx + hyy);
+        const double EN = E * Nc, EwN = EN * w, e = EwN * Nc;
+        wx = -(EN * wya);
+        wy = EN * wxa;
+        xw = -(EwN * yb);
+        yw = EwN * xb;
+        xx = D66 * hxx + (D11 * hyy + e);
+        xy = -(D66 * hxy + D12 * hyx);
+        yx = -(D12 * hxy + D66 * hyx);
+        yy = D11 * hxx + (D66 * hyy + e);
+        zz = s.kzz;
+    }
+    template <bool CLEAR>
+    __device__ __forceinline__ void add(double *st, int na, int nb) const {
+        t3_add2<CLEAR>(st, na, nb, 0, 0, uu, uv);
+        t3_add2<CLEAR>(st, na, nb, 1, 0, vu, vv);
+        t3_add2<CLEAR>(st, na, nb, 2, 2, ww, wx);
+        t3_add<CLEAR>(st, na, nb, 2, 4, wy);
+        t3_add2<CLEAR>(st, na, nb, 3, 2, xw, xx);
+        t3_add<CLEAR>(st, na, nb, 3, 4, xy);
+        t3_add2<CLEAR>(st, na, nb, 4, 2, yw, yx);
+        t3_add<CLEAR>(st, na, nb, 4, 4, yy);
+        if (na == nb) {
+            t3_add<CLEAR>(st, na, nb, 5, 5, zz);
+        } else {
+            t3_add2<CLEAR>(st, nb, na, 0, 0, uu, vu);
+            t3_add2<CLEAR>(st, nb, na, 1, 0, uv, vv);
+            t3_add2<CLEAR>(st, nb, na, 2, 2, ww, xw);
+            t3_add<CLEAR>(st, nb, na, 2, 4, yw);
+            t3_add2<CLEAR>(st, nb, na, 3, 2, wx, xx);
+            t3_add<CLEAR>(st, nb, na, 3, 4, yx);
+            t3_add2<CLEAR>(st, nb, na, 4, 2, wy, xy);
+            t3_add<CLEAR>(st, nb, na, 4, 4, yy);
+        }
+    }
+};
+
+// Node-pair block K_ab (a <= b) of the element and its transpose onto the
+// staged values.  Of the drilling rotations update_KC0 keeps rz_a - rz_a only.
+template <bool ROT, bool B0>
+__device__ __forceinline__ void t3_pair_add(const T3Elem &s, double *st, int na, int nb) {
+    constexpr bool CLEAR = false;
+    const double Nc = 0.33333333333333333333;
+    const double w = s.w, xb = s.Nx[nb], yb = s.Ny[nb];
+    const double wxa = w * s.Nx[na], wya = w * s.Ny[na];
+    double H[3][3];  // derivatives only
+    H[1][1] = wxa * xb;
+    H[1][2] = wxa * yb;
+    H[2][1] = wya * xb;
+    H[2][2] = wya * yb;
+    const double E44 = s.es[0], E45 = s.es[1], E55 = s.es[2];
+    const double *A = s.A, *B = s.B, *D = s.D, *R = s.R;
+    const double wN = w * Nc, xa0 = wxa * Nc, ya0 = wya * Nc, x0b = wN * xb, y0b = wN * yb, nn = wN * Nc;
+    const bool diag = na == nb;
+    const double kzz = diag ? s.kzz : 0.;
+    double P[3][3], Q[3][3];
+#pragma unroll
+    for (int hb = 0; hb < 2; hb++) {
+        if (hb == 0) {
+            P[0][0] = couple<0, 2, 0, 2>(A, s.ap, H);
+            P[0][1] = couple<0, 2, 2, 1>(A, s.am, H);
+            P[1][0] = couple<2, 1, 0, 2>(A, s.am, H);
+            P[1][1] = couple<2, 1, 2, 1>(A, s.ap, H);
+            P[2][2] = E44 * H[2][2] + E45 * (H[2][1] + H[1][2]) + E55 * H[1][1];
+            if (!B0) {
+                Q[0][0] = -couple<0, 2, 2, 1>(B, B[5], H);
+                Q[0][1] = couple<0, 2, 0, 2>(B, B[5], H);
+                Q[1][0] = -couple<2, 1, 2, 1>(B, B[5], H);
+                Q[1][1] = couple<2, 1, 0, 2>(B, B[5], H);
+            }
+            Q[2][0] = -(E44 * ya0 + E45 * xa0);
+            Q[2][1] = E45 * ya0 + E55 * xa0;
+        } else {
+            if (!B0) {
+                P[0][0] = -couple<2, 1, 0, 2>(B, B[5], H);
+                P[0][1] = -couple<2, 1, 2, 1>(B, B[5], H);
+                P[1][0] = couple<0, 2, 0, 2>(B, B[5], H);
+                P[1][1] = couple<0, 2, 2, 1>(B, B[5], H);
+            }
+            P[0][2] = -(E44 * y0b + E45 * x0b);
+            P[1][2] = E45 * y0b + E55 * x0b;
+            const double e45 = E45 * nn;
+            Q[0][0] = couple<2, 1, 2, 1>(D, D[5], H) + E44 * nn;
+            Q[0][1] = -(couple<2, 1, 0, 2>(D, D[5], H) + e45);
+            Q[1][0] = -(couple<0, 2, 2, 1>(D, D[5], H) + e45);
+            Q[1][1] = couple<0, 2, 0, 2>(D, D[5], H) + E55 * nn;
+            Q[2][2] = kzz;
+        }
+        if (!ROT) {
+            if (hb == 0) {
+                t3_add2<CLEAR>(st, na, nb, 0, 0, P[0][0], P[0][1]);
+                t3_add2<CLEAR>(st, na, nb, 1, 0, P[1][0], P[1][1]);
+                t3_add2<CLEAR>(st, na, nb, 2, 2, P[2][2], Q[2][0]);
+                t3_add<CLEAR>(st, na, nb, 2, 4, Q[2][1]);
+                if (!B0) {
+                    for (int i = 0; i < 2; i++) {
+                        t3_add<CLEAR>(st, na, nb, i, 3, Q[i][0]);
+                        t3_add<CLEAR>(st, na, nb, i, 4, Q[i][1]);
+                    }
+                }
+                if (!diag) {
+                    t3_add2<CLEAR>(st, nb, na, 0, 0, P[0][0], P[1][0]);
+                    t3_add2<CLEAR>(st, nb, na, 1, 0, P[0][1], P[1][1]);
+                    t3_add<CLEAR>(st, nb, na, 2, 2, P[2][2]);
+                    t3_add<CLEAR>(st, nb, na, 3, 2, Q[2][0]);
+                    t3_add<CLEAR>(st, nb, na, 4, 2, Q[2][1]);
+                    if (!B0)
+                        for (int i = 0; i < 2; i++) t3_add2<CLEAR>(st, nb, na, 3 + i, 0, Q[0][i], Q[1][i]);
+                }
+            } else {
+                if (!B0)
+                    for (int i = 0; i < 2; i++) t3_add2<CLEAR>(st, na, nb, 3 + i, 0, P[i][0], P[i][1]);
+                t3_add2<CLEAR>(st, na, nb, 3, 2, P[0][2], Q[0][0]);
+                t3_add<CLEAR>(st, na, nb, 3, 4, Q[0][1]);
+                t3_add2<CLEAR>(st, na, nb, 4, 2, P[1][2], Q[1][0]);
+                t3_add<CLEAR>(st, na, nb, 4, 4, Q[1][1]);
+                if (diag) {
+                    t3_add<CLEAR>(st, na, nb, 5, 5, Q[2][2]);
+                } else {
+                    t3_add<CLEAR>(st, nb, na, 2, 3, P[0][2]);
+                    t3_add<CLEAR>(st, nb, na, 2, 4, P[1][2]);
+                    for (int i = 0; i < 2; i++) {
+                        t3_add<CLEAR>(st, nb, na, 3 + i, 3, Q[0][i]);
+                        t3_add<CLEAR>(st, nb, na, 3 + i, 4, Q[1][i]);
+                        if (!B0) {
+                            t3_add<CLEAR>(st, nb, na, i, 3, P[0][i]);
+                            t3_add<CLEAR>(st, nb, na, i, 4, P[1][i]);
+                        }
+                    }
+                }
+            }
+        } else {
+            // R K of the part's non-zeros (no rz but the rz_a - rz_a term)
+            double tp[3][3], tq[3][3], op[3][3], oq[3][3];
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                const double x = R[3 * i], y = R[3 * i + 1], z = R[3 * i + 2];
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    tp[i][j] = hb == 0 || !B0 ? x * P[0][j] + y * P[1][j] : 0.;
+                    tq[i][j] = hb == 1 ? x * Q[0][j] + y * Q[1][j]
+                               : B0 ? z * Q[2][j] : x * Q[0][j] + y * Q[1][j] + z * Q[2][j];
+                }
+                tp[i][2] = hb == 0 ? z * P[2][2] : x * P[0][2] + y * P[1][2];
+                tq[i][2] = hb == 1 ? z * Q[2][2] : 0.;
+            }
+            turn(R, tp, op);
+            turn(R, tq, oq);
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                t3_add2<CLEAR>(st, na, nb, 3 * hb + i, 0, op[i][0], op[i][1]);
+                t3_add2<CLEAR>(st, na, nb, 3 * hb + i, 2, op[i][2], oq[i][0]);
+                t3_add2<CLEAR>(st, na, nb, 3 * hb + i, 4, oq[i][1], oq[i][2]);
+            }
+            if (!diag) {
+#pragma unroll
+                for (int i = 0; i < 3; i++)
+#pragma unroll
+                    for (int j = 0; j < 3; j++) {
+                        t3_add<CLEAR>(st, nb, na, j, 3 * hb + i, op[i][j]);
+                        t3_add<CLEAR>(st, nb, na, 3 + j, 3 * hb + i, oq[i][j]);
+                    }
+            }
+        }
+    }
+}
+
+// Whether everything that the warp's lanes add to is zero (the whole blocks:
+// entries a lane leaves alone only make the answer false more often).
+__device__ __forceinline__ bool t3_clear(double *st, int na, int nb) {
+    unsigned long long any = 0;
+#pragma unroll
+    for (int m = 0; m < 6; m++)
+#pragma unroll
+        for (int n = 0; n < 6; n += 2) {
+            const double2 o = *reinterpret_cast<const double2 *>(t3_at(st, na, nb, m, n));
+            const double2 q = *reinterpret_cast<const double2 *>(t3_at(st, nb, na, m, n));
+            any |= (dbits(o.x) << 1) | (dbits(o.y) << 1) | (dbits(q.x) << 1) | (dbits(q.y) << 1);
+        }
+    return any == 0;
+}
+
+__global__ void __launch_bounds__(TNT, TMINB) t3_kc0_kernel(RSArgs a, int vec16) {
+    extern __shared__ __align__(16) unsigned char t3_raw[];
+    T3Smem &S = *reinterpret_cast<T3Smem *>(t3_raw);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // tiles of TTE interleaved over the CTAs, then one smaller tile each that
+    // shares what is left evenly
+    const int64_t full = a.E / ((int64_t)TTE * gridDim.x), rest0 = full * TTE * gridDim.x, left = a.E - rest0;
+    auto first = [&](int64_t t) {
+        return t < full ? (t * gridDim.x + blockIdx.x) * TTE : rest0 + left * blockIdx.x / gridDim.x;
+    };
+    auto count = [&](int64_t t) {
+        if (t < full) return TTE;
+        return t > full ? 0 : (int)(left * (blockIdx.x + 1) / gridDim.x - left * blockIdx.x / gridDim.x);
+    };
+    auto phase_a = [&](int64_t t, int buf) {
+        if (warp != TCW || lane >= TTE) return;
+        if (lane < count(t)) t3_phase_a(a, first(t) + lane, S.el[buf][lane]);
+        else S.el[buf][lane].flags = 0;
+    };
+    phase_a(0, 0);
+    int buf = 0, n;
+    const int j = lane / 6, pr = lane - 6 * j;  // element of the warp and node pair of the lane
+    const int pa = pr < 3 ? 0 : pr < 5 ? 1 : 2, pb = pr < 3 ? pr : pr < 5 ? pr - 2 : 2;
+    for (int64_t t = 0; (n = count(t)) > 0; t++, buf ^= 1) {
+        __syncthreads();
+        if (warp == TCW) {
+            phase_a(t + 1, buf ^ 1);
+            continue;
+        }
+        // a short last tile spreads over the warps
+        const int per = (n + TCW - 1) / TCW, e0 = warp * per;
+        const int cnt = n - e0 < per ? n - e0 : per;
+        if (cnt <= 0) continue;
+        const T3Elem *els = S.el[buf] + e0;
+        double(*stage)[TSP] = S.stage[warp];
+        for (int k = 0; k < cnt; k++) {
+            if (!(els[k].flags & TF_VALID)) continue;
+            const double *kv = a.Kv + els[k].init_k;
+            if (vec16 && !(els[k].init_k & 1)) {
+#pragma unroll
+                for (int i = 0; i < 6; i++)
+                    if (lane + 32 * i < 162) cp_async16(stage[k] + 2 * (lane + 32 * i), kv + 2 * (lane + 32 * i));
+            } else {
+                for (int i = lane; i < 324; i += 32) cp_async8(stage[k] + i, kv + i);
+            }
+        }
+        cp_async_commit();
+        const int fl = j < cnt ? els[j].flags : 0;
+        const T3Elem &s = els[fl ? j : 0];
+        double *st = stage[fl ? j : 0];
+        if (__all_sync(0xffffffffu, !(fl & TF_VALID) || (fl & TF_ISO))) {
+            const T3Iso K(s, pa, pb);
+            cp_async_wait_all();
+            __syncwarp();
+            const bool clear = __all_sync(0xffffffffu, !(fl & TF_VALID) || t3_clear(st, pa, pb));
+            __syncwarp();
+            if (fl & TF_VALID) {
+                if (clear) K.add<true>(st, pa, pb);
+                else K.add<false>(st, pa, pb);
+            }
+        } else {
+            cp_async_wait_all();
+            __syncwarp();
+            if (fl & TF_ROTATE) {
+                if (fl & TF_B0) t3_pair_add<true, true>(s, st, pa, pb);
+                else t3_pair_add<true, false>(s, st, pa, pb);
+            } else if (fl & TF_VALID) {
+                if (fl & TF_B0) t3_pair_add<false, true>(s, st, pa, pb);
+                else t3_pair_add<false, false>(s, st, pa, pb);
+            }
+        }
+        __syncwarp();
+        for (int k = 0; k < cnt; k++) {
+            const T3Elem &e = els[k];
+            if (!(e.flags & TF_VALID)) continue;
+            const double *sv = stage[k];
+            const long long k0 = e.init_k;
+            if (vec16 && !(k0 & 1)) {
+                // slots q, q + 1, q = 2 lane + 64 i: 64 = 3 rows and 10 columns
+                int q = 2 * lane, row = q / 18, col = q - 18 * row;
+#pragma unroll
+                for (int i = 0; i < 6; i++, q += 64) {
+                    if (q < 324) {
+                        *reinterpret_cast<double2 *>(a.Kv + k0 + q) = *reinterpret_cast<const double2 *>(sv + q);
+                        if (!a.values_only) {
+                            const int ra = row / 6, cb = col / 6;
+                            const long long r = e.c[ra] + (row - 6 * ra), c = e.c[cb] + (col - 6 * cb);
+                            *reinterpret_cast<longlong2 *>(a.Kr + k0 + q) = make_longlong2(r, r);
+                            *reinterpret_cast<longlong2 *>(a.Kc + k0 + q) = make_longlong2(c, c + 1);
+                        }
+                    }
+                    row += 3;
+                    col += 10;
+                    if (col >= 18) {
+                        col -= 18;
+                        row += 1;
+                    }
+                }
+            } else {
+                for (int q = lane; q < 324; q += 32) {
+                    const int row = q / 18, col = q - 18 * row;
+                    a.Kv[k0 + q] = sv[q];
+                    if (!a.values_only) {
+                        a.Kr[k0 + q] = e.c[row / 6] + row % 6;
+                        a.Kc[k0 + q] = e.c[col / 6] + col % 6;
+                    }
+                }
+            }
+        }
+        __syncwarp();
+    }
+}
+
+int launch_t3_kc0(const RSArgs &a, cudaStream_t st) {
+    FE3D_CUDA(cudaFuncSetAttribute(t3_kc0_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(T3Smem)));
+    const auto al16 = [](const void *q) { return ((uintptr_t)q & 15u) == 0; };
+    const int vec16 = al16(a.Kv) && (a.values_only || (al16(a.Kr) && al16(a.Kc)));
+    // one wave of CTAs; small meshes spread over the SMs (6 elements a CTA)
+    const int64_t g = (a.E + 5) / 6, cap = (int64_t)kSMs * TMINB;
+    t3_kc0_kernel<<<(int)(g < cap ? g : cap), TNT, sizeof(T3Smem), st>>>(a, vec16);
+    FE3D_CHECK_LAUNCH();
+    return FE3D_OK;
+}
+
 int rs_check_common(int64_t E, const int64_t *cdof, const double *x, const double *xmat, int xmat_stride,
                     const double *R, const double *m, const double *xe, const double *area, const double *props,
                     int64_t nprops, const double *k6rot, int k6rot_stride) {
@@ -1232,7 +1750,7 @@ extern "C" int fe3d_tria3r_kc0(int64_t E, const int64_t *cdof, const int64_t *in
     if (!values_only && (!Kr || !Kc)) return FE3D_ERR_ARG;
     RSArgs a{E, cdof, init_k, x, nx, xmat, xmat_stride, R, m, xe, area, props, nprops, pid, k6rot, k6rot_stride,
              alpha, alpha_stride, Kr, Kc, Kv, nk, values_only, err};
-    return launch_rs_kc0<3>(a, as_stream(stream));
+    return launch_t3_kc0(a, as_stream(stream));
 }
 
 extern "C" int fe3d_quad4r_kc0(int64_t E, const int64_t *cdof, const int64_t *init_k, const double *x, int64_t nx,

@@ -83,3 +83,37 @@ def test_csr_matches_triplets(gpulib, nx, ny, section):
         batch.quad4_update_KC0_csr(vals, fmap, m.x, rec, mode=mode)
         got = vals - start if mode == 'add' else vals
         assert float((got - want).abs().max()) <= 1e-14 * scale, (mode, start)
+
+
+@pytest.mark.parametrize('E', [1, 5, 7, 29, 31, 1823, 1825, 9121])
+@pytest.mark.parametrize('start', ['clear', 'mixed', 'random'])
+def test_tria_tiles_sections_and_current_values(gpulib, oracle, E, start):
+    """Tria3R at the edges of its tiles (6 elements a CTA, 5 a warp, 30 a tile, one full wave)."""
+    import torch
+    from pyfe3d_gb300 import batch
+    x4, _, recs, pid, rng = _elements(E, 3 * E)
+    x = x4.reshape(E, 4, 3)[:, :3].copy()
+    x[rng.random(E) < 0.6, :, 2] = 0.
+    x = x.ravel()
+    cdof = 6 * np.arange(3 * E, dtype=np.int64).reshape(E, 3)
+    k6, alpha = rng.uniform(10., 200., E), rng.uniform(0.2, 1., E)
+    off = 1 if E % 2 else 0  # odd: the 8-byte path
+    n = 324 * E + 2
+    v0 = np.zeros(n)
+    if start != 'clear':
+        v0[:] = rng.normal(size=n)
+    if start == 'mixed':
+        v0[:324 * (E // 2)] = 0.
+        v0[rng.random(n) < 0.5] = 0.
+    r = torch.zeros(n, dtype=torch.int64, device='cuda')
+    c, v = torch.zeros_like(r), torch.from_numpy(v0).cuda()
+    ik = 324 * np.arange(E, dtype=np.int64)
+    batch.tria3r_update_KC0(r, c, v, x, cdof, ik + off, recs, pid=pid, k6rot=k6, alpha=alpha)
+    r0, c0, k0 = oracle.t3_kc0_batch(cdof, ik, x, recs, pid=pid, k6rot=k6, alpha=alpha)
+    s = slice(off, off + 324 * E)
+    assert (r.cpu().numpy()[s] == r0).all() and (c.cpu().numpy()[s] == c0).all()
+    got = v.cpu().numpy()
+    assert blockwise_rel_err(got[s] - v0[s], k0, 324) < REL_TOL
+    out = np.ones(n, bool)
+    out[s] = False
+    assert (got[out] == v0[out]).all()
