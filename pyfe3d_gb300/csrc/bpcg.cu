@@ -23,6 +23,15 @@
 // instance changes), rebuilt between chunks whenever a quarter of the listed
 // instances has finished, so converged plates stop costing bandwidth.
 //
+// Resident teams (precision 0): where every active instance's rows are contiguous
+// and its vectors fit the shared memory of the blocks it gets, the instances run
+// in one cooperative launch, each on a team of blocks of its own (team_pcg.cu),
+// without lockstep: blocks are dealt out by the expected time of each instance's
+// remaining iterations, and dealt out anew when a fifth of them has nothing left
+// to do.  48 plates of 8..40 elements a side to 1e-10: lockstep 139 ms (three
+// launches and the slowest plate's iterations, stored zeros and all), teams
+// 51 ms.
+//
 // Work split (precision 0): instances whose rows are contiguous and at most
 // `split_rows` in number are instead solved each by one thread block of a
 // block-resident kernel (bcta_kernel) on a second stream, concurrently with
@@ -33,7 +42,10 @@
 #include <limits.h>
 #include <math.h>
 
+#include <algorithm>
+#include <queue>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
@@ -627,6 +639,15 @@ __global__ void __launch_bounds__(CT) bcta_kernel(CtaArgs a) {
     }
 }
 
+// bw[inst] = how far the columns of an instance's rows reach from the diagonal.
+__global__ void inst_reach_kernel(int64_t n, const int64_t *rowptr, const int32_t *colind, const int32_t *inst,
+                                  int32_t *bw) {
+    const int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (row >= n || rowptr[row + 1] <= rowptr[row]) return;
+    const int lo = (int)row - colind[rowptr[row]], hi = colind[rowptr[row + 1] - 1] - (int)row;
+    atomicMax(bw + inst[row], lo > hi ? lo : hi);
+}
+
 // Counts entries that couple two different instances.
 __global__ void coupling_kernel(int64_t n, const int64_t *rowptr, const int32_t *colind, const int32_t *inst,
                                 int *bad) {
@@ -660,7 +681,10 @@ struct fe3d_bsolver {
     // instances whose rows are contiguous (0 otherwise), the size limit, and
     // the block-resident solver's list, results and stream
     int32_t *rlo = nullptr, *rhi = nullptr, *nlo = nullptr, *nhi = nullptr, *rcnt = nullptr, *ncnt = nullptr;
-    std::vector<int64_t> contig_rows;
+    std::vector<int64_t> contig_rows, first_row;
+    fe3d_team *team = nullptr;     // resident teams, made by the first solve that can use them
+    int team_tried = 0;
+    std::vector<int32_t> reach;    // column reach of each instance
     int64_t split_rows = 0;
     int32_t *cta_list = nullptr;
     int *cta_status = nullptr;
@@ -787,6 +811,7 @@ int autotune(fe3d_bsolver *b, const VT *vals, PT *p, PT *q, int *best) {
 extern "C" int fe3d_bsolver_free(fe3d_bsolver *b) {
     if (!b) return FE3D_OK;
     drop_graphs(b);
+    team_free(b->team);
     cudaFree(b->inst); cudaFree(b->node_inst); cudaFree(b->active); cudaFree(b->flag); cudaFree(b->bad);
     cudaFree(b->pq); cudaFree(b->rz); cudaFree(b->rr); cudaFree(b->ff); cudaFree(b->rt);
     cudaFree(b->rowlist); cudaFree(b->nodelist); cudaFree(b->lcount); cudaFree(b->blockcount);
@@ -880,6 +905,7 @@ extern "C" int fe3d_bsolver_create(const fe3d_pattern *pat, int block_size, int6
             return FE3D_ERR_CUDA;
         }
         b->contig_rows.assign(ninst, 0);
+        b->first_row.assign(lo.begin(), lo.end());
         for (int64_t i = 0; i < ninst; i++)
             if (cnt[i] > 0 && (int64_t)hi[i] - lo[i] + 1 == cnt[i]) b->contig_rows[i] = cnt[i];
     }
@@ -898,8 +924,9 @@ extern "C" int fe3d_bsolver_setup(fe3d_bsolver *b, const double *vals, int mixed
     // the private stream must see the block inverses written on the caller's stream
     FE3D_CUDA(cudaEventRecord(s->ev_in, as_stream(stream)));
     FE3D_CUDA(cudaStreamWaitEvent(s->stream, s->ev_in, 0));
-    if ((rc = autotune<double, double>(b, s->vals, s->p, s->q, &b->lanes[0]))) return rc;
-    if (mixed && (rc = autotune<float, float>(b, s->vals32, s->p32, s->q32, &b->lanes[1]))) return rc;
+    // (the pattern decides: once per solver)
+    if (!b->lanes[0] && (rc = autotune<double, double>(b, s->vals, s->p, s->q, &b->lanes[0]))) return rc;
+    if (mixed && !b->lanes[1] && (rc = autotune<float, float>(b, s->vals32, s->p32, s->q32, &b->lanes[1]))) return rc;
     return FE3D_OK;
 }
 
@@ -923,6 +950,75 @@ extern "C" int fe3d_bsolver_set_split(fe3d_bsolver *b, int64_t max_rows, int64_t
 }
 
 namespace {
+
+// Expected microseconds of one iteration of an instance on g blocks: exchanges,
+// then 28 + 7 FP64 instructions of 16 cycles an SM per 32 rows.
+double team_cost(int64_t rows, int g) { return 5. + (g > 1 ? 1.5 : 0.) + 0.009 * (double)rows / g; }
+
+// Deals the blocks out to the instances todo (their remaining iterations left,
+// relative): the longest first as long as each gets the blocks it needs, then
+// the spare blocks one by one to whatever would finish last.
+std::vector<TeamPart> deal(const fe3d_bsolver *b, const std::vector<int64_t> &todo, const std::vector<double> &left) {
+    std::vector<std::pair<double, int64_t>> order;
+    for (int64_t i : todo) order.push_back({left[i] * team_cost(b->contig_rows[i], 1), i});
+    std::sort(order.begin(), order.end(), [](const auto &x, const auto &y) {
+        return x.first != y.first ? x.first > y.first : x.second < y.second;
+    });
+    std::vector<TeamPart> parts;
+    int used = 0;
+    for (const auto &q : order) {
+        const int64_t i = q.second, n = b->contig_rows[i];
+        int g = 1;
+        while (g <= b->team->blocks && team_smem((n + g - 1) / g + 6, b->reach[i]) > b->team->smem_max) g++;
+        if (used + g > b->team->blocks) continue;
+        parts.push_back({b->first_row[i], b->first_row[i] + n, i, g});
+        used += g;
+    }
+    auto cost = [&](size_t k) {
+        return left[parts[k].sys] * team_cost(parts[k].row1 - parts[k].row0, parts[k].blocks);
+    };
+    std::priority_queue<std::pair<double, size_t>> heap;
+    for (size_t k = 0; k < parts.size(); k++) heap.push({cost(k), k});
+    for (; used < b->team->blocks && !heap.empty();) {
+        const size_t k = heap.top().second;
+        heap.pop();
+        if ((int64_t)parts[k].blocks * kTeamRows >= parts[k].row1 - parts[k].row0) continue;  // no gain from more
+        parts[k].blocks++;
+        used++;
+        heap.push({cost(k), k});
+    }
+    return parts;
+}
+
+// Whether the instances act can run on teams (makes the teams at first use).
+bool teams_ready(fe3d_bsolver *b, const std::vector<int> &act, cudaStream_t st) {
+    fe3d_solver *s = b->base;
+    if (!b->team_tried) {
+        b->team_tried = 1;
+        b->team = team_create(s, b->ninst, st);
+        if (b->team) {
+            b->reach.assign(b->ninst, 0);
+            bool ok = cudaMemsetAsync(b->rcnt, 0, sizeof(int32_t) * b->ninst, st) == cudaSuccess;
+            inst_reach_kernel<<<bgrid(s->n, 256, 1 << 30), 256, 0, st>>>(s->n, s->pat->rowptr, s->pat->colind, b->inst,
+                                                                         b->rcnt);
+            ok = ok && cudaMemcpyAsync(b->reach.data(), b->rcnt, sizeof(int32_t) * b->ninst, cudaMemcpyDeviceToHost,
+                                       st) == cudaSuccess &&
+                 cudaStreamSynchronize(st) == cudaSuccess;
+            if (!ok) {
+                (void)cudaGetLastError();
+                team_free(b->team);
+                b->team = nullptr;
+            }
+        }
+    }
+    if (!b->team) return false;
+    for (int64_t i = 0; i < b->ninst; i++)
+        if (act[i] && (b->contig_rows[i] <= 0 ||
+                       team_smem((b->contig_rows[i] + b->team->blocks - 1) / b->team->blocks + 6, b->reach[i]) >
+                           b->team->smem_max))
+            return false;
+    return true;
+}
 
 template <typename VT, typename PT>
 int bsolve(fe3d_bsolver *b, double *fu, double *uu, const fe3d_solve_opts *o, int prec, const VT *vals,
@@ -975,13 +1071,32 @@ int bsolve(fe3d_bsolver *b, double *fu, double *uu, const fe3d_solve_opts *o, in
         return FE3D_OK;
     };
     const double tol2 = o->tol * o->tol;
+    int rc;
+    // FP64 residuals of the iterates, statuses of the instances that were cut
+    // short, and the totals
+    auto finish = [&](int64_t its, int64_t repl) -> int {
+        std::vector<int> all(K, 1);
+        if ((rc = true_res(all))) return rc;
+        total->status = 0;
+        total->iterations = its;
+        total->replacements = repl;
+        double worst = 0.;
+        for (int64_t i = 0; i < K; i++) {
+            const double rel = hff[i] > 0. ? sqrt(hrt[i] / hff[i]) : 0.;
+            if (hact[i]) status[i] = rel <= o->tol ? 0 : 1;
+            if (status[i] > total->status) total->status = status[i];
+            if (rel > worst || !(rel == rel)) worst = rel;
+            relres[i] = rel;
+        }
+        total->relres = worst;
+        return FE3D_OK;
+    };
     // right-hand-side norms; instances with f = 0 get u = 0
     FE3D_CUDA(cudaMemsetAsync(b->ff, 0, sizeof(double) * K, st));
     bnorm_kernel<<<vg, BS, 0, st>>>(n, b->inst, fu, b->ff);
     FE3D_CHECK_LAUNCH();
     FE3D_CUDA(cudaMemcpyAsync(hff.data(), b->ff, sizeof(double) * K, cudaMemcpyDeviceToHost, st));
     FE3D_CUDA(cudaStreamSynchronize(st));
-    int rc;
     for (int64_t i = 0; i < K; i++) hflag[i] = hff[i] == 0.;
     if ((rc = upload(b->flag, hflag))) return rc;
     bzero_kernel<<<vg, BS, 0, st>>>(n, b->inst, b->flag, uu, 0, nullptr);
@@ -1039,11 +1154,84 @@ int bsolve(fe3d_bsolver *b, double *fu, double *uu, const fe3d_solve_opts *o, in
     }
     if ((rc = upload(b->flag, hact))) return rc;
     if ((rc = precondition(1))) return rc;
+    const int chunk = o->check_every < 2 ? 2 : (int)(o->check_every & ~1);
+    int64_t it = 0;
+    // resident teams: every instance iterates on its own, nothing in lockstep
+    if (prec == 0 && !nested && b->split_rows == 0 && nactive > 0 && o->maxiter > 0 && teams_ready(b, hact, st) &&
+        team_inverses(b->team, s, st) == FE3D_OK) {
+        fe3d_team *t = b->team;
+        std::vector<double> left(K), rr0(hrt);
+        std::vector<int64_t> todo;
+        std::vector<TeamPart> parts, was;
+        for (int64_t i = 0; i < K; i++) left[i] = sqrt((double)b->contig_rows[i]);
+        while (nactive > 0) {
+            todo.clear();
+            for (int64_t i = 0; i < K; i++)
+                if (hact[i] && iters[i] < o->maxiter) todo.push_back(i);
+            if (todo.empty()) break;
+            parts = deal(b, todo, left);
+            const bool same = parts.size() == was.size() &&
+                              std::equal(parts.begin(), parts.end(), was.begin(), [](const auto &x, const auto &y) {
+                                  return x.sys == y.sys && x.blocks == y.blocks;
+                              });
+            if (!same) {
+                unsigned long long total[2] = {0, 0};
+                if ((rc = team_split(t, s, parts, st)) || (rc = team_plan(t, s, st))) break;
+                FE3D_CUDA(cudaMemcpyAsync(total, t->total, sizeof(total), cudaMemcpyDeviceToHost, st));
+                FE3D_CUDA(cudaStreamSynchronize(st));
+                if ((rc = team_build(t, s, total[0], total[1], st))) break;
+                was = parts;
+            }
+            std::vector<TeamSys> sys(K, TeamSys{0., 0, 0, 0, 0});
+            for (const TeamPart &q : parts)
+                sys[q.sys] = {tol2 * hff[q.sys],
+                              (int)(o->maxiter - iters[q.sys] < kTeamIters ? o->maxiter - iters[q.sys] : kTeamIters),
+                              (int)(iters[q.sys] % chunk), 0, 0};
+            const int enough = parts.size() == 1 ? INT_MAX : t->G / 5 > 8 ? t->G / 5 : 8;
+            if ((rc = team_run(t, s, uu, b->rz + par * K, b->rr, sys, chunk, enough, st))) return rc;
+            FE3D_CUDA(cudaMemcpyAsync(hrr.data(), b->rr, sizeof(double) * K, cudaMemcpyDeviceToHost, st));
+            FE3D_CUDA(cudaStreamSynchronize(st));
+            std::vector<int> check(K, 0);
+            int ncheck = 0;
+            for (const TeamPart &q : parts) {
+                const int64_t i = q.sys;
+                iters[i] += sys[i].iters;
+                if (iters[i] > it) it = iters[i];
+                const double goal = tol2 * hff[i];
+                if (!(hrr[i] == hrr[i]) || isinf(hrr[i])) {
+                    hact[i] = 0;
+                    status[i] = 3;
+                    nactive--;
+                } else if (hrr[i] <= goal && (iters[i] % chunk == 0 || iters[i] >= o->maxiter)) {
+                    check[i] = 1;
+                    ncheck++;
+                }
+                // what is left of the way to the tolerance, in orders of magnitude
+                const double way = log(rr0[i] / goal), rest = hrr[i] > goal ? log(hrr[i] / goal) : 0.;
+                left[i] = sqrt((double)b->contig_rows[i]) * (way > 0. && rest < way ? fmax(rest / way, 0.05) : 1.);
+            }
+            if (!ncheck) continue;
+            if ((rc = true_res(check))) return rc;
+            for (int64_t i = 0; i < K; i++)
+                if (check[i] && hrt[i] <= tol2 * hff[i]) {
+                    hact[i] = 0;
+                    status[i] = 0;
+                    nactive--;
+                    check[i] = 0;
+                }
+            // a false convergence restarts from the FP64 residual
+            if ((rc = upload(b->flag, check))) return rc;
+            if ((rc = precondition(1))) return rc;
+        }
+        if (rc == FE3D_OK) return finish(it, 0);
+        // no memory for a split: the lockstep recurrence needs none
+        if (rc != FE3D_ERR_NOMEM) return rc;
+        if ((rc = upload(b->flag, hact)) || (rc = precondition(1))) return rc;
+    }
     FE3D_CUDA(cudaMemsetAsync(b->pq, 0, sizeof(double) * K, st));
     if ((rc = upload(b->active, hact))) return rc;
     if ((rc = compact(b, st))) return rc;
     int compacted_at = nactive;  // active instances when the lists were built
-    const int chunk = o->check_every < 2 ? 2 : (int)(o->check_every & ~1);
     auto launch_iteration = [&](int pr) {
         double *rz_cur = b->rz + pr * K, *rz_nxt = b->rz + (pr ^ 1) * K;
         launch_bspmv<VT, PT>(lanes, sg, st, n, b, vals, p, q, rz_nxt, b->rr);
@@ -1053,7 +1241,7 @@ int bsolve(fe3d_bsolver *b, double *fu, double *uu, const fe3d_solve_opts *o, in
         bdirection_kernel<PT><<<vg, BS, 0, st>>>(n, b->inst, b->active, rz_nxt, rz_cur, z, p, b->pq, K, b->rowlist,
                                                  b->lcount);
     };
-    int64_t it = 0, since = 0, replacements = 0;
+    int64_t since = 0, replacements = 0;
     std::vector<double> last_rt(K, 0.);
     std::vector<int> stall(K, 0);
     std::vector<double> rr_start(hrt);       // nested: FP64 residual at the instance's last restart
@@ -1174,21 +1362,7 @@ int bsolve(fe3d_bsolver *b, double *fu, double *uu, const fe3d_solve_opts *o, in
             if (ci[i] > it_all) it_all = ci[i];
         }
     }
-    std::vector<int> all(K, 1);
-    if ((rc = true_res(all))) return rc;
-    total->status = 0;
-    total->iterations = it_all;
-    total->replacements = replacements;
-    double worst = 0.;
-    for (int64_t i = 0; i < K; i++) {
-        const double rel = hff[i] > 0. ? sqrt(hrt[i] / hff[i]) : 0.;
-        if (hact[i]) status[i] = rel <= o->tol ? 0 : 1;
-        if (status[i] > total->status) total->status = status[i];
-        if (rel > worst || !(rel == rel)) worst = rel;
-        relres[i] = rel;
-    }
-    total->relres = worst;
-    return FE3D_OK;
+    return finish(it_all, replacements);
 }
 
 }  // namespace

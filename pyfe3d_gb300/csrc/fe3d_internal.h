@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 // Free-row layout of one node in a pattern built from element connectivity:
 // its free rows are consecutive, start at CSR position rs (-1 when the node
 // has no free DOF) and all have L entries; fm holds the free-DOF bits.
@@ -62,31 +64,51 @@ struct fe3d_fmap {
     fe3d_fmap_group g[kFmapMaxGroups];
 };
 
-// Resident PCG of one system (team_pcg.cu): its split over co-resident blocks,
-// the slice layout of the non-zero values and the exchange words.
+// Resident PCG (team_pcg.cu): the split of one or more systems over co-resident
+// blocks, the slice layout of the non-zero values and the exchange words.
 // Rows per block wanted while blocks are left: 16 rather than 64 at 2,166 rows
 // takes 6.2 instead of 8.0 us per iteration (fewer FP64 instructions per block
 // against a slower exchange).
 constexpr int kTeamRows = 16;
-constexpr int64_t kTeamMaxRows = 1 << 20;
+constexpr int64_t kTeamIters = 4096;   // iterations of one resident launch at most (a quarter of a second)
+
+// One system of a launch: limits in, iterations out.
+struct TeamSys {
+    double stop2;   // r.r at which to stop
+    int maxiter;    // iterations of this launch at most
+    int phase;      // convergence is looked at where phase + iterations is a multiple of chunk
+    int iters;      // iterations run
+    int pad;
+};
+
+// Rows [row0, row1) of system sys on so many blocks.
+struct TeamPart {
+    int64_t row0, row1, sys;
+    int blocks;
+};
 
 struct fe3d_team {
-    int G = 0, L = 1;                  // blocks, lanes per row
+    int blocks = 0;                    // blocks of a launch at most
+    size_t smem_max = 0;
+    int G = 0, L = 1;                  // blocks in use, lanes per row
     int nmax = 0, wmax = 0;            // largest row count and column window of a block
     size_t smem = 0;
     bool reg = false;                  // the rows fit the blocks' registers
-    int32_t *r0 = nullptr;             // [G + 1] first row of each block
-    int32_t *slice0 = nullptr;         // [G + 1] first slice
-    int32_t *cmin = nullptr, *cmax = nullptr;  // [G] column window
+    int32_t *ints = nullptr;           // the per-block arrays below
+    int32_t *rbeg = nullptr, *rend = nullptr, *slice0 = nullptr, *cmin = nullptr, *cmax = nullptr;
+    int32_t *tfirst = nullptr, *tcount = nullptr, *tsys = nullptr;
+    int64_t slices = 0;                // allocated in slen, soff
     int32_t *slen = nullptr;
     int64_t *soff = nullptr;
     double *sval = nullptr;
     uint16_t *scol = nullptr;
-    int64_t cap = 0;
+    int64_t cap = 0;                   // entries allocated in sval, scol
     unsigned long long *total = nullptr;
     ulonglong2 *z = nullptr, *slots = nullptr;
     double *dval = nullptr;            // [6][n] non-zeros of the rows of the block inverses
     uint32_t *dinf = nullptr;          // [n]
+    TeamSys *sys = nullptr;
+    int *done = nullptr;
     unsigned epoch = 1;
 };
 
@@ -146,16 +168,19 @@ struct fe3d_solver {
 
 namespace fe3d {
 void team_free(fe3d_team *t);
-fe3d_team *team_create(const fe3d_solver *s, cudaStream_t st);
+fe3d_team *team_create(const fe3d_solver *s, int64_t nsys, cudaStream_t st);
+size_t team_smem(int64_t rows, int64_t bw);
+int team_split(fe3d_team *t, const fe3d_solver *s, const std::vector<TeamPart> &parts, cudaStream_t st);
 // Counts the non-zeros into t->total (and the longest slice into t->total[1]);
-// team_build lays them out once the caller has read both.
+// team_build lays them out once the caller has read both; team_inverses takes
+// the block inverses.
 int team_plan(fe3d_team *t, const fe3d_solver *s, cudaStream_t st);
 int team_build(fe3d_team *t, const fe3d_solver *s, unsigned long long total, unsigned long long longest,
                cudaStream_t st);
-// Up to maxiter iterations from s->r, s->p, u and scal[rz_index], ended where
-// phase + iterations is a multiple of chunk and r.r <= stop2 or not finite;
-// scal[2] = r.r, scal[6] = iterations run, scal[7] = 1 when a block gave up
-// waiting.
-int team_run(fe3d_team *t, const fe3d_solver *s, double *u, int rz_index, int maxiter, int chunk, int phase,
-             double stop2, cudaStream_t st);
+int team_inverses(fe3d_team *t, const fe3d_solver *s, cudaStream_t st);
+// Iterations of every system of the split from s->r, s->p, u and rz (per
+// system), until its limits are met or the teams of enough blocks have
+// finished; rr per system, sys updated (synchronises).
+int team_run(fe3d_team *t, const fe3d_solver *s, double *u, double *rz, double *rr, std::vector<TeamSys> &sys,
+             int chunk, int enough, cudaStream_t st);
 }  // namespace fe3d

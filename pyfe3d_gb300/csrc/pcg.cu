@@ -31,6 +31,8 @@
 //   scalars stay FP64; every `replace_every` iterations the true residual
 //   replaces the recurrence residual (reliable updates), and convergence is
 //   decided on that residual only.
+#include <limits.h>
+
 #include "common.cuh"
 #include "fe3d_internal.h"
 
@@ -1113,8 +1115,6 @@ int sell_build(fe3d_solver *s, unsigned long long total, cudaStream_t st) {
     return FE3D_OK;
 }
 
-constexpr int64_t kTeamIters = 4096;  // iterations of one resident launch at most (a quarter of a second)
-
 // FP64 residual r = f - K u; returns ||r||^2 (synchronises).
 int true_residual(fe3d_solver *s, const double *f, double *u, cudaStream_t st, double *rr) {
     // the increment u since the last replacement joins the double-double
@@ -1154,8 +1154,17 @@ int run_cg(fe3d_solver *s, const double *f, double *u, const fe3d_solve_opts *o,
     // plain FP64 recurrence: resident iterations where the system fits
     const bool resident = prec == 0 && !o->flexible;
     if (resident && !s->team_tried) {
-        s->team = team_create(s, st);
+        // the split follows from the pattern: made once, kept with the solver
         s->team_tried = 1;
+        s->team = n <= (1 << 20) ? team_create(s, 1, st) : nullptr;
+        if (s->team) {
+            int64_t g = (n + kTeamRows - 1) / kTeamRows;
+            if (g > s->team->blocks) g = s->team->blocks;
+            if (team_split(s->team, s, {{0, n, 0, (int)g}}, st)) {
+                team_free(s->team);
+                s->team = nullptr;
+            }
+        }
     }
     fe3d_team *team = nullptr;
     {
@@ -1174,7 +1183,8 @@ int run_cg(fe3d_solver *s, const double *f, double *u, const fe3d_solve_opts *o,
                                       cudaMemcpyDeviceToHost, st));
         FE3D_CUDA(cudaStreamSynchronize(st));
         // no memory for the copy: the launch-per-kernel iteration needs none
-        if (team && ff != 0. && team_build(team, s, total[0], total[1], st)) team = nullptr;
+        if (team && ff != 0. && (team_build(team, s, total[0], total[1], st) || team_inverses(team, s, st)))
+            team = nullptr;
         else if (!team && prec == 0 && ff != 0. && (rc = sell_build(s, total[0], st))) return rc;
     }
     stats->iterations = 0;
@@ -1310,15 +1320,13 @@ int run_cg(fe3d_solver *s, const double *f, double *u, const fe3d_solve_opts *o,
         if (team) {
             // many chunks in one launch: it ends where the host has to act
             // (the conditions below), at kTeamIters iterations at most
-            double h[8];
             const int64_t most = (o->maxiter - it) < kTeamIters ? (o->maxiter - it) : kTeamIters;
-            const double stop2 = target > inner2 * rr_replaced ? target : inner2 * rr_replaced;
-            if ((rc = team_run(team, s, u, par, (int)most, chunk, (int)(it % chunk), stop2, st))) return rc;
-            FE3D_CUDA(cudaMemcpyAsync(h, s->scal, sizeof(h), cudaMemcpyDeviceToHost, st));
+            std::vector<TeamSys> one{{target > inner2 * rr_replaced ? target : inner2 * rr_replaced, (int)most,
+                                      (int)(it % chunk), 0, 0}};
+            if ((rc = team_run(team, s, u, s->scal + par, s->scal + 2, one, chunk, INT_MAX, st))) return rc;
+            FE3D_CUDA(cudaMemcpyAsync(&rr, s->scal + 2, sizeof(double), cudaMemcpyDeviceToHost, st));
             FE3D_CUDA(cudaStreamSynchronize(st));
-            if (h[7] != 0.) return FE3D_ERR_LAUNCH;
-            rr = h[2];
-            len = (int64_t)h[6];
+            len = one[0].iters;
         } else {
             if ((rc = run_chunk((int)len))) return rc;
             FE3D_CUDA(cudaMemcpyAsync(&rr, s->scal + 2, sizeof(double), cudaMemcpyDeviceToHost, st));

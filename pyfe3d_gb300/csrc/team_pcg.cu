@@ -11,6 +11,11 @@
 // columns its rows reach; p = z + beta p is recomputed by every block for its
 // own window, so z is the only vector that travels.
 //
+// Several independent systems run in one launch, each on a team of its own
+// blocks (bpcg.cu); teams do not wait for one another, and once the blocks of
+// finished teams pass a share of the grid the others stop at their next look at
+// the residual, so that the host can deal the blocks out anew.
+//
 // Exchange: every value that crosses blocks (z, the partial sums of p.q, r.z
 // and r.r) travels as two 8-byte words, each holding half of the double and
 // the iteration's number.  A reader polls the words themselves: no fence, no
@@ -33,6 +38,10 @@
 // resident: 486 rows 20.8 / 5.9, 2,166 rows 20.8 / 6.2, 9,126 rows 22.2 / 8.2,
 // 58,806 rows 25.5 / 11.6, 237,606 rows 43 / 25, 536,406 rows 69.5 / 60 (there
 // the matrix no longer fits L2 and bounds both).
+#include <limits.h>
+
+#include <vector>
+
 #include "common.cuh"
 #include "fe3d_internal.h"
 
@@ -125,7 +134,9 @@ __device__ __forceinline__ double team_add(const double (&v)[TEAM_WORDS], int G)
 }
 
 struct TeamArgs {
-    const int32_t *r0, *slice0, *cmin, *cmax;  // per block: first row, first slice, column window
+    // per block: rows, first slice, column window, and its team: first block,
+    // number of blocks and system
+    const int32_t *rbeg, *rend, *slice0, *cmin, *cmax, *tfirst, *tcount, *tsys;
     const int32_t *slen;
     const int64_t *soff;
     const double *sval;
@@ -138,15 +149,15 @@ struct TeamArgs {
     const uint32_t *dinf;    // [n] their number and, 3 bits each, their columns
     double *u, *r, *p;
     int64_t n;
-    double *scal;        // [rz_index] rz in / out, [2] r.r out, [6] iterations run, [7] 1: a poll gave up
-    int rz_index;
-    ulonglong2 *z;       // [n]
-    ulonglong2 *slots;   // [3][TEAM_MAX] slots: p.q, r.z, r.r
-    unsigned epoch;      // of the launch's first iteration
-    int maxiter;         // iterations of this launch at most
-    int chunk, phase;    // convergence is looked at where phase + iterations is a multiple of chunk
-    double stop2;        // r.r at which to stop
-    int wmax, nmax;      // largest window and row count of a block
+    double *rz, *rr;         // per system: r.z in and out, r.r out
+    TeamSys *sys;            // per system: limits in, iterations run out
+    ulonglong2 *z;           // [n]
+    ulonglong2 *slots;       // [3][blocks] slots: p.q, r.z, r.r
+    unsigned epoch;          // of the launch's first iteration
+    int chunk;               // convergence is looked at every chunk iterations
+    int wmax, nmax;          // largest window and row count of a block
+    int *done;               // [0] blocks of finished teams, [1] a poll gave up
+    int enough;              // finished blocks at which the other teams stop too
 };
 
 // Entries per lane that a block of at most TT / L rows keeps in registers.
@@ -156,16 +167,20 @@ template <int L, bool REG>
 __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
     extern __shared__ __align__(16) double sm[];
     __shared__ double red[TT + 4];
-    __shared__ double bc[3];
-    __shared__ int fail, fresh, dmax;  // a poll gave up; beta = 0; most non-zeros in a row of the block inverses
-    const int tid = threadIdx.x, G = gridDim.x, bid = blockIdx.x;
-    const int r0 = a.r0[bid], n = a.r0[bid + 1] - r0, c0 = a.cmin[bid], W = n > 0 ? a.cmax[bid] - c0 + 1 : 0;
-    const int s0 = a.slice0[bid];
+    __shared__ double bc[4];
+    // a poll gave up; beta = 0; most non-zeros in a row of the block inverses; others finished
+    __shared__ int fail, fresh, dmax, yield;
+    const int tid = threadIdx.x, G = a.tcount[blockIdx.x], t0 = a.tfirst[blockIdx.x], bid = blockIdx.x - t0;
+    const int sys = a.tsys[blockIdx.x];
+    const int r0 = a.rbeg[blockIdx.x], n = a.rend[blockIdx.x] - r0, c0 = a.cmin[blockIdx.x];
+    const int W = n > 0 ? a.cmax[blockIdx.x] - c0 + 1 : 0, s0 = a.slice0[blockIdx.x];
+    const TeamSys lim = a.sys[sys];
     double *pw = sm, *rs = pw + a.wmax, *us = rs + a.nmax, *qs = us + a.nmax;
     int *rfirst = reinterpret_cast<int *>(qs + a.nmax);  // first row of the row's node
     uint32_t *rinf = reinterpret_cast<uint32_t *>(rfirst + a.nmax);
     const int own = r0 - c0;  // window index of the block's first row
-    ulonglong2 *slot_pq = a.slots, *slot_rz = slot_pq + SLOT * TEAM_MAX, *slot_rr = slot_rz + SLOT * TEAM_MAX;
+    ulonglong2 *slot_pq = a.slots + SLOT * t0, *slot_rz = slot_pq + SLOT * gridDim.x,
+               *slot_rr = slot_rz + SLOT * gridDim.x;
     if (tid == 0) {
         fail = 0;
         dmax = 0;
@@ -179,7 +194,7 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
         rinf[i] = a.dinf[r0 + i];
         atomicMax(&dmax, (int)(rinf[i] & 7));
     }
-    double rz = a.scal[a.rz_index], rr = 0., irz = 0.;
+    double rz = a.rz[sys], rr = 0., irz = 0.;
     const int rows32 = (n * L + 31) & ~31;
     // REG: the block's rows of the matrix and of the block inverses stay in registers
     constexpr int MK = REG ? team_regs(L) : 4;
@@ -206,8 +221,8 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
         }
     }
     __syncthreads();
-    int it = 0, left = a.chunk - a.phase;  // iterations to the next look at convergence
-    bool stop = it >= a.maxiter;
+    int it = 0, left = a.chunk - lim.phase;  // iterations to the next look at convergence
+    bool stop = it >= lim.maxiter;
     const bool few = dmax <= 3;
     const int nwq = max(1, min(rows32, TT) >> 5), nwz = max(1, (min(n, TT) + 31) >> 5);
     while (!stop) {
@@ -262,7 +277,7 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
         __syncthreads();
         // z = Minv r, r.z (and r.r where convergence is looked at)
         it++;
-        const bool look = --left == 0 || it >= a.maxiter;
+        const bool look = --left == 0 || it >= lim.maxiter;
         if (left == 0) left = a.chunk;
         double lrz = 0., lrr = 0.;
         for (int i = tid; i < n; i += REG ? (1 << 20) : TT) {
@@ -289,16 +304,20 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
         if (look) {
             __syncthreads();
             lrr = team_block_sum(lrr, nwz, 1, red);
-            if (tid == 0) ll_store(slot_rr + SLOT * bid, lrr, ep);
+            if (tid == 0) {
+                ll_store(slot_rr + SLOT * bid, lrr, ep);
+                // the team's first block decides for all whether others have finished
+                if (bid == 0) ll_store(slot_rr + 1, *(volatile int *)a.done >= a.enough ? 1. : 0., ep);
+            }
         }
         for (int i = tid; i < n; i += REG ? (1 << 20) : TT) us[i] += alpha * pw[own + i];
         // p = z + beta p over the window.  The words of z are asked for once
         // r.z has come from every block: polling them earlier would crowd the
         // lines that their owners are about to write
-        double zv[4], vz[TEAM_WORDS], vr[TEAM_WORDS];
+        double zv[4], vz[TEAM_WORDS], vr[TEAM_WORDS], vy[1];
         if (tid >= TZ) {
             if (!team_poll(slot_rz, G, ep, vz)) fail = 1;
-            if (look && !team_poll(slot_rr, G, ep, vr)) fail = 1;
+            if (look && !(team_poll(slot_rr, G, ep, vr) && ll_poll(slot_rr + 1, 0, 1, 1, ep, vy))) fail = 1;
         }
         __syncthreads();
         if (tid < TZ) {
@@ -311,6 +330,7 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
                 fresh = be == 0.;
                 bc[1] = rzn;
                 bc[2] = s;
+                if (look) yield = vy[0] != 0.;
             }
         }
         __syncthreads();
@@ -332,18 +352,19 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
             }
         }
         __syncthreads();
-        stop = fail || it >= a.maxiter || (look && !(rr > a.stop2 && rr <= 1.7e308));
+        stop = fail || it >= lim.maxiter || (look && (yield || !(rr > lim.stop2 && rr <= 1.7e308)));
     }
     for (int i = tid; i < n; i += TT) {
         a.u[r0 + i] = us[i];
         a.r[r0 + i] = rs[i];
         a.p[r0 + i] = pw[own + i];
     }
-    if (fail && tid == 0) a.scal[7] = 1.;
+    if (fail && tid == 0) a.done[1] = 1;
     if (bid == 0 && tid == 0) {
-        a.scal[a.rz_index] = rz;
-        a.scal[2] = rr;
-        a.scal[6] = (double)it;
+        a.rz[sys] = rz;
+        a.rr[sys] = rr;
+        a.sys[sys].iters = it;
+        atomicAdd(a.done, G);
     }
 }
 
@@ -369,31 +390,25 @@ __global__ void __launch_bounds__(256) team_blocks_kernel(int64_t n, const int64
     dinf[row] = inf | (uint32_t)cnt;
 }
 
-// Block boundaries: rows split by stored entries, moved back to the first row
-// of the node they fall in.
-__global__ void team_split_kernel(int G, int64_t n, int64_t nnz, const int64_t *rowptr, const int64_t *dof_of_row,
-                                  const int32_t *start, int bs, int32_t *r0) {
+// First rows of the blocks: the wanted ones moved back to the first row of the
+// node they fall in (a team's first block keeps the system's first row); a
+// block ends where the next of its team begins.
+__global__ void team_split_kernel(int B, const int32_t *want, const int32_t *tfirst, const int32_t *tcount,
+                                  const int32_t *tend, const int64_t *dof_of_row, const int32_t *start, int bs,
+                                  int32_t *rbeg, int32_t *rend) {
     const int b = threadIdx.x;
-    if (b > G) return;
-    if (b == 0 || b == G) {
-        r0[b] = b == 0 ? 0 : (int32_t)n;
-        return;
-    }
-    const int64_t want = nnz / G * b;
-    int64_t lo = 0, hi = n;  // first row whose entries start at or after want
-    while (lo < hi) {
-        const int64_t m = (lo + hi) / 2;
-        if (rowptr[m] < want) lo = m + 1;
-        else hi = m;
-    }
-    r0[b] = lo < n ? start[dof_of_row[lo] / bs] : (int32_t)n;
+    auto at = [&](int i) { return i == tfirst[i] ? want[i] : start[dof_of_row[want[i]] / bs]; };
+    if (b >= B) return;
+    rbeg[b] = at(b);
+    rend[b] = b + 1 < tfirst[b] + tcount[b] ? at(b + 1) : tend[b];
 }
 
 // Column window of each block: its rows' columns and its own rows.
-__global__ void __launch_bounds__(256) team_window_kernel(const int32_t *r0, const int64_t *rowptr,
+__global__ void __launch_bounds__(256) team_window_kernel(const int32_t *rbeg, const int32_t *rend,
+                                                          const int64_t *rowptr,
                                                           const int32_t *colind, int32_t *cmin, int32_t *cmax) {
     __shared__ int lo, hi;
-    const int a = r0[blockIdx.x], e = r0[blockIdx.x + 1];
+    const int a = rbeg[blockIdx.x], e = rend[blockIdx.x];
     if (threadIdx.x == 0) {
         lo = a;
         hi = e - 1;
@@ -415,10 +430,11 @@ __global__ void __launch_bounds__(256) team_window_kernel(const int32_t *r0, con
 }
 
 // Lengths (entries per lane) and places of a block's slices.
-__global__ void __launch_bounds__(256) team_count_kernel(const int32_t *r0, const int32_t *slice0, int L,
+__global__ void __launch_bounds__(256) team_count_kernel(const int32_t *rbeg, const int32_t *rend, const int32_t *slice0,
+                                                         int L,
                                                          const int64_t *rowptr, const double *vals, int32_t *slen,
                                                          int64_t *soff, unsigned long long *total) {
-    const int a = r0[blockIdx.x], e = r0[blockIdx.x + 1], s0 = slice0[blockIdx.x], s1 = slice0[blockIdx.x + 1];
+    const int a = rbeg[blockIdx.x], e = rend[blockIdx.x], s0 = slice0[blockIdx.x], s1 = slice0[blockIdx.x + 1];
     const int lane = threadIdx.x & 31, per = 32 / L;
     for (int s = s0 + (threadIdx.x >> 5); s < s1; s += blockDim.x >> 5) {
         int longest = 0;
@@ -441,11 +457,12 @@ __global__ void __launch_bounds__(256) team_count_kernel(const int32_t *r0, cons
 
 // Entry k of a row goes to lane k % L of its L lanes; lanes that end early
 // repeat the row's last column with the value 0.
-__global__ void __launch_bounds__(256) team_fill_kernel(const int32_t *r0, const int32_t *slice0, int L,
+__global__ void __launch_bounds__(256) team_fill_kernel(const int32_t *rbeg, const int32_t *rend, const int32_t *slice0,
+                                                         int L,
                                                         const int64_t *rowptr, const uint16_t *col16,
                                                         const double *vals, const int32_t *slen,
                                                         const int64_t *soff, double *sval, uint16_t *scol) {
-    const int a = r0[blockIdx.x], e = r0[blockIdx.x + 1], s0 = slice0[blockIdx.x], s1 = slice0[blockIdx.x + 1];
+    const int a = rbeg[blockIdx.x], e = rend[blockIdx.x], s0 = slice0[blockIdx.x], s1 = slice0[blockIdx.x + 1];
     const int lane = threadIdx.x & 31, per = 32 / L;
     for (int s = s0 + (threadIdx.x >> 5); s < s1; s += blockDim.x >> 5) {
         const int row = a + (s - s0) * per + lane / L, sub = lane % L, len = slen[s];
@@ -495,27 +512,25 @@ bool get(T **p, size_t n) {
 
 void team_free(fe3d_team *t) {
     if (!t) return;
-    cudaFree(t->r0);
-    cudaFree(t->slice0);
-    cudaFree(t->cmin);
-    cudaFree(t->cmax);
+    cudaFree(t->ints);
     cudaFree(t->slen);
     cudaFree(t->soff);
     cudaFree(t->sval);
     cudaFree(t->scol);
     cudaFree(t->total);
     cudaFree(t->z);
+    cudaFree(t->slots);
     cudaFree(t->dval);
     cudaFree(t->dinf);
-    cudaFree(t->slots);
+    cudaFree(t->sys);
+    cudaFree(t->done);
     delete t;
 }
 
-// Splits the solver's system over blocks; nullptr where it does not fit (or
-// memory is short): the launch-per-kernel iteration is used then.
-fe3d_team *team_create(const fe3d_solver *s, cudaStream_t st) {
-    const fe3d_pattern *p = s->pat;
-    if (s->n < 1 || s->n > kTeamMaxRows || !p->col16) return nullptr;
+// Memory for up to nsys systems of the solver's matrix; nullptr where the
+// device or the pattern does not allow it or memory is short.
+fe3d_team *team_create(const fe3d_solver *s, int64_t nsys, cudaStream_t st) {
+    if (s->n < 1 || s->n > INT32_MAX || !s->pat->col16) return nullptr;
     int dev = 0, sms = 0, coop = 0, optin = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
@@ -523,66 +538,22 @@ fe3d_team *team_create(const fe3d_solver *s, cudaStream_t st) {
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess || !coop)
         return nullptr;
     fe3d_team *t = new fe3d_team();
-    const int64_t g = (s->n + kTeamRows - 1) / kTeamRows;
-    t->G = (int)(g < 1 ? 1 : g > TEAM_MAX ? TEAM_MAX : g);
-    if (t->G > sms) t->G = sms;
-    const int G = t->G;
-    int32_t h[3 * (TEAM_MAX + 1)];
-    bool ok = get(&t->r0, G + 1) && get(&t->slice0, G + 1) && get(&t->cmin, G) && get(&t->cmax, G) &&
-              get(&t->total, 2) && get(&t->z, s->n) && get(&t->slots, 3 * SLOT * TEAM_MAX) &&
-              get(&t->dval, 6 * s->n) && get(&t->dinf, s->n);
-    if (ok) {
-        team_split_kernel<<<1, TEAM_MAX + 8, 0, st>>>(G, s->n, p->nnz, p->rowptr, p->dof_of_row, s->start, s->bs, t->r0);
-        team_window_kernel<<<G, 256, 0, st>>>(t->r0, p->rowptr, p->colind, t->cmin, t->cmax);
-        ok = cudaMemcpyAsync(h, t->r0, sizeof(int32_t) * (G + 1), cudaMemcpyDeviceToHost, st) == cudaSuccess &&
-             cudaMemcpyAsync(h + G + 1, t->cmin, sizeof(int32_t) * G, cudaMemcpyDeviceToHost, st) == cudaSuccess &&
-             cudaMemcpyAsync(h + 2 * G + 1, t->cmax, sizeof(int32_t) * G, cudaMemcpyDeviceToHost, st) == cudaSuccess &&
-             cudaMemsetAsync(t->z, 0, sizeof(ulonglong2) * s->n, st) == cudaSuccess &&
-             cudaMemsetAsync(t->slots, 0, sizeof(ulonglong2) * 3 * SLOT * TEAM_MAX, st) == cudaSuccess &&
-             cudaStreamSynchronize(st) == cudaSuccess;
-    }
-    if (ok) {
-        for (int b = 0; b < G; b++) {
-            const int n = h[b + 1] - h[b], w = n > 0 ? h[2 * G + 1 + b] - h[G + 1 + b] + 1 : 0;
-            if (n < 0) ok = false;
-            if (n > t->nmax) t->nmax = n;
-            if (w > t->wmax) t->wmax = w;
-        }
-        t->smem = sizeof(double) * ((size_t)t->wmax + 3 * (size_t)t->nmax) + 2 * sizeof(int) * (size_t)t->nmax;
-        ok = ok && t->smem + 8192 <= (size_t)optin;
-    }
-    if (ok) {
-        // lanes per row: the fewest FP64 instructions on one sub-partition's
-        // warps for a row of 27 non-zeros (a node of a flat plate's inside)
-        int best = 1 << 30;
-        for (int L = 1; L <= 8; L *= 2) {
-            int cost = 28 / L + 1, lg = L;
-            while (lg > 1) {
-                cost++;
-                lg /= 2;
-            }
-            cost *= (t->nmax * L + 127) / 128;
-            if (cost < best) {
-                best = cost;
-                t->L = L;
-            }
-        }
-        const int per = 32 / t->L;
-        int32_t first[TEAM_MAX + 1];
-        first[0] = 0;
-        for (int b = 0; b < G; b++) first[b + 1] = first[b] + (h[b + 1] - h[b] + per - 1) / per;
-        ok = get(&t->slen, first[G]) && get(&t->soff, first[G]) &&
-             cudaMemcpyAsync(t->slice0, first, sizeof(int32_t) * (G + 1), cudaMemcpyHostToDevice, st) == cudaSuccess &&
-             cudaStreamSynchronize(st) == cudaSuccess;
+    t->blocks = sms < TEAM_MAX ? sms : TEAM_MAX;
+    t->smem_max = (size_t)optin - 8192;
+    const size_t slots = 3 * SLOT * TEAM_MAX;
+    bool ok = get(&t->ints, 10 * (TEAM_MAX + 1)) && get(&t->total, 2) && get(&t->z, s->n) && get(&t->slots, slots) &&
+              get(&t->dval, 6 * s->n) && get(&t->dinf, s->n) && get(&t->sys, nsys) && get(&t->done, 2) &&
+              cudaMemsetAsync(t->z, 0, sizeof(ulonglong2) * s->n, st) == cudaSuccess &&
+              cudaMemsetAsync(t->slots, 0, sizeof(ulonglong2) * slots, st) == cudaSuccess;
+    for (int L = 1; ok && L <= 8; L *= 2)
         for (int reg = 0; ok && reg < 2; reg++) {
             int res = 0;
-            ok = cudaFuncSetAttribute(team_kernel(t->L, reg), cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 8192) ==
-                     cudaSuccess &&
-                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res, team_kernel(t->L, reg), TT, t->smem) ==
+            ok = cudaFuncSetAttribute(team_kernel(L, reg), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)t->smem_max) == cudaSuccess &&
+                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res, team_kernel(L, reg), TT, t->smem_max) ==
                      cudaSuccess &&
                  res >= 1;
         }
-    }
     if (!ok) {
         (void)cudaGetLastError();
         team_free(t);
@@ -591,10 +562,94 @@ fe3d_team *team_create(const fe3d_solver *s, cudaStream_t st) {
     return t;
 }
 
+// Shared memory of a block of rows rows whose columns reach bw rows further on
+// either side.
+size_t team_smem(int64_t rows, int64_t bw) { return sizeof(double) * (size_t)(4 * rows + 2 * bw) + 8 * (size_t)rows; }
+
+// Deals the systems out: part i on parts[i].blocks blocks.  Returns 0, or
+// FE3D_ERR_TOO_LARGE where a block's rows do not fit shared memory.
+int team_split(fe3d_team *t, const fe3d_solver *s, const std::vector<TeamPart> &parts, cudaStream_t st) {
+    constexpr int S = TEAM_MAX + 1;
+    std::vector<int32_t> h(10 * S, 0);
+    int32_t *want = &h[0], *tfirst = &h[S], *tcount = &h[2 * S], *tend = &h[3 * S], *tsys = &h[4 * S];
+    int B = 0;
+    for (const TeamPart &q : parts) {
+        const int first = B;
+        for (int j = 0; j < q.blocks; j++, B++) {
+            if (B >= t->blocks) return FE3D_ERR_ARG;
+            want[B] = (int32_t)(q.row0 + (q.row1 - q.row0) * j / q.blocks);
+            tfirst[B] = first;
+            tcount[B] = q.blocks;
+            tend[B] = (int32_t)q.row1;
+            tsys[B] = (int32_t)q.sys;
+        }
+    }
+    t->G = B;
+    int32_t *d = t->ints;
+    t->tfirst = d + S;
+    t->tcount = d + 2 * S;
+    t->tsys = d + 4 * S;
+    t->rbeg = d + 5 * S;
+    t->rend = d + 6 * S;
+    t->cmin = d + 7 * S;
+    t->cmax = d + 8 * S;
+    t->slice0 = d + 9 * S;
+    FE3D_CUDA(cudaMemcpyAsync(d, h.data(), sizeof(int32_t) * 5 * S, cudaMemcpyHostToDevice, st));
+    team_split_kernel<<<1, TEAM_MAX + 8, 0, st>>>(B, d, t->tfirst, t->tcount, d + 3 * S, s->pat->dof_of_row, s->start,
+                                                  s->bs, t->rbeg, t->rend);
+    team_window_kernel<<<B, 256, 0, st>>>(t->rbeg, t->rend, s->pat->rowptr, s->pat->colind, t->cmin, t->cmax);
+    FE3D_CHECK_LAUNCH();
+    FE3D_CUDA(cudaMemcpyAsync(&h[5 * S], t->rbeg, sizeof(int32_t) * 4 * S, cudaMemcpyDeviceToHost, st));
+    FE3D_CUDA(cudaStreamSynchronize(st));
+    t->nmax = t->wmax = 0;
+    for (int b = 0; b < B; b++) {
+        const int n = h[6 * S + b] - h[5 * S + b], w = n > 0 ? h[8 * S + b] - h[7 * S + b] + 1 : 0;
+        if (n < 0) return FE3D_ERR_ARG;
+        if (n > t->nmax) t->nmax = n;
+        if (w > t->wmax) t->wmax = w;
+    }
+    t->smem = sizeof(double) * ((size_t)t->wmax + 3 * (size_t)t->nmax) + 2 * sizeof(int) * (size_t)t->nmax;
+    if (t->smem > t->smem_max) return FE3D_ERR_TOO_LARGE;
+    // lanes per row: the fewest FP64 instructions on one sub-partition's warps
+    // for a row of 27 non-zeros (a node of a flat plate's inside)
+    int best = 1 << 30;
+    for (int L = 1; L <= 8; L *= 2) {
+        int cost = 28 / L + 1, lg = L;
+        while (lg > 1) {
+            cost++;
+            lg /= 2;
+        }
+        cost *= (t->nmax * L + 127) / 128;
+        if (cost < best) {
+            best = cost;
+            t->L = L;
+        }
+    }
+    const int per = 32 / t->L;
+    int32_t *slice0 = &h[9 * S];
+    slice0[0] = 0;
+    for (int b = 0; b < B; b++) slice0[b + 1] = slice0[b] + (h[6 * S + b] - h[5 * S + b] + per - 1) / per;
+    if (slice0[B] > t->slices) {
+        cudaFree(t->slen);
+        cudaFree(t->soff);
+        t->slen = nullptr;
+        t->soff = nullptr;
+        t->slices = 0;
+        if (!get(&t->slen, slice0[B]) || !get(&t->soff, slice0[B])) {
+            (void)cudaGetLastError();
+            return FE3D_ERR_NOMEM;
+        }
+        t->slices = slice0[B];
+    }
+    FE3D_CUDA(cudaMemcpyAsync(t->slice0, slice0, sizeof(int32_t) * (B + 1), cudaMemcpyHostToDevice, st));
+    FE3D_CUDA(cudaStreamSynchronize(st));
+    return FE3D_OK;
+}
+
 int team_plan(fe3d_team *t, const fe3d_solver *s, cudaStream_t st) {
     FE3D_CUDA(cudaMemsetAsync(t->total, 0, 2 * sizeof(unsigned long long), st));
-    team_count_kernel<<<t->G, 256, 0, st>>>(t->r0, t->slice0, t->L, s->pat->rowptr, s->vals, t->slen, t->soff,
-                                            t->total);
+    team_count_kernel<<<t->G, 256, 0, st>>>(t->rbeg, t->rend, t->slice0, t->L, s->pat->rowptr, s->vals, t->slen,
+                                            t->soff, t->total);
     FE3D_CHECK_LAUNCH();
     return FE3D_OK;
 }
@@ -615,31 +670,44 @@ int team_build(fe3d_team *t, const fe3d_solver *s, unsigned long long total, uns
         }
         t->cap = entries;
     }
-    team_fill_kernel<<<t->G, 256, 0, st>>>(t->r0, t->slice0, t->L, s->pat->rowptr, s->pat->col16, s->vals, t->slen,
-                                           t->soff, t->sval, t->scol);
+    team_fill_kernel<<<t->G, 256, 0, st>>>(t->rbeg, t->rend, t->slice0, t->L, s->pat->rowptr, s->pat->col16, s->vals,
+                                           t->slen, t->soff, t->sval, t->scol);
+    FE3D_CHECK_LAUNCH();
+    return FE3D_OK;
+}
+
+int team_inverses(fe3d_team *t, const fe3d_solver *s, cudaStream_t st) {
     team_blocks_kernel<<<(unsigned)((s->n + 255) / 256), 256, 0, st>>>(s->n, s->pat->dof_of_row, s->start, s->size,
                                                                        s->bs, s->Dinv, t->dval, t->dinf);
     FE3D_CHECK_LAUNCH();
     return FE3D_OK;
 }
 
-int team_run(fe3d_team *t, const fe3d_solver *s, double *u, int rz_index, int maxiter, int chunk, int phase,
-             double stop2, cudaStream_t st) {
-    if (t->epoch > 0xffffffffu - (unsigned)maxiter - 2u) {
+int team_run(fe3d_team *t, const fe3d_solver *s, double *u, double *rz, double *rr, std::vector<TeamSys> &sys,
+             int chunk, int enough, cudaStream_t st) {
+    int most = 0;
+    for (const TeamSys &q : sys)
+        if (q.maxiter > most) most = q.maxiter;
+    if (t->epoch > 0xffffffffu - (unsigned)most - 2u) {
         FE3D_CUDA(cudaMemsetAsync(t->z, 0, sizeof(ulonglong2) * s->n, st));
         FE3D_CUDA(cudaMemsetAsync(t->slots, 0, sizeof(ulonglong2) * 3 * SLOT * TEAM_MAX, st));
         t->epoch = 1;
     }
-    TeamArgs a{t->r0, t->slice0, t->cmin, t->cmax, t->slen, t->soff, t->sval, t->scol, s->pat->colbase,
-               s->pat->dof_of_row, s->start, s->bs, t->dval, t->dinf, u, s->r, s->p, s->n, s->scal, rz_index,
-               t->z, t->slots, t->epoch, maxiter, chunk, phase, stop2, t->wmax, t->nmax};
-    t->epoch += (unsigned)maxiter + 1u;
-    FE3D_CUDA(cudaMemsetAsync(s->scal + 6, 0, 2 * sizeof(double), st));
+    FE3D_CUDA(cudaMemcpyAsync(t->sys, sys.data(), sizeof(TeamSys) * sys.size(), cudaMemcpyHostToDevice, st));
+    FE3D_CUDA(cudaMemsetAsync(t->done, 0, 2 * sizeof(int), st));
+    TeamArgs a{t->rbeg, t->rend, t->slice0, t->cmin, t->cmax, t->tfirst, t->tcount, t->tsys, t->slen, t->soff,
+               t->sval, t->scol, s->pat->colbase, s->pat->dof_of_row, s->start, s->bs, t->dval, t->dinf, u, s->r,
+               s->p, s->n, rz, rr, t->sys, t->z, t->slots, t->epoch, chunk, t->wmax, t->nmax, t->done, enough};
+    t->epoch += (unsigned)most + 1u;
     void *args[] = {&a};
-    if (cudaLaunchCooperativeKernel((const void *)team_kernel(t->L, t->reg), dim3(t->G), dim3(TT), args, t->smem, st) !=
-        cudaSuccess)
+    if (cudaLaunchCooperativeKernel((const void *)team_kernel(t->L, t->reg), dim3(t->G), dim3(TT), args, t->smem,
+                                    st) != cudaSuccess)
         return FE3D_ERR_LAUNCH;
-    return FE3D_OK;
+    int done[2] = {0, 0};
+    FE3D_CUDA(cudaMemcpyAsync(sys.data(), t->sys, sizeof(TeamSys) * sys.size(), cudaMemcpyDeviceToHost, st));
+    FE3D_CUDA(cudaMemcpyAsync(done, t->done, sizeof(done), cudaMemcpyDeviceToHost, st));
+    FE3D_CUDA(cudaStreamSynchronize(st));
+    return done[1] ? FE3D_ERR_LAUNCH : FE3D_OK;
 }
 
 }  // namespace fe3d

@@ -1,0 +1,52 @@
+"""Batched solves on teams of blocks: more instances than blocks, one instance far larger than the others, iteration
+caps and initial guesses, against the lockstep recurrence (which a work split of no instance selects)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _batch(sizes, seed):
+    import torch
+    from pyfe3d_gb300 import batch
+    from pyfe3d_gb300.meshes import BatchedPlates
+    from pyfe3d_gb300.solver import ElementPattern, FusedMap
+    rng = np.random.default_rng(seed)
+    nx, ny = np.array(sizes).T
+    P = len(sizes)
+    bp = BatchedPlates.__new__(BatchedPlates)
+    bp._build(nx, ny, rng.uniform(0.5, 2., P), rng.uniform(0.5, 2., P), rng.uniform(5e10, 2e11, P),
+              rng.uniform(0.25, 0.35, P), rng.uniform(0.005, 0.02, P), rng.integers(0, 2, P).astype(bool))
+    pat = ElementPattern([bp.cdof], bp.N, bp.bk)
+    fmap = FusedMap(pat, [bp.cdof])
+    vals = batch.quad4_update_KC0_csr(fmap.new_values(), fmap, bp.x, bp.props, pid=bp.pid)
+    f = torch.from_numpy(bp.f).cuda()
+    return bp, pat, vals, pat.reduce(f)
+
+
+@pytest.mark.parametrize('sizes', [[(3, 3)], [(2, 5), (60, 40)], [(2 + i % 5, 3 + i % 4) for i in range(200)],
+                                   [(50, 50)] + [(4, 4 + i % 3) for i in range(160)]], ids=['one', 'two', 'many', 'uneven'])
+def test_teams_match_lockstep(gpulib, sizes):
+    from pyfe3d_gb300.solver import BatchSolver
+    bp, pat, vals, f = _batch(sizes, len(sizes))
+    teams = BatchSolver(pat, bp.inst_of_dof, bp.P).setup(vals)
+    lock = BatchSolver(pat, bp.inst_of_dof, bp.P).setup(vals)
+    assert lock.set_split(1) == 0
+    u, st = teams.solve(f, tol=1e-10)
+    v, sl = lock.solve(f, tol=1e-10)
+    assert (st['inst_status'] == 0).all() and (sl['inst_status'] == 0).all()
+    assert (st['inst_relres'] <= 1e-10).all()
+    inst = teams.inst_of_row.cpu().numpy()
+    d, w = (u - v).cpu().numpy(), v.cpu().numpy()
+    err = np.sqrt(np.bincount(inst, d * d) / np.bincount(inst, w * w))
+    assert err.max() <= 1e-7, err.max()
+    # the same recurrence: the iteration counts agree up to rounding and the check interval
+    assert (abs(st['inst_iters'] - sl['inst_iters']) <= 100 + 0.05 * sl['inst_iters']).all()
+    # a cap ends every unfinished instance there; its iterate continues
+    u1, s1 = teams.solve(f, tol=1e-10, maxiter=30, check_every=20)
+    assert s1['inst_iters'].max() <= 30 and (s1['inst_iters'][s1['inst_status'] == 1] == 30).all()
+    u2, s2 = teams.solve(f, u0=u1, tol=1e-10)
+    assert (s2['inst_status'] == 0).all()
+    # nothing left to do
+    _, s3 = teams.solve(f, u0=u2, tol=1e-9)
+    assert (s3['inst_status'] == 0).all() and s3['inst_iters'].max() == 0
