@@ -91,8 +91,8 @@ struct fe3d_team {
     int blocks = 0;                    // blocks of a launch at most
     size_t smem_max = 0;
     int G = 0, L = 1;                  // blocks in use, lanes per row
-    int nmax = 0, wmax = 0;            // largest row count and column window of a block
-    size_t smem = 0;
+    int nmax = 0;                      // largest row count of a block
+    size_t smem = 0;                   // of the block that needs most
     bool reg = false;                  // the rows fit the blocks' registers
     int32_t *ints = nullptr;           // the per-block arrays below
     int32_t *rbeg = nullptr, *rend = nullptr, *slice0 = nullptr, *cmin = nullptr, *cmax = nullptr;

@@ -155,7 +155,6 @@ struct TeamArgs {
     ulonglong2 *slots;       // [3][blocks] slots: p.q, r.z, r.r
     unsigned epoch;          // of the launch's first iteration
     int chunk;               // convergence is looked at every chunk iterations
-    int wmax, nmax;          // largest window and row count of a block
     int *done;               // [0] blocks of finished teams, [1] a poll gave up
     int enough;              // finished blocks at which the other teams stop too
 };
@@ -175,9 +174,9 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
     const int r0 = a.rbeg[blockIdx.x], n = a.rend[blockIdx.x] - r0, c0 = a.cmin[blockIdx.x];
     const int W = n > 0 ? a.cmax[blockIdx.x] - c0 + 1 : 0, s0 = a.slice0[blockIdx.x];
     const TeamSys lim = a.sys[sys];
-    double *pw = sm, *rs = pw + a.wmax, *us = rs + a.nmax, *qs = us + a.nmax;
-    int *rfirst = reinterpret_cast<int *>(qs + a.nmax);  // first row of the row's node
-    uint32_t *rinf = reinterpret_cast<uint32_t *>(rfirst + a.nmax);
+    double *pw = sm, *rs = pw + W, *us = rs + n, *qs = us + n;
+    int *rfirst = reinterpret_cast<int *>(qs + n);  // first row of the row's node
+    uint32_t *rinf = reinterpret_cast<uint32_t *>(rfirst + n);
     const int own = r0 - c0;  // window index of the block's first row
     ulonglong2 *slot_pq = a.slots + SLOT * t0, *slot_rz = slot_pq + SLOT * gridDim.x,
                *slot_rr = slot_rz + SLOT * gridDim.x;
@@ -601,14 +600,15 @@ int team_split(fe3d_team *t, const fe3d_solver *s, const std::vector<TeamPart> &
     FE3D_CHECK_LAUNCH();
     FE3D_CUDA(cudaMemcpyAsync(&h[5 * S], t->rbeg, sizeof(int32_t) * 4 * S, cudaMemcpyDeviceToHost, st));
     FE3D_CUDA(cudaStreamSynchronize(st));
-    t->nmax = t->wmax = 0;
+    t->nmax = 0;
+    t->smem = 0;
     for (int b = 0; b < B; b++) {
         const int n = h[6 * S + b] - h[5 * S + b], w = n > 0 ? h[8 * S + b] - h[7 * S + b] + 1 : 0;
         if (n < 0) return FE3D_ERR_ARG;
         if (n > t->nmax) t->nmax = n;
-        if (w > t->wmax) t->wmax = w;
+        const size_t need = sizeof(double) * ((size_t)w + 3 * (size_t)n) + 2 * sizeof(int) * (size_t)n;
+        if (need > t->smem) t->smem = need;
     }
-    t->smem = sizeof(double) * ((size_t)t->wmax + 3 * (size_t)t->nmax) + 2 * sizeof(int) * (size_t)t->nmax;
     if (t->smem > t->smem_max) return FE3D_ERR_TOO_LARGE;
     // lanes per row: the fewest FP64 instructions on one sub-partition's warps
     // for a row of 27 non-zeros (a node of a flat plate's inside)
@@ -697,7 +697,7 @@ int team_run(fe3d_team *t, const fe3d_solver *s, double *u, double *rz, double *
     FE3D_CUDA(cudaMemsetAsync(t->done, 0, 2 * sizeof(int), st));
     TeamArgs a{t->rbeg, t->rend, t->slice0, t->cmin, t->cmax, t->tfirst, t->tcount, t->tsys, t->slen, t->soff,
                t->sval, t->scol, s->pat->colbase, s->pat->dof_of_row, s->start, s->bs, t->dval, t->dinf, u, s->r,
-               s->p, s->n, rz, rr, t->sys, t->z, t->slots, t->epoch, chunk, t->wmax, t->nmax, t->done, enough};
+               s->p, s->n, rz, rr, t->sys, t->z, t->slots, t->epoch, chunk, t->done, enough};
     t->epoch += (unsigned)most + 1u;
     void *args[] = {&a};
     if (cudaLaunchCooperativeKernel((const void *)team_kernel(t->L, t->reg), dim3(t->G), dim3(TT), args, t->smem,

@@ -25,7 +25,8 @@ def _batch(sizes, seed):
 
 
 @pytest.mark.parametrize('sizes', [[(3, 3)], [(2, 5), (60, 40)], [(2 + i % 5, 3 + i % 4) for i in range(200)],
-                                   [(50, 50)] + [(4, 4 + i % 3) for i in range(160)]], ids=['one', 'two', 'many', 'uneven'])
+                                   [(50, 50)] + [(4, 4 + i % 3) for i in range(160)],
+                                   [(260, 30), (30, 260), (150, 150), (140, 180), (250, 60), (200, 90)]], ids=['one', 'two', 'many', 'uneven', 'long'])
 def test_teams_match_lockstep(gpulib, sizes):
     from pyfe3d_gb300.solver import BatchSolver
     bp, pat, vals, f = _batch(sizes, len(sizes))
