@@ -52,6 +52,9 @@ extern "C" {
 #define FE3D_BEAMC_M_SIZE 144
 
 int fe3d_version(void);
+
+/* Waits until the work queued on the stream has finished. */
+int fe3d_stream_synchronize(void *stream);
 const char *fe3d_error_string(int code);
 
 /* ------------------------------------------------------------------ Quad4

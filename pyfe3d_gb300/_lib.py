@@ -4,8 +4,10 @@ The library is a plain C ABI (``include/fe3d_gb300.h``) loaded with ctypes.
 PyTorch only provides device memory and the current CUDA stream.  There is no
 CPU fallback: every entry point raises if the library or a GPU is missing.
 """
+import collections
 import ctypes
 import os
+import threading
 
 import numpy as np
 
@@ -33,6 +35,7 @@ c_vp = ctypes.c_void_p
 # argument signatures of the exported entry points (see include/fe3d_gb300.h)
 _SIGS = {
     'fe3d_version': ([], c_int),
+    'fe3d_stream_synchronize': ([c_vp], c_int),
     'fe3d_quad4_frame': ([c_i64, c_vp, c_vp, c_i64, c_vp, c_int, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp], c_int),
     'fe3d_quad4_probe_xe': ([c_i64, c_vp, c_vp, c_i64, c_vp, c_vp, c_vp, c_vp, c_vp], c_int),
     'fe3d_quad4_probe_ue': ([c_i64, c_vp, c_vp, c_i64, c_vp, c_vp, c_vp, c_vp], c_int),
@@ -158,33 +161,99 @@ def register(name, args, res=c_int):
         f.restype = res
 
 
+_torch = None
+_available = False
+
+
 def torch_mod():
-    import torch
-    return torch
+    global _torch
+    if _torch is None:
+        import torch
+        _torch = torch
+    return _torch
+
+
+def _device_index():
+    """Index of the current CUDA device; raises when no GPU is available."""
+    global _available
+    torch = torch_mod()
+    if not _available:
+        if not torch.cuda.is_available():
+            raise Fe3dError('pyfe3d_gb300 needs a CUDA device (GB300, sm_103a); none is available')
+        _available = True
+    return torch.cuda.current_device()
 
 
 def device():
     """The current CUDA device; raises when no GPU is available."""
+    return torch_mod().device('cuda', _device_index())
+
+
+def _raw_stream():
     torch = torch_mod()
-    if not torch.cuda.is_available():
-        raise Fe3dError('pyfe3d_gb300 needs a CUDA device (GB300, sm_103a); none is available')
-    return torch.device('cuda', torch.cuda.current_device())
+    raw = getattr(torch._C, '_cuda_getCurrentRawStream', None)
+    return raw(torch.cuda.current_device()) if raw is not None else torch.cuda.current_stream().cuda_stream
 
 
 def stream_ptr():
-    torch = torch_mod()
-    return c_vp(torch.cuda.current_stream().cuda_stream)
+    return c_vp(_raw_stream())
 
 
 def err_word():
-    """Per-device int32 error word the kernels OR their error bits into."""
+    """Per-device int32 error word the kernels OR their error bits into: pinned
+    host memory, which kernels touch only to report an error and the host
+    reads without a copy once it has synchronised the stream."""
     torch = torch_mod()
-    dev = device()
-    w = _err_words.get(dev.index)
+    idx = _device_index()
+    w = _err_words.get(idx)
     if w is None:
-        w = torch.zeros(1, dtype=torch.int32, device=dev)
-        _err_words[dev.index] = w
+        w = torch.zeros(1, dtype=torch.int32).pin_memory()
+        _err_words[idx] = w
     return w
+
+
+class _Constants:
+    """Small constant device tensors (a scalar, zero record indices) kept per
+    device and stream, so that a call that needs one neither copies from the
+    host nor fills.  A tensor is only ever used on the stream it was made on,
+    which also orders its release; at most 64 tensors of 16 MB are kept, the
+    least recently used released first.  Nothing is kept during a graph
+    capture, whose memory belongs to the graph."""
+
+    def __init__(self):
+        self._kept = collections.OrderedDict()
+        self._lock = threading.Lock()
+
+    def get(self, kind, n, make):
+        """make(m) returns a tensor of m equal entries; the result has n of them."""
+        if n > (1 << 21) or torch_mod().cuda.is_current_stream_capturing():
+            return make(n)
+        key = (kind, _device_index(), _raw_stream())
+        with self._lock:
+            t = self._kept.get(key)
+            if t is None or t.numel() < n:
+                t = self._kept[key] = make(max(n, 1024))
+                if len(self._kept) > 64:
+                    self._kept.popitem(last=False)
+            self._kept.move_to_end(key)
+        return t[:n]
+
+
+_constants = _Constants()
+
+
+def scalar_f64(v):
+    """A one-entry float64 device tensor holding v."""
+    torch = torch_mod()
+    v = float(v)
+    return _constants.get(('f64', v.hex()), 1,
+                          lambda m: torch.full((m,), v, dtype=torch.float64, device=device()))
+
+
+def zeros_i32(n):
+    """n int32 zeros on the device (not to be written)."""
+    torch = torch_mod()
+    return _constants.get('i32', n, lambda m: torch.zeros(m, dtype=torch.int32, device=device()))
 
 
 def ptr(t):
@@ -205,16 +274,24 @@ def keep(t):
     return ptr(t)
 
 
+def synchronize():
+    """Wait for the current stream."""
+    rc = load().fe3d_stream_synchronize(stream_ptr())
+    if rc != 0:
+        raise Fe3dError('%s (status %d)' % (FE3D_ERRORS.get(rc, 'unknown'), rc))
+
+
 def check(rc, what='', err=None):
     """Raise on a negative status; with ``err``, synchronise and check the device word."""
     if _kept:
-        torch_mod().cuda.current_stream().synchronize()
+        synchronize()
         del _kept[:]
     if rc != 0:
         raise Fe3dError('%s: %s (status %d)' % (what, FE3D_ERRORS.get(rc, 'unknown'), rc))
     if err is not None:
-        v = int(err.item())
-        if v:
+        synchronize()
+        if ctypes.c_int32.from_address(err.data_ptr()).value:
+            v = int(err.item())
             err.zero_()
             raise Fe3dError('%s: device reported error bits 0x%x (an offset outside the '
                             'caller\'s buffers)' % (what, v))
@@ -223,21 +300,29 @@ def check(rc, what='', err=None):
 _NP_TO_TORCH = None
 
 
+def _torch_dtype(dtype):
+    global _NP_TO_TORCH
+    if _NP_TO_TORCH is None:
+        torch = torch_mod()
+        _NP_TO_TORCH = {np.float64: torch.float64, np.int64: torch.int64, np.int32: torch.int32,
+                        np.float32: torch.float32, np.uint8: torch.uint8}
+    return _NP_TO_TORCH[dtype] if dtype in _NP_TO_TORCH else _NP_TO_TORCH[np.dtype(dtype).type]
+
+
 def to_device(a, dtype):
     """numpy array or torch tensor -> contiguous CUDA tensor of ``dtype`` (numpy dtype)."""
     torch = torch_mod()
-    tdt = {np.float64: torch.float64, np.int64: torch.int64, np.int32: torch.int32,
-           np.float32: torch.float32, np.uint8: torch.uint8}[np.dtype(dtype).type]
-    dev = device()
+    tdt = _torch_dtype(dtype)
     if isinstance(a, torch.Tensor):
         t = a
         if t.dtype != tdt:
             t = t.to(tdt)
-        if t.device != dev:
-            t = t.to(dev)
+        idx = _device_index()
+        if not t.is_cuda or t.get_device() != idx:
+            t = t.to(device())
         return t.contiguous()
     arr = np.ascontiguousarray(a, dtype=dtype)
-    return torch.from_numpy(arr).to(dev)
+    return torch.from_numpy(arr).to(device())
 
 
 def is_cuda_tensor(a):

@@ -41,8 +41,7 @@ def _pid(pid, P, E):
     elements, otherwise record e belongs to element e."""
     if pid is None:
         if P.shape[0] == 1 and E > 1:
-            torch = _lib.torch_mod()
-            return torch.zeros(E, dtype=torch.int32, device=P.device)
+            return _lib.zeros_i32(E)
         return None
     return _dev(pid, np.int32)
 
@@ -477,6 +476,8 @@ def beamc_update_M(Mr, Mc, Mv, x, cdof, init_k, vxy, props, pid=None, mtype=0, c
 # friends below are the Quad4 functions.
 
 def _per_elem(v, E, width, name):
+    if width == 1 and isinstance(v, (int, float)):
+        return _lib.scalar_f64(v), 0
     t = _dev(np.asarray(v, dtype=np.float64) if not _lib.is_cuda_tensor(v) else v, np.float64).reshape(-1)
     if t.numel() == width:
         return t.contiguous(), 0

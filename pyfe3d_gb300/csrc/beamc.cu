@@ -636,6 +636,11 @@ extern "C" int fe3d_beamc_fint(int64_t E, const int64_t *cdof, const double *R, 
 
 extern "C" int fe3d_version(void) { return 1; }
 
+extern "C" int fe3d_stream_synchronize(void *stream) {
+    FE3D_CUDA(cudaStreamSynchronize(as_stream(stream)));
+    return FE3D_OK;
+}
+
 extern "C" const char *fe3d_error_string(int code) {
     switch (code) {
         case FE3D_OK: return "ok";
