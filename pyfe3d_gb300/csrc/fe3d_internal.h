@@ -162,6 +162,14 @@ struct fe3d_solver {
     unsigned long long *sell_total = nullptr;
     int sell_on = 0;
     int sell_grid = 0;                    // blocks of the slice kernels (one wave of resident ones)
+    // row-wise update: rows of each 32-node chunk, and each row's non-zeros of
+    // the block inverses (rebuilt by every solve)
+    int32_t *chunk_row = nullptr;         // [nchunks + 1]
+    int64_t nchunks = 0;
+    int upd_grid = 0;
+    double *dval = nullptr;               // [6][n]
+    uint32_t *dinf = nullptr;             // [n]
+    int *xnz = nullptr;                   // [0] non-zero initial guess, [1] non-finite matrix value
     fe3d_team *team = nullptr;            // resident iterations (FP64, systems that fit)
     int team_tried = 0;
 };

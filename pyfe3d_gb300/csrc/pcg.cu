@@ -155,22 +155,28 @@ __global__ void __launch_bounds__(RED_BS) spmv_kernel(int64_t n, const int64_t *
 __global__ void __launch_bounds__(RED_BS) sell_count_kernel(int64_t n, const int64_t *__restrict__ rowptr,
                                                             const double *__restrict__ vals,
                                                             int32_t *__restrict__ slen, int64_t *__restrict__ soff,
-                                                            unsigned long long *total) {
+                                                            unsigned long long *total, int *nonfinite) {
     const int64_t slice = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     if (slice * 32 >= n) return;
     const int lane = threadIdx.x & 31;
     const int64_t row = slice * 32 + lane;
     const int64_t rb = rowptr[row < n ? row : n], re = rowptr[row < n ? row + 1 : n];
     unsigned longest = 0;
-    // row by row with the lanes along the entries: coalesced reads
+    bool bad = false;
+    // row by row with the lanes along the entries: coalesced reads (bits, not
+    // doubles: comparisons would take the FP64 pipe)
 #pragma unroll 4
     for (int r = 0; r < 32; r++) {
         const int64_t b = __shfl_sync(0xffffffffu, rb, r), e = __shfl_sync(0xffffffffu, re, r);
         unsigned cnt = 0;
-        for (int64_t k = b; k < e; k += 32)
-            cnt += __popc(__ballot_sync(0xffffffffu, k + lane < e && vals[k + lane < e ? k + lane : b] != 0.));
+        for (int64_t k = b; k < e; k += 32) {
+            const long long v = k + lane < e ? __double_as_longlong(vals[k + lane]) << 1 : 0;
+            bad |= (unsigned long long)v >= 0xffe0000000000000ull;
+            cnt += __popc(__ballot_sync(0xffffffffu, v != 0));
+        }
         longest = cnt > longest ? cnt : longest;
     }
+    if (bad) *nonfinite = 1;
     if (lane == 0) {
         slen[slice] = (int32_t)longest;
         soff[slice] = (int64_t)atomicAdd(total, (unsigned long long)longest);
@@ -179,6 +185,8 @@ __global__ void __launch_bounds__(RED_BS) sell_count_kernel(int64_t n, const int
 
 // Fills the slices; a row shorter than its slice repeats its last column with
 // the value 0 (a non-finite x there is met by the row's own entry as well).
+// A lane reads its row entry by entry: 0.39 ms at 501x501 nodes; rows turned in
+// shared memory for coalesced reads took 0.63 ms (a serial ballot per row).
 __global__ void __launch_bounds__(RED_BS) sell_fill_kernel(int64_t n, const int64_t *__restrict__ rowptr,
                                                            const uint16_t *__restrict__ col16,
                                                            const double *__restrict__ vals,
@@ -198,7 +206,7 @@ __global__ void __launch_bounds__(RED_BS) sell_fill_kernel(int64_t n, const int6
         const int64_t re = rowptr[row + 1];
         for (int64_t k = rowptr[row]; k < re; k++) {
             const double v = vals[k];
-            if (v != 0.) {
+            if ((__double_as_longlong(v) << 1) != 0) {
                 c = col16[k];
                 sv[32 * at] = v;
                 sc[32 * at] = c;
@@ -605,6 +613,120 @@ __global__ void __launch_bounds__(RED_BS) update_kernel(int64_t nnodes, const in
     }
 }
 
+// ---- row-wise update (FP64 recurrence, plain) -----------------------------
+// update_kernel with one thread per row: a block takes the rows of 32
+// consecutive nodes (at most UPD_BS), so every vector is read and written
+// coalesced, and of a row of the block inverse only the non-zeros are read and
+// multiplied (a flat plate's inverses couple (u, v, rz) and (w, rx, ry) only: 3
+// of 6).  84 bytes and 7 FP64 instructions per row, where a thread per node
+// made 104 bytes in 48-byte strides and 10 instructions.  501x501-node plate:
+// 62 -> 36 us.
+constexpr int UPD_NODES = 32, UPD_BS = 6 * UPD_NODES;
+
+// First row of each chunk of UPD_NODES nodes.
+__global__ void chunk_rows_kernel(int64_t nchunks, int64_t n, int bs, const int64_t *dof_of_row, int32_t *row) {
+    const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (c > nchunks) return;
+    const int64_t dof = c * UPD_NODES * bs;
+    int64_t lo = 0, hi = n;
+    while (lo < hi) {
+        const int64_t m = (lo + hi) / 2;
+        if (dof_of_row[m] < dof) lo = m + 1;
+        else hi = m;
+    }
+    row[c] = (int32_t)(c == nchunks ? n : lo);
+}
+
+// Non-zeros of each row of the block inverses: their number, their columns (3
+// bits each) and the row's place in its node (bits 21 on).
+__global__ void inverse_rows_kernel(int64_t n, const int64_t *dof_of_row, const int32_t *start, const int8_t *size,
+                                    int bs, const double *Dinv, double *dval, uint32_t *dinf) {
+    const int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (row >= n) return;
+    const int64_t node = dof_of_row[row] / bs;
+    const int i = (int)(row - start[node]), b = size[node];
+    int cnt = 0;
+    uint32_t inf = (uint32_t)i << 21;
+    for (int k = 0; k < b; k++) {
+        const double v = Dinv[36 * node + 6 * i + k];
+        if (v != 0.) {
+            dval[cnt * n + row] = v;
+            cnt++;
+            inf |= (uint32_t)k << (3 * cnt);
+        }
+    }
+    dinf[row] = inf | (uint32_t)cnt;
+}
+
+__global__ void __launch_bounds__(UPD_BS) update_rows_kernel(int64_t nchunks, int64_t n,
+                                                             const int32_t *__restrict__ chunk_row,
+                                                             const double *__restrict__ dval,
+                                                             const uint32_t *__restrict__ dinf,
+                                                             const double *alpha_in, const double *rz_cur,
+                                                             const double *__restrict__ p,
+                                                             const double *__restrict__ q, double *__restrict__ u,
+                                                             double *__restrict__ r, double *__restrict__ z,
+                                                             double *prz, double *prr, unsigned int *counter,
+                                                             double *rz_new, double *rr_out, double *beta_out) {
+    __shared__ double sh[34];
+    __shared__ double rs[2][UPD_BS];
+    const double alpha = *alpha_in;
+    double rz = 0., rr = 0.;
+    int buf = 0;
+    for (int64_t c = blockIdx.x; c < nchunks; c += gridDim.x, buf ^= 1) {
+        const int64_t row = chunk_row[c] + threadIdx.x;
+        const bool in = row < chunk_row[c + 1];
+        double ri = 0., d[6];
+        uint32_t inf = 0;
+        if (in) {
+            inf = dinf[row];
+            const double pi = p[row], qi = q[row], ui = u[row];
+            ri = r[row];
+#pragma unroll
+            for (int k = 0; k < 6; k++) d[k] = k < (int)(inf & 7u) ? dval[k * n + row] : 0.;
+            u[row] = ui + alpha * pi;
+            ri -= alpha * qi;
+            r[row] = ri;
+            rs[buf][threadIdx.x] = ri;
+        }
+        // (two buffers: a row of the next chunk is written after this barrier,
+        // one of the chunk after that only after the next)
+        __syncthreads();
+        const double *rn = rs[buf] + (in ? (int)threadIdx.x - (int)(inf >> 21) : 0);
+        const int most = __reduce_max_sync(0xffffffffu, (int)(inf & 7u));
+        double acc = 0.;
+        if (most > 3) {
+#pragma unroll
+            for (int k = 0; k < 6; k++) acc += d[k] * rn[(inf >> (3 + 3 * k)) & 7u];
+        } else {
+#pragma unroll
+            for (int k = 0; k < 3; k++) acc += d[k] * rn[(inf >> (3 + 3 * k)) & 7u];
+        }
+        if (in) {
+            z[row] = acc;
+            rz += ri * acc;
+            rr += ri * ri;
+        }
+    }
+    __syncthreads();
+    const double s1 = block_sum(rz, sh);
+    __syncthreads();
+    if (threadIdx.x == 0) prz[blockIdx.x] = s1;
+    const double s2 = block_sum(rr, sh);
+    if (threadIdx.x == 0) prr[blockIdx.x] = s2;
+    if (last_block(counter)) {
+        const double rzn = reduce_partials_l2(prz, gridDim.x, sh);
+        const double rrn = reduce_partials_l2(prr, gridDim.x, sh);
+        if (threadIdx.x == 0) {
+            const double rzc = *rz_cur;
+            *rz_new = rzn;
+            *rr_out = rrn;
+            *beta_out = rzc != 0. ? rzn / rzc : 0.;
+            *counter = 0u;
+        }
+    }
+}
+
 // K3: p = z + beta p (beta from the update kernel's last block; a restart
 // sets p = z without reading p: fresh allocations hold garbage).
 template <typename PT>
@@ -733,6 +855,27 @@ __global__ void __launch_bounds__(RED_BS) dd_residual_sell_kernel(int64_t n, con
 __global__ void combine_kernel(int64_t n, const double *xhi, const double *xlo, double *u) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         u[i] = xhi[i] + xlo[i];
+}
+
+// flag = 1 where x holds a non-zero (or NaN).
+__global__ void any_nonzero_kernel(int64_t n, const double *x, int *flag) {
+    bool any = false;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        any |= (__double_as_longlong(x[i]) << 1) != 0;
+    if (__any_sync(__activemask(), any) && (threadIdx.x & 31) == 0) *flag = 1;
+}
+
+// The residual of a zero iterate, r = f, with partial sums of r.r.
+__global__ void __launch_bounds__(RED_BS) zero_residual_kernel(int64_t n, const double *f, double *r,
+                                                               double *partial_rr) {
+    __shared__ double sh[33];
+    double rr = 0.;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        r[i] = f[i];
+        rr += f[i] * f[i];
+    }
+    const double s = block_sum(rr, sh);
+    if (threadIdx.x == 0) partial_rr[blockIdx.x] = s;
 }
 
 __global__ void finalize_sum_kernel(const double *partials, int n, double *out) {
@@ -921,6 +1064,7 @@ extern "C" int fe3d_solver_free(fe3d_solver *s) {
     cudaFree(s->prr); cudaFree(s->prf); cudaFree(s->scal); cudaFree(s->nonpos);
     cudaFree(s->vals2); cudaFree(s->p2);
     team_free(s->team);
+    cudaFree(s->chunk_row); cudaFree(s->dval); cudaFree(s->dinf); cudaFree(s->xnz);
     cudaFree(s->soff); cudaFree(s->slen); cudaFree(s->sval); cudaFree(s->scol); cudaFree(s->sell_total);
     delete s;
     return FE3D_OK;
@@ -1073,11 +1217,13 @@ int sell_plan(fe3d_solver *s, cudaStream_t st) {
     if (!s->sell_total) {
         const int res = resident_per_sm(spmv_sell_kernel, RED_BS, 0);
         s->sell_grid = grid_cap(s->n, RED_BS, kSMs * (res < 8 ? res : 8));
-        if (alloc(&s->slen, slices) || alloc(&s->soff, slices) || alloc(&s->sell_total, 1)) return FE3D_ERR_NOMEM;
+        if (alloc(&s->slen, slices) || alloc(&s->soff, slices) || alloc(&s->xnz, 2) || alloc(&s->sell_total, 1))
+            return FE3D_ERR_NOMEM;
     }
+    FE3D_CUDA(cudaMemsetAsync(s->xnz, 0, 2 * sizeof(int), st));
     FE3D_CUDA(cudaMemsetAsync(s->sell_total, 0, sizeof(unsigned long long), st));
     sell_count_kernel<<<grid_cap(slices * 32, RED_BS, 1 << 30), RED_BS, 0, st>>>(s->n, s->pat->rowptr, s->vals,
-                                                                                 s->slen, s->soff, s->sell_total);
+                                                                                 s->slen, s->soff, s->sell_total, s->xnz + 1);
     FE3D_CHECK_LAUNCH();
     return FE3D_OK;
 }
@@ -1107,8 +1253,28 @@ int sell_build(fe3d_solver *s, unsigned long long total, cudaStream_t st) {
                 s->graph[0][j] = nullptr;
             }
     }
+    if (on && !s->chunk_row) {
+        s->nchunks = (s->nnodes + UPD_NODES - 1) / UPD_NODES;
+        const int res = resident_per_sm(update_rows_kernel, UPD_BS, 0);
+        s->upd_grid = grid_cap(s->nchunks, 1, kSMs * (res < 8 ? res : 8));
+        if (alloc(&s->dval, 6 * s->n) || alloc(&s->dinf, s->n) || alloc(&s->chunk_row, s->nchunks + 1)) {
+            (void)cudaGetLastError();
+            cudaFree(s->dval);
+            cudaFree(s->dinf);
+            s->dval = nullptr;
+            s->dinf = nullptr;
+            on = 0;
+        } else {
+            chunk_rows_kernel<<<grid_cap(s->nchunks + 1, 256, 1 << 30), 256, 0, st>>>(
+                s->nchunks, s->n, s->bs, s->pat->dof_of_row, s->chunk_row);
+            FE3D_CHECK_LAUNCH();
+        }
+    }
     s->sell_on = on;
     if (!on) return FE3D_OK;
+    inverse_rows_kernel<<<grid_cap(s->n, 256, 1 << 30), 256, 0, st>>>(s->n, s->pat->dof_of_row, s->start, s->size,
+                                                                     s->bs, s->Dinv, s->dval, s->dinf);
+    FE3D_CHECK_LAUNCH();
     sell_fill_kernel<<<grid_cap((s->n + 31) / 32 * 32, RED_BS, 1 << 30), RED_BS, 0, st>>>(
         s->n, s->pat->rowptr, s->pat->col16, s->vals, s->slen, s->soff, s->sval, s->scol);
     FE3D_CHECK_LAUNCH();
@@ -1167,12 +1333,14 @@ int run_cg(fe3d_solver *s, const double *f, double *u, const fe3d_solve_opts *o,
         }
     }
     fe3d_team *team = nullptr;
+    bool zero_start = false;  // u = 0 and every value finite: the residual is f
     {
         // ||f||, and the non-zero count of the FP64 recurrence's matrix
         unsigned long long total[2] = {0, 0};
         s->sell_on = 0;
         team = resident ? s->team : nullptr;
         if (team ? (rc = team_plan(team, s, st)) : prec == 0 && (rc = sell_plan(s, st))) return rc;
+        if (!team && prec == 0 && s->xnz) any_nonzero_kernel<<<s->vec_grid, RED_BS, 0, st>>>(n, u, s->xnz);
         precond_kernel<double, double><<<s->node_grid, RED_BS, 0, st>>>(
             s->nnodes, s->start, s->size, s->Dinv, f, s->z, s->prz, s->prr, nullptr, nullptr);
         finalize_sum_kernel<<<1, RED_BS, 0, st>>>(s->prr, s->node_grid, s->scal + 4);
@@ -1181,7 +1349,11 @@ int run_cg(fe3d_solver *s, const double *f, double *u, const fe3d_solve_opts *o,
         if (team || (prec == 0 && s->sell_total))
             FE3D_CUDA(cudaMemcpyAsync(total, team ? team->total : s->sell_total, (team ? 2 : 1) * sizeof(total[0]),
                                       cudaMemcpyDeviceToHost, st));
+        int xnz[2] = {1, 0};
+        if (!team && prec == 0 && s->xnz)
+            FE3D_CUDA(cudaMemcpyAsync(xnz, s->xnz, sizeof(xnz), cudaMemcpyDeviceToHost, st));
         FE3D_CUDA(cudaStreamSynchronize(st));
+        zero_start = !xnz[0] && !xnz[1];
         // no memory for the copy: the launch-per-kernel iteration needs none
         if (team && ff != 0. && (team_build(team, s, total[0], total[1], st) || team_inverses(team, s, st)))
             team = nullptr;
@@ -1205,7 +1377,15 @@ int run_cg(fe3d_solver *s, const double *f, double *u, const fe3d_solve_opts *o,
         FE3D_CUDA(cudaMemsetAsync(u, 0, sizeof(double) * n, st));
     }
     double rr = 0.;
-    if ((rc = true_residual(s, f, u, st, &rr))) return rc;
+    if (zero_start) {
+        zero_residual_kernel<<<s->vec_grid, RED_BS, 0, st>>>(n, f, s->r, s->prr);
+        finalize_sum_kernel<<<1, RED_BS, 0, st>>>(s->prr, s->vec_grid, s->scal + 2);
+        FE3D_CHECK_LAUNCH();
+        FE3D_CUDA(cudaMemcpyAsync(&rr, s->scal + 2, sizeof(double), cudaMemcpyDeviceToHost, st));
+        FE3D_CUDA(cudaStreamSynchronize(st));
+    } else if ((rc = true_residual(s, f, u, st, &rr))) {
+        return rc;
+    }
     if (!(rr == rr)) {
         combine_kernel<<<s->vec_grid, RED_BS, 0, st>>>(n, s->xhi, s->xlo, u);
         FE3D_CHECK_LAUNCH();
@@ -1252,7 +1432,14 @@ int run_cg(fe3d_solver *s, const double *f, double *u, const fe3d_solve_opts *o,
                                                              s->scal + pr, s->scal + 3);
         else
             launch_spmv<VT, PT>(lanes, st, n, s->pat, vals_k, p, q, s->ppq, s->counter, s->scal + pr, s->scal + 3);
-        update_kernel<PT, PT><<<s->node_grid, RED_BS, 0, st>>>(s->nnodes, s->start, s->size, Dk, s->scal + 3,
+        if (s->sell_on && !prf)
+            update_rows_kernel<<<s->upd_grid, UPD_BS, 0, st>>>(s->nchunks, n, s->chunk_row, s->dval, s->dinf,
+                                                               s->scal + 3, s->scal + pr, (const double *)p,
+                                                               (const double *)q, u, s->r, (double *)z, s->prz,
+                                                               s->prr, s->counter, s->scal + (pr ^ 1), s->scal + 2,
+                                                               s->scal + 5);
+        else
+            update_kernel<PT, PT><<<s->node_grid, RED_BS, 0, st>>>(s->nnodes, s->start, s->size, Dk, s->scal + 3,
                                                                s->scal + pr, p, q, u, s->r, z, s->prz, s->prr, prf,
                                                                sck, isck, s->counter, s->scal + (pr ^ 1), s->scal + 2,
                                                                s->scal + 5);

@@ -80,3 +80,39 @@ def test_numbering_and_partial_nodes(gpulib, nodes, order):
     u2, st2 = s.solve(torch.from_numpy(f).cuda(), u0=u1, tol=1e-13, check_every=7)
     assert st2['status'] == 'converged'
     assert np.linalg.norm(u2.cpu().numpy() - ref) <= 1e-11 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize('nodes', [2731, 2752, 9001])
+@pytest.mark.parametrize('coupled', [False, True])
+def test_row_wise_update(gpulib, nodes, coupled):
+    """Launch-by-launch FP64 iterations (a system whose columns reach too far for resident blocks): chunks of nodes with
+    fixed DOFs and of whole nodes, from zero and from a given iterate."""
+    import torch
+    from scipy.sparse.linalg import spsolve
+    from pyfe3d_gb300.solver import CSRPattern, Solver
+    rng = np.random.default_rng(nodes)
+    r, c, v = _triplets(nodes, coupled, 5)
+    # a weak coupling of the first and the last node widens every window beyond shared memory when n is large
+    far = np.array([0, 6 * nodes - 6])
+    r, c, v = np.concatenate([r, far, far[::-1]]), np.concatenate([c, far, far]), np.concatenate([v, [1., 1., .1, .1]])
+    bk = rng.random(6 * nodes) < 0.15
+    bk[far] = False
+    bk[600:900] = True
+    perm = rng.permutation(nodes)
+    r, c = 6 * perm[r // 6] + r % 6, 6 * perm[c // 6] + c % 6
+    pat = CSRPattern(r, c, 6 * nodes, bk)
+    vals = pat.assemble(v)
+    s = Solver(pat).setup(vals)
+    f = rng.normal(size=pat.nrows)
+    ref = spsolve(pat.to_scipy(vals).tocsc(), f)
+    fd = torch.from_numpy(f).cuda()
+    u, st = s.solve(fd, tol=1e-13)
+    assert st['status'] == 'converged'
+    assert np.linalg.norm(u.cpu().numpy() - ref) <= 1e-11 * np.linalg.norm(ref)
+    u1, _ = s.solve(fd, tol=1e-300, maxiter=4, check_every=2)
+    u2, st2 = s.solve(fd, u0=u1, tol=1e-13)
+    assert st2['status'] == 'converged'
+    assert np.linalg.norm(u2.cpu().numpy() - ref) <= 1e-11 * np.linalg.norm(ref)
+    vals[5] = float('nan')
+    _, st3 = s.solve(fd, tol=1e-13, maxiter=100)
+    assert st3['status'] == 'non-finite'
