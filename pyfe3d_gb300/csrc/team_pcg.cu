@@ -21,23 +21,24 @@
 // the iteration's number.  A reader polls the words themselves: no fence, no
 // counter, one trip through L2 per exchange, two exchanges per iteration.  A
 // slot is written again only after every reader of its previous value has
-// sent something that the writer waited for.  Sums over blocks are taken in a
-// fixed order by each block, so all blocks hold the same scalars and the
-// result does not depend on scheduling.  Every poll is bounded; a block that
+// sent something that the writer waited for.  Each block makes the same sum over
+// blocks, so all hold the same scalars and the result does not depend on
+// scheduling.  Every poll is bounded; a block that
 // gives up raises a flag and returns.  The partial sums sit a 128-byte line
 // apart: 152 blocks exchange a value in 3.1k cycles, 5.8k with four to a line.
 //
 // Matrix: the non-zero values in slices of 32 / L rows, L lanes per row (L
 // grows as the rows per block shrink), anchored at the block's first row.  An
 // FP64 instruction holds its sub-partition's pipe for 64 cycles whatever its
-// active lanes, so reductions go through shared memory to one warp per
-// sub-partition instead of shuffles in all warps, comparisons of doubles are
-// left to one warp, and blocks of few rows keep them in registers.
+// active lanes, so sums over lanes and blocks are made with integer reductions
+// (fixed_sum), comparisons of doubles are left to one warp, and blocks of few
+// rows keep them in registers.
 //
 // Measured on clamped perturbed plates, us per iteration, three launches /
-// resident: 486 rows 20.8 / 5.9, 2,166 rows 20.8 / 6.2, 9,126 rows 22.2 / 8.2,
-// 58,806 rows 25.5 / 11.6, 237,606 rows 43 / 25, 536,406 rows 69.5 / 60 (there
-// the matrix no longer fits L2 and bounds both).
+// resident with shuffle trees / with fixed_sum: 486 rows 20.8 / 5.9 / 5.9,
+// 2,166 rows 20.8 / 6.7 / 6.2, 9,126 rows 22.2 / 8.2 / 7.6, 58,806 rows 25.5 /
+// 11.6 / 10.2, 237,606 rows 43 / 25 / 23.7, 536,406 rows 69.5 / 60 / 57 (there
+// the matrix no longer fits L2 and bounds all).
 #include <limits.h>
 
 #include <vector>
@@ -89,48 +90,84 @@ __device__ __forceinline__ bool ll_poll(const ulonglong2 *base, int i0, int step
     return all;
 }
 
-// Sum over the block of values held by its first nw warps (by the lanes that
-// are multiples of lo in a group of more than four), valid in warp 0.  red:
-// TT + 4 doubles; a block-wide barrier has to come before the next use.
-__device__ __forceinline__ double team_block_sum(double v, int nw, int lo, double *red) {
-    const int warp = threadIdx.x >> 5;
-    if (nw > 4) {
-        red[threadIdx.x] = v;
-        __syncthreads();
-        v = threadIdx.x < 128
-                ? (red[threadIdx.x] + red[threadIdx.x + 128]) + (red[threadIdx.x + 256] + red[threadIdx.x + 384]) : 0.;
-        nw = 4;
-        lo = 1;
-    }
-    if (warp < nw) {
-        for (int o = 16; o >= lo; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if ((threadIdx.x & 31) == 0) red[TT + warp] = v;
-    }
-    __syncthreads();
-    v = 0.;
-    if (warp == 0) {
-        v = red[TT];
-        for (int w = 1; w < nw; w++) v += red[TT + w];
-    }
+// Sum of N doubles a lane over the warp (all lanes get it), in fixed point
+// relative to the largest: every mantissa is shifted to 61 bits below the
+// largest exponent, split into three limbs, and the limbs are added with the
+// warp's integer reductions.  Exact but for 2^-61 of the largest term per term
+// and the final rounding, whatever the order, and free of the FP64 pipe, where
+// a tree of five additions takes 450 cycles and this 150.  Infinities, NaN and
+// sums near the denormal range are left to such a tree (plain_sum, a call, so
+// that the compiler does not predicate its additions into the common path).
+__device__ __noinline__ double plain_sum(double v) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
+}
+__device__ __noinline__ double plain_add(double a, double b) { return a + b; }
+template <int N>
+__device__ __forceinline__ double fixed_sum(const double (&v)[N]) {
+    int emax = 0;
+#pragma unroll
+    for (int j = 0; j < N; j++) emax = max(emax, (int)((unsigned)__double2hiint(v[j]) >> 20 & 0x7ffu));
+    emax = (int)__reduce_max_sync(0xffffffffu, (unsigned)emax);
+    if (emax == 0x7ff || emax < 128) {
+        double s = v[0];
+        for (int j = 1; j < N; j++) s = plain_add(s, v[j]);
+        return plain_sum(s);
+    }
+    unsigned lo = 0, mid = 0;
+    int hi = 0;
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        const long long b = __double_as_longlong(v[j]);
+        const int e = (int)(b >> 52) & 0x7ff, d = emax - e;
+        long long m = ((b & 0xfffffffffffffll) | (1ll << 52)) << 8;
+        m = e == 0 || d > 60 ? 0 : m >> d;
+        if (b < 0) m = -m;
+        lo += (unsigned)m & 0x1fffffu;
+        mid += (unsigned)(m >> 21) & 0x1fffffu;
+        hi += (int)(m >> 42);
+    }
+    lo = __reduce_add_sync(0xffffffffu, lo);
+    mid = __reduce_add_sync(0xffffffffu, mid);
+    hi = __reduce_add_sync(0xffffffffu, hi);
+    // total = T 2^21 + lo in units of 2^(emax - 1023 - 60); the top 63 bits of it
+    const long long T = ((long long)hi << 21) + mid + (lo >> 21);
+    const long long V = T * 4096 + (long long)((lo & 0x1fffffu) >> 9);  // units of 2^(emax - 1023 - 51)
+    if (V == 0) return 0.;
+    const unsigned long long a = (unsigned long long)(V < 0 ? -V : V);
+    const int lz = __clzll((long long)a);
+    unsigned long long m = a << lz;  // leading one at bit 63
+    const int e = emax - 51 + 63 - lz;  // its exponent (biased), at least 77
+    const unsigned long long r = m & 0x7ffull;
+    m >>= 11;
+    if (r > 0x400ull || (r == 0x400ull && (m & 1))) m++;  // to nearest; a carry moves into the exponent
+    const unsigned long long bits = ((unsigned long long)(e - 1) << 52) + m;
+    return __longlong_as_double((long long)(bits | (V < 0 ? 1ull << 63 : 0ull)));
+}
+
+// Sum over the block of values held by its first nw warps, valid in warp 0.
+// red: 16 doubles; a block-wide barrier has to come before the next use.
+__device__ __forceinline__ double team_block_sum(double v, int nw, double *red) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const double one[1] = {v};
+    if (warp < nw) {
+        v = fixed_sum(one);
+        if (nw == 1) return v;
+        if (lane == 0) red[warp] = v;
+    }
+    if (nw == 1) return 0.;
+    __syncthreads();
+    if (warp != 0) return 0.;
+    const double all[1] = {lane < nw ? red[lane] : 0.};
+    return fixed_sum(all);
 }
 
 constexpr int TEAM_WORDS = (TEAM_MAX + 31) / 32;
 
-// One warp: the blocks' partial sums, then their sum in a fixed order (lane 0).
+// One warp: the blocks' partial sums.
 __device__ __forceinline__ bool team_poll(const ulonglong2 *slots, int G, unsigned ep, double (&v)[TEAM_WORDS],
                                           int limit = POLL_MAX) {
     return ll_poll(slots, SLOT * (int)(threadIdx.x & 31), SLOT * 32, SLOT * G, ep, v, limit);
-}
-__device__ __forceinline__ double team_add(const double (&v)[TEAM_WORDS], int G) {
-    double s = v[0];
-#pragma unroll
-    for (int j = 1; j < TEAM_WORDS; j++)
-        if (32 * j < G) s += v[j];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        if (o < G) s += __shfl_xor_sync(0xffffffffu, s, o);
-    return s;
 }
 
 struct TeamArgs {
@@ -165,7 +202,7 @@ constexpr int team_regs(int L) { return L == 1 ? 28 : L == 2 ? 16 : 8; }
 template <int L, bool REG>
 __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
     extern __shared__ __align__(16) double sm[];
-    __shared__ double red[TT + 4];
+    __shared__ double red[TT / 32];
     __shared__ double bc[4];
     // a poll gave up; beta = 0; most non-zeros in a row of the block inverses; others finished
     __shared__ int fail, fresh, dmax, yield;
@@ -260,12 +297,12 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
                 if (L == 1 || (t & (L - 1)) == 0) dot += pw[own + i] * acc;
             }
         }
-        dot = team_block_sum(dot, nwq, L, red);
+        dot = team_block_sum(dot, nwq, red);
         if (tid < 32) {
             if (tid == 0) ll_store(slot_pq + SLOT * bid, dot, ep);
             double v[TEAM_WORDS];
             if (!team_poll(slot_pq, G, ep, v, it == 0 ? POLL_FIRST : POLL_MAX)) fail = 1;
-            const double pq = team_add(v, G);
+            const double pq = fixed_sum(v);
             if (tid == 0) bc[0] = pq != 0. ? rz / pq : 0.;
         } else if (tid >= TZ) {
             irz = fabs(rz) > 1e-290 ? 1. / rz : 0.;  // for beta, while alpha is waited for
@@ -298,11 +335,11 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
             lrz += rs[i] * acc;
             if (look) lrr += rs[i] * rs[i];
         }
-        lrz = team_block_sum(lrz, nwz, 1, red);
+        lrz = team_block_sum(lrz, nwz, red);
         if (tid == 0) ll_store(slot_rz + SLOT * bid, lrz, ep);
         if (look) {
             __syncthreads();
-            lrr = team_block_sum(lrr, nwz, 1, red);
+            lrr = team_block_sum(lrr, nwz, red);
             if (tid == 0) {
                 ll_store(slot_rr + SLOT * bid, lrr, ep);
                 // the team's first block decides for all whether others have finished
@@ -322,7 +359,7 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
         if (tid < TZ) {
             if (!ll_poll(a.z + c0, tid, TZ, W, ep, zv)) fail = 1;
         } else {
-            const double rzn = team_add(vz, G), s = look ? team_add(vr, G) : 0.;
+            const double rzn = fixed_sum(vz), s = look ? fixed_sum(vr) : 0.;
             if (tid == TZ) {
                 const double be = rz == 0. ? 0. : irz != 0. ? rzn * irz : rzn / rz;
                 bc[0] = be;

@@ -51,3 +51,18 @@ def test_teams_match_lockstep(gpulib, sizes):
     # nothing left to do
     _, s3 = teams.solve(f, u0=u2, tol=1e-9)
     assert (s3['inst_status'] == 0).all() and s3['inst_iters'].max() == 0
+
+
+@pytest.mark.parametrize('size', [(2, 3), (9, 8), (40, 31)], ids=str)
+@pytest.mark.parametrize('exponent', [-475, -240, 0, 240, 480])
+def test_loads_of_any_scale(gpulib, size, exponent):
+    """Inner products near both ends of the range of a double (their sums over lanes and blocks are made in fixed
+    point, next to those ends by plain additions): the solution scales with the load."""
+    from pyfe3d_gb300.solver import Solver
+    _, pat, vals, f = _batch([size], 3)
+    s = Solver(pat).setup(vals)
+    u, st = s.solve(f, tol=1e-10)
+    v, sv = s.solve(f * 2. ** exponent, tol=1e-10)
+    assert st['status'] == sv['status'] == 'converged' and sv['relres'] <= 1e-10
+    w = v * 2. ** -exponent
+    assert ((w - u).norm() <= 1e-7 * u.norm()).item()
