@@ -244,7 +244,8 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
         for (int k = 0; k < 6; k++) dreg[k] = k < (int)(dinf & 7) ? a.dval[k * a.n + r0 + tid] : 0.;
         if (tid < rows32) {
             mylen = a.slen[s0 + (tid >> 5)];
-            cb = tid / L < n ? a.colbase[r0 + tid / L] - c0 : 0;
+            // (a row without entries has the base 0, which the window may not hold)
+            cb = tid / L < n ? max(a.colbase[r0 + tid / L] - c0, 0) : 0;
         }
         const int64_t o = tid < rows32 ? a.soff[s0 + (tid >> 5)] * 32 + (tid & 31) : 0;
         uint32_t c = 0;
@@ -286,7 +287,7 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
                 const int64_t o = __ldg(a.soff + slice) * 32 + (t & 31);
                 const double *sv = a.sval + o;
                 const uint16_t *sc = a.scol + o;
-                const double *xb = pw + (i < n ? __ldg(a.colbase + r0 + i) - c0 : 0);
+                const double *xb = pw + (i < n ? max(__ldg(a.colbase + r0 + i) - c0, 0) : 0);
 #pragma unroll 9
                 for (int k = 0; k < len; k++) acc += __ldg(sv + 32 * k) * xb[__ldg(sc + 32 * k)];
             }

@@ -116,3 +116,26 @@ def test_row_wise_update(gpulib, nodes, coupled):
     vals[5] = float('nan')
     _, st3 = s.solve(fd, tol=1e-13, maxiter=100)
     assert st3['status'] == 'non-finite'
+
+
+@pytest.mark.parametrize('nodes', [40, 400, 5000])
+def test_rows_without_entries(gpulib, nodes):
+    """Nodes that no element meets: their rows are empty and their unloaded DOFs stay zero."""
+    import torch
+    from scipy.sparse.linalg import spsolve
+    from pyfe3d_gb300.solver import CSRPattern, Solver
+    r, c, v = _triplets(nodes, True, 3)
+    alone = np.zeros(nodes, bool)
+    alone[[nodes // 2, nodes // 2 + 1, nodes - 9, nodes - 1]] = True
+    keep = ~(alone[r // 6] | alone[c // 6])
+    pat = CSRPattern(r[keep], c[keep], 6 * nodes, None)
+    vals = pat.assemble(v[keep])
+    f = np.random.default_rng(1).normal(size=6 * nodes)
+    free = np.repeat(~alone, 6)
+    f[~free] = 0.
+    u, st = Solver(pat).setup(vals).solve(torch.from_numpy(f).cuda(), tol=1e-13, check_every=2)
+    assert st['status'] == 'converged'
+    u = u.cpu().numpy()
+    assert (u[~free] == 0.).all()
+    ref = spsolve(pat.to_scipy(vals).tocsr()[free][:, free].tocsc(), f[free])
+    assert np.linalg.norm(u[free] - ref) <= 1e-11 * np.linalg.norm(ref)  # condition number below 100
