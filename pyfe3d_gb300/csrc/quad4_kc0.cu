@@ -414,8 +414,6 @@ struct CentreH<true> {
         b[2] = o[5 + nb].f;
     }
     __device__ __forceinline__ double operator()(int p, int q) const { return ff_to_double(ff_mul(a[p], b[q])); }
-    // H0^xx + H0^yy
-    __device__ __forceinline__ double trace() const { return ff_to_double(ff_fma(a[1], b[1], ff_mul(a[2], b[2]))); }
 };
 template <>
 struct CentreH<false> {
@@ -495,13 +493,18 @@ __device__ __forceinline__ void pair_add_iso(const KElem &s, const double H[3][3
     add2<CLEAR, false, true>(st, na, nb, 5, 4, 0., H[0][0]);
     // bending and transverse shear: rows and columns w, rx, ry
     const double D11 = s.D[0], D12 = s.D[1], D66 = s.D[5], E = s.es[0];
-    const double ec = E * h0(0, 0);
-    add2<CLEAR>(st, na, nb, 2, 2, E * ((s.flags & KF_THICK) ? H[1][1] + H[2][2] : h0.trace()), -E * h0(2, 0));
+    const double c00 = h0(0, 0);
+    // The shear terms dominate and cancel in bending: each is a product rounded
+    // once into its entry.  H0^xx + H0^yy summed in float-float and E c00 rounded
+    // by itself save three instructions, and plate solutions lose 0.15 digits.
+    const bool thick = s.flags & KF_THICK;
+    const double sx = thick ? H[1][1] : h0(1, 1), sy = thick ? H[2][2] : h0(2, 2);
+    add2<CLEAR>(st, na, nb, 2, 2, E * sy + E * sx, -E * h0(2, 0));
     add2<CLEAR, true, false>(st, na, nb, 2, 4, E * h0(1, 0), 0.);
-    add2<CLEAR>(st, na, nb, 3, 2, -E * h0(0, 2), D66 * H[1][1] + (D11 * H[2][2] + ec));
+    add2<CLEAR>(st, na, nb, 3, 2, -E * h0(0, 2), D66 * H[1][1] + D11 * H[2][2] + E * c00);
     add2<CLEAR, true, false>(st, na, nb, 3, 4, -(D66 * H[1][2] + D12 * H[2][1]), 0.);
     add2<CLEAR>(st, na, nb, 4, 2, E * h0(0, 1), -(D12 * H[1][2] + D66 * H[2][1]));
-    add2<CLEAR, true, false>(st, na, nb, 4, 4, D11 * H[1][1] + (D66 * H[2][2] + ec), 0.);
+    add2<CLEAR, true, false>(st, na, nb, 4, 4, D11 * H[1][1] + D66 * H[2][2] + E * c00, 0.);
 }
 
 // Adds the general 6x6 block K_ab onto the staged values, three rows at a
