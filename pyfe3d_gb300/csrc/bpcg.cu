@@ -1179,7 +1179,7 @@ int bsolve(fe3d_bsolver *b, double *fu, double *uu, const fe3d_solve_opts *o, in
                 if ((rc = team_split(t, s, parts, st)) || (rc = team_plan(t, s, st))) break;
                 FE3D_CUDA(cudaMemcpyAsync(total, t->total, sizeof(total), cudaMemcpyDeviceToHost, st));
                 FE3D_CUDA(cudaStreamSynchronize(st));
-                if ((rc = team_build(t, s, total[0], total[1], st))) break;
+                if ((rc = team_build(t, s, total, st))) break;
                 was = parts;
             }
             std::vector<TeamSys> sys(K, TeamSys{0., 0, 0, 0, 0});

@@ -92,8 +92,9 @@ struct fe3d_team {
     size_t smem_max = 0;
     int G = 0, L = 1;                  // blocks in use, lanes per row
     int nmax = 0;                      // largest row count of a block
-    size_t smem = 0;                   // of the block that needs most
-    bool reg = false;                  // the rows fit the blocks' registers
+    size_t smem = 0;                   // of the block that needs most, without matrix entries
+    size_t smem_run = 0;               // of a launch
+    int rows = 0;                      // where the matrix rows are kept (team_pcg.cu)
     int32_t *ints = nullptr;           // the per-block arrays below
     int32_t *rbeg = nullptr, *rend = nullptr, *slice0 = nullptr, *cmin = nullptr, *cmax = nullptr;
     int32_t *tfirst = nullptr, *tcount = nullptr, *tsys = nullptr;
@@ -179,12 +180,11 @@ void team_free(fe3d_team *t);
 fe3d_team *team_create(const fe3d_solver *s, int64_t nsys, cudaStream_t st);
 size_t team_smem(int64_t rows, int64_t bw);
 int team_split(fe3d_team *t, const fe3d_solver *s, const std::vector<TeamPart> &parts, cudaStream_t st);
-// Counts the non-zeros into t->total (and the longest slice into t->total[1]);
+// Counts into t->total the entries of all slices and of the block with most;
 // team_build lays them out once the caller has read both; team_inverses takes
 // the block inverses.
 int team_plan(fe3d_team *t, const fe3d_solver *s, cudaStream_t st);
-int team_build(fe3d_team *t, const fe3d_solver *s, unsigned long long total, unsigned long long longest,
-               cudaStream_t st);
+int team_build(fe3d_team *t, const fe3d_solver *s, const unsigned long long (&total)[2], cudaStream_t st);
 int team_inverses(fe3d_team *t, const fe3d_solver *s, cudaStream_t st);
 // Iterations of every system of the split from s->r, s->p, u and rz (per
 // system), until its limits are met or the teams of enough blocks have

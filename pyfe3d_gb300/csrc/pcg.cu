@@ -1355,7 +1355,7 @@ int run_cg(fe3d_solver *s, const double *f, double *u, const fe3d_solve_opts *o,
         FE3D_CUDA(cudaStreamSynchronize(st));
         zero_start = !xnz[0] && !xnz[1];
         // no memory for the copy: the launch-per-kernel iteration needs none
-        if (team && ff != 0. && (team_build(team, s, total[0], total[1], st) || team_inverses(team, s, st)))
+        if (team && ff != 0. && (team_build(team, s, total, st) || team_inverses(team, s, st)))
             team = nullptr;
         else if (!team && prec == 0 && ff != 0. && (rc = sell_build(s, total[0], st))) return rc;
     }

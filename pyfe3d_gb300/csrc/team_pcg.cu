@@ -28,17 +28,22 @@
 // apart: 152 blocks exchange a value in 3.1k cycles, 5.8k with four to a line.
 //
 // Matrix: the non-zero values in slices of 32 / L rows, L lanes per row (L
-// grows as the rows per block shrink), anchored at the block's first row.  An
-// FP64 instruction holds its sub-partition's pipe for 64 cycles whatever its
-// active lanes, so sums over lanes and blocks are made with integer reductions
-// (fixed_sum), comparisons of doubles are left to one warp, and blocks of few
-// rows keep them in registers.
+// grows as the rows per block shrink), anchored at the block's first row and
+// copied to shared memory where they fit.  An FP64 instruction holds its
+// sub-partition's pipe for 64 cycles whatever its active lanes, so sums over
+// lanes and blocks are made with integer reductions (fixed_sum), comparisons of
+// doubles with integer operations, and rare FP64 work stands behind branches
+// and calls.  While alpha is waited for, blocks of up to a row per thread apply
+// the preconditioner to r and to q: z = Minv r - alpha Minv q then follows
+// alpha with one instruction.
 //
 // Measured on clamped perturbed plates, us per iteration, three launches /
-// resident with shuffle trees / with fixed_sum: 486 rows 20.8 / 5.9 / 5.9,
-// 2,166 rows 20.8 / 6.7 / 6.2, 9,126 rows 22.2 / 8.2 / 7.6, 58,806 rows 25.5 /
-// 11.6 / 10.2, 237,606 rows 43 / 25 / 23.7, 536,406 rows 69.5 / 60 / 57 (there
-// the matrix no longer fits L2 and bounds all).
+// resident, rows in registers and FP64 sums / now: 486 rows 20.8 / 5.9 / 4.9,
+// 2,166 rows 20.8 / 6.7 / 5.1, 9,126 rows 22.2 / 8.2 / 6.4, 58,806 rows 25.5 /
+// 11.6 / 9.5, 237,606 rows 43 / 25 / 22.6, 536,406 rows 69.5 / 60 / 44 (there the
+// matrix no longer fits L2).  At 20,886 rows a block's 12,300 cycles are: product
+// 3,300, sums over the block 2,800, waiting for p.q 1,800, for r.z and z 3,000,
+// sums over blocks and division 1,900 -- of which the FP64 pipe needs 3,900.
 #include <limits.h>
 
 #include <vector>
@@ -77,14 +82,16 @@ __device__ __forceinline__ bool ll_poll(const ulonglong2 *base, int i0, int step
         unsigned long long a[N], b[N];
 #pragma unroll
         for (int j = 0; j < N; j++) {
-            const ulonglong2 *p = base + (i0 + j * step < lim ? i0 + j * step : i0);
-            asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a[j]), "=l"(b[j]) : "l"(p) : "memory");
+            a[j] = b[j] = (unsigned long long)ep << 32;
+            if (i0 + j * step < lim)
+                asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];"
+                             : "=l"(a[j]), "=l"(b[j]) : "l"(base + i0 + j * step) : "memory");
         }
         all = true;
 #pragma unroll
         for (int j = 0; j < N; j++) {
             all &= (unsigned)(a[j] >> 32) == ep && (unsigned)(b[j] >> 32) == ep;
-            if (i0 + j * step < lim) v[j] = __hiloint2double((int)(unsigned)b[j], (int)(unsigned)a[j]);
+            v[j] = __hiloint2double((int)(unsigned)b[j], (int)(unsigned)a[j]);
         }
     }
     return all;
@@ -104,7 +111,7 @@ __device__ __noinline__ double plain_sum(double v) {
 }
 __device__ __noinline__ double plain_add(double a, double b) { return a + b; }
 template <int N>
-__device__ __forceinline__ double fixed_sum(const double (&v)[N]) {
+__device__ __forceinline__ double fixed_sum_of(const double (&v)[N]) {
     int emax = 0;
 #pragma unroll
     for (int j = 0; j < N; j++) emax = max(emax, (int)((unsigned)__double2hiint(v[j]) >> 20 & 0x7ffu));
@@ -145,24 +152,65 @@ __device__ __forceinline__ double fixed_sum(const double (&v)[N]) {
     return __longlong_as_double((long long)(bits | (V < 0 ? 1ull << 63 : 0ull)));
 }
 
+constexpr int TEAM_WORDS = (TEAM_MAX + 31) / 32;
+
+// Calls, not inlined: the iteration's code runs once per iteration in one warp
+// at a time, and the less of it there is the more stays in the instruction cache.
+__device__ __noinline__ double fixed_sum(double v) {
+    const double one[1] = {v};
+    return fixed_sum_of(one);
+}
+__device__ __noinline__ double fixed_sum(double a, double b, double c, double d, double e) {
+    const double five[5] = {a, b, c, d, e};
+    return fixed_sum_of(five);
+}
+__device__ __forceinline__ double fixed_sum(const double (&v)[TEAM_WORDS]) {
+    static_assert(TEAM_WORDS == 5, "words per lane");
+    return fixed_sum(v[0], v[1], v[2], v[3], v[4]);
+}
+
 // Sum over the block of values held by its first nw warps, valid in warp 0.
 // red: 16 doubles; a block-wide barrier has to come before the next use.
 __device__ __forceinline__ double team_block_sum(double v, int nw, double *red) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const double one[1] = {v};
     if (warp < nw) {
-        v = fixed_sum(one);
+        v = fixed_sum(v);
         if (nw == 1) return v;
         if (lane == 0) red[warp] = v;
     }
     if (nw == 1) return 0.;
     __syncthreads();
     if (warp != 0) return 0.;
-    const double all[1] = {lane < nw ? red[lane] : 0.};
-    return fixed_sum(all);
+    if (nw > 4) return fixed_sum(lane < nw ? red[lane] : 0.);
+    v = red[0];
+#pragma unroll 1
+    for (int w = 1; w < nw; w++) v += red[w];  // 64 cycles each, fixed_sum 320
+    return v;
 }
 
-constexpr int TEAM_WORDS = (TEAM_MAX + 31) / 32;
+__device__ __forceinline__ int exponent_of(double v) { return (int)((unsigned)__double2hiint(v) >> 20 & 0x7ffu); }
+__device__ __forceinline__ bool bits_zero(double v) { return (__double_as_longlong(v) << 1) == 0; }
+
+// a / b, 0 where b is 0: an approximate reciprocal (20 bits), one Newton step,
+// and the quotient by it corrected once by its residual; the division with a
+// comparison takes 830 cycles.  The ends of the range are left to the division.
+__device__ __noinline__ double plain_quotient(double a, double b) { return b != 0. ? a / b : 0.; }
+__device__ __forceinline__ double quotient(double a, double b) {
+    const int e = exponent_of(b);
+    if (e <= 64 || e >= 1984) return plain_quotient(a, b);
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    y = fma(fma(-b, y, 1.), y, y);
+    const double q = a * y, c = fma(fma(-q, b, a), y, q);
+    return exponent_of(c) < 0x7ff ? c : q;
+}
+
+// acc + d0 r[c0] + d1 r[c1] + d2 r[c2], columns 3 bits each from inf (a call,
+// so that its FP64 instructions are not predicated into the path without them).
+__device__ __noinline__ double three_more(double acc, double d0, double d1, double d2, const double *rn, uint32_t inf) {
+    return acc + d0 * rn[inf & 7] + d1 * rn[(inf >> 3) & 7] + d2 * rn[(inf >> 6) & 7];
+}
+
 
 // One warp: the blocks' partial sums.
 __device__ __forceinline__ bool team_poll(const ulonglong2 *slots, int G, unsigned ep, double (&v)[TEAM_WORDS],
@@ -196,10 +244,17 @@ struct TeamArgs {
     int enough;              // finished blocks at which the other teams stop too
 };
 
-// Entries per lane that a block of at most TT / L rows keeps in registers.
-constexpr int team_regs(int L) { return L == 1 ? 28 : L == 2 ? 16 : 8; }
+// Where a block's rows of the matrix are between two iterations, and how they
+// are read: from shared memory where they fit; else from L1 and L2 in a plain
+// loop (NEAR), or a chunk ahead of their use where all rows together exceed what
+// L2 holds next to the vectors (FAR, above kFarEntries entries of 10 bytes).  us
+// per iteration: 58,806 rows SHARED 9.5, NEAR 9.9, FAR 10.5; 84,966 rows 12.5,
+// 13.7, 14.5; 133,206 rows (too many for SHARED) NEAR 14.4, FAR 16.2; 237,606
+// rows 22.6, 24.5; 314,646 rows 30.4, 30.0; 536,406 rows 48, 44.
+enum { SHARED, NEAR, FAR };
+constexpr int64_t kFarEntries = 8400000;
 
-template <int L, bool REG>
+template <int L, int ROWS>
 __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
     extern __shared__ __align__(16) double sm[];
     __shared__ double red[TT / 32];
@@ -212,8 +267,11 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
     const int W = n > 0 ? a.cmax[blockIdx.x] - c0 + 1 : 0, s0 = a.slice0[blockIdx.x];
     const TeamSys lim = a.sys[sys];
     double *pw = sm, *rs = pw + W, *us = rs + n, *qs = us + n;
-    int *rfirst = reinterpret_cast<int *>(qs + n);  // first row of the row's node
+    const int ns = (n * L + 31) >> 5;
+    int64_t *sinf = reinterpret_cast<int64_t *>(qs + n);  // offset << 16 | length of the block's slices
+    int *rfirst = reinterpret_cast<int *>(sinf + ns);     // first row of the row's node
     uint32_t *rinf = reinterpret_cast<uint32_t *>(rfirst + n);
+    uint16_t *rbase = reinterpret_cast<uint16_t *>(rinf + n);  // window index of the row's column base
     const int own = r0 - c0;  // window index of the block's first row
     ulonglong2 *slot_pq = a.slots + SLOT * t0, *slot_rz = slot_pq + SLOT * gridDim.x,
                *slot_rr = slot_rz + SLOT * gridDim.x;
@@ -228,36 +286,72 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
         us[i] = a.u[r0 + i];
         rfirst[i] = a.start[a.dof_of_row[r0 + i] / a.bs] - r0;
         rinf[i] = a.dinf[r0 + i];
+        // (a row without entries has the base 0, which the window may not hold)
+        rbase[i] = (uint16_t)max(a.colbase[r0 + i] - c0, 0);
         atomicMax(&dmax, (int)(rinf[i] & 7));
     }
-    double rz = a.rz[sys], rr = 0., irz = 0.;
-    const int rows32 = (n * L + 31) & ~31;
-    // REG: the block's rows of the matrix and of the block inverses stay in registers
-    constexpr int MK = REG ? team_regs(L) : 4;
-    double dreg[6], vreg[MK];
-    uint32_t creg[MK / 2], dinf = 0;
-    int mylen = 0, dfirst = 0, cb = 0;
-    if (REG) {
-        dinf = tid < n ? a.dinf[r0 + tid] : 0;
-        dfirst = tid < n ? a.start[a.dof_of_row[r0 + tid] / a.bs] - r0 : 0;
-#pragma unroll
-        for (int k = 0; k < 6; k++) dreg[k] = k < (int)(dinf & 7) ? a.dval[k * a.n + r0 + tid] : 0.;
-        if (tid < rows32) {
-            mylen = a.slen[s0 + (tid >> 5)];
-            // (a row without entries has the base 0, which the window may not hold)
-            cb = tid / L < n ? max(a.colbase[r0 + tid / L] - c0, 0) : 0;
+    for (int i = tid; i < ns; i += TT) sinf[i] = a.soff[s0 + i] << 16 | a.slen[s0 + i];
+    double *mv = nullptr;      // SHARED: the block's slices, and their places in sinf
+    uint16_t *mc = nullptr;
+    if (ROWS == SHARED) {
+        const size_t base = (reinterpret_cast<char *>(rbase + n) - reinterpret_cast<char *>(sm) + 7) & ~(size_t)7;
+        mv = reinterpret_cast<double *>(reinterpret_cast<char *>(sm) + base);
+        __syncthreads();
+        int at = 0, tot = 0;
+        for (int i = 0; i < ns; i++) tot += (int)(sinf[i] & 0xffff);
+        mc = reinterpret_cast<uint16_t *>(mv + 32 * tot);
+        for (int i = 0; i < ns; i++) {
+            const int64_t si = sinf[i];
+            const int len = (int)(si & 0xffff);
+            if ((i & (TT / 32 - 1)) == tid >> 5)
+                for (int e = 0; e < len; e++) {
+                    const int64_t o = 32 * ((si >> 16) + e) + (tid & 31);
+                    mv[32 * (at + e) + (tid & 31)] = a.sval[o];
+                    mc[32 * (at + e) + (tid & 31)] = a.scol[o];
+                }
+            at += len;
         }
-        const int64_t o = tid < rows32 ? a.soff[s0 + (tid >> 5)] * 32 + (tid & 31) : 0;
-        uint32_t c = 0;
-#pragma unroll
-        for (int k = 0; k < MK; k++) {
-            vreg[k] = k < mylen ? a.sval[o + 32 * k] : 0.;
-            if (k < mylen) c = cb + a.scol[o + 32 * k];  // window index (the window has at most 28,000 columns)
-            if (k & 1) creg[k / 2] |= c << 16;
-            else creg[k / 2] = c;
+        __syncthreads();
+        if (tid == 0) {
+            at = 0;
+            for (int i = 0; i < ns; i++) {
+                const int len = (int)(sinf[i] & 0xffff);
+                sinf[i] = (int64_t)at << 16 | len;
+                at += len;
+            }
         }
     }
+    double rz = a.rz[sys], rr = 0., irz = 0.;
     __syncthreads();
+    const int rows32 = (n * L + 31) & ~31;
+    double dreg[6];
+    // the thread's first row of the block inverses
+    const bool single = n <= TT;
+    const uint32_t dinf = tid < n ? rinf[tid] : 0;
+    const int dfirst = tid < n ? rfirst[tid] : 0;
+#pragma unroll
+    for (int k = 0; k < 6; k++) dreg[k] = k < (int)(dinf & 7) ? a.dval[k * a.n + r0 + tid] : 0.;
+    __syncthreads();
+    // FAR: CH entries a lane of the warp's slice from entry k on, loaded one
+    // chunk ahead of their use (the first of an iteration at the end of the one
+    // before), past the slice's end its last entry again
+    constexpr int CH = 7;
+    double cv[CH];
+    uint16_t cc[CH];
+    auto fetch = [&](int64_t si, int k, double(&v)[CH], uint16_t(&c)[CH]) {
+        const int last = (int)(si & 0xffff) - 1;
+        if (k > last) return;
+        const double *sv = a.sval + 32 * (si >> 16) + (tid & 31);
+        const uint16_t *sc = a.scol + 32 * (si >> 16) + (tid & 31);
+#pragma unroll
+        for (int j = 0; j < CH; j++) {
+            const int e = 32 * min(k + j, last);
+            v[j] = __ldg(sv + e);
+            c[j] = __ldg(sc + e);
+        }
+    };
+    for (int j = 0; j < CH; j++) cv[j] = 0., cc[j] = 0;
+    if (ROWS == FAR && tid < rows32) fetch(sinf[tid >> 5], 0, cv, cc);
     int it = 0, left = a.chunk - lim.phase;  // iterations to the next look at convergence
     bool stop = it >= lim.maxiter;
     const bool few = dmax <= 3;
@@ -266,80 +360,159 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
         const unsigned ep = a.epoch + (unsigned)it;
         // q = K p over the block's rows, and p.q
         double dot = 0.;
-        for (int t = tid; t < rows32; t += REG ? (1 << 20) : TT) {
-            const int i = t / L;
-            double acc = 0.;
-            if (REG) {
-                // four entries at a time; those past the slice's end are zeros
+        if (ROWS == SHARED) {
+            for (int t = tid; t < rows32; t += TT) {
+                const int i = t / L, len = (int)(sinf[t >> 5] & 0xffff), o = 32 * (int)(sinf[t >> 5] >> 16) + (t & 31);
+                const double *xb = pw + (i < n ? rbase[i] : 0), *sv = mv + o;
+                const uint16_t *sc = mc + o;
+                double acc = 0.;
+#pragma unroll 7
+                for (int k = 0; k < len; k++) acc += sv[32 * k] * xb[sc[32 * k]];
 #pragma unroll
-                for (int k = 0; k < MK; k += 4)
-                    if (k < mylen) {
-                        const double x0 = pw[creg[k / 2] & 0xffff], x1 = pw[creg[k / 2] >> 16];
-                        const double x2 = pw[creg[k / 2 + 1] & 0xffff], x3 = pw[creg[k / 2 + 1] >> 16];
-                        acc += vreg[k] * x0;
-                        acc += vreg[k + 1] * x1;
-                        acc += vreg[k + 2] * x2;
-                        acc += vreg[k + 3] * x3;
-                    }
-            } else {
-                const int slice = s0 + (t >> 5);
-                const int len = __ldg(a.slen + slice);
-                const int64_t o = __ldg(a.soff + slice) * 32 + (t & 31);
-                const double *sv = a.sval + o;
+                for (int o2 = L / 2; o2 > 0; o2 >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o2);
+                if (i < n) {
+                    qs[i] = acc;
+                    if (L == 1 || (t & (L - 1)) == 0) dot += pw[own + i] * acc;
+                }
+            }
+        }
+        if (ROWS == NEAR) {
+            for (int t = tid; t < rows32; t += TT) {
+                const int i = t / L, len = (int)(sinf[t >> 5] & 0xffff);
+                const int64_t o = 32 * (sinf[t >> 5] >> 16) + (t & 31);
+                const double *xb = pw + (i < n ? rbase[i] : 0), *sv = a.sval + o;
                 const uint16_t *sc = a.scol + o;
-                const double *xb = pw + (i < n ? max(__ldg(a.colbase + r0 + i) - c0, 0) : 0);
+                double acc = 0.;
 #pragma unroll 9
                 for (int k = 0; k < len; k++) acc += __ldg(sv + 32 * k) * xb[__ldg(sc + 32 * k)];
-            }
 #pragma unroll
-            for (int o2 = L / 2; o2 > 0; o2 >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o2);
-            if (i < n) {
-                qs[i] = acc;
-                if (L == 1 || (t & (L - 1)) == 0) dot += pw[own + i] * acc;
+                for (int o2 = L / 2; o2 > 0; o2 >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o2);
+                if (i < n) {
+                    qs[i] = acc;
+                    if (L == 1 || (t & (L - 1)) == 0) dot += pw[own + i] * acc;
+                }
+            }
+        }
+        if (ROWS == FAR) {
+            int t = tid, k = 0;
+            int64_t si = t < rows32 ? sinf[t >> 5] : 0;
+            double acc = 0.;
+#pragma unroll 1
+            while (t < rows32) {
+                const int i = t / L, m = (int)(si & 0xffff) - k;
+                const double *xb = pw + (i < n ? rbase[i] : 0);
+                double nv[CH];
+                uint16_t nc[CH];
+                int64_t sn = si;
+                const bool end = m <= CH;
+                k += CH;
+                if (end) {
+                    t += TT;
+                    k = 0;
+                    if (t < rows32) sn = sinf[t >> 5];
+                }
+                if (t < rows32) fetch(sn, k, nv, nc);
+                double x[CH];
+#pragma unroll
+                for (int j = 0; j < CH; j++) x[j] = m > 0 ? xb[cc[j]] : 0.;  // an empty slice has no columns
+                // (a jump into the additions: predicated-off ones would take the FP64 pipe)
+                switch (m < CH ? m : CH) {
+                case 7: acc += cv[6] * x[6]; [[fallthrough]];
+                case 6: acc += cv[5] * x[5]; [[fallthrough]];
+                case 5: acc += cv[4] * x[4]; [[fallthrough]];
+                case 4: acc += cv[3] * x[3]; [[fallthrough]];
+                case 3: acc += cv[2] * x[2]; [[fallthrough]];
+                case 2: acc += cv[1] * x[1]; [[fallthrough]];
+                case 1: acc += cv[0] * x[0];
+                }
+                if (end) {
+#pragma unroll
+                    for (int o2 = L / 2; o2 > 0; o2 >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o2);
+                    if (i < n) {
+                        qs[i] = acc;
+                        if (L == 1 || (tid & (L - 1)) == 0) dot += pw[own + i] * acc;
+                    }
+                    acc = 0.;
+                }
+#pragma unroll
+                for (int j = 0; j < CH; j++) cv[j] = nv[j], cc[j] = nc[j];
+                si = sn;
             }
         }
         dot = team_block_sum(dot, nwq, red);
+        if (tid == 0) ll_store(slot_pq + SLOT * bid, dot, ep);
+        // a row per thread: Minv r and Minv q while alpha is waited for (z = Minv r - alpha Minv q)
+        double zr = 0., zq = 0.;
+        if (nwq == 1) __syncwarp();  // q from this warp's own lanes (a barrier came otherwise)
+        if (single && tid < n) {
+            const double *rn = rs + dfirst, *qn = qs + dfirst;
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                const int c = (dinf >> (3 + 3 * k)) & 7;
+                zr += dreg[k] * rn[c];
+                zq += dreg[k] * qn[c];
+            }
+            if (!few) {
+                zr = three_more(zr, dreg[3], dreg[4], dreg[5], rn, dinf >> 12);
+                zq = three_more(zq, dreg[3], dreg[4], dreg[5], qn, dinf >> 12);
+            }
+        }
         if (tid < 32) {
-            if (tid == 0) ll_store(slot_pq + SLOT * bid, dot, ep);
             double v[TEAM_WORDS];
             if (!team_poll(slot_pq, G, ep, v, it == 0 ? POLL_FIRST : POLL_MAX)) fail = 1;
             const double pq = fixed_sum(v);
-            if (tid == 0) bc[0] = pq != 0. ? rz / pq : 0.;
+            if (tid == 0) bc[0] = quotient(rz, pq);
         } else if (tid >= TZ) {
-            irz = fabs(rz) > 1e-290 ? 1. / rz : 0.;  // for beta, while alpha is waited for
+            irz = exponent_of(rz) > 64 && exponent_of(rz) < 1984 ? 1. / rz : 0.;  // for beta
         }
         __syncthreads();
+        // z = Minv r, r.z
         const double alpha = bc[0];
-        for (int i = tid; i < n; i += REG ? (1 << 20) : TT) rs[i] -= alpha * qs[i];
-        __syncthreads();
-        // z = Minv r, r.z (and r.r where convergence is looked at)
-        it++;
-        const bool look = --left == 0 || it >= lim.maxiter;
-        if (left == 0) left = a.chunk;
-        double lrz = 0., lrr = 0.;
-        for (int i = tid; i < n; i += REG ? (1 << 20) : TT) {
-            const uint32_t inf = REG ? dinf : rinf[i];
-            const double *rn = rs + (REG ? dfirst : rfirst[i]);
-            double acc = 0.;
-            if (REG) {
-#pragma unroll
-                for (int k = 0; k < 3; k++) acc += dreg[k] * rn[(inf >> (3 + 3 * k)) & 7];
-                if (!few) {
-#pragma unroll
-                    for (int k = 3; k < 6; k++) acc += dreg[k] * rn[(inf >> (3 + 3 * k)) & 7];
-                }
-            } else {
-                const int cnt = inf & 7;
-                for (int k = 0; k < cnt; k++) acc += __ldg(a.dval + k * a.n + r0 + i) * rn[(inf >> (3 + 3 * k)) & 7];
+        double lrz = 0.;
+        if (single) {
+            if (tid < n) {
+                const double rv = rs[tid] - alpha * qs[tid];
+                zr -= alpha * zq;
+                ll_store(a.z + r0 + tid, zr, ep);
+                lrz = rv * zr;
+                rs[tid] = rv;
             }
-            ll_store(a.z + r0 + i, acc, ep);
-            lrz += rs[i] * acc;
-            if (look) lrr += rs[i] * rs[i];
+        } else {
+            for (int i = tid; i < n; i += TT) rs[i] -= alpha * qs[i];
+            __syncthreads();
+            // the first three entries of a row of the block inverses are asked for a row ahead
+            double d[3] = {dreg[0], dreg[1], dreg[2]};
+            uint32_t inf = dinf;
+#pragma unroll 1
+            for (int i = tid; i < n; i += TT) {
+                const uint32_t ninf = i + TT < n ? rinf[i + TT] : 0;
+                double nd[3];
+#pragma unroll
+                for (int k = 0; k < 3; k++)
+                    nd[k] = k < (int)(ninf & 7) ? __ldg(a.dval + k * a.n + r0 + i + TT) : 0.;
+                const double *rn = rs + rfirst[i];
+                double acc = 0.;
+#pragma unroll
+                for (int k = 0; k < 3; k++) acc += d[k] * rn[(inf >> (3 + 3 * k)) & 7];
+#pragma unroll 1
+                for (int k = 3; k < (int)(inf & 7); k++)
+                    acc += __ldg(a.dval + k * a.n + r0 + i) * rn[(inf >> (3 + 3 * k)) & 7];
+                ll_store(a.z + r0 + i, acc, ep);
+                lrz += rs[i] * acc;
+#pragma unroll
+                for (int k = 0; k < 3; k++) d[k] = nd[k];
+                inf = ninf;
+            }
         }
         lrz = team_block_sum(lrz, nwz, red);
         if (tid == 0) ll_store(slot_rz + SLOT * bid, lrz, ep);
+        it++;
+        const bool look = --left == 0 || it >= lim.maxiter;
+        if (left == 0) left = a.chunk;
         if (look) {
             __syncthreads();
+            double lrr = 0.;
+            for (int i = tid; i < n; i += TT) lrr += rs[i] * rs[i];
             lrr = team_block_sum(lrr, nwz, red);
             if (tid == 0) {
                 ll_store(slot_rr + SLOT * bid, lrr, ep);
@@ -347,47 +520,54 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
                 if (bid == 0) ll_store(slot_rr + 1, *(volatile int *)a.done >= a.enough ? 1. : 0., ep);
             }
         }
-        for (int i = tid; i < n; i += REG ? (1 << 20) : TT) us[i] += alpha * pw[own + i];
-        // p = z + beta p over the window.  The words of z are asked for once
-        // r.z has come from every block: polling them earlier would crowd the
-        // lines that their owners are about to write
-        double zv[4], vz[TEAM_WORDS], vr[TEAM_WORDS], vy[1];
-        if (tid >= TZ) {
-            if (!team_poll(slot_rz, G, ep, vz)) fail = 1;
-            if (look && !(team_poll(slot_rr, G, ep, vr) && ll_poll(slot_rr + 1, 0, 1, 1, ep, vy))) fail = 1;
-        }
-        __syncthreads();
+        for (int i = tid; i < n; i += TT) us[i] += alpha * pw[own + i];
+        // p = z + beta p over the window
+        constexpr int ZW = ROWS == FAR ? 4 : 6;  // words a thread asks for at a time
+        double zv[ZW];
         if (tid < TZ) {
             if (!ll_poll(a.z + c0, tid, TZ, W, ep, zv)) fail = 1;
         } else {
-            const double rzn = fixed_sum(vz), s = look ? fixed_sum(vr) : 0.;
+            double vz[TEAM_WORDS], vr[TEAM_WORDS], vy[1];
+            if (!team_poll(slot_rz, G, ep, vz)) fail = 1;
+            if (look && !(team_poll(slot_rr, G, ep, vr) && ll_poll(slot_rr + 1, 0, 1, 1, ep, vy))) fail = 1;
+            const double rzn = fixed_sum(vz);
+            double s = 0.;
+            if (look) s = fixed_sum(vr);
             if (tid == TZ) {
-                const double be = rz == 0. ? 0. : irz != 0. ? rzn * irz : rzn / rz;
-                bc[0] = be;
-                fresh = be == 0.;
-                bc[1] = rzn;
-                bc[2] = s;
+                const double be = bits_zero(irz) ? plain_quotient(rzn, rz) : rzn * irz;
+                bc[1] = be;
+                fresh = bits_zero(be);
+                bc[2] = rzn;
+                bc[3] = s;
                 if (look) yield = vy[0] != 0.;
             }
         }
         __syncthreads();
         // (comparisons of doubles run on the FP64 pipe too: one warp makes them)
-        const double beta = bc[0];
+        const double beta = bc[1];
         const bool reset = fresh;
-        rz = bc[1];
-        if (look) rr = bc[2];
-        if (tid < TZ && tid < W) {
+        rz = bc[2];
+        if (look) rr = bc[3];
+        if (W <= TZ) {
+            if (tid < W) pw[tid] = reset ? zv[0] : zv[0] + beta * pw[tid];
+        } else if (W <= 2 * TZ) {
+            // (a path of its own: predicated-off FP64 instructions take the pipe too)
+            if (tid < TZ) pw[tid] = reset ? zv[0] : zv[0] + beta * pw[tid];
+            if (tid + TZ < W && tid < TZ) pw[tid + TZ] = reset ? zv[1] : zv[1] + beta * pw[tid + TZ];
+        } else if (tid < TZ) {
             for (int c1 = tid;;) {
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
+                for (int j = 0; j < ZW; j++) {
                     const int c = c1 + j * TZ;
+                    if (c1 - tid + j * TZ >= W) break;  // (for the whole block: a branch, not predicates)
                     if (c < W) pw[c] = reset ? zv[j] : zv[j] + beta * pw[c];
                 }
-                c1 += 4 * TZ;
+                c1 += ZW * TZ;
                 if (c1 >= W) break;
                 if (!ll_poll(a.z + c0, c1, TZ, W, ep, zv)) fail = 1;
             }
         }
+        if (ROWS == FAR && tid < rows32) fetch(sinf[tid >> 5], 0, cv, cc);
         __syncthreads();
         stop = fail || it >= lim.maxiter || (look && (yield || !(rr > lim.stop2 && rr <= 1.7e308)));
     }
@@ -473,6 +653,9 @@ __global__ void __launch_bounds__(256) team_count_kernel(const int32_t *rbeg, co
                                                          int64_t *soff, unsigned long long *total) {
     const int a = rbeg[blockIdx.x], e = rend[blockIdx.x], s0 = slice0[blockIdx.x], s1 = slice0[blockIdx.x + 1];
     const int lane = threadIdx.x & 31, per = 32 / L;
+    __shared__ int all;
+    if (threadIdx.x == 0) all = 0;
+    __syncthreads();
     for (int s = s0 + (threadIdx.x >> 5); s < s1; s += blockDim.x >> 5) {
         int longest = 0;
         for (int j = 0; j < per; j++) {
@@ -487,9 +670,11 @@ __global__ void __launch_bounds__(256) team_count_kernel(const int32_t *rbeg, co
         if (lane == 0) {
             slen[s] = longest;
             soff[s] = (int64_t)atomicAdd(total, (unsigned long long)longest);
-            atomicMax(total + 1, (unsigned long long)longest);
+            atomicAdd(&all, longest);
         }
     }
+    __syncthreads();
+    if (threadIdx.x == 0) atomicMax(total + 1, (unsigned long long)all);
 }
 
 // Entry k of a row goes to lane k % L of its L lanes; lanes that end early
@@ -531,13 +716,14 @@ __global__ void __launch_bounds__(256) team_fill_kernel(const int32_t *rbeg, con
 
 typedef void (*TeamKernel)(TeamArgs);
 
-TeamKernel team_kernel(int L, bool reg) {
-    switch (L) {
-        case 1: return reg ? team_pcg_kernel<1, true> : team_pcg_kernel<1, false>;
-        case 2: return reg ? team_pcg_kernel<2, true> : team_pcg_kernel<2, false>;
-        case 4: return reg ? team_pcg_kernel<4, true> : team_pcg_kernel<4, false>;
-        default: return reg ? team_pcg_kernel<8, true> : team_pcg_kernel<8, false>;
-    }
+template <int L>
+TeamKernel team_kernel(int rows) {
+    return rows == SHARED ? team_pcg_kernel<L, SHARED> : rows == NEAR ? team_pcg_kernel<L, NEAR>
+                                                                      : team_pcg_kernel<L, FAR>;
+}
+TeamKernel team_kernel(int L, int rows) {
+    return L == 1 ? team_kernel<1>(rows) : L == 2 ? team_kernel<2>(rows) : L == 4 ? team_kernel<4>(rows)
+                                                                                 : team_kernel<8>(rows);
 }
 
 template <typename T>
@@ -583,11 +769,11 @@ fe3d_team *team_create(const fe3d_solver *s, int64_t nsys, cudaStream_t st) {
               cudaMemsetAsync(t->z, 0, sizeof(ulonglong2) * s->n, st) == cudaSuccess &&
               cudaMemsetAsync(t->slots, 0, sizeof(ulonglong2) * slots, st) == cudaSuccess;
     for (int L = 1; ok && L <= 8; L *= 2)
-        for (int reg = 0; ok && reg < 2; reg++) {
+        for (int rows = SHARED; ok && rows <= FAR; rows++) {
             int res = 0;
-            ok = cudaFuncSetAttribute(team_kernel(L, reg), cudaFuncAttributeMaxDynamicSharedMemorySize,
+            ok = cudaFuncSetAttribute(team_kernel(L, rows), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)t->smem_max) == cudaSuccess &&
-                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res, team_kernel(L, reg), TT, t->smem_max) ==
+                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res, team_kernel(L, rows), TT, t->smem_max) ==
                      cudaSuccess &&
                  res >= 1;
         }
@@ -601,7 +787,9 @@ fe3d_team *team_create(const fe3d_solver *s, int64_t nsys, cudaStream_t st) {
 
 // Shared memory of a block of rows rows whose columns reach bw rows further on
 // either side.
-size_t team_smem(int64_t rows, int64_t bw) { return sizeof(double) * (size_t)(4 * rows + 2 * bw) + 8 * (size_t)rows; }
+size_t team_smem(int64_t rows, int64_t bw) {
+    return sizeof(double) * (size_t)(4 * rows + 2 * bw + rows / 4 + 1) + 10 * (size_t)rows;
+}
 
 // Deals the systems out: part i on parts[i].blocks blocks.  Returns 0, or
 // FE3D_ERR_TOO_LARGE where a block's rows do not fit shared memory.
@@ -639,15 +827,11 @@ int team_split(fe3d_team *t, const fe3d_solver *s, const std::vector<TeamPart> &
     FE3D_CUDA(cudaMemcpyAsync(&h[5 * S], t->rbeg, sizeof(int32_t) * 4 * S, cudaMemcpyDeviceToHost, st));
     FE3D_CUDA(cudaStreamSynchronize(st));
     t->nmax = 0;
-    t->smem = 0;
     for (int b = 0; b < B; b++) {
-        const int n = h[6 * S + b] - h[5 * S + b], w = n > 0 ? h[8 * S + b] - h[7 * S + b] + 1 : 0;
+        const int n = h[6 * S + b] - h[5 * S + b];
         if (n < 0) return FE3D_ERR_ARG;
         if (n > t->nmax) t->nmax = n;
-        const size_t need = sizeof(double) * ((size_t)w + 3 * (size_t)n) + 2 * sizeof(int) * (size_t)n;
-        if (need > t->smem) t->smem = need;
     }
-    if (t->smem > t->smem_max) return FE3D_ERR_TOO_LARGE;
     // lanes per row: the fewest FP64 instructions on one sub-partition's warps
     // for a row of 27 non-zeros (a node of a flat plate's inside)
     int best = 1 << 30;
@@ -663,6 +847,14 @@ int team_split(fe3d_team *t, const fe3d_solver *s, const std::vector<TeamPart> &
             t->L = L;
         }
     }
+    t->smem = 0;
+    for (int b = 0; b < B; b++) {
+        const size_t n = h[6 * S + b] - h[5 * S + b], w = n > 0 ? h[8 * S + b] - h[7 * S + b] + 1 : 0;
+        const size_t need = sizeof(double) * (w + 3 * n + (n * t->L + 31) / 32) +
+                            (2 * sizeof(int) + sizeof(uint16_t)) * n;
+        if (need > t->smem) t->smem = need;
+    }
+    if (t->smem > t->smem_max) return FE3D_ERR_TOO_LARGE;
     const int per = 32 / t->L;
     int32_t *slice0 = &h[9 * S];
     slice0[0] = 0;
@@ -692,10 +884,11 @@ int team_plan(fe3d_team *t, const fe3d_solver *s, cudaStream_t st) {
     return FE3D_OK;
 }
 
-int team_build(fe3d_team *t, const fe3d_solver *s, unsigned long long total, unsigned long long longest,
-               cudaStream_t st) {
-    t->reg = t->nmax * t->L <= TT && (int64_t)longest <= team_regs(t->L);
-    const int64_t entries = 32 * (int64_t)total;
+int team_build(fe3d_team *t, const fe3d_solver *s, const unsigned long long (&total)[2], cudaStream_t st) {
+    const size_t shared = ((t->smem + 7) & ~(size_t)7) + 32 * (sizeof(double) + sizeof(uint16_t)) * (size_t)total[1];
+    const int64_t entries = 32 * (int64_t)total[0];
+    t->rows = shared <= t->smem_max ? SHARED : entries <= kFarEntries ? NEAR : FAR;
+    t->smem_run = t->rows == SHARED ? shared : t->smem;
     if (entries > t->cap) {
         cudaFree(t->sval);
         cudaFree(t->scol);
@@ -738,8 +931,8 @@ int team_run(fe3d_team *t, const fe3d_solver *s, double *u, double *rz, double *
                s->p, s->n, rz, rr, t->sys, t->z, t->slots, t->epoch, chunk, t->done, enough};
     t->epoch += (unsigned)most + 1u;
     void *args[] = {&a};
-    if (cudaLaunchCooperativeKernel((const void *)team_kernel(t->L, t->reg), dim3(t->G), dim3(TT), args, t->smem,
-                                    st) != cudaSuccess)
+    if (cudaLaunchCooperativeKernel((const void *)team_kernel(t->L, t->rows), dim3(t->G), dim3(TT), args,
+                                    t->smem_run, st) != cudaSuccess)
         return FE3D_ERR_LAUNCH;
     int done[2] = {0, 0};
     FE3D_CUDA(cudaMemcpyAsync(sys.data(), t->sys, sizeof(TeamSys) * sys.size(), cudaMemcpyDeviceToHost, st));

@@ -66,3 +66,15 @@ def test_loads_of_any_scale(gpulib, size, exponent):
     assert st['status'] == sv['status'] == 'converged' and sv['relres'] <= 1e-10
     w = v * 2. ** -exponent
     assert ((w - u).norm() <= 1e-7 * u.norm()).item()
+
+
+@pytest.mark.parametrize('size', [(3, 2), (21, 20), (75, 74), (126, 125), (133, 131), (244, 240)], ids=str)
+def test_rows_in_shared_memory_and_streamed(gpulib, size):
+    """Blocks that keep their rows in shared memory (up to and above a row per thread), read them from L2 and load
+    them ahead: the recurrence's residual is confirmed by the compensated residual f - K u, which is evaluated by
+    other kernels (a wrong product would part the two)."""
+    from pyfe3d_gb300.solver import Solver
+    _, pat, vals, f = _batch([size], 5)
+    s = Solver(pat).setup(vals)
+    _, st = s.solve(f, tol=1e-8)
+    assert st['status'] == 'converged' and st['relres'] <= 1e-8
