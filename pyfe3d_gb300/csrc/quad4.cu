@@ -79,16 +79,26 @@ __global__ void quad4_probe_xe_kernel(int64_t E, const int64_t *cdof, const doub
 // Phase A: one warp forms the frame, ue and the material-frame A and B of
 // the tile's 32 elements; phase A2: warp g evaluates Gauss point g (the
 // in-plane stress resultants and the vectors detJ Nmat grad N_a) of all 32;
-// phase B: one lane per node pair forms the 3x3 translational block
-// r_m3 r_n3 G_ab of the row-major 12x12 layout, and the warp adds it onto
-// the caller's values, which cp.async has copied to shared memory while the
-// blocks were formed.  Elements flat in the global x-y plane have
-// r13 = r23 = 0: only their 16 (w, w) values change.
+// phase B: G_ab = G_ba of the 10 node pairs, a lane per element and a pair per
+// warp pass; then the 3x3 translational block r_m3 r_n3 G_ab of the row-major
+// 12x12 layout is added onto the caller's values.  Elements flat in the global
+// x-y plane have r13 = r23 = 0: only their 16 (w, w) values change, which are
+// read into registers before phase A2 and, where all are zeros, stored instead
+// of added to; the other elements' values come through shared memory.
+//
+// Bound by the chain through its phases (90,000 flat isotropic elements with
+// indices: phase A 36 us, A2 25, B 28, write-out 46, of 139; the bytes take 41).
+// So phase A's indices are loaded a tile ahead and all that they point to is
+// asked for at once, five CTAs share an SM, and what takes the FP64 pipe (64
+// cycles a warp instruction) is left out: comparisons of doubles, 6 of the 16
+// pairs, additions onto zeros, a zero A16 and A26.  139 -> 120 us.
 constexpr int KG_ROW = 13;
 constexpr int KG_FLATZ = 8;  // element flag: flat with normal along global z
 constexpr int KG_FF = 16;    // element flag: Jacobian and derivatives in float-float
 constexpr int KG_NOB = 32;   // element flag: B = 0, the resultants need no curvatures
-struct __align__(16) KGElemS {
+constexpr int KG_A16 = 64;   // element flag: A16, A26 or B not zero
+// (79 doubles, odd: lanes reading one field of 32 elements hit distinct banks)
+struct KGElemS {
     double rr[9];      // r_m3 r_n3 (translational block pattern)
     double g[4][16];   // per Gauss point: Nx[4], Ny[4], then per node a the
                        // vector detJ Nmat grad N_a (x and y components)
@@ -150,22 +160,15 @@ __device__ __forceinline__ void kg_point_ff(const ff *xyf, const ff (*sh)[2][4],
     }
 }
 
-// The caller's 144 values of the two elements (el0, el0 + 1) of a warp's
-// round, copied into shared memory ahead of the block computation so that
-// the += does not wait on one global load per slot.
+// The caller's 144 values of those of the two elements (el0, el0 + 1) of a
+// warp's round that are not flat in z, copied into shared memory ahead of the
+// block computation so that the += does not wait on one global load per slot.
 __device__ __forceinline__ void kg_prefetch(const Q4Args &a, const KGElemS *se, double (*old)[144], int el0,
                                             int lane) {
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         const KGElemS &t = se[el0 + h];
-        if (!(t.flags & F_VALID)) continue;
-        if (t.flags & KG_FLATZ) {
-            if (lane < 16) {
-                const int i = (3 * (lane >> 2) + 2) * 12 + 3 * (lane & 3) + 2;
-                cp_async8(&old[h][i], a.Kv + t.init_k + i);
-            }
-            continue;
-        }
+        if (!(t.flags & F_VALID) || (t.flags & KG_FLATZ)) continue;
         for (int i = lane; i < 144; i += 32) cp_async8(&old[h][i], a.Kv + t.init_k + i);
     }
     cp_async_commit();
@@ -193,30 +196,49 @@ __device__ __forceinline__ void kg_point_vectors(double *o, double nxx, double n
 // the material direction.  Returns false (nothing written) otherwise.
 __device__ __forceinline__ bool kg_setup_global(const Q4Args &a, const long long *c, int64_t p, const double *u,
                                                 KGElemS &s, KGScratch &q) {
-    const double *p0 = a.x + c[0] / 2, *p1 = a.x + c[1] / 2, *p2 = a.x + c[2] / 2, *p3 = a.x + c[3] / 2;
-    if (p2[2] != p0[2] || p1[2] != p3[2]) return false;
-    const double cz = (p1[0] - p3[0]) * (p2[1] - p0[1]) - (p1[1] - p3[1]) * (p2[0] - p0[0]);
+    // every value is asked for before the first test: one trip to memory, not four
+    double X[4], Y[4], Z[4], U[4], V[4], A[6], B[6];
     const double *P = a.props + (int64_t)SP_STRIDE * p;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const double *q0 = a.x + c[i] / 2;
+        X[i] = q0[0];
+        Y[i] = q0[1];
+        Z[i] = q0[2];
+        U[i] = u[c[i]];
+        V[i] = u[c[i] + 1];
+    }
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+        A[i] = P[SP_A11 + i];
+        B[i] = P[SP_B11 + i];
+    }
+    if (!is_eq(Z[2], Z[0]) || !is_eq(Z[1], Z[3])) return false;
+    const double cz = (X[1] - X[3]) * (Y[2] - Y[0]) - (Y[1] - Y[3]) * (X[2] - X[0]);
     const double eps = 64. * 2.220446049250313e-16;
-    bool g = cz > 0. && P[SP_A16] == 0. && P[SP_A26] == 0. && P[SP_A11] == P[SP_A22] &&
-             fabs(P[SP_A66] - 0.5 * (P[SP_A11] - P[SP_A12])) <= eps * fabs(P[SP_A11]);
-    for (int i = 0; i < 6; i++) g &= P[SP_B11 + i] == 0.;
+    // (|x| <= y of non-negative doubles compares their bits)
+    // (A packed as 11 12 16 22 26 66)
+    bool g = is_pos(cz) && is_zero(A[2]) && is_zero(A[4]) && is_eq(A[0], A[3]) &&
+             dbits(fabs(A[5] - 0.5 * (A[0] - A[1]))) <= dbits(eps * fabs(A[0]));
+#pragma unroll
+    for (int i = 0; i < 6; i++) g &= is_zero(B[i]);
     if (!g) return false;
-    const double *pp[4] = {p0, p1, p2, p3};
     bool ffok = true;
     double d[8];
+#pragma unroll
     for (int i = 0; i < 4; i++) {
-        q.xy[2 * i] = pp[i][0];
-        q.xy[2 * i + 1] = pp[i][1];
-        d[2 * i] = pp[i][0] - p0[0];
-        d[2 * i + 1] = pp[i][1] - p0[1];
+        q.xy[2 * i] = X[i];
+        q.xy[2 * i + 1] = Y[i];
+        d[2 * i] = X[i] - X[0];
+        d[2 * i + 1] = Y[i] - Y[0];
         ffok &= ff_safe(d[2 * i]) && ff_safe(d[2 * i + 1]);
-        q.ue[6 * i] = u[c[i]];
-        q.ue[6 * i + 1] = u[c[i] + 1];
+        q.ue[6 * i] = U[i];
+        q.ue[6 * i + 1] = V[i];
     }
     if (ffok)
         for (int i = 0; i < 8; i++) q.xyf[i] = ff_from_double(d[i]);
-    for (int i = 0; i < 6; i++) q.ab[i] = P[SP_A11 + i];
+#pragma unroll
+    for (int i = 0; i < 6; i++) q.ab[i] = A[i];
     for (int i = 0; i < 9; i++) s.rr[i] = i == 8 ? 1. : 0.;
     s.flags = F_VALID | KG_FLATZ | KG_NOB | (ffok ? KG_FF : 0);
     return true;
@@ -246,7 +268,7 @@ __device__ __forceinline__ void kg_write_indices(const Q4Args &a, const KGElemS 
 // With nstress (update_KG_given_stress, quad4.pyx:2259-3081): the stress
 // resultants are the given constants (Nxx, Nyy, Nxy) of the element
 // (nstress + ns_stride e) at every Gauss point instead of those of ue.
-__global__ void __launch_bounds__(NT, 4) quad4_kg_kernel(Q4Args a, const double *u, int64_t nu,
+__global__ void __launch_bounds__(NT, 5) quad4_kg_kernel(Q4Args a, const double *u, int64_t nu,
                                                       const double *ue_in, const double *nstress,
                                                       int ns_stride) {
     __shared__ KGElemS se[TILE];
@@ -254,10 +276,13 @@ __global__ void __launch_bounds__(NT, 4) quad4_kg_kernel(Q4Args a, const double 
     // values of each warp's round reuse its memory (static total under 48 KB)
     __shared__ union {
         KGScratch sq[TILE];
-        double oldv[NT / 32][2][144];
+        struct {
+            double oldv[NT / 32][2][144];
+            double gs[TILE][17];  // G_ab, times r_33^2 for elements flat in z
+        } b;
     } su;
     KGScratch *sq = su.sq;
-    double(*oldv)[2][144] = su.oldv;
+    double(*oldv)[2][144] = su.b.oldv, (*gs)[17] = su.b.gs;
     __shared__ double stage[NT / 32][2][12 * KG_ROW];
     // dN/dxi and dN/deta of the 4 nodes at the 4 Gauss points, float-float
     __shared__ ff shf[4][2][4];
@@ -270,6 +295,16 @@ __global__ void __launch_bounds__(NT, 4) quad4_kg_kernel(Q4Args a, const double 
         shf[g][d][i] = ff_from_double(d == 0 ? 0.25 * sx * (1 + sy * eta) : 0.25 * sy * (1 + sx * xi));
     }
     const int64_t ntiles = (a.E + TILE - 1) / TILE;
+    // phase A's indices are loaded a tile ahead
+    long long nc[4] = {0, 0, 0, 0}, nk0 = 0, np = 0;
+    auto ask = [&](int64_t e) {
+        if (tid >= TILE || e >= a.E) return;
+#pragma unroll
+        for (int i = 0; i < 4; i++) nc[i] = a.cdof[4 * e + i];
+        nk0 = a.init_k[e];
+        np = a.pid ? (long long)a.pid[e] : e;
+    };
+    ask((int64_t)blockIdx.x * TILE + tid);
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int64_t e0 = tile * TILE;
         __syncthreads();
@@ -278,19 +313,18 @@ __global__ void __launch_bounds__(NT, 4) quad4_kg_kernel(Q4Args a, const double 
             s.flags = 0;
             const int64_t e = e0 + tid;
             if (e < a.E) {
-                long long c[4];
+                const long long c[4] = {nc[0], nc[1], nc[2], nc[3]}, k0 = nk0;
+                const int64_t p = np;
+                ask(e + (int64_t)gridDim.x * TILE);
                 bool ok = true;
                 for (int i = 0; i < 4; i++) {
-                    c[i] = a.cdof[4 * e + i];
                     s.c[i] = c[i];
                     if (c[i] < 0) ok = false;
                     if (a.x && c[i] / 2 + 3 > a.nx) ok = false;
                     if (a.x && !nstress && c[i] + 6 > nu) ok = false;
                 }
-                const long long k0 = a.init_k[e];
                 s.init_k = k0;
                 if (k0 < 0 || k0 + 144 > a.nk) ok = false;
-                const int64_t p = a.pid ? (int64_t)a.pid[e] : e;
                 if (!nstress && (p < 0 || p >= a.nprops)) ok = false;
                 if (!ok) {
                     raise_error(a.err, kErrBounds);
@@ -340,7 +374,7 @@ __global__ void __launch_bounds__(NT, 4) quad4_kg_kernel(Q4Args a, const double 
                         }
                         for (int mm = 0; mm < 3; mm++)
                             for (int nn = 0; nn < 3; nn++) s.rr[3 * mm + nn] = R[3 * mm + 2] * R[3 * nn + 2];
-                        bool nob = false;
+                        bool nob = false, a16 = true;
                         if (nstress) {
                             const double *ns = nstress + (int64_t)ns_stride * e;
                             q.ab[0] = ns[0];
@@ -358,17 +392,28 @@ __global__ void __launch_bounds__(NT, 4) quad4_kg_kernel(Q4Args a, const double 
                                 rotate_plane(m[0], m[1], m[2], m[3], P + SP_B11, q.ab + 6);
                             }
                             nob = true;
-                            for (int i = 0; i < 6; i++) nob &= q.ab[6 + i] == 0.;
+                            for (int i = 0; i < 6; i++) nob &= is_zero(q.ab[6 + i]);
+                            a16 = !(nob && is_zero(q.ab[2]) && is_zero(q.ab[4]));
                         }
                         // flat in the global x-y plane: r13 = r23 = 0, so r_m3 r_n3 is
                         // zero but for (w, w) and 128 of the 144 entries are zeros
                         s.flags = F_VALID | ((R[2] == 0. && R[5] == 0.) ? KG_FLATZ : 0) | (ffok ? KG_FF : 0) |
-                                  (nob ? KG_NOB : 0);
+                                  (nob ? KG_NOB : 0) | (a16 ? KG_A16 : 0);
                     }
                 }
             }
         }
         __syncthreads();
+        // the (w, w) values of the flat elements that this lane will write
+        const int half = lane >> 4, pair = lane & 15, na = pair >> 2, nb = pair & 3;
+        const int ww = (3 * na + 2) * 12 + 3 * nb + 2;
+        double old[TILE / 8];
+#pragma unroll
+        for (int r = 0; r < TILE / 8; r++) {
+            const KGElemS &t = se[r * 8 + warp * 2 + half];
+            const bool mine = (t.flags & (F_VALID | KG_FLATZ)) == (F_VALID | KG_FLATZ);
+            old[r] = mine ? a.Kv[t.init_k + ww] : 0.;
+        }
         // phase A2: warp g evaluates Gauss point g of the tile's 32 elements
         // (full warps; the four points run on the four sub-partitions)
         for (int w = tid; w < TILE * 4; w += NT) {
@@ -401,75 +446,87 @@ __global__ void __launch_bounds__(NT, 4) quad4_kg_kernel(Q4Args a, const double 
                     s.g[g][i] = Nx[i];
                     s.g[g][4 + i] = Ny[i];
                 }
-                double nxx = A[0] * exx + A[1] * eyy + A[2] * gxy;
-                double nyy = A[1] * exx + A[3] * eyy + A[4] * gxy;
-                double nxy = A[2] * exx + A[4] * eyy + A[5] * gxy;
-                if (!(s.flags & KG_NOB)) {
-                    double kxx = 0, kyy = 0, kxy = 0;
-                    for (int i = 0; i < 4; i++) {
-                        const double *ui = q.ue + 6 * i;
-                        kxx += Nx[i] * ui[4];
-                        kyy -= Ny[i] * ui[3];
-                        kxy += Ny[i] * ui[4] - Nx[i] * ui[3];
+                double nxx = A[0] * exx + A[1] * eyy;
+                double nyy = A[1] * exx + A[3] * eyy;
+                double nxy = A[5] * gxy;
+                if (s.flags & KG_A16) {
+                    nxx += A[2] * gxy;
+                    nyy += A[4] * gxy;
+                    nxy = A[2] * exx + A[4] * eyy + A[5] * gxy;
+                    if (!(s.flags & KG_NOB)) {
+                        double kxx = 0, kyy = 0, kxy = 0;
+                        for (int i = 0; i < 4; i++) {
+                            const double *ui = q.ue + 6 * i;
+                            kxx += Nx[i] * ui[4];
+                            kyy -= Ny[i] * ui[3];
+                            kxy += Ny[i] * ui[4] - Nx[i] * ui[3];
+                        }
+                        nxx = nxx + B[0] * kxx + B[1] * kyy + B[2] * kxy;
+                        nyy = nyy + B[1] * kxx + B[3] * kyy + B[4] * kxy;
+                        nxy = nxy + B[2] * kxx + B[4] * kyy + B[5] * kxy;
                     }
-                    nxx = nxx + B[0] * kxx + B[1] * kyy + B[2] * kxy;
-                    nyy = nyy + B[1] * kxx + B[3] * kyy + B[4] * kxy;
-                    nxy = nxy + B[2] * kxx + B[4] * kyy + B[5] * kxy;
                 }
                 kg_point_vectors(s.g[g], detJ * nxx, detJ * nyy, detJ * nxy);
             }
         }
         __syncthreads();
-        const int half = lane >> 4, pair = lane & 15, na = pair >> 2, nb = pair & 3;
-        for (int round = 0; round < TILE / 8; round++) {
-            kg_prefetch(a, se, oldv[warp], round * 8 + warp * 2, lane);
-            const int el = round * 8 + warp * 2 + half;
+        // phase B: the pair of pass w / 32 (the warps that make three passes
+        // change places with the tiles, each stays on its sub-partition)
+        const int shift = 64 * (int)((tile / gridDim.x + blockIdx.x / kSMs) & 1);
+        for (int w = (tid + shift) % NT; w < 10 * TILE; w += NT) {
+            const int el = w & (TILE - 1), k = w / TILE;
+            const int pa = k < 4 ? 0 : k < 7 ? 1 : k < 9 ? 2 : 3, pb = k < 4 ? k : k < 7 ? k - 3 : k < 9 ? k - 5 : 3;
             const KGElemS &s = se[el];
-            if (s.flags & F_VALID) {
-                double G = 0.;
+            if (!(s.flags & F_VALID)) continue;
+            double G = 0.;
 #pragma unroll
-                for (int g = 0; g < 4; g++) {
-                    const double *o = s.g[g];
-                    G += o[nb] * o[8 + 2 * na] + o[4 + nb] * o[9 + 2 * na];
-                }
-                double *st = stage[warp][half];
-                if (s.flags & KG_FLATZ) {
-                    st[(3 * na + 2) * KG_ROW + 3 * nb + 2] = s.rr[8] * G;
-                } else {
+            for (int g = 0; g < 4; g++) {
+                const double *o = s.g[g];
+                G += o[pb] * o[8 + 2 * pa] + o[4 + pb] * o[9 + 2 * pa];
+            }
+            if (s.flags & KG_FLATZ) G *= s.rr[8];
+            gs[el][4 * pa + pb] = G;
+            gs[el][4 * pb + pa] = G;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int round = 0; round < TILE / 8; round++) {
+            const int el0 = round * 8 + warp * 2, el = el0 + half;
+            const KGElemS &s = se[el];
+            const bool mine = (s.flags & (F_VALID | KG_FLATZ)) == (F_VALID | KG_FLATZ);
+            const double G = gs[el][pair];
+            // other values of flat elements stay as they are (+= 0)
+            if (__all_sync(0xffffffffu, !mine || is_zero(old[round]))) {
+                if (mine) a.Kv[s.init_k + ww] = G;
+            } else if (mine) {
+                a.Kv[s.init_k + ww] = old[round] + G;
+            }
+            if (__any_sync(0xffffffffu, (s.flags & F_VALID) && !mine)) {
+                kg_prefetch(a, se, oldv[warp], el0, lane);
+                if ((s.flags & F_VALID) && !mine) {
+                    double *st = stage[warp][half];
 #pragma unroll
                     for (int mm = 0; mm < 3; mm++)
 #pragma unroll
                         for (int nn = 0; nn < 3; nn++)
                             st[(3 * na + mm) * KG_ROW + 3 * nb + nn] = s.rr[3 * mm + nn] * G;
                 }
+                cp_async_wait_all();
+                __syncwarp();
             }
-            cp_async_wait_all();
-            __syncwarp();
-#pragma unroll
+#pragma unroll 1
             for (int h = 0; h < 2; h++) {
-                const KGElemS &t = se[round * 8 + warp * 2 + h];
+                const KGElemS &t = se[el0 + h];
                 if (!(t.flags & F_VALID)) continue;
                 const long long k0 = t.init_k;
-                const double *st = stage[warp][h];
-                if (t.flags & KG_FLATZ) {
-                    // the 16 (w, w) values on lanes 0..15 (one FP64 addition per
-                    // warp); the other values stay as they are (+= 0), and all
-                    // 144 indices are written
-                    if (lane < 16) {
-                        const int i = (3 * (lane >> 2) + 2) * 12 + 3 * (lane & 3) + 2;
-                        a.Kv[k0 + i] = oldv[warp][h][i] + st[(i / 12) * KG_ROW + i % 12];
-                    }
-                    if (a.Kr) kg_write_indices(a, t, k0, lane);
-                    continue;
-                }
-                for (int i = lane; i < 144; i += 32) {
-                    const int row = i / 12, col = i - row * 12;
-                    a.Kv[k0 + i] = oldv[warp][h][i] + st[row * KG_ROW + col];
-                    if (a.Kr) {
-                        a.Kr[k0 + i] = t.c[row / 3] + row % 3;
-                        a.Kc[k0 + i] = t.c[col / 3] + col % 3;
+                if (!(t.flags & KG_FLATZ)) {
+                    const double *st = stage[warp][h];
+                    for (int i = lane; i < 144; i += 32) {
+                        const int row = i / 12, col = i - row * 12;
+                        a.Kv[k0 + i] = oldv[warp][h][i] + st[row * KG_ROW + col];
                     }
                 }
+                if (a.Kr) kg_write_indices(a, t, k0, lane);
             }
             __syncwarp();
         }
@@ -849,7 +906,7 @@ extern "C" int fe3d_quad4_kg(int64_t E, const int64_t *cdof, const int64_t *init
     Q4Args a{E, cdof, init_k, x, nx, xmat, xmat_stride, R, m, xe, nullptr, props, nprops, pid,
              Kr, Kc, Kv, nk, 0, err};
     a.vec16 = Kr && ((uintptr_t)Kr & 15u) == 0 && ((uintptr_t)Kc & 15u) == 0;
-    quad4_kg_kernel<<<grid_for(E, 4), NT, 0, as_stream(stream)>>>(a, u, nu, ue, nullptr, 0);
+    quad4_kg_kernel<<<grid_for(E, 5), NT, 0, as_stream(stream)>>>(a, u, nu, ue, nullptr, 0);
     FE3D_CHECK_LAUNCH();
     return FE3D_OK;
 }
@@ -869,7 +926,7 @@ extern "C" int fe3d_quad4_kg_given_stress(int64_t E, const int64_t *cdof, const 
     Q4Args a{E, cdof, init_k, x, nx, xmat, xmat_stride, R, nullptr, xe, nullptr, nullptr, 0, nullptr,
              Kr, Kc, Kv, nk, 0, err};
     a.vec16 = Kr && ((uintptr_t)Kr & 15u) == 0 && ((uintptr_t)Kc & 15u) == 0;
-    quad4_kg_kernel<<<grid_for(E, 4), NT, 0, as_stream(stream)>>>(a, nullptr, 0, nullptr, nstress,
+    quad4_kg_kernel<<<grid_for(E, 5), NT, 0, as_stream(stream)>>>(a, nullptr, 0, nullptr, nstress,
                                                                   nstress_stride);
     FE3D_CHECK_LAUNCH();
     return FE3D_OK;
