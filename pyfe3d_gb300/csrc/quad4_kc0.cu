@@ -30,9 +30,9 @@
 // and write out, four elements each per tile, with one barrier per tile.  (With
 // phase A on a warp of the same tile the others waited for it: 20,000 of a
 // tile's 70,000 cycles.)  1,000,000 flat isotropic elements with indices onto
-// cleared values 3.56 -> 3.09 ms, 0.88 of the 2.95 ms that reading and writing
-// the values and writing the indices take with the same stores and no element
-// work; DRAM at 5.8 TB/s.  90,000 elements into CSR 0.73 -> 0.50 ms, 28,800
+// cleared values 3.56 -> 3.06 ms, against 2.95 ms for reading and writing the
+// values and writing the indices with the same stores and no element work; DRAM
+// at 6.0 TB/s.  90,000 elements into CSR 0.73 -> 0.50 ms, 28,800
 // laminated elements of a cylinder 0.42 -> 0.38 ms.
 //
 // Flat elements whose normal is +Z (r13 = r23 = r31 = r32 = 0) are evaluated
