@@ -67,7 +67,7 @@ struct fe3d_fmap {
 // Resident PCG (team_pcg.cu): the split of one or more systems over co-resident
 // blocks, the slice layout of the non-zero values and the exchange words.
 // Rows per block wanted while blocks are left: 16 rather than 64 at 2,166 rows
-// takes 6.2 instead of 8.0 us per iteration (fewer FP64 instructions per block
+// took 6.2 instead of 8.0 us per iteration (fewer FP64 instructions per block
 // against a slower exchange).
 constexpr int kTeamRows = 16;
 constexpr int64_t kTeamIters = 4096;   // iterations of one resident launch at most (a quarter of a second)

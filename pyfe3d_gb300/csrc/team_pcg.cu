@@ -33,16 +33,14 @@
 // sub-partition's pipe for 64 cycles whatever its active lanes, so sums over
 // lanes and blocks are made with integer reductions (fixed_sum), comparisons of
 // doubles with integer operations, and rare FP64 work stands behind branches
-// and calls.  While alpha is waited for, blocks of up to a row per thread apply
-// the preconditioner to r and to q: z = Minv r - alpha Minv q then follows
-// alpha with one instruction.
+// and calls.
 //
 // Measured on clamped perturbed plates, us per iteration, three launches /
-// resident, rows in registers and FP64 sums / now: 486 rows 20.8 / 5.9 / 4.9,
-// 2,166 rows 20.8 / 6.7 / 5.1, 9,126 rows 22.2 / 8.2 / 6.4, 58,806 rows 25.5 /
-// 11.6 / 9.5, 237,606 rows 43 / 25 / 22.6, 536,406 rows 69.5 / 60 / 44 (there the
-// matrix no longer fits L2).  At 20,886 rows a block's 12,300 cycles are: product
-// 3,300, sums over the block 2,800, waiting for p.q 1,800, for r.z and z 3,000,
+// resident, rows in registers and FP64 sums / now: 486 rows 20.8 / 5.9 / 5.9,
+// 2,166 rows 20.8 / 6.7 / 5.6, 9,126 rows 22.2 / 8.2 / 6.6, 58,806 rows 25.5 /
+// 11.6 / 9.6, 237,606 rows 43 / 25 / 22.4, 536,406 rows 69.5 / 60 / 44 (there the
+// matrix no longer fits L2).  At 20,886 rows a block's 12,700 cycles are: product
+// 3,300, sums over the block 2,800, waiting for p.q 1,800, for r.z and z 3,000, z 400,
 // sums over blocks and division 1,900 -- of which the FP64 pipe needs 3,900.
 #include <limits.h>
 
@@ -205,13 +203,6 @@ __device__ __forceinline__ double quotient(double a, double b) {
     return exponent_of(c) < 0x7ff ? c : q;
 }
 
-// acc + d0 r[c0] + d1 r[c1] + d2 r[c2], columns 3 bits each from inf (a call,
-// so that its FP64 instructions are not predicated into the path without them).
-__device__ __noinline__ double three_more(double acc, double d0, double d1, double d2, const double *rn, uint32_t inf) {
-    return acc + d0 * rn[inf & 7] + d1 * rn[(inf >> 3) & 7] + d2 * rn[(inf >> 6) & 7];
-}
-
-
 // One warp: the blocks' partial sums.
 __device__ __forceinline__ bool team_poll(const ulonglong2 *slots, int G, unsigned ep, double (&v)[TEAM_WORDS],
                                           int limit = POLL_MAX) {
@@ -259,8 +250,8 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
     extern __shared__ __align__(16) double sm[];
     __shared__ double red[TT / 32];
     __shared__ double bc[4];
-    // a poll gave up; beta = 0; most non-zeros in a row of the block inverses; others finished
-    __shared__ int fail, fresh, dmax, yield;
+    // a poll gave up; beta = 0; others finished
+    __shared__ int fail, fresh, yield;
     const int tid = threadIdx.x, G = a.tcount[blockIdx.x], t0 = a.tfirst[blockIdx.x], bid = blockIdx.x - t0;
     const int sys = a.tsys[blockIdx.x];
     const int r0 = a.rbeg[blockIdx.x], n = a.rend[blockIdx.x] - r0, c0 = a.cmin[blockIdx.x];
@@ -275,10 +266,7 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
     const int own = r0 - c0;  // window index of the block's first row
     ulonglong2 *slot_pq = a.slots + SLOT * t0, *slot_rz = slot_pq + SLOT * gridDim.x,
                *slot_rr = slot_rz + SLOT * gridDim.x;
-    if (tid == 0) {
-        fail = 0;
-        dmax = 0;
-    }
+    if (tid == 0) fail = 0;
     __syncthreads();
     for (int c = tid; c < W; c += TT) pw[c] = a.p[c0 + c];
     for (int i = tid; i < n; i += TT) {
@@ -288,7 +276,6 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
         rinf[i] = a.dinf[r0 + i];
         // (a row without entries has the base 0, which the window may not hold)
         rbase[i] = (uint16_t)max(a.colbase[r0 + i] - c0, 0);
-        atomicMax(&dmax, (int)(rinf[i] & 7));
     }
     for (int i = tid; i < ns; i += TT) sinf[i] = a.soff[s0 + i] << 16 | a.slen[s0 + i];
     double *mv = nullptr;      // SHARED: the block's slices, and their places in sinf
@@ -324,13 +311,11 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
     double rz = a.rz[sys], rr = 0., irz = 0.;
     __syncthreads();
     const int rows32 = (n * L + 31) & ~31;
-    double dreg[6];
-    // the thread's first row of the block inverses
-    const bool single = n <= TT;
+    double dreg[3];
+    // the first entries of the thread's first row of the block inverses
     const uint32_t dinf = tid < n ? rinf[tid] : 0;
-    const int dfirst = tid < n ? rfirst[tid] : 0;
 #pragma unroll
-    for (int k = 0; k < 6; k++) dreg[k] = k < (int)(dinf & 7) ? a.dval[k * a.n + r0 + tid] : 0.;
+    for (int k = 0; k < 3; k++) dreg[k] = k < (int)(dinf & 7) ? a.dval[k * a.n + r0 + tid] : 0.;
     __syncthreads();
     // FAR: CH entries a lane of the warp's slice from entry k on, loaded one
     // chunk ahead of their use (the first of an iteration at the end of the one
@@ -354,7 +339,6 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
     if (ROWS == FAR && tid < rows32) fetch(sinf[tid >> 5], 0, cv, cc);
     int it = 0, left = a.chunk - lim.phase;  // iterations to the next look at convergence
     bool stop = it >= lim.maxiter;
-    const bool few = dmax <= 3;
     const int nwq = max(1, min(rows32, TT) >> 5), nwz = max(1, (min(n, TT) + 31) >> 5);
     while (!stop) {
         const unsigned ep = a.epoch + (unsigned)it;
@@ -440,24 +424,11 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
             }
         }
         dot = team_block_sum(dot, nwq, red);
-        if (tid == 0) ll_store(slot_pq + SLOT * bid, dot, ep);
-        // a row per thread: Minv r and Minv q while alpha is waited for (z = Minv r - alpha Minv q)
-        double zr = 0., zq = 0.;
-        if (nwq == 1) __syncwarp();  // q from this warp's own lanes (a barrier came otherwise)
-        if (single && tid < n) {
-            const double *rn = rs + dfirst, *qn = qs + dfirst;
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                const int c = (dinf >> (3 + 3 * k)) & 7;
-                zr += dreg[k] * rn[c];
-                zq += dreg[k] * qn[c];
-            }
-            if (!few) {
-                zr = three_more(zr, dreg[3], dreg[4], dreg[5], rn, dinf >> 12);
-                zq = three_more(zq, dreg[3], dreg[4], dreg[5], qn, dinf >> 12);
-            }
-        }
         if (tid < 32) {
+            // (the word leaves before the warp's other lanes start to poll, which
+            // they otherwise may do first: 0.4 us per iteration)
+            if (tid == 0) ll_store(slot_pq + SLOT * bid, dot, ep);
+            __syncwarp();
             double v[TEAM_WORDS];
             if (!team_poll(slot_pq, G, ep, v, it == 0 ? POLL_FIRST : POLL_MAX)) fail = 1;
             const double pq = fixed_sum(v);
@@ -469,43 +440,37 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
         // z = Minv r, r.z
         const double alpha = bc[0];
         double lrz = 0.;
-        if (single) {
-            if (tid < n) {
-                const double rv = rs[tid] - alpha * qs[tid];
-                zr -= alpha * zq;
-                ll_store(a.z + r0 + tid, zr, ep);
-                lrz = rv * zr;
-                rs[tid] = rv;
-            }
-        } else {
-            for (int i = tid; i < n; i += TT) rs[i] -= alpha * qs[i];
-            __syncthreads();
-            // the first three entries of a row of the block inverses are asked for a row ahead
-            double d[3] = {dreg[0], dreg[1], dreg[2]};
-            uint32_t inf = dinf;
+        // (z from the new r, not as Minv r - alpha Minv q made while alpha is waited
+        // for: 0.4 us less, but where r drops by orders of magnitude in one
+        // iteration, as with one node or uncoupled ones, that z has no correct digit)
+        for (int i = tid; i < n; i += TT) rs[i] -= alpha * qs[i];
+        __syncthreads();
+        // the first three entries of a row of the block inverses are asked for a row ahead
+        double d[3] = {dreg[0], dreg[1], dreg[2]};
+        uint32_t inf = dinf;
 #pragma unroll 1
-            for (int i = tid; i < n; i += TT) {
-                const uint32_t ninf = i + TT < n ? rinf[i + TT] : 0;
-                double nd[3];
+        for (int i = tid; i < n; i += TT) {
+            const uint32_t ninf = i + TT < n ? rinf[i + TT] : 0;
+            double nd[3];
 #pragma unroll
-                for (int k = 0; k < 3; k++)
-                    nd[k] = k < (int)(ninf & 7) ? __ldg(a.dval + k * a.n + r0 + i + TT) : 0.;
-                const double *rn = rs + rfirst[i];
-                double acc = 0.;
+            for (int k = 0; k < 3; k++)
+                nd[k] = k < (int)(ninf & 7) ? __ldg(a.dval + k * a.n + r0 + i + TT) : 0.;
+            const double *rn = rs + rfirst[i];
+            double acc = 0.;
 #pragma unroll
-                for (int k = 0; k < 3; k++) acc += d[k] * rn[(inf >> (3 + 3 * k)) & 7];
+            for (int k = 0; k < 3; k++) acc += d[k] * rn[(inf >> (3 + 3 * k)) & 7];
 #pragma unroll 1
-                for (int k = 3; k < (int)(inf & 7); k++)
-                    acc += __ldg(a.dval + k * a.n + r0 + i) * rn[(inf >> (3 + 3 * k)) & 7];
-                ll_store(a.z + r0 + i, acc, ep);
-                lrz += rs[i] * acc;
+            for (int k = 3; k < (int)(inf & 7); k++)
+                acc += __ldg(a.dval + k * a.n + r0 + i) * rn[(inf >> (3 + 3 * k)) & 7];
+            ll_store(a.z + r0 + i, acc, ep);
+            lrz += rs[i] * acc;
 #pragma unroll
-                for (int k = 0; k < 3; k++) d[k] = nd[k];
-                inf = ninf;
-            }
+            for (int k = 0; k < 3; k++) d[k] = nd[k];
+            inf = ninf;
         }
         lrz = team_block_sum(lrz, nwz, red);
         if (tid == 0) ll_store(slot_rz + SLOT * bid, lrz, ep);
+        __syncwarp();
         it++;
         const bool look = --left == 0 || it >= lim.maxiter;
         if (left == 0) left = a.chunk;

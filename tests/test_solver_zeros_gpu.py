@@ -139,3 +139,21 @@ def test_rows_without_entries(gpulib, nodes):
     assert (u[~free] == 0.).all()
     ref = spsolve(pat.to_scipy(vals).tocsr()[free][:, free].tocsc(), f[free])
     assert np.linalg.norm(u[free] - ref) <= 1e-11 * np.linalg.norm(ref)  # condition number below 100
+
+
+@pytest.mark.parametrize('nodes', [1, 2, 40, 700])
+@pytest.mark.parametrize('exponent', [-300, 0, 300])
+def test_residual_that_drops_at_once(gpulib, nodes, exponent):
+    """Uncoupled nodes: the preconditioner is the inverse, the first iteration leaves rounding and the others of the
+    check interval run on it."""
+    import torch
+    from pyfe3d_gb300.solver import CSRPattern, Solver
+    r, c, v = _triplets(nodes, True, 3)
+    keep = r // 6 == c // 6
+    pat = CSRPattern(r[keep], c[keep], 6 * nodes, None)
+    vals = pat.assemble(v[keep])
+    f = torch.from_numpy(np.random.default_rng(1).normal(size=6 * nodes)).cuda() * 2. ** exponent
+    for check in (2, 50, 1000):
+        u, st = Solver(pat).setup(vals).solve(f, tol=1e-12, check_every=check)
+        assert st['status'] == 'converged' and st['relres'] <= 1e-12
+        assert torch.isfinite(u).all()
