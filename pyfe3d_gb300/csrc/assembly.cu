@@ -119,10 +119,13 @@ __global__ void widen_kernel(int64_t n, const int32_t *a, int64_t *b) {
 
 // ---- runs of entries ----------------------------------------------------
 // A run is entries s, s + 1, .. of one row and one node's columns whose
-// segments are as long and whose slots are each one further.  Record: {first
+// segments are as long and whose slots are each one further.  It ends with the
+// node, whichever of the node's DOFs are free, so it has at most RUN_MAX entries,
+// which is what the lanes of a run write.  Record: {first
 // entry, length | slots per entry << 8, 0, first place in perm}, {its first
 // four slots}.
 constexpr int RUN_SLOTS = 4;
+constexpr int RUN_MAX = 6, RUN_LANES = RUN_MAX / 2;
 
 // flag[s] = 1 where entry s does not continue the run of entry s - 1 (rows:
 // run_rows_kernel).
@@ -133,7 +136,8 @@ __global__ void run_flags_kernel(int64_t nnz, const int32_t *seg, const int32_t 
     bool head = s == 0;
     if (!head) {
         const int32_t b = seg[s], e = seg[s + 1], a = seg[s - 1];
-        head = e - b != b - a || colind[s] != colind[s - 1] + 1 || dof_of_row[colind[s]] % 6 == 0;
+        head = e - b != b - a || colind[s] != colind[s - 1] + 1 ||
+               dof_of_row[colind[s]] / RUN_MAX != dof_of_row[colind[s - 1]] / RUN_MAX;
         for (int32_t t = 0; !head && t < e - b; t++) head = perm[b + t] != perm[a + t] + 1;
     }
     flag[s] = head;
@@ -208,8 +212,8 @@ __global__ void __launch_bounds__(256) assemble_runs_kernel(int64_t nruns, const
                                                             const int32_t *__restrict__ perm,
                                                             const double *__restrict__ Kv, double *__restrict__ vals,
                                                             int vec16) {
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, r = t / 3;
-    const int j = 2 * (int)(t - 3 * r);
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, r = t / RUN_LANES;
+    const int j = 2 * (int)(t - RUN_LANES * r);
     int4 h = make_int4(0, 0, 0, 0), q = h;
     if (r < nruns) {
         h = __ldg(runs + 2 * r);
@@ -511,7 +515,7 @@ extern "C" int fe3d_assemble(const fe3d_pattern *p, const double *Kv, double *va
     if (p->nnz > 0 && !p->perm) return FE3D_ERR_STATE;  // pattern built from elements: no COO slots
     if (p->nnz == 0) return FE3D_OK;
     if (p->nruns) {
-        assemble_runs_kernel<<<nblk(3 * p->nruns), 256, 0, as_stream(stream)>>>(p->nruns, p->runs, p->perm, Kv, vals,
+        assemble_runs_kernel<<<nblk(RUN_LANES * p->nruns), 256, 0, as_stream(stream)>>>(p->nruns, p->runs, p->perm, Kv, vals,
                                                                                ((uintptr_t)Kv & 15u) == 0);
         FE3D_CHECK_LAUNCH();
         return FE3D_OK;
