@@ -121,9 +121,8 @@ __global__ void widen_kernel(int64_t n, const int32_t *a, int64_t *b) {
 // A run is entries s, s + 1, .. of one row and one node's columns whose
 // segments are as long and whose slots are each one further.  It ends with the
 // node, whichever of the node's DOFs are free, so it has at most RUN_MAX entries,
-// which is what the lanes of a run write.  Record: {first
-// entry, length | slots per entry << 8, 0, first place in perm}, {its first
-// four slots}.
+// which is what the lanes of a run write.  Record: {first entry, length, slots
+// per entry, first place in perm}, {its first four slots}.
 constexpr int RUN_SLOTS = 4;
 constexpr int RUN_MAX = 6, RUN_LANES = RUN_MAX / 2;
 
@@ -155,7 +154,7 @@ __global__ void run_fill_kernel(int64_t nnz, const int32_t *flag, const int32_t 
     const int32_t b = seg[s], k = seg[s + 1] - b;
     int32_t q[RUN_SLOTS];
     for (int t = 0; t < RUN_SLOTS; t++) q[t] = t < k ? perm[b + t] : 0;
-    runs[2 * (int64_t)scan[s]] = make_int4((int)s, k << 8, 0, b);
+    runs[2 * (int64_t)scan[s]] = make_int4((int)s, 0, k, b);
     runs[2 * (int64_t)scan[s] + 1] = make_int4(q[0], q[1], q[2], q[3]);
 }
 
@@ -163,7 +162,7 @@ __global__ void run_lengths_kernel(int64_t nruns, int64_t nnz, int4 *runs) {
     const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (r >= nruns) return;
     const int next = r + 1 < nruns ? runs[2 * (r + 1)].x : (int)nnz;
-    runs[2 * r].y |= next - runs[2 * r].x;
+    runs[2 * r].y = next - runs[2 * r].x;
 }
 
 // Sorts every RUN_CHUNK runs by their slots per entry (4 and more, 3, 2, 1;
@@ -181,7 +180,7 @@ __global__ void __launch_bounds__(RUN_CHUNK) run_sort_kernel(int64_t nruns, int4
         h = runs[2 * r];
         q = runs[2 * r + 1];
     }
-    const int k = h.y >> 8, cls = !in ? -1 : k >= 4 ? 0 : 4 - k;
+    const int k = h.z, cls = !in ? -1 : k >= 4 ? 0 : 4 - k;
     int below = 0;
     for (int c = 0; c < 4; c++) {
         const unsigned m = __ballot_sync(0xffffffffu, cls == c);
@@ -219,7 +218,7 @@ __global__ void __launch_bounds__(256) assemble_runs_kernel(int64_t nruns, const
         h = __ldg(runs + 2 * r);
         q = __ldg(runs + 2 * r + 1);
     }
-    const int len = h.y & 0xff, k = h.y >> 8;
+    const int len = h.y, k = h.z;
     const bool in = j < len, two = j + 1 < len;
     // one path per warp, its loads in flight together
     const int most = __reduce_max_sync(0xffffffffu, in ? k : 0);

@@ -87,3 +87,15 @@ def test_entries_of_a_sparse_matrix(gpulib, n, density):
     _check(A.row.astype(np.int64), A.col.astype(np.int64), n, None)
     bk = np.random.default_rng(2).random(n) < 0.5
     _check(A.row.astype(np.int64), A.col.astype(np.int64), n, bk)
+
+
+def test_many_slots_per_entry(gpulib):
+    """A run of two entries with 2^23 slots each."""
+    import torch
+    from pyfe3d_gb300.solver import CSRPattern
+    n = 1 << 24
+    c = torch.arange(n, device='cuda') & 1
+    pat = CSRPattern(torch.zeros_like(c), c, 6, None)
+    out = torch.full((2,), float('nan'), dtype=torch.float64, device='cuda')
+    pat.assemble(torch.ones(n, dtype=torch.float64, device='cuda'), out=out)
+    assert out.tolist() == [n / 2, n / 2]
