@@ -48,6 +48,7 @@
 
 #include "common.cuh"
 #include "fe3d_internal.h"
+#include "fixed_sum.h"
 
 namespace fe3d {
 namespace {
@@ -96,13 +97,11 @@ __device__ __forceinline__ bool ll_poll(const ulonglong2 *base, int i0, int step
 }
 
 // Sum of N doubles a lane over the warp (all lanes get it), in fixed point
-// relative to the largest: every mantissa is shifted to 61 bits below the
-// largest exponent, split into three limbs, and the limbs are added with the
-// warp's integer reductions.  Exact but for 2^-61 of the largest term per term
-// and the final rounding, whatever the order, and free of the FP64 pipe, where
-// a tree of five additions takes 450 cycles and this 150.  Infinities, NaN and
-// sums near the denormal range are left to such a tree (plain_sum, a call, so
-// that the compiler does not predicate its additions into the common path).
+// relative to the largest (fixed_sum.h), the limbs added with the warp's integer
+// reductions: free of the FP64 pipe, where a tree of five additions takes 450
+// cycles and this 150.  Infinities, NaN and sums near the denormal range are left
+// to such a tree (plain_sum, a call, so that the compiler does not predicate its
+// additions into the common path).
 __device__ __noinline__ double plain_sum(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
@@ -110,44 +109,23 @@ __device__ __noinline__ double plain_sum(double v) {
 __device__ __noinline__ double plain_add(double a, double b) { return a + b; }
 template <int N>
 __device__ __forceinline__ double fixed_sum_of(const double (&v)[N]) {
-    int emax = 0;
+    unsigned top = 0;
 #pragma unroll
-    for (int j = 0; j < N; j++) emax = max(emax, (int)((unsigned)__double2hiint(v[j]) >> 20 & 0x7ffu));
-    emax = (int)__reduce_max_sync(0xffffffffu, (unsigned)emax);
-    if (emax == 0x7ff || emax < 128) {
+    for (int j = 0; j < N; j++) top = max(top, (unsigned)__double2hiint(v[j]) & 0x7fffffffu);
+    const int emax = (int)(__reduce_max_sync(0xffffffffu, top) >> 20);
+    if (emax == 0x7ff || emax < FS_EMIN) {
         double s = v[0];
         for (int j = 1; j < N; j++) s = plain_add(s, v[j]);
         return plain_sum(s);
     }
-    unsigned lo = 0, mid = 0;
-    int hi = 0;
+    static_assert(32 * N <= FS_TERMS, "terms of a fixed-point sum");
+    FixedLimbs f{0u, 0u, 0};
 #pragma unroll
-    for (int j = 0; j < N; j++) {
-        const long long b = __double_as_longlong(v[j]);
-        const int e = (int)(b >> 52) & 0x7ff, d = emax - e;
-        long long m = ((b & 0xfffffffffffffll) | (1ll << 52)) << 8;
-        m = e == 0 || d > 60 ? 0 : m >> d;
-        if (b < 0) m = -m;
-        lo += (unsigned)m & 0x1fffffu;
-        mid += (unsigned)(m >> 21) & 0x1fffffu;
-        hi += (int)(m >> 42);
-    }
-    lo = __reduce_add_sync(0xffffffffu, lo);
-    mid = __reduce_add_sync(0xffffffffu, mid);
-    hi = __reduce_add_sync(0xffffffffu, hi);
-    // total = T 2^21 + lo in units of 2^(emax - 1023 - 60); the top 63 bits of it
-    const long long T = ((long long)hi << 21) + mid + (lo >> 21);
-    const long long V = T * 4096 + (long long)((lo & 0x1fffffu) >> 9);  // units of 2^(emax - 1023 - 51)
-    if (V == 0) return 0.;
-    const unsigned long long a = (unsigned long long)(V < 0 ? -V : V);
-    const int lz = __clzll((long long)a);
-    unsigned long long m = a << lz;  // leading one at bit 63
-    const int e = emax - 51 + 63 - lz;  // its exponent (biased), at least 77
-    const unsigned long long r = m & 0x7ffull;
-    m >>= 11;
-    if (r > 0x400ull || (r == 0x400ull && (m & 1))) m++;  // to nearest; a carry moves into the exponent
-    const unsigned long long bits = ((unsigned long long)(e - 1) << 52) + m;
-    return __longlong_as_double((long long)(bits | (V < 0 ? 1ull << 63 : 0ull)));
+    for (int j = 0; j < N; j++) fixed_add(f, __double_as_longlong(v[j]), emax);
+    f.lo = __reduce_add_sync(0xffffffffu, f.lo);
+    f.mid = __reduce_add_sync(0xffffffffu, f.mid);
+    f.hi = __reduce_add_sync(0xffffffffu, f.hi);
+    return __longlong_as_double((long long)fixed_round(f, emax));
 }
 
 constexpr int TEAM_WORDS = (TEAM_MAX + 31) / 32;
