@@ -19,8 +19,11 @@
 namespace fe3d {
 
 constexpr int FS_TERMS = 256;  // terms at most: limbs of 21 bits, 32-bit sums
-// biased exponents of the largest term for which nothing leaves the normal range
-constexpr int FS_EMIN = 128;
+// biased exponents of the largest term for which no sum of FS_TERMS terms leaves
+// the normal range: it is below 2^9 times the power of two at or below that term
+constexpr int FS_EMIN = 128, FS_EMAX = 0x7fe - 9;
+
+FS_FN bool fixed_range(int emax) { return (unsigned)(emax - FS_EMIN) <= (unsigned)(FS_EMAX - FS_EMIN); }
 
 struct FixedLimbs {
     uint32_t lo, mid;  // 21 bits each
@@ -39,7 +42,7 @@ FS_FN uint64_t fixed_shift(uint64_t m, int d) {
 }
 
 // Adds the term with the bits b to f; emax: the largest term's biased exponent,
-// at least FS_EMIN (a zero or denormal term then moves out entirely).
+// in fixed_range (a zero or denormal term then moves out entirely).
 FS_FN void fixed_add(FixedLimbs &f, int64_t b, int emax) {
     int64_t m = (int64_t)fixed_shift((uint64_t)((b & 0xfffffffffffffll) | (1ll << 52)) << 10,
                                      emax - ((int)(b >> 52) & 0x7ff));

@@ -99,9 +99,9 @@ __device__ __forceinline__ bool ll_poll(const ulonglong2 *base, int i0, int step
 // Sum of N doubles a lane over the warp (all lanes get it), in fixed point
 // relative to the largest (fixed_sum.h), the limbs added with the warp's integer
 // reductions: free of the FP64 pipe, where a tree of five additions takes 450
-// cycles and this 150.  Infinities, NaN and sums near the denormal range are left
-// to such a tree (plain_sum, a call, so that the compiler does not predicate its
-// additions into the common path).
+// cycles and this 150.  Infinities, NaN and sums near the ends of the range are
+// left to such a tree (plain_sum, a call, so that the compiler does not predicate
+// its additions into the common path).
 __device__ __noinline__ double plain_sum(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
@@ -113,7 +113,7 @@ __device__ __forceinline__ double fixed_sum_of(const double (&v)[N]) {
 #pragma unroll
     for (int j = 0; j < N; j++) top = max(top, (unsigned)__double2hiint(v[j]) & 0x7fffffffu);
     const int emax = (int)(__reduce_max_sync(0xffffffffu, top) >> 20);
-    if (emax == 0x7ff || emax < FS_EMIN) {
+    if (!fixed_range(emax)) {
         double s = v[0];
         for (int j = 1; j < N; j++) s = plain_add(s, v[j]);
         return plain_sum(s);

@@ -25,6 +25,7 @@ extern "C" int fixed_sum(const int64_t *b, int n, int64_t *out) {
     *out = fe3d::fixed_round(f, emax);
     return fe3d::FS_TERMS;
 }
+extern "C" int fixed_range(int emax) { return fe3d::fixed_range(emax); }
 '''
 
 
@@ -37,13 +38,15 @@ def fixed_sum(tmp_path_factory):
     src, lib = d / 'shim.cpp', d / 'shim.so'
     src.write_text(SHIM)
     subprocess.run([cxx, '-O1', '-std=c++17', '-shared', '-fPIC', '-I' + CSRC, str(src), '-o', str(lib)], check=True)
-    f = ctypes.CDLL(str(lib)).fixed_sum
+    h = ctypes.CDLL(str(lib))
+    f = h.fixed_sum
 
     def call(v):
         v = np.ascontiguousarray(v, dtype=np.float64)
         out = np.zeros(1)
         assert v.size <= f(v.ctypes.data_as(ctypes.c_void_p), v.size, out.ctypes.data_as(ctypes.c_void_p))
         return out[0]
+    call.range = h.fixed_range
     return call
 
 
@@ -83,3 +86,18 @@ def test_against_exact_sums(fixed_sum, n, decades, signs):
             elif signs == 'cancel':
                 v[n // 2:] = -v[:n - n // 2] * (1. + 2. ** -40)
             _check(fixed_sum, v)
+
+
+def test_ends_of_the_range(fixed_sum):
+    """Where the fixed-point sum is taken it neither overflows (256 terms of the largest size) nor ends below the
+    normal numbers (all but the last bit cancelled); infinities, NaN and the rest are left to plain additions."""
+    big = 2. - 2. ** -52
+    for e in range(2048):
+        if not fixed_sum.range(e):
+            continue
+        for v in (256 * [math.ldexp(big, e - 1023)], 256 * [math.ldexp(-big, e - 1023)],
+                  [math.ldexp(big, e - 1023), math.ldexp(-(2. - 2. ** -51), e - 1023)]):
+            got = fixed_sum(v)
+            assert math.isfinite(got) and got == math.fsum(v) and abs(got) >= 2. ** -1022
+    assert fixed_sum.range(1023 - 800) and fixed_sum.range(1023) and fixed_sum.range(1023 + 1000)
+    assert not any(fixed_sum.range(e) for e in (0, 1, 2040, 2046, 2047))
