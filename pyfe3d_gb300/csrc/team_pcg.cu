@@ -49,6 +49,7 @@
 #include "common.cuh"
 #include "fe3d_internal.h"
 #include "fixed_sum.h"
+#include "quotient.cuh"
 
 namespace fe3d {
 namespace {
@@ -162,23 +163,6 @@ __device__ __forceinline__ double team_block_sum(double v, int nw, double *red) 
 #pragma unroll 1
     for (int w = 1; w < nw; w++) v += red[w];  // 64 cycles each, fixed_sum 320
     return v;
-}
-
-__device__ __forceinline__ int exponent_of(double v) { return (int)((unsigned)__double2hiint(v) >> 20 & 0x7ffu); }
-__device__ __forceinline__ bool bits_zero(double v) { return (__double_as_longlong(v) << 1) == 0; }
-
-// a / b, 0 where b is 0: an approximate reciprocal (20 bits), one Newton step,
-// and the quotient by it corrected once by its residual; the division with a
-// comparison takes 830 cycles.  The ends of the range are left to the division.
-__device__ __noinline__ double plain_quotient(double a, double b) { return b != 0. ? a / b : 0.; }
-__device__ __forceinline__ double quotient(double a, double b) {
-    const int e = exponent_of(b);
-    if (e <= 64 || e >= 1984) return plain_quotient(a, b);
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    y = fma(fma(-b, y, 1.), y, y);
-    const double q = a * y, c = fma(fma(-q, b, a), y, q);
-    return exponent_of(c) < 0x7ff ? c : q;
 }
 
 // One warp: the blocks' partial sums.
@@ -412,7 +396,7 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
             const double pq = fixed_sum(v);
             if (tid == 0) bc[0] = quotient(rz, pq);
         } else if (tid >= TZ) {
-            irz = exponent_of(rz) > 64 && exponent_of(rz) < 1984 ? 1. / rz : 0.;  // for beta
+            irz = quotient_range(rz) ? 1. / rz : 0.;  // for beta
         }
         __syncthreads();
         // z = Minv r, r.z
@@ -477,7 +461,7 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
             double s = 0.;
             if (look) s = fixed_sum(vr);
             if (tid == TZ) {
-                const double be = bits_zero(irz) ? plain_quotient(rzn, rz) : rzn * irz;
+                const double be = bits_zero(irz) ? plain_quotient(rzn, rz) : quotient_by(rzn, rz, irz);
                 bc[1] = be;
                 fresh = bits_zero(be);
                 bc[2] = rzn;
