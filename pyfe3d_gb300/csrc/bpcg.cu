@@ -663,36 +663,6 @@ __global__ void coupling_kernel(int64_t n, const int64_t *rowptr, const int32_t 
 
 using namespace fe3d;
 
-struct fe3d_bsolver {
-    fe3d_solver *base = nullptr;  // node blocks, block inverses, work vectors, stream
-    int64_t ninst = 0;
-    int32_t *inst = nullptr;       // [nrows] instance of each reduced row
-    int32_t *node_inst = nullptr;  // [nnodes]
-    int *active = nullptr, *flag = nullptr;
-    int *bad = nullptr;
-    double *pq = nullptr, *rz = nullptr /* [2][ninst] */, *rr = nullptr, *ff = nullptr, *rt = nullptr;
-    int lanes[2] = {0, 0};  // autotuned lanes per row [precision]
-    int32_t *rowlist = nullptr, *nodelist = nullptr;  // rows / nodes of active instances
-    int *lcount = nullptr;                            // [0] rows, [1] nodes in the lists
-    int *blockcount = nullptr;                        // compaction scratch [2][kCompactGrid]
-    cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [precision][parity]
-    int graph_chunk[2][2] = {{0, 0}, {0, 0}};
-    // work split: row and node ranges per instance, the rows of the
-    // instances whose rows are contiguous (0 otherwise), the size limit, and
-    // the block-resident solver's list, results and stream
-    int32_t *rlo = nullptr, *rhi = nullptr, *nlo = nullptr, *nhi = nullptr, *rcnt = nullptr, *ncnt = nullptr;
-    std::vector<int64_t> contig_rows, first_row;
-    fe3d_team *team = nullptr;     // resident teams, made by the first solve that can use them
-    int team_tried = 0;
-    std::vector<int32_t> reach;    // column reach of each instance
-    int64_t split_rows = 0;
-    int32_t *cta_list = nullptr;
-    int *cta_status = nullptr;
-    int64_t *cta_iters = nullptr;
-    cudaStream_t cta_stream = nullptr;
-    cudaEvent_t cta_start = nullptr, cta_done = nullptr;
-};
-
 namespace {
 
 void drop_graphs(fe3d_bsolver *b) {
@@ -1188,7 +1158,7 @@ int bsolve(fe3d_bsolver *b, double *fu, double *uu, const fe3d_solve_opts *o, in
                               (int)(o->maxiter - iters[q.sys] < kTeamIters ? o->maxiter - iters[q.sys] : kTeamIters),
                               (int)(iters[q.sys] % chunk), 0, 0};
             const int enough = parts.size() == 1 ? INT_MAX : t->G / 5 > 8 ? t->G / 5 : 8;
-            if ((rc = team_run(t, s, uu, b->rz + par * K, b->rr, sys, chunk, enough, st))) return rc;
+            if ((rc = team_run(t, s, uu, b->rz + par * K, b->rr, sys, chunk, enough, st))) break;
             FE3D_CUDA(cudaMemcpyAsync(hrr.data(), b->rr, sizeof(double) * K, cudaMemcpyDeviceToHost, st));
             FE3D_CUDA(cudaStreamSynchronize(st));
             std::vector<int> check(K, 0);
@@ -1224,9 +1194,14 @@ int bsolve(fe3d_bsolver *b, double *fu, double *uu, const fe3d_solve_opts *o, in
             if ((rc = precondition(1))) return rc;
         }
         if (rc == FE3D_OK) return finish(it, 0);
-        // no memory for a split: the lockstep recurrence needs none
-        if (rc != FE3D_ERR_NOMEM) return rc;
-        if ((rc = upload(b->flag, hact)) || (rc = precondition(1))) return rc;
+        // no memory for a split, a launch refused or an exchange that did not end:
+        // the lockstep recurrence needs none of them and goes on from the iterates
+        if (rc != FE3D_ERR_NOMEM && rc != FE3D_ERR_LAUNCH) return rc;
+        if (rc == FE3D_ERR_LAUNCH) {
+            team_free(b->team);
+            b->team = nullptr;
+        }
+        if ((rc = true_res(hact)) || (rc = precondition(1))) return rc;
     }
     FE3D_CUDA(cudaMemsetAsync(b->pq, 0, sizeof(double) * K, st));
     if ((rc = upload(b->active, hact))) return rc;

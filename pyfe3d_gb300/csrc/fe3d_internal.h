@@ -111,6 +111,10 @@ struct fe3d_team {
     TeamSys *sys = nullptr;
     int *done = nullptr;
     unsigned epoch = 1;
+    // polls of one word before a block gives up: about a second, and about a
+    // minute at the first exchange, where blocks may still wait for SMs that
+    // another stream's kernel holds
+    int poll = 1 << 21, poll_first = 1 << 27;
 };
 
 // Block-Jacobi PCG state (pcg.cu); the batched solver (bpcg.cu) reuses its
@@ -175,6 +179,37 @@ struct fe3d_solver {
     int team_tried = 0;
 };
 
+// Batched PCG state (bpcg.cu).
+struct fe3d_bsolver {
+    fe3d_solver *base = nullptr;  // node blocks, block inverses, work vectors, stream
+    int64_t ninst = 0;
+    int32_t *inst = nullptr;       // [nrows] instance of each reduced row
+    int32_t *node_inst = nullptr;  // [nnodes]
+    int *active = nullptr, *flag = nullptr;
+    int *bad = nullptr;
+    double *pq = nullptr, *rz = nullptr /* [2][ninst] */, *rr = nullptr, *ff = nullptr, *rt = nullptr;
+    int lanes[2] = {0, 0};  // autotuned lanes per row [precision]
+    int32_t *rowlist = nullptr, *nodelist = nullptr;  // rows / nodes of active instances
+    int *lcount = nullptr;                            // [0] rows, [1] nodes in the lists
+    int *blockcount = nullptr;                        // compaction scratch [2][kCompactGrid]
+    cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [precision][parity]
+    int graph_chunk[2][2] = {{0, 0}, {0, 0}};
+    // work split: row and node ranges per instance, the rows of the
+    // instances whose rows are contiguous (0 otherwise), the size limit, and
+    // the block-resident solver's list, results and stream
+    int32_t *rlo = nullptr, *rhi = nullptr, *nlo = nullptr, *nhi = nullptr, *rcnt = nullptr, *ncnt = nullptr;
+    std::vector<int64_t> contig_rows, first_row;
+    fe3d_team *team = nullptr;     // resident teams, made by the first solve that can use them
+    int team_tried = 0;
+    std::vector<int32_t> reach;    // column reach of each instance
+    int64_t split_rows = 0;
+    int32_t *cta_list = nullptr;
+    int *cta_status = nullptr;
+    int64_t *cta_iters = nullptr;
+    cudaStream_t cta_stream = nullptr;
+    cudaEvent_t cta_start = nullptr, cta_done = nullptr;
+};
+
 namespace fe3d {
 void team_free(fe3d_team *t);
 fe3d_team *team_create(const fe3d_solver *s, int64_t nsys, cudaStream_t st);
@@ -188,7 +223,9 @@ int team_build(fe3d_team *t, const fe3d_solver *s, const unsigned long long (&to
 int team_inverses(fe3d_team *t, const fe3d_solver *s, cudaStream_t st);
 // Iterations of every system of the split from s->r, s->p, u and rz (per
 // system), until its limits are met or the teams of enough blocks have
-// finished; rr per system, sys updated (synchronises).
+// finished; rr per system, sys updated (synchronises).  FE3D_ERR_LAUNCH where
+// the launch is refused or a poll gave up: u is then an earlier iterate in some
+// or all rows, and r, p and rz do not belong to it.
 int team_run(fe3d_team *t, const fe3d_solver *s, double *u, double *rz, double *rr, std::vector<TeamSys> &sys,
              int chunk, int enough, cudaStream_t st);
 }  // namespace fe3d

@@ -1510,7 +1510,17 @@ int run_cg(fe3d_solver *s, const double *f, double *u, const fe3d_solve_opts *o,
             const int64_t most = (o->maxiter - it) < kTeamIters ? (o->maxiter - it) : kTeamIters;
             std::vector<TeamSys> one{{target > inner2 * rr_replaced ? target : inner2 * rr_replaced, (int)most,
                                       (int)(it % chunk), 0, 0}};
-            if ((rc = team_run(team, s, u, s->scal + par, s->scal + 2, one, chunk, INT_MAX, st))) return rc;
+            rc = team_run(team, s, u, s->scal + par, s->scal + 2, one, chunk, INT_MAX, st);
+            if (rc == FE3D_ERR_LAUNCH) {
+                // refused, or an exchange did not end: a launch per kernel from
+                // the iterate, here and in later solves
+                team_free(team);
+                team = s->team = nullptr;
+                if ((rc = true_residual(s, f, u, st, &rr_replaced)) || (rc = restart())) return rc;
+                since_replace = 0;
+                continue;
+            }
+            if (rc) return rc;
             FE3D_CUDA(cudaMemcpyAsync(&rr, s->scal + 2, sizeof(double), cudaMemcpyDeviceToHost, st));
             FE3D_CUDA(cudaStreamSynchronize(st));
             len = one[0].iters;

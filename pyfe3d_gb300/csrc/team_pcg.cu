@@ -56,10 +56,6 @@ namespace {
 
 constexpr int TT = 512;               // threads per block
 constexpr int TEAM_MAX = kSMs;        // blocks of one system
-// Polls of one word before a block gives up: about a second, and about a
-// minute at the first exchange, where blocks may still wait for SMs that
-// another stream's kernel holds.
-constexpr int POLL_MAX = 1 << 21, POLL_FIRST = 1 << 27;
 constexpr int TZ = TT - 32;           // threads that fetch z; the last warp sums r.z meanwhile
 constexpr int SLOT = 8;               // words (16 bytes) per slot: a 128-byte line each
 
@@ -73,7 +69,7 @@ __device__ __forceinline__ void ll_store(ulonglong2 *p, double v, unsigned ep) {
 // all loads of a round in flight together; false when one did not arrive.
 template <int N>
 __device__ __forceinline__ bool ll_poll(const ulonglong2 *base, int i0, int step, int lim, unsigned ep,
-                                        double (&v)[N], int limit = POLL_MAX) {
+                                        double (&v)[N], int limit) {
 #pragma unroll
     for (int j = 0; j < N; j++) v[j] = 0.;
     if (i0 >= lim) return true;
@@ -167,7 +163,7 @@ __device__ __forceinline__ double team_block_sum(double v, int nw, double *red) 
 
 // One warp: the blocks' partial sums.
 __device__ __forceinline__ bool team_poll(const ulonglong2 *slots, int G, unsigned ep, double (&v)[TEAM_WORDS],
-                                          int limit = POLL_MAX) {
+                                          int limit) {
     return ll_poll(slots, SLOT * (int)(threadIdx.x & 31), SLOT * 32, SLOT * G, ep, v, limit);
 }
 
@@ -195,6 +191,7 @@ struct TeamArgs {
     int chunk;               // convergence is looked at every chunk iterations
     int *done;               // [0] blocks of finished teams, [1] a poll gave up
     int enough;              // finished blocks at which the other teams stop too
+    int poll, poll_first;    // polls of a word before a block gives up, and at the first exchange
 };
 
 // Where a block's rows of the matrix are between two iterations, and how they
@@ -392,7 +389,7 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
             if (tid == 0) ll_store(slot_pq + SLOT * bid, dot, ep);
             __syncwarp();
             double v[TEAM_WORDS];
-            if (!team_poll(slot_pq, G, ep, v, it == 0 ? POLL_FIRST : POLL_MAX)) fail = 1;
+            if (!team_poll(slot_pq, G, ep, v, it == 0 ? a.poll_first : a.poll)) fail = 1;
             const double pq = fixed_sum(v);
             if (tid == 0) bc[0] = quotient(rz, pq);
         } else if (tid >= TZ) {
@@ -452,11 +449,12 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
         constexpr int ZW = ROWS == FAR ? 4 : 6;  // words a thread asks for at a time
         double zv[ZW];
         if (tid < TZ) {
-            if (!ll_poll(a.z + c0, tid, TZ, W, ep, zv)) fail = 1;
+            if (!ll_poll(a.z + c0, tid, TZ, W, ep, zv, a.poll)) fail = 1;
         } else {
             double vz[TEAM_WORDS], vr[TEAM_WORDS], vy[1];
-            if (!team_poll(slot_rz, G, ep, vz)) fail = 1;
-            if (look && !(team_poll(slot_rr, G, ep, vr) && ll_poll(slot_rr + 1, 0, 1, 1, ep, vy))) fail = 1;
+            if (!team_poll(slot_rz, G, ep, vz, a.poll)) fail = 1;
+            if (look && !(team_poll(slot_rr, G, ep, vr, a.poll) && ll_poll(slot_rr + 1, 0, 1, 1, ep, vy, a.poll)))
+                fail = 1;
             const double rzn = fixed_sum(vz);
             double s = 0.;
             if (look) s = fixed_sum(vr);
@@ -491,19 +489,23 @@ __global__ void __launch_bounds__(TT, 1) team_pcg_kernel(TeamArgs a) {
                 }
                 c1 += ZW * TZ;
                 if (c1 >= W) break;
-                if (!ll_poll(a.z + c0, c1, TZ, W, ep, zv)) fail = 1;
+                if (!ll_poll(a.z + c0, c1, TZ, W, ep, zv, a.poll)) fail = 1;
             }
         }
         if (ROWS == FAR && tid < rows32) fetch(sinf[tid >> 5], 0, cv, cc);
         __syncthreads();
         stop = fail || it >= lim.maxiter || (look && (yield || !(rr > lim.stop2 && rr <= 1.7e308)));
     }
+    if (fail) {
+        // the rows keep the u of before the launch, from which the host restarts
+        if (tid == 0) a.done[1] = 1;
+        return;
+    }
     for (int i = tid; i < n; i += TT) {
         a.u[r0 + i] = us[i];
         a.r[r0 + i] = rs[i];
         a.p[r0 + i] = pw[own + i];
     }
-    if (fail && tid == 0) a.done[1] = 1;
     if (bid == 0 && tid == 0) {
         a.rz[sys] = rz;
         a.rr[sys] = rr;
@@ -855,12 +857,14 @@ int team_run(fe3d_team *t, const fe3d_solver *s, double *u, double *rz, double *
     FE3D_CUDA(cudaMemsetAsync(t->done, 0, 2 * sizeof(int), st));
     TeamArgs a{t->rbeg, t->rend, t->slice0, t->cmin, t->cmax, t->tfirst, t->tcount, t->tsys, t->slen, t->soff,
                t->sval, t->scol, s->pat->colbase, s->pat->dof_of_row, s->start, s->bs, t->dval, t->dinf, u, s->r,
-               s->p, s->n, rz, rr, t->sys, t->z, t->slots, t->epoch, chunk, t->done, enough};
+               s->p, s->n, rz, rr, t->sys, t->z, t->slots, t->epoch, chunk, t->done, enough, t->poll, t->poll_first};
     t->epoch += (unsigned)most + 1u;
     void *args[] = {&a};
     if (cudaLaunchCooperativeKernel((const void *)team_kernel(t->L, t->rows), dim3(t->G), dim3(TT), args,
-                                    t->smem_run, st) != cudaSuccess)
+                                    t->smem_run, st) != cudaSuccess) {
+        (void)cudaGetLastError();
         return FE3D_ERR_LAUNCH;
+    }
     int done[2] = {0, 0};
     FE3D_CUDA(cudaMemcpyAsync(sys.data(), t->sys, sizeof(TeamSys) * sys.size(), cudaMemcpyDeviceToHost, st));
     FE3D_CUDA(cudaMemcpyAsync(done, t->done, sizeof(done), cudaMemcpyDeviceToHost, st));
