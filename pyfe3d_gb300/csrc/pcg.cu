@@ -862,7 +862,7 @@ __global__ void any_nonzero_kernel(int64_t n, const double *x, int *flag) {
     bool any = false;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         any |= (__double_as_longlong(x[i]) << 1) != 0;
-    if (__any_sync(__activemask(), any) && (threadIdx.x & 31) == 0) *flag = 1;
+    if (any) *flag = 1;
 }
 
 // The residual of a zero iterate, r = f, with partial sums of r.r.
