@@ -1200,8 +1200,8 @@ extern "C" int fe3d_spmv(const fe3d_pattern *p, const double *vals, const double
 namespace {
 
 // Slice layout of the solve's values: counts the non-zeros on st (sell_plan),
-// and once the caller has read *sell_total and synchronised, decides and
-// fills it (sell_build).  The layout is used when it holds at most 3/4 of the
+// and once the caller has read *sell_total (NULL without memory for the counts) and
+// synchronised, decides and fills it (sell_build).  The layout is used when it holds at most 3/4 of the
 // stored entries; otherwise (curved shells, laminates with coupling) the CSR
 // kernels read the caller's values as they are.  Below kSellMinRows one row
 // per lane leaves too few warps and the row's serial FP64 chain shows (clamped
@@ -1217,8 +1217,18 @@ int sell_plan(fe3d_solver *s, cudaStream_t st) {
     if (!s->sell_total) {
         const int res = resident_per_sm(spmv_sell_kernel, RED_BS, 0);
         s->sell_grid = grid_cap(s->n, RED_BS, kSMs * (res < 8 ? res : 8));
-        if (alloc(&s->slen, slices) || alloc(&s->soff, slices) || alloc(&s->xnz, 2) || alloc(&s->sell_total, 1))
-            return FE3D_ERR_NOMEM;
+        if (alloc(&s->slen, slices) || alloc(&s->soff, slices) || alloc(&s->xnz, 2) || alloc(&s->sell_total, 1)) {
+            // no room for the counts: the CSR kernels need none
+            (void)cudaGetLastError();
+            cudaFree(s->slen);
+            cudaFree(s->soff);
+            cudaFree(s->xnz);
+            s->slen = nullptr;
+            s->soff = nullptr;
+            s->xnz = nullptr;
+            s->sell_total = nullptr;
+            return FE3D_OK;
+        }
     }
     FE3D_CUDA(cudaMemsetAsync(s->xnz, 0, 2 * sizeof(int), st));
     FE3D_CUDA(cudaMemsetAsync(s->sell_total, 0, sizeof(unsigned long long), st));
@@ -1230,7 +1240,7 @@ int sell_plan(fe3d_solver *s, cudaStream_t st) {
 
 int sell_build(fe3d_solver *s, unsigned long long total, cudaStream_t st) {
     const int64_t entries = 32 * (int64_t)total;
-    int on = s->pat->col16 && s->n >= kSellMinRows && 4 * entries <= 3 * s->pat->nnz;
+    int on = s->sell_total && 4 * entries <= 3 * s->pat->nnz;
     if (on && entries > s->sell_cap) {
         cudaFree(s->sval);
         cudaFree(s->scol);
