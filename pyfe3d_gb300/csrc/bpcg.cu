@@ -615,11 +615,14 @@ __global__ void __launch_bounds__(CT) bcta_kernel(CtaArgs a) {
                     status = 3;
                     break;
                 }
-                if (rr <= lim) {
-                    // 5 % below the tolerance: the reported residual is summed in
-                    // another order, which moves it by up to a percent here
+                // 5 % below the tolerance: the residual f - K u differs from the
+                // recurrence's, and the reported one, summed in another order, from
+                // both, by up to a percent here.  (A margin on f - K u itself makes
+                // false convergences, whose restarts lose the direction, of every
+                // iterate that stops within it.)
+                if (rr <= 0.9 * lim || (rr <= lim && it >= a.maxiter)) {
                     const double rt = cta_rows(a, r0, r1, a.u, 0, a.r, 0, a.f, red);
-                    if (rt <= 0.9 * lim) {
+                    if (rt <= lim) {
                         status = 0;
                         break;
                     }
