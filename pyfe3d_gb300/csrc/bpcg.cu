@@ -595,13 +595,13 @@ __global__ void __launch_bounds__(CT) bcta_kernel(CtaArgs a) {
     for (int li = blockIdx.x; li < a.nlist; li += gridDim.x) {
         const int inst = a.list[li];
         const int64_t r0 = a.rlo[inst], r1 = a.rhi[inst], n0 = a.nlo[inst], n1 = a.nhi[inst];
-        const double lim = a.tol2 * a.ff[inst];
+        const double goal = 0.9 * a.tol2 * a.ff[inst];
         double rr = cta_rows(a, r0, r1, a.u, 0, a.r, 0, a.f, red);
         int status = 1;
         int64_t it = 0;
         if (!(rr == rr) || isinf(rr)) {
             status = 3;
-        } else if (rr <= lim) {
+        } else if (rr <= a.tol2 * a.ff[inst]) {
             status = 0;
         } else {
             double rr_r;
@@ -620,9 +620,9 @@ __global__ void __launch_bounds__(CT) bcta_kernel(CtaArgs a) {
                 // both, by up to a percent here.  (A margin on f - K u itself makes
                 // false convergences, whose restarts lose the direction, of every
                 // iterate that stops within it.)
-                if (rr <= 0.9 * lim || (rr <= lim && it >= a.maxiter)) {
+                if (rr <= goal || (it >= a.maxiter && rr <= a.tol2 * a.ff[inst])) {
                     const double rt = cta_rows(a, r0, r1, a.u, 0, a.r, 0, a.f, red);
-                    if (rt <= lim) {
+                    if (rt <= a.tol2 * a.ff[inst]) {
                         status = 0;
                         break;
                     }
