@@ -362,8 +362,10 @@ __global__ void bzero_kernel(int64_t n, const int32_t *inst, const int *flag, do
 // (so the iteration kernels walk rows and nodes in memory order and an
 // instance stays contiguous), *count = their number.  Block g owns the items
 // [g per, (g + 1) per): pass 1 counts its kept items, one block scans the
-// counts, pass 2 writes each block's items at its offset in order.
+// counts, pass 2 writes each block's items at its offset in order.  A node
+// without free DOFs has the instance -1 and is never kept.
 constexpr int kCompactGrid = kSMs * 8;
+__device__ __forceinline__ bool kept(const int *active, int inst) { return inst >= 0 && active[inst] != 0; }
 
 __global__ void __launch_bounds__(BS) bcount_kernel(int64_t n, const int32_t *__restrict__ inst,
                                                     const int *__restrict__ active, int *blockcount) {
@@ -371,7 +373,7 @@ __global__ void __launch_bounds__(BS) bcount_kernel(int64_t n, const int32_t *__
     const int64_t per = (n + gridDim.x - 1) / gridDim.x;
     const int64_t c0 = blockIdx.x * per, c1 = c0 + per < n ? c0 + per : n;
     int cnt = 0;
-    for (int64_t i = c0 + threadIdx.x; i < c1; i += blockDim.x) cnt += active[inst[i]] != 0;
+    for (int64_t i = c0 + threadIdx.x; i < c1; i += blockDim.x) cnt += kept(active, inst[i]);
     for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
     if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = cnt;
     __syncthreads();
@@ -419,7 +421,7 @@ __global__ void __launch_bounds__(BS) bscatter_kernel(int64_t n, const int32_t *
     int base = blockoff[blockIdx.x];
     for (int64_t t0 = c0; t0 < c1; t0 += blockDim.x) {
         const int64_t i = t0 + threadIdx.x;
-        const bool keep = i < c1 && active[inst[i]] != 0;
+        const bool keep = i < c1 && kept(active, inst[i]);
         const unsigned m = __ballot_sync(0xffffffffu, keep);
         if (lane == 0) wsum[warp] = __popc(m);
         __syncthreads();
