@@ -965,6 +965,22 @@ std::vector<TeamPart> deal(const fe3d_bsolver *b, const std::vector<int64_t> &to
     return parts;
 }
 
+// Whether the nactive instances act are better solved on teams than in lockstep.
+// A launch of teams takes 152 instances at most and costs about 0.5 ms besides its
+// iterations, of 5 us at least; a lockstep iteration takes 20 us and 0.33 ns per
+// active row, however many instances there are.  Plates to 1e-8, mean rows per
+// plate, plates from which on lockstep was the faster: 29 and 43 rows 570, 79 rows
+// 2,430, 157 rows 6,000, 257 rows 12,500, 341 rows 18,000; teams / lockstep, ms: 4,864 of 42
+// rows 20.7 / 6.0, 4,864 of 78 rows 31 / 21, 9,728 of 154 rows 125 / 100, 1,216 of 157
+// rows 13 / 29, 1,024 of 348 rows 29 / 76, 16,384 of 1,442 rows 3,120 / 6,600.
+bool teams_pay(const fe3d_bsolver *b, const std::vector<int> &act, int nactive) {
+    int64_t rows = 0;
+    for (int64_t i = 0; i < b->ninst; i++)
+        if (act[i]) rows += b->contig_rows[i];
+    const double mean = nactive > 0 ? (double)rows / nactive : 0.;
+    return nactive > 0 && nactive <= 500. + 55. * (mean > 40. ? mean - 40. : 0.);
+}
+
 // Whether the instances act can run on teams (makes the teams at first use).
 bool teams_ready(fe3d_bsolver *b, const std::vector<int> &act, cudaStream_t st) {
     fe3d_solver *s = b->base;
@@ -1131,11 +1147,17 @@ int bsolve(fe3d_bsolver *b, double *fu, double *uu, const fe3d_solve_opts *o, in
     if ((rc = precondition(1))) return rc;
     const int chunk = o->check_every < 2 ? 2 : (int)(o->check_every & ~1);
     int64_t it = 0;
-    // resident teams: every instance iterates on its own, nothing in lockstep
-    if (prec == 0 && !nested && b->split_rows == 0 && nactive > 0 && o->maxiter > 0 && teams_ready(b, hact, st) &&
-        team_inverses(b->team, s, st) == FE3D_OK) {
+    bool teams = prec == 0 && !nested && b->split_rows == 0 && o->maxiter > 0;  // not tried in vain
+    // resident teams: every active instance iterates on its own from its r, p and
+    // rz, nothing in lockstep; done is false where the lockstep recurrence has to
+    // go on instead
+    auto run_teams = [&](bool &done) -> int {
+        done = false;
+        teams = teams_ready(b, hact, st) && team_inverses(b->team, s, st) == FE3D_OK;
+        if (!teams) return FE3D_OK;
+        int rc = FE3D_OK;
         fe3d_team *t = b->team;
-        std::vector<double> left(K), rr0(hrt);
+        std::vector<double> left(K), rr0(hrr);
         std::vector<int64_t> todo;
         std::vector<TeamPart> parts, was;
         for (int64_t i = 0; i < K; i++) left[i] = sqrt((double)b->contig_rows[i]);
@@ -1198,20 +1220,34 @@ int bsolve(fe3d_bsolver *b, double *fu, double *uu, const fe3d_solve_opts *o, in
             if ((rc = upload(b->flag, check))) return rc;
             if ((rc = precondition(1))) return rc;
         }
-        if (rc == FE3D_OK) return finish(it, 0);
+        done = rc == FE3D_OK;
         // no memory for a split, a launch refused or an exchange that did not end:
         // the lockstep recurrence needs none of them and goes on from the iterates
         if (rc != FE3D_ERR_NOMEM && rc != FE3D_ERR_LAUNCH) return rc;
+        teams = false;
         if (rc == FE3D_ERR_LAUNCH) {
             team_free(b->team);
             b->team = nullptr;
         }
         if ((rc = true_res(hact)) || (rc = precondition(1))) return rc;
+        return FE3D_OK;
+    };
+    int64_t since = 0, replacements = 0;
+    bool done = false;
+    hrr = hrt;
+    if (teams && teams_pay(b, hact, nactive)) {
+        if ((rc = run_teams(done))) return rc;
+        if (done) return finish(it, replacements);
     }
-    FE3D_CUDA(cudaMemsetAsync(b->pq, 0, sizeof(double) * K, st));
-    if ((rc = upload(b->active, hact))) return rc;
-    if ((rc = compact(b, st))) return rc;
-    int compacted_at = nactive;  // active instances when the lists were built
+    int compacted_at = 0;  // active instances when the lists were built
+    auto begin_lockstep = [&]() -> int {
+        FE3D_CUDA(cudaMemsetAsync(b->pq, 0, sizeof(double) * K, st));
+        int e = upload(b->active, hact);
+        if (!e) e = compact(b, st);
+        compacted_at = nactive;
+        return e;
+    };
+    if ((rc = begin_lockstep())) return rc;
     auto launch_iteration = [&](int pr) {
         double *rz_cur = b->rz + pr * K, *rz_nxt = b->rz + (pr ^ 1) * K;
         launch_bspmv<VT, PT>(lanes, sg, st, n, b, vals, p, q, rz_nxt, b->rr);
@@ -1221,7 +1257,6 @@ int bsolve(fe3d_bsolver *b, double *fu, double *uu, const fe3d_solve_opts *o, in
         bdirection_kernel<PT><<<vg, BS, 0, st>>>(n, b->inst, b->active, rz_nxt, rz_cur, z, p, b->pq, K, b->rowlist,
                                                  b->lcount);
     };
-    int64_t since = 0, replacements = 0;
     std::vector<double> last_rt(K, 0.);
     std::vector<int> stall(K, 0);
     std::vector<double> rr_start(hrt);       // nested: FP64 residual at the instance's last restart
@@ -1317,6 +1352,14 @@ int bsolve(fe3d_bsolver *b, double *fu, double *uu, const fe3d_solve_opts *o, in
                 replacements++;
                 since = 0;
             }
+        }
+        if (teams && nactive > 0 && it < o->maxiter && teams_pay(b, hact, nactive)) {
+            for (int64_t i = 0; i < K; i++)
+                if (hact[i]) iters[i] = it;
+            if ((rc = run_teams(done))) return rc;
+            if (done) return finish(it, replacements);
+            if ((rc = begin_lockstep())) return rc;
+            continue;
         }
         if ((rc = upload(b->active, hact))) return rc;
         // drop the rows of finished instances from the lists once a quarter
