@@ -9,8 +9,8 @@
 // Brockman's hourglass stiffness on u, v, w, rx, ry with the twist mode
 // gamma_a = N_a,xy at the centre (quad4r.pyx:1936-1981).
 //
-// Quad4R KC0 kernel (Tria3R's: t3_kc0_kernel): phase A (one thread per element, plus one per Quad4R drilling
-// point) stages the element's frame, constitutive data and shape-function
+// Quad4R KC0 kernel (Tria3R's: t3_kc0_kernel): phase A (one thread per element,
+// plus one per drilling point) stages the element's frame, constitutive data and shape-function
 // derivatives in shared memory; phase B gives each thread one node pair
 // a <= b, builds the 6x6 block (and its transpose) and stages it; phase C
 // streams every element's (6 NN)^2 slots with all threads of the block,
@@ -594,11 +594,8 @@ __device__ __forceinline__ void rs_block(const RSElem<NN> &s, const ff (*sh)[3][
 // elements staged per pass: 8 keep the shared memory of a block small enough
 // for 3 blocks per SM (measured faster than 12 at 2 blocks per SM, whose passes
 // keep more threads busy)
-#ifndef FE3D_RS_TB4
-#define FE3D_RS_TB4 8
-#endif
-template <int NN>
 struct RSTile {
+    static constexpr int NN = 4;                     // Quad4R
     static constexpr int S = 6 * NN;                 // rows of the element matrix
     static constexpr int S2 = S * S;                 // slots per element
     // staged row and element strides (doubles): rows 16-byte aligned; the
@@ -611,12 +608,12 @@ struct RSTile {
     // charges a warp instruction whatever its active lanes); the blocks are
     // staged TB elements at a time
     static constexpr int TE = 32;
-    static constexpr int TB = FE3D_RS_TB4;
+    static constexpr int TB = 8;
     static constexpr size_t smem = (size_t)TB * SP * sizeof(double) + (size_t)TE * sizeof(RSElem<NN>);
 };
 
-template <int NN>
 __device__ __forceinline__ void pair_of(int p, int &a, int &b) {
+    constexpr int NN = RSTile::NN;
     // p-th pair (a, b), a <= b, in row order
     a = 0;
     int rem = p;
@@ -630,9 +627,8 @@ __device__ __forceinline__ void pair_of(int p, int &a, int &b) {
 // The caller's current values of elements e0 .. e0 + nel - 1, copied into
 // the stage with cp.async (16-byte pieces where the element's slots are
 // 16-byte aligned, else 8-byte pieces).
-template <int NN>
 __device__ __forceinline__ void rs_prefetch(const RSArgs &a, int64_t e0, int nel, double *stage, int tid) {
-    using Tl = RSTile<NN>;
+    using Tl = RSTile;
     constexpr int H = Tl::S2 / 2;  // 16-byte pieces per element
     for (int i = tid; i < nel * H; i += RNT) {
         const int el = i / H, j = i - el * H;
@@ -653,36 +649,34 @@ __device__ __forceinline__ void rs_prefetch(const RSArgs &a, int64_t e0, int nel
     cp_async_commit();
 }
 
-template <int NN>
 __global__ void __launch_bounds__(RNT) rs_kc0_kernel(RSArgs a) {
-    using Tl = RSTile<NN>;
+    using Tl = RSTile;
+    constexpr int NN = Tl::NN;
     extern __shared__ __align__(16) double rs_smem[];
     double *stage = rs_smem;
     RSElem<NN> *se = reinterpret_cast<RSElem<NN> *>(rs_smem + (size_t)Tl::TB * Tl::SP);
     __shared__ ff sh[4][3][4];
     const int tid = threadIdx.x;
-    if (NN == 4) rs_shape_table(sh, tid);
+    rs_shape_table(sh, tid);
     const int64_t ntiles = (a.E + Tl::TE - 1) / Tl::TE;
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int64_t e0 = tile * Tl::TE;
         __syncthreads();
-        rs_prefetch<NN>(a, e0, Tl::TB, stage, tid);
+        rs_prefetch(a, e0, Tl::TB, stage, tid);
         if (tid < Tl::TE) {
             se[tid].flags = 0;
             if (e0 + tid < a.E) rs_phase_a<NN>(a, e0 + tid, se[tid], Tl::S2, true);
         }
-        if (NN == 4) {
-            __syncthreads();
-            if (tid < 4 * Tl::TE) {
-                RSElem<NN> &s = se[tid >> 2];
-                if (s.flags & RF_VALID) rs_drill_point<NN>(s, sh, tid & 3);
-            }
+        __syncthreads();
+        if (tid < 4 * Tl::TE) {
+            RSElem<NN> &s = se[tid >> 2];
+            if (s.flags & RF_VALID) rs_drill_point<NN>(s, sh, tid & 3);
         }
         for (int r0 = 0; r0 < Tl::TE; r0 += Tl::TB) {
             const int nb = Tl::TE - r0 < Tl::TB ? Tl::TE - r0 : Tl::TB;
             if (r0 > 0) {
                 __syncthreads();  // the previous pass's write-out has read the stage
-                rs_prefetch<NN>(a, e0 + r0, nb, stage, tid);
+                rs_prefetch(a, e0 + r0, nb, stage, tid);
             }
             // the element data and (first pass of the tile) the prefetches of every thread
             cp_async_wait_all();
@@ -692,7 +686,7 @@ __global__ void __launch_bounds__(RNT) rs_kc0_kernel(RSArgs a) {
                 const RSElem<NN> &s = se[r0 + el];
                 if (s.flags & RF_VALID) {
                     int pa, pb;
-                    pair_of<NN>(tid - el * Tl::P, pa, pb);
+                    pair_of(tid - el * Tl::P, pa, pb);
                     double K[6][6];
                     rs_block<NN>(s, sh, pa, pb, K);
                     if (s.flags & RF_ROTATE) rotate_block(s.R, K);
@@ -1141,23 +1135,21 @@ inline int rs_grid(int64_t E, int per_block, int per_sm) {
     return (int)g;
 }
 
-template <int NN>
 int launch_rs_kc0(const RSArgs &a, cudaStream_t st) {
-    using Tl = RSTile<NN>;
+    using Tl = RSTile;
     static bool attr = false;
     static int per_sm = 1;  // resident blocks per SM (registers and shared memory)
     if (!attr) {
-        FE3D_CUDA(cudaFuncSetAttribute(rs_kc0_kernel<NN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tl::smem));
+        FE3D_CUDA(cudaFuncSetAttribute(rs_kc0_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tl::smem));
         int n = 0;
-        FE3D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rs_kc0_kernel<NN>, RNT, Tl::smem));
+        FE3D_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rs_kc0_kernel, RNT, Tl::smem));
         per_sm = n > 0 ? n : 1;
         attr = true;
     }
-    rs_kc0_kernel<NN><<<rs_grid(a.E, Tl::TE, per_sm), RNT, Tl::smem, st>>>(a);
+    rs_kc0_kernel<<<rs_grid(a.E, Tl::TE, per_sm), RNT, Tl::smem, st>>>(a);
     FE3D_CHECK_LAUNCH();
     return FE3D_OK;
 }
-
 
 // ------------------------------------------------------------ Tria3R KC0
 // CTAs of 7 warps, two per SM: the last warp runs phase A (one lane per
@@ -1418,10 +1410,10 @@ struct T3Iso {
 };
 
 // Node-pair block K_ab (a <= b) of the element and its transpose onto the
-// staged values.  Of the drilling rotations update_KC0 keeps rz_a - rz_a only.
+// staged values, zeros or not (only isotropic elements look).  Of the drilling
+// rotations update_KC0 keeps rz_a - rz_a only.
 template <bool ROT, bool B0>
 __device__ __forceinline__ void t3_pair_add(const T3Elem &s, double *st, int na, int nb) {
-    constexpr bool CLEAR = false;
     const double Nc = 0.33333333333333333333;
     const double w = s.w, xb = s.Nx[nb], yb = s.Ny[nb];
     const double wxa = w * s.Nx[na], wya = w * s.Ny[na];
@@ -1470,43 +1462,43 @@ __device__ __forceinline__ void t3_pair_add(const T3Elem &s, double *st, int na,
         }
         if (!ROT) {
             if (hb == 0) {
-                t3_add2<CLEAR>(st, na, nb, 0, 0, P[0][0], P[0][1]);
-                t3_add2<CLEAR>(st, na, nb, 1, 0, P[1][0], P[1][1]);
-                t3_add2<CLEAR>(st, na, nb, 2, 2, P[2][2], Q[2][0]);
-                t3_add<CLEAR>(st, na, nb, 2, 4, Q[2][1]);
+                t3_add2<false>(st, na, nb, 0, 0, P[0][0], P[0][1]);
+                t3_add2<false>(st, na, nb, 1, 0, P[1][0], P[1][1]);
+                t3_add2<false>(st, na, nb, 2, 2, P[2][2], Q[2][0]);
+                t3_add<false>(st, na, nb, 2, 4, Q[2][1]);
                 if (!B0) {
                     for (int i = 0; i < 2; i++) {
-                        t3_add<CLEAR>(st, na, nb, i, 3, Q[i][0]);
-                        t3_add<CLEAR>(st, na, nb, i, 4, Q[i][1]);
+                        t3_add<false>(st, na, nb, i, 3, Q[i][0]);
+                        t3_add<false>(st, na, nb, i, 4, Q[i][1]);
                     }
                 }
                 if (!diag) {
-                    t3_add2<CLEAR>(st, nb, na, 0, 0, P[0][0], P[1][0]);
-                    t3_add2<CLEAR>(st, nb, na, 1, 0, P[0][1], P[1][1]);
-                    t3_add<CLEAR>(st, nb, na, 2, 2, P[2][2]);
-                    t3_add<CLEAR>(st, nb, na, 3, 2, Q[2][0]);
-                    t3_add<CLEAR>(st, nb, na, 4, 2, Q[2][1]);
+                    t3_add2<false>(st, nb, na, 0, 0, P[0][0], P[1][0]);
+                    t3_add2<false>(st, nb, na, 1, 0, P[0][1], P[1][1]);
+                    t3_add<false>(st, nb, na, 2, 2, P[2][2]);
+                    t3_add<false>(st, nb, na, 3, 2, Q[2][0]);
+                    t3_add<false>(st, nb, na, 4, 2, Q[2][1]);
                     if (!B0)
-                        for (int i = 0; i < 2; i++) t3_add2<CLEAR>(st, nb, na, 3 + i, 0, Q[0][i], Q[1][i]);
+                        for (int i = 0; i < 2; i++) t3_add2<false>(st, nb, na, 3 + i, 0, Q[0][i], Q[1][i]);
                 }
             } else {
                 if (!B0)
-                    for (int i = 0; i < 2; i++) t3_add2<CLEAR>(st, na, nb, 3 + i, 0, P[i][0], P[i][1]);
-                t3_add2<CLEAR>(st, na, nb, 3, 2, P[0][2], Q[0][0]);
-                t3_add<CLEAR>(st, na, nb, 3, 4, Q[0][1]);
-                t3_add2<CLEAR>(st, na, nb, 4, 2, P[1][2], Q[1][0]);
-                t3_add<CLEAR>(st, na, nb, 4, 4, Q[1][1]);
+                    for (int i = 0; i < 2; i++) t3_add2<false>(st, na, nb, 3 + i, 0, P[i][0], P[i][1]);
+                t3_add2<false>(st, na, nb, 3, 2, P[0][2], Q[0][0]);
+                t3_add<false>(st, na, nb, 3, 4, Q[0][1]);
+                t3_add2<false>(st, na, nb, 4, 2, P[1][2], Q[1][0]);
+                t3_add<false>(st, na, nb, 4, 4, Q[1][1]);
                 if (diag) {
-                    t3_add<CLEAR>(st, na, nb, 5, 5, Q[2][2]);
+                    t3_add<false>(st, na, nb, 5, 5, Q[2][2]);
                 } else {
-                    t3_add<CLEAR>(st, nb, na, 2, 3, P[0][2]);
-                    t3_add<CLEAR>(st, nb, na, 2, 4, P[1][2]);
+                    t3_add<false>(st, nb, na, 2, 3, P[0][2]);
+                    t3_add<false>(st, nb, na, 2, 4, P[1][2]);
                     for (int i = 0; i < 2; i++) {
-                        t3_add<CLEAR>(st, nb, na, 3 + i, 3, Q[0][i]);
-                        t3_add<CLEAR>(st, nb, na, 3 + i, 4, Q[1][i]);
+                        t3_add<false>(st, nb, na, 3 + i, 3, Q[0][i]);
+                        t3_add<false>(st, nb, na, 3 + i, 4, Q[1][i]);
                         if (!B0) {
-                            t3_add<CLEAR>(st, nb, na, i, 3, P[0][i]);
-                            t3_add<CLEAR>(st, nb, na, i, 4, P[1][i]);
+                            t3_add<false>(st, nb, na, i, 3, P[0][i]);
+                            t3_add<false>(st, nb, na, i, 4, P[1][i]);
                         }
                     }
                 }
@@ -1530,17 +1522,17 @@ __device__ __forceinline__ void t3_pair_add(const T3Elem &s, double *st, int na,
             turn(R, tq, oq);
 #pragma unroll
             for (int i = 0; i < 3; i++) {
-                t3_add2<CLEAR>(st, na, nb, 3 * hb + i, 0, op[i][0], op[i][1]);
-                t3_add2<CLEAR>(st, na, nb, 3 * hb + i, 2, op[i][2], oq[i][0]);
-                t3_add2<CLEAR>(st, na, nb, 3 * hb + i, 4, oq[i][1], oq[i][2]);
+                t3_add2<false>(st, na, nb, 3 * hb + i, 0, op[i][0], op[i][1]);
+                t3_add2<false>(st, na, nb, 3 * hb + i, 2, op[i][2], oq[i][0]);
+                t3_add2<false>(st, na, nb, 3 * hb + i, 4, oq[i][1], oq[i][2]);
             }
             if (!diag) {
 #pragma unroll
                 for (int i = 0; i < 3; i++)
 #pragma unroll
                     for (int j = 0; j < 3; j++) {
-                        t3_add<CLEAR>(st, nb, na, j, 3 * hb + i, op[i][j]);
-                        t3_add<CLEAR>(st, nb, na, 3 + j, 3 * hb + i, oq[i][j]);
+                        t3_add<false>(st, nb, na, j, 3 * hb + i, op[i][j]);
+                        t3_add<false>(st, nb, na, 3 + j, 3 * hb + i, oq[i][j]);
                     }
             }
         }
@@ -1767,7 +1759,7 @@ extern "C" int fe3d_quad4r_kc0(int64_t E, const int64_t *cdof, const int64_t *in
     if (!values_only && (!Kr || !Kc)) return FE3D_ERR_ARG;
     RSArgs a{E, cdof, init_k, x, nx, xmat, xmat_stride, R, m, xe, area, props, nprops, pid, k6rot, k6rot_stride,
              hgfactors, hg_stride, Kr, Kc, Kv, nk, values_only, err};
-    return launch_rs_kc0<4>(a, as_stream(stream));
+    return launch_rs_kc0(a, as_stream(stream));
 }
 
 extern "C" int fe3d_tria3r_finte(int64_t E, const int64_t *cdof, const double *R, const double *m, const double *xe,
