@@ -878,7 +878,7 @@ def bench_batch(args):
     """Many independent uneven plates at the stated distribution (nx, ny
     uniform in [8, batch-nmax] elements): the block-diagonal pattern built
     from the elements, the fused KC0 of all plates into it, and the batched
-    PCG.  The whole batch runs a capped number of lockstep iterations (rate
+    PCG.  The whole batch runs a capped number of iterations (rate
     per iteration); a seeded sample of plates is solved to 1e-8 batched and
     one plate at a time (plain FP64 PCG on the same GPU)."""
     import torch
@@ -926,7 +926,7 @@ def bench_batch(args):
     ms = ev0.elapsed_time(ev1)
     out['all_plates_capped'] = {'maxiter': cap, 'ms': ms, 'ms_per_lockstep_iteration': ms / max(st['iterations'], 1),
                                 'converged': int((st['inst_status'] == 0).sum()),
-                                'note': 'every plate of the batch for a capped number of lockstep FP64 iterations'}
+                                'note': 'every plate of the batch for a capped number of FP64 iterations, on teams of blocks'}
     del bs, ur, vals, fm, pat
     torch.cuda.empty_cache()
     # seeded sample of the same plates: batched and one at a time, to 1e-8
@@ -978,9 +978,10 @@ def bench_batch(args):
 
 
 def bench_work_split():
-    """The batched solver's work split on many small plates: every plate in
-    the lockstep recurrence, against every plate solved by one thread block
-    of the block-resident kernel, to 1e-8 in FP64; with the SpMV FMAs each
+    """The batched solver's paths on many small plates: every plate on a team
+    of blocks (the default), in the lockstep recurrence (a work split that no
+    plate meets), and solved by one thread block of the block-resident kernel,
+    to 1e-8 in FP64; with the SpMV FMAs each
     run performed (sum over plates of iterations x nonzeros) and their rate."""
     import torch
     from pyfe3d_gb300 import batch
@@ -1001,7 +1002,7 @@ def bench_work_split():
     out = {'workload': '%d isotropic plates, nx, ny uniform in [4, 12] elements, seeded' % bp.P,
            'free_dofs': int(pat.nrows), 'nnz': int(pat.nnz), 'max_plate_rows': int(rows.max())}
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    for name, split in (('lockstep', 0), ('block_resident', int(rows.max()))):
+    for name, split in (('teams', 0), ('lockstep', 1), ('block_resident', int(rows.max()))):
         bs.set_split(split)
         bs.solve(fr, tol=1e-8, check_every=50, maxiter=50)
         torch.cuda.synchronize()
@@ -1014,9 +1015,10 @@ def bench_work_split():
         out[name] = {'ms': ms, 'solves_per_s': bp.P * 1e3 / ms, 'converged': int((st['inst_status'] == 0).sum()),
                      'max_relres': float(st['inst_relres'].max()), 'max_plate_iterations': int(st['inst_iters'].max()),
                      'spmv_fp64_fma': fma, 'spmv_fp64_tflops': 2 * fma / (ms / 1e3) / 1e12}
-    out['note'] = ('both paths are bound by the slowest plates: their iterations times the latency of one '
-                   'iteration (lockstep: three graph-launched kernels; block-resident: dependent row trips '
-                   'inside one block), not by FP64 throughput or bandwidth (see spmv_fp64_tflops)')
+    out['note'] = ('lockstep and block-resident plates are bound by the slowest ones: their iterations times the '
+                   'latency of one iteration (lockstep: three graph-launched kernels; block-resident: dependent row '
+                   'trips inside one block), not by FP64 throughput or bandwidth (see spmv_fp64_tflops); teams share '
+                   'out the blocks by what each plate has left')
     return out
 
 

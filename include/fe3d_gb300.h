@@ -561,13 +561,17 @@ int fe3d_dense_gemm_tall(int64_t n, int k, int m, const double *X, const double 
  * Every instance runs its own CG recurrence and convergence test.  Create
  * fails with FE3D_ERR_BOUNDS when an instance is out of range or a node's
  * rows span two instances, and with FE3D_ERR_ARG when the matrix couples two
- * instances.  Per-instance dot products use FP64 atomics: the last bits of
- * the iterates can differ from run to run. */
+ * instances.  In precision 0 instances whose rows are contiguous run on teams of
+ * blocks of one cooperative launch, many tiny ones in lockstep first; the others
+ * in lockstep.  Per-instance dot products in lockstep use FP64 atomics, and when
+ * the blocks are dealt out anew depends on timing: the last bits of the iterates
+ * can differ from run to run. */
 typedef struct fe3d_bsolver fe3d_bsolver;
 int fe3d_bsolver_create(const fe3d_pattern *p, int block_size, int64_t ninst, const int32_t *inst_of_row,
                         fe3d_bsolver **out);
 /* As fe3d_solver_setup; also times the SpMV lanes-per-row candidates
- * (4, 8, 16, 32) on this matrix and keeps the fastest per precision. */
+ * (4, 8, 16, 32) on this matrix and keeps the fastest per precision (at the
+ * first set-up: the pattern decides). */
 int fe3d_bsolver_setup(fe3d_bsolver *b, const double *vals, int mixed, int *nonpos_blocks, void *stream);
 /* Lanes per row chosen at setup (0 when that precision was not prepared). */
 int fe3d_bsolver_info(const fe3d_bsolver *b, int *lanes_fp64, int *lanes_fp32);
@@ -576,8 +580,8 @@ int fe3d_bsolver_info(const fe3d_bsolver *b, int *lanes_fp64, int *lanes_fp32);
  * block of a block-resident FP64 PCG kernel (block-level reductions in a fixed
  * order, convergence confirmed on the FP64 residual; the search direction
  * and its product in shared memory), on a second stream
- * concurrently with the lockstep recurrence of the other instances; 0 (the
- * default) sends every instance to the lockstep recurrence.  eligible (host,
+ * concurrently with the lockstep recurrence of the other instances; 0 is the
+ * default (no split).  eligible (host,
  * may be NULL) receives the number of instances the limit selects. */
 int fe3d_bsolver_set_split(fe3d_bsolver *b, int64_t max_rows, int64_t *eligible);
 /* Largest max_rows: the block keeps the instance's search direction and its
@@ -587,8 +591,8 @@ int fe3d_bsolver_set_split(fe3d_bsolver *b, int64_t max_rows, int64_t *eligible)
  * converged, 1 iteration cap, 3 non-finite, 4 stagnated in precision 1),
  * inst_iters and inst_relres
  * (FP64 ||f - K u|| / ||f|| per instance) are host arrays of ninst, each may
- * be NULL; total gets the worst status and relative residual and the number
- * of lockstep iterations.  Synchronises `stream`. */
+ * be NULL; total gets the worst status and relative residual and the largest
+ * number of iterations.  Synchronises `stream`. */
 int fe3d_bsolver_solve(fe3d_bsolver *b, const double *f, double *u, const fe3d_solve_opts *opts,
                        int *inst_status, int64_t *inst_iters, double *inst_relres, fe3d_solve_stats *total,
                        void *stream);

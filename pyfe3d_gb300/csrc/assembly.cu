@@ -14,9 +14,9 @@
 // result is deterministic.  The six (free) columns of a node in a row of the
 // matrix come from six consecutive slots of every element that has both nodes,
 // so the segments of neighbouring entries are the same slots shifted by one:
-// the pattern describes such a run by one 32-byte record, and the numeric
-// assembly reads 5 instead of 11 bytes of indices per entry and two slots per
-// load.
+// the pattern describes such a run, which ends with the node, by one 32-byte
+// record, and the numeric assembly reads 5 instead of 11 bytes of indices per entry
+// and two slots per load.
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 

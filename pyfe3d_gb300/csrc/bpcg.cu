@@ -28,9 +28,11 @@
 // in one cooperative launch, each on a team of blocks of its own (team_pcg.cu),
 // without lockstep: blocks are dealt out by the expected time of each instance's
 // remaining iterations, and dealt out anew when a fifth of them has nothing left
-// to do.  48 plates of 8..40 elements a side to 1e-10: lockstep 139 ms (three
-// launches and the slowest plate's iterations, stored zeros and all), teams
-// 51 ms.
+// to do (which depends on timing, as the sums' order in lockstep does: the last
+// bits of the iterates differ from run to run).  48 plates of 8..40 elements a side
+// to 1e-10: lockstep 139 ms (three launches and the slowest plate's iterations,
+// stored zeros and all), teams 43 ms.  Many tiny instances start in lockstep and
+// change to teams when few enough are left (teams_pay).
 //
 // Work split (precision 0): instances whose rows are contiguous and at most
 // `split_rows` in number are instead solved each by one thread block of a
@@ -38,7 +40,8 @@
 // the lockstep iterations of the others: the whole PCG recurrence of a small
 // plate runs inside one block (block-level reductions in a fixed order, no
 // host round trips, no launches per iteration), and the block moves on to
-// the next small instance when its plate has converged.
+// the next small instance when its plate has converged.  1,024 plates of 4..12
+// elements a side to 1e-8: block-resident 86 ms, lockstep 76 ms, teams 29 ms.
 #include <limits.h>
 #include <math.h>
 

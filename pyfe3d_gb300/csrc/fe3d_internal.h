@@ -66,9 +66,10 @@ struct fe3d_fmap {
 
 // Resident PCG (team_pcg.cu): the split of one or more systems over co-resident
 // blocks, the slice layout of the non-zero values and the exchange words.
-// Rows per block wanted while blocks are left: 16 rather than 64 at 2,166 rows
-// took 6.2 instead of 8.0 us per iteration (fewer FP64 instructions per block
-// against a slower exchange).
+// Rows per block wanted while blocks are left, fewer FP64 instructions per block
+// against a slower exchange: us per iteration with 8 / 16 / 32 / 64 rows, 486 rows
+// 5.5 / 5.9 / 6.3 / 6.1, 2,166 rows 5.6 / 5.7 / 5.6 / 6.0, 9,126 rows 6.8 / 6.8 /
+// 6.8 / 6.9.
 constexpr int kTeamRows = 16;
 constexpr int64_t kTeamIters = 4096;   // iterations of one resident launch at most (a quarter of a second)
 

@@ -147,8 +147,8 @@ __global__ void __launch_bounds__(RED_BS) spmv_kernel(int64_t n, const int64_t *
 // zeros cost neither bytes nor FP64 instructions (an FP64 instruction takes
 // the pipe for 64 cycles per sub-partition whatever its active lanes), loads
 // are coalesced and a row needs no shuffle reduction.  501x501-node plate
-// (80.5 M stored entries): one PCG iteration 0.286 -> 0.17 ms, 50 iterations
-// with set-up and residuals 18.5 -> 10.5 ms.
+// (80.5 M stored entries): one PCG iteration 0.286 -> 0.131 ms with the row-wise
+// update, 50 iterations with set-up and residuals 18.4 -> 8.3 ms.
 
 // Longest non-zero row of each slice, its place in the slice layout (taken
 // from *total, so the slices' order may vary but not what they hold).
@@ -1203,7 +1203,12 @@ namespace {
 // and once the caller has read *sell_total (NULL without memory for the counts) and
 // synchronised, decides and fills it (sell_build).  The layout is used when it holds at most 3/4 of the
 // stored entries; otherwise (curved shells, laminates with coupling) the CSR
-// kernels read the caller's values as they are.  Below kSellMinRows one row
+// kernels read the caller's values as they are: the bound keeps the copy, of 10
+// bytes per entry, from systems whose product it does not halve.  (The iterations
+// alone would be shorter there too.  us per iteration CSR / slices, no zeros
+// stored: cylinder 171,360 rows 57 / 50, 689,754 rows 140 / 127, laminated panel
+// 241,204 rows 71 / 55, 1,503,004 rows 281 / 190; half zeros, plate 1,494,006 rows
+// 286 / 131.)  Below kSellMinRows one row
 // per lane leaves too few warps and the row's serial FP64 chain shows (clamped
 // perturbed plates, us per iteration CSR / slices: 2,166 rows 20.8 / 23.3,
 // 9,126 rows 22.2 / 24.1, 14,406 rows 24.0 / 23.8, 20,886 rows 25.5 / 24.2,

@@ -22,8 +22,9 @@
 // counter, one trip through L2 per exchange, two exchanges per iteration.  A
 // slot is written again only after every reader of its previous value has
 // sent something that the writer waited for.  Each block makes the same sum over
-// blocks, so all hold the same scalars and the result does not depend on
-// scheduling.  Every poll is bounded; a block that
+// blocks, so all hold the same scalars, and the result of a launch with one system
+// does not depend on scheduling (with several, when a team stops for the blocks to
+// be dealt out anew depends on when the others finish).  Every poll is bounded; a block that
 // gives up raises a flag and returns.  The partial sums sit a 128-byte line
 // apart: 152 blocks exchange a value in 3.1k cycles, 5.8k with four to a line.
 //
@@ -36,10 +37,14 @@
 // and calls.
 //
 // Measured on clamped perturbed plates, us per iteration, three launches /
-// resident, rows in registers and FP64 sums / now: 486 rows 20.8 / 5.9 / 5.9,
-// 2,166 rows 20.8 / 6.7 / 5.6, 9,126 rows 22.2 / 8.2 / 6.6, 58,806 rows 25.5 /
-// 11.6 / 9.6, 237,606 rows 43 / 25 / 22.4, 536,406 rows 69.5 / 60 / 44 (there the
-// matrix no longer fits L2).  At 20,886 rows a block's 12,700 cycles are: product
+// resident, rows in registers and FP64 sums / now: 486 rows 20.8 / 5.9 / 5.8,
+// 2,166 rows 20.8 / 6.7 / 5.7, 9,126 rows 22.2 / 8.2 / 6.6, 58,806 rows 25.5 /
+// 11.6 / 9.8, 237,606 rows 43 / 25 / 22.6, 536,406 rows 69.5 / 60 / 45 (there the
+// matrix no longer fits L2).  Other matrices, three launches / resident: laminated
+// cylinder (54 non-zeros a row) 1,080 rows 20.1 / 6.2, 42,480 rows 28.3 / 12.8,
+// 387,714 rows 91 / 66; laminated panel 616,324 rows 131 / 90; lattice of nodes with
+// 3 DOFs 81,000 rows 25.3 / 15.3; plate with shuffled nodes 20,184 rows 25.6 / 13.9;
+// chain with one node joined to 200 others (rows of 1,200 entries) 6,000 rows 44 / 46.  At 20,886 rows a block's 12,700 cycles are: product
 // 3,300, sums over the block 2,800, waiting for p.q 1,800, for r.z and z 3,000, z 400,
 // sums over blocks and division 1,900 -- of which the FP64 pipe needs 3,900.
 #include <limits.h>
@@ -198,9 +203,9 @@ struct TeamArgs {
 // are read: from shared memory where they fit; else from L1 and L2 in a plain
 // loop (NEAR), or a chunk ahead of their use where all rows together exceed what
 // L2 holds next to the vectors (FAR, above kFarEntries entries of 10 bytes).  us
-// per iteration: 58,806 rows SHARED 9.5, NEAR 9.9, FAR 10.5; 84,966 rows 12.5,
-// 13.7, 14.5; 133,206 rows (too many for SHARED) NEAR 14.4, FAR 16.2; 237,606
-// rows 22.6, 24.5; 314,646 rows 30.4, 30.0; 536,406 rows 48, 44.
+// per iteration: 58,806 rows SHARED 10.2, NEAR 10.6, FAR 11.1; 84,966 rows 12.7,
+// 13.6, 14.0; 133,206 rows (too many for SHARED) NEAR 14.8, FAR 16.6; 237,606
+// rows 23.4, 25.9; 314,646 rows 31.2, 32.0; 536,406 rows 50, 47.
 enum { SHARED, NEAR, FAR };
 constexpr int64_t kFarEntries = 8400000;
 
@@ -762,7 +767,13 @@ int team_split(fe3d_team *t, const fe3d_solver *s, const std::vector<TeamPart> &
         if (n > t->nmax) t->nmax = n;
     }
     // lanes per row: the fewest FP64 instructions on one sub-partition's warps
-    // for a row of 27 non-zeros (a node of a flat plate's inside)
+    // for a row of 27 non-zeros (a node of a flat plate's inside).  us per
+    // iteration with 1 / 2 / 4 / 8 lanes, * the chosen ones: plate 2,166 rows 6.4 /
+    // 5.9 / 5.7* / 5.7, 9,126 rows 7.0 / 6.5* / 6.5 / 6.9, 20,886 rows 7.2* / 7.3 /
+    // 7.9 / 8.9, 237,606 rows 23* / 27 / 34 / 45; rows of 54: cylinder 1,080 rows 7.7 /
+    // 6.7 / 6.2* / 6.1, 10,440 rows 8.9* / 8.0 / 7.9 / 8.7, 42,480 rows 11.8 / 12.9* /
+    // 13.0 / 14.4, 387,714 rows 67* / 73 / 78 / 90, panel 21,964 rows 8.6 / 8.5* / 9.4 /
+    // 10.0
     int best = 1 << 30;
     for (int L = 1; L <= 8; L *= 2) {
         int cost = 28 / L + 1, lg = L;

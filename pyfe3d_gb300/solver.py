@@ -403,7 +403,8 @@ class BatchSolver:
         """Work split of FP64 solves: instances of at most ``max_rows``
         contiguous reduced rows are solved each by one thread block of a
         block-resident PCG kernel, concurrently with the lockstep recurrence of
-        the others (0: all lockstep).  Returns how many instances qualify."""
+        the others (0, the default: no split; instances run on teams of
+        blocks, many tiny ones in lockstep first).  Returns how many qualify."""
         e = ctypes.c_int64()
         _lib.check(_lib.load().fe3d_bsolver_set_split(self._h, int(max_rows), ctypes.byref(e)),
                    'fe3d_bsolver_set_split')
